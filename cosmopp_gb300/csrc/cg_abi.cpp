@@ -118,7 +118,7 @@ size_t staging_bytes(int N, int lmax, int max_batch)
            sizeof(int) * Bm;
 }
 
-void fill_plan(const cg_ctx* shape, size_t budget, cg_memory_plan* p)
+void fill_plan(cg_ctx* shape, size_t budget, cg_memory_plan* p)
 {
     size_t fixed = staging_bytes(shape->N, shape->lmax, shape->max_batch), per = 0;
     if (shape->precision == CG_PREC_MIXED) {
@@ -126,7 +126,14 @@ void fill_plan(const cg_ctx* shape, size_t budget, cg_memory_plan* p)
         cg::mixed_bytes(shape, &f, &per);
         fixed += f;
     } else {
-        per = cg::fp64_bytes_per_element(shape);
+        size_t f = 0;
+        cg::fp64_bytes(shape, &f, &per);
+        const size_t reserve = ((size_t)256 << 20) + budget / 100;
+        if (shape->harm && fixed + f + per + reserve > budget) {  // the gradient's route that needs less memory
+            shape->harm = false;
+            cg::fp64_bytes(shape, &f, &per);
+        }
+        fixed += f;
     }
     p->bytes_fixed = fixed;
     p->bytes_per_element = per;
@@ -160,6 +167,7 @@ int shape_of(const cg_config* cfg, cg_ctx* shape)
     shape->lmax = cfg->lmax;
     shape->max_batch = cfg->max_batch;
     shape->precision = cfg->precision;
+    shape->harm = cg::fp64_harmonics_ok(n, shape->nt, shape->lmax, cfg->dirs);
     return CG_OK;
 }
 
@@ -227,6 +235,7 @@ extern "C" int cg_create(cg_ctx** out, const cg_config* cfg)
     ctx->recenter = cfg->recenter;
     ctx->recenter_radius = cfg->recenter_radius > 0 ? cfg->recenter_radius : 1.0;
     ctx->device = cfg->device;
+    ctx->harm = cg::fp64_harmonics_ok(ctx->n, ctx->nt, ctx->lmax, cfg->dirs);
 
     // beam: Utils::readPixelWindowFunction with a unit window (f[l] = 1, f[l] *= B_l)
     ctx->leg.beam.resize(ctx->lmax + 1);
@@ -660,9 +669,7 @@ extern "C" int cg_stage_times(cg_ctx* ctx, double* ms)
 
 struct cg_lik {
     cg_ctx ctx;                  // device, sizes, stream and error text
-    double* A = nullptr;         // tiled C + F + N, then L, then C^-1
-    double* M = nullptr;
-    double* Dinv = nullptr;
+    double* A = nullptr;         // tiled C + F + N, then C^-1
     double* diag = nullptr;
     double* tmp = nullptr;       // [4][N] vectors + scalars
     int* st = nullptr;
@@ -677,7 +684,7 @@ extern "C" void cg_likelihood_destroy(cg_lik* lik)
     if (!lik) return;
     cudaSetDevice(lik->ctx.device);
     if (lik->ctx.stream) cudaStreamSynchronize(lik->ctx.stream);
-    cudaFree(lik->A); cudaFree(lik->M); cudaFree(lik->Dinv); cudaFree(lik->diag); cudaFree(lik->tmp); cudaFree(lik->st);
+    cudaFree(lik->A); cudaFree(lik->diag); cudaFree(lik->tmp); cudaFree(lik->st);
     cudaFree(lik->Ninv);
     if (lik->ctx.stream) cudaStreamDestroy(lik->ctx.stream);
     delete lik;
@@ -699,23 +706,26 @@ extern "C" int cg_likelihood_create(cg_lik** out, int n, const double* c_packed,
     if (!device_ok(device, &ctx.sm_count, why)) { g_create_error = why; return CG_ERR_NO_DEVICE; }
     ctx.device = device;
     ctx.n = n;
-    ctx.nt = (n + cg::TS - 1) / cg::TS;
+    ctx.nt = 2 * ((n + 2 * cg::TS - 1) / (2 * cg::TS));
     ctx.N = ctx.nt * cg::TS;
     cudaSetDevice(device);
     if (cudaStreamCreateWithFlags(&ctx.stream, cudaStreamNonBlocking) != cudaSuccess) { g_create_error = "stream"; return CG_ERR_CUDA; }
     const size_t np = (size_t)n * (n + 1) / 2, tiled = cg::tiled_elems(ctx.nt);
-    double* dpk = nullptr;
-    if (!dalloc(&lik->A, tiled) || !dalloc(&lik->M, tiled) || !dalloc(&lik->Dinv, (size_t)ctx.nt * cg::TILE_ELEMS) ||
-        !dalloc(&lik->diag, (size_t)ctx.N) || !dalloc(&lik->tmp, 4 * (size_t)ctx.N + 8) || !dalloc(&lik->st, 1) ||
+    double *dpk = nullptr, *M = nullptr;
+    unsigned char* work = nullptr;
+    // the factorisation's scratch (M = L^-1 and the digit images) is given back when it is done
+    auto free_scratch = [&] { cudaFree(dpk); cudaFree(M); cudaFree(work); };
+    if (!dalloc(&lik->A, tiled) || !dalloc(&M, tiled) || !dalloc(&work, cg::digit_bytes(ctx.nt, ctx.nt)) ||
+        !dalloc(&lik->diag, (size_t)ctx.N) || !dalloc(&lik->tmp, 4 * (size_t)ctx.N + 8) || !dalloc(&lik->st, 2) ||
         !dalloc(&dpk, 3 * np)) {
-        cudaFree(dpk);
+        free_scratch();
         g_create_error = "device allocation failed";
         cg_likelihood_destroy(lik.release());
         return CG_ERR_ALLOC;
     }
     for (size_t k = 0; k < np; ++k)
         if (!std::isfinite(c_packed[k]) || !std::isfinite(noise_packed[k]) || (fid_packed && !std::isfinite(fid_packed[k]))) {
-            cudaFree(dpk);
+            free_scratch();
             g_create_error = "non-finite matrix entry";
             cg_likelihood_destroy(lik.release());
             return CG_ERR_NONFINITE;
@@ -724,23 +734,26 @@ extern "C" int cg_likelihood_create(cg_lik** out, int n, const double* c_packed,
     cudaMemcpyAsync(dpk, c_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
     if (fid_packed) cudaMemcpyAsync(dpk + np, fid_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dpk + 2 * np, noise_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(lik->st, 0, sizeof(int), s);
+    cudaMemsetAsync(lik->st, 0, 2 * sizeof(int), s);
     cg::fp64_packed_to_tiled(n, ctx.nt, dpk, fid_packed ? dpk + np : nullptr, dpk + 2 * np, lik->A, s);
-    int rc = cg::tiled_cholesky<double>(&ctx, 1, ctx.nt, lik->A, lik->Dinv, lik->diag, lik->st, tiled, s);
-    if (!rc) {
-        cg::fp64_logdet(1, n, ctx.N, lik->diag, lik->tmp + 4 * (size_t)ctx.N, s);
-        rc = cg::tiled_trtri<double>(&ctx, 1, ctx.nt, lik->A, lik->Dinv, lik->M, tiled, s);
-    }
-    if (!rc) rc = cg::tiled_lauum<double>(&ctx, 1, ctx.nt, lik->M, lik->A, tiled, s);
-    int st = 0;
+    int rc = cg::fp64_identity_rows(&ctx, 1, ctx.nt, M, tiled, s);
+    if (!rc)
+        rc = cg::digit_factor(&ctx, 1, ctx.nt, ctx.nt, cg::DIGIT_EXT_IDENTITY, lik->A, tiled, M, tiled, lik->diag,
+                              lik->st, work, lik->st + 1, s);
+    if (!rc) cg::fp64_logdet(1, n, ctx.N, lik->diag, lik->tmp + 4 * (size_t)ctx.N, s);
+    int st[2] = {0, 0};
     if (!rc) {
         cudaMemcpyAsync(&lik->logdet, lik->tmp + 4 * (size_t)ctx.N, sizeof(double), cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(&st, lik->st, sizeof(int), cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(st, lik->st, 2 * sizeof(int), cudaMemcpyDeviceToHost, s);
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) { ctx.err = cudaGetErrorString(e); rc = CG_ERR_CUDA; }
     }
-    cudaFree(dpk);
-    if (!rc && st) {
+    free_scratch();
+    if (!rc && st[1]) {
+        ctx.err = "a device wait gave up";
+        rc = CG_ERR_TIMEOUT;
+    }
+    if (!rc && st[0]) {
         // source/likelihood.cpp:120-125: "The covariance matrix must be positive definite."
         ctx.err = "The covariance matrix is not positive definite.";
         rc = CG_ERR_NOT_PD;

@@ -50,16 +50,19 @@ struct DevBuf {
 // ---- plain FP64 path workspace -------------------------------------------
 struct Fp64Work {
     int cap = 0;                 // batch capacity
-    double* A = nullptr;         // [cap][tiled]  C, then L, then C^-1
-    double* M = nullptr;         // [cap][tiled]  L^-1
-    double* Dinv = nullptr;      // [cap][nt][TS*TS] inverses of the diagonal L tiles
+    double* A = nullptr;         // [cap][tiled]  C, then its factor's scratch (C^-1 with DIGIT_EXT_IDENTITY)
+    double* E = nullptr;         // [cap][ext_elems] the factorisation's extra rows (k_digit.cu)
+    size_t ext_elems = 0;        // doubles of E per element
+    unsigned char* dig = nullptr;  // digit images, digit_bytes per element
+    size_t dig_bytes = 0;        // per element
+    double* Yt = nullptr;        // [ext tiles] harmonics x B_l of the pixels, shared by every element
     double* diag = nullptr;      // [cap][N] diagonal of L
-    double* clc = nullptr;       // [cap][lmax+1] cl_l (2l+1)/(4 pi)
     double* dvec = nullptr;      // [cap][N] data maps (padded)
-    double* alpha = nullptr;     // [cap][N]
-    double* gpart = nullptr;     // [cap][nblk][lmax+1] adjoint partial sums
+    double* alpha = nullptr;     // [cap][N] L^-1 d, or C^-1 d
+    double* gpart = nullptr;     // [cap][gpart_elems] gradient partial sums
     int* st = nullptr;           // [cap] status
     double* ld = nullptr;        // [cap] ln det
+    int* err = nullptr;          // [1] a bounded device wait gave up
 };
 
 // ---- mixed path workspace ------------------------------------------------
@@ -168,6 +171,7 @@ struct cg_ctx {
     double* d_cl = nullptr;      // staging [max_batch][lmax+1]
     double* d_out = nullptr;     // staging for outputs
     size_t d_out_bytes = 0;
+    bool harm = false;           // FP64 gradient through the harmonics (else through C^-1 and the P_l)
     cg::Fp64Work w64;
     cg::MixedWork wmx;
     cg::Tune tune;
@@ -218,11 +222,15 @@ inline void stage_mark(cg_ctx* ctx, int stage, cudaStream_t s)
 }
 inline void count_launch(cg_ctx* ctx, long long k = 1) { ctx->launches += k; }
 // plain FP64 path (k_fp64.cu)
-int fp64_ensure(cg_ctx* ctx, int B);
-size_t fp64_bytes_per_element(const cg_ctx* ctx);
+// device bytes: *fixed for the harmonics of the pixels, *per_element for one element's workspace
+void fp64_bytes(const cg_ctx* ctx, size_t* fixed, size_t* per_element);
+// whether the gradient goes through the harmonics of the pixels (xyz [n][3], unit vectors only)
+bool fp64_harmonics_ok(int n, int nt, int lmax, const double* xyz);
+// real spherical harmonics times B_l at the pixels into Y [nharm_pad(lmax)][N] (k_mixed.cu)
+size_t ylm_rows(int lmax);
+int ylm_fill(cg_ctx* ctx, double* Y, cudaStream_t s);
 // mixed path device bytes: reference point + table, and one batch element's workspace
 void mixed_bytes(const cg_ctx* ctx, size_t* fixed, size_t* per_element);
-int fp64_build_tiled(cg_ctx* ctx, int B, const double* d_cl, bool add_noise, cudaStream_t s);
 int fp64_build_tiled_into(cg_ctx* ctx, int B, const double* d_cl, bool add_noise, double* A, cudaStream_t s);
 int fp64_build_packed(cg_ctx* ctx, int B, const double* d_cl, double* d_out, cudaStream_t s);
 // polarisation likelihood set-up: M = N^-1 + N^-1 C N^-1 for packed C and dense N^-1 (ld x ld,
@@ -243,6 +251,16 @@ int fp64_build_fiducial(cg_ctx* ctx, int lo, int hi, const double* d_tables, dou
                         cudaStream_t s);
 int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int d_stride, double* d_m2lnl,
                  double* d_chi2, double* d_logdet, double* d_grad, int* d_status, cudaStream_t s);
+// FP64 factorisation with its products on the tensor cores (k_digit.cu).  A: lower 64 x 64 tiles, nt
+// (even) block rows; E: ne (even) block rows of extra right-hand sides, which end as E L^-T.
+//   DIGIT_EXT_ROWS      E's tile (eb, k) at eb nt + k, element (r, c) at r + 64 c; diag = diagonal of L
+//   DIGIT_EXT_IDENTITY  ne = nt, E holds the identity, tile (eb, k >= eb) at tile_index(k, eb); it ends
+//                       as scratch and A as the inverse
+// work: digit_bytes(nt, ne) per matrix, 16-byte aligned; *err is set if a bounded wait gives up.
+enum DigitExt { DIGIT_EXT_ROWS = 0, DIGIT_EXT_IDENTITY = 1 };
+size_t digit_bytes(int nt, int ne);
+int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t strideA, double* E,
+                 size_t strideE, double* diag, int* status, unsigned char* work, int* err, cudaStream_t s);
 // generic tiled FP64 / FP32 factorisation entry points (k_chol.cu)
 template <typename T>
 int tiled_cholesky(cg_ctx* ctx, int B, int nt, T* A, T* Dinv, T* diag, int* status, size_t strideA, cudaStream_t s);
@@ -302,6 +320,8 @@ void mixed_free(cg_ctx* ctx);
 int mixed_ensure(cg_ctx* ctx, int B);
 void fp64_free(cg_ctx* ctx);
 // small FP64 launchers used by the Likelihood drop-in (k_fp64.cu)
+// E = identity of DIGIT_EXT_IDENTITY (lower tiles of the batch)
+int fp64_identity_rows(cg_ctx* ctx, int B, int nt, double* E, size_t strideE, cudaStream_t s);
 void fp64_packed_to_tiled(int n, int nt, const double* c, const double* f, const double* nz, double* A, cudaStream_t s);
 void fp64_symv(int B, int nt, int N, const double* V, const double* dv, double* alpha, cudaStream_t s);
 void fp64_logdet(int B, int n, int N, const double* diag, double* out, cudaStream_t s);

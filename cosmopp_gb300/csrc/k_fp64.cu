@@ -14,6 +14,9 @@
 // the factor's diagonal, explicit inverse, chi2 = d^T C^-1 d.  The adjoint
 // gradient (no reference counterpart) is
 //   d(-2lnL)/dC_l = sum_ij (C^-1 - a a^T)_ij (2l+1)/(4pi) B_l^2 P_l(x_ij),  a = C^-1 d.
+#include <algorithm>
+#include <cmath>
+
 #include "cg_internal.h"
 
 namespace cg {
@@ -369,10 +372,11 @@ __global__ void check_inputs(int B, int lmax, const double* __restrict__ cl, int
     status[b] = st;
 }
 
-__global__ void copy_status(int B, const int* __restrict__ src, int* __restrict__ dst)
+// a bounded device wait that gave up (*err) marks every element of the batch
+__global__ void copy_status(int B, const int* __restrict__ src, const int* __restrict__ err, int* __restrict__ dst)
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < B) dst[b] = src[b];
+    if (b < B) dst[b] = *err ? CG_ERR_TIMEOUT : src[b];
 }
 
 // A = c + fid + noise from packed host-layout arrays into the tiled layout,
@@ -594,6 +598,127 @@ __global__ void sim_means(int nsims, int n, const double* __restrict__ sims, dou
     mean[j] = __ddiv_rn(s, (double)nsims);
 }
 
+// E = identity of DIGIT_EXT_IDENTITY: tile (eb, k) at tile_index(k, eb); grid (tiles, B)
+__global__ void __launch_bounds__(kThreads) identity_rows(double* __restrict__ E, size_t strideE)
+{
+    int k, eb;
+    tile_coords(blockIdx.x, k, eb);
+    double* tile = E + (size_t)blockIdx.y * strideE + (size_t)blockIdx.x * TILE_ELEMS;
+    for (int e = threadIdx.x; e < TILE_ELEMS; e += kThreads) tile[e] = (k == eb && e % TS == e / TS) ? 1.0 : 0.0;
+}
+
+// the harmonics' rows [h][N] as E's tiles (eb, k), zero beyond nharm; grid (nt, ne)
+__global__ void __launch_bounds__(kThreads) harmonic_tiles(int N, int nt, int nharm, const double* __restrict__ Y,
+                                                           double* __restrict__ Yt)
+{
+    __shared__ double s[TS][TS + 1];
+    const int k = blockIdx.x, eb = blockIdx.y;
+    for (int e = threadIdx.x; e < TILE_ELEMS; e += kThreads) {
+        const int c = e % TS, r = e / TS, h = eb * TS + r;
+        s[r][c] = h < nharm ? Y[(size_t)h * N + k * TS + c] : 0.0;
+    }
+    __syncthreads();
+    double* tile = Yt + ((size_t)eb * nt + k) * TILE_ELEMS;
+    for (int e = threadIdx.x; e < TILE_ELEMS; e += kThreads) tile[e] = s[e % TS][e / TS];
+}
+
+// E's rows at the start: the harmonics (Yt, nullable) and the map as row drow; grid (nt, ne, B)
+__global__ void __launch_bounds__(kThreads) ext_rows(int n, int nt, int drow, const double* __restrict__ Yt,
+                                                     const double* __restrict__ d, int d_stride,
+                                                     double* __restrict__ E, size_t strideE)
+{
+    const int k = blockIdx.x, eb = blockIdx.y, b = blockIdx.z;
+    const size_t off = ((size_t)eb * nt + k) * TILE_ELEMS;
+    double* tile = E + (size_t)b * strideE + off;
+    const int rd = drow - eb * TS;
+    for (int e = threadIdx.x; e < TILE_ELEMS; e += kThreads) {
+        double v = Yt ? Yt[off + e] : 0.0;
+        if (e % TS == rd) {
+            const int i = k * TS + e / TS;
+            v = i < n ? d[(size_t)b * d_stride + i] : 0.0;
+        }
+        tile[e] = v;
+    }
+}
+
+// y = L^-1 d from E's row drow, chi2 = y . y, m2lnl = chi2 + logdet; grid B
+__global__ void __launch_bounds__(kThreads) chi2_rows(int nt, int drow, const double* __restrict__ E, size_t strideE,
+                                                      const double* __restrict__ logdet, double* __restrict__ y,
+                                                      double* __restrict__ m2lnl, double* __restrict__ chi2)
+{
+    __shared__ double red[kThreads];
+    const int b = blockIdx.x, N = nt * TS;
+    const double* Eb = E + (size_t)b * strideE + (size_t)(drow / TS) * nt * TILE_ELEMS + drow % TS;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < N; i += kThreads) {
+        const double v = Eb[(size_t)i * TS];  // tile i / 64, column i % 64: consecutive columns of the block row
+        y[(size_t)b * N + i] = v;
+        s = fma(v, v, s);
+    }
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = kThreads / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        if (chi2) chi2[b] = red[0];
+        m2lnl[b] = red[0] + logdet[b];
+    }
+}
+
+// Gradient through the harmonics: with Z = L^-1 Y (Y_l the 2l + 1 harmonics of l times B_l at the
+// pixels, dC/dC_l = Y_l Y_l^T by the addition theorem) and y = L^-1 d,
+//   d(-2lnL)/dC_l = tr(C^-1 Y_l Y_l^T) - |Y_l^T C^-1 d|^2 = sum_{h in l} (|Z_h|^2 - (Z_h . y)^2).
+// part[b][z][0 / 1][h] = the sums over block columns k = z, z + kHarmSplit, ...; grid (ne, kHarmSplit, B)
+constexpr int kHarmSplit = 8;
+__global__ void __launch_bounds__(kThreads) harmonic_sums(int nt, int ne, const double* __restrict__ E, size_t strideE,
+                                                          const double* __restrict__ y, double* __restrict__ part)
+{
+    __shared__ double red[2][4][TS];
+    const int eb = blockIdx.x, z = blockIdx.y, b = blockIdx.z, r = threadIdx.x % TS, q = threadIdx.x / TS;
+    const double* Eb = E + (size_t)b * strideE + (size_t)eb * nt * TILE_ELEMS;
+    const double* yb = y + (size_t)b * nt * TS;
+    double zz = 0.0, zy = 0.0;
+    for (int k = z; k < nt; k += kHarmSplit)
+#pragma unroll 8
+        for (int c = q; c < TS; c += 4) {
+            const double v = Eb[(size_t)k * TILE_ELEMS + r + TS * c];
+            zz = fma(v, v, zz);
+            zy = fma(v, yb[k * TS + c], zy);
+        }
+    red[0][q][r] = zz;
+    red[1][q][r] = zy;
+    __syncthreads();
+    if (q < 2) {
+        const size_t nh = (size_t)ne * TS;
+        part[(((size_t)b * kHarmSplit + z) * 2 + q) * nh + eb * TS + r] =
+            ((red[q][0][r] + red[q][1][r]) + red[q][2][r]) + red[q][3][r];
+    }
+}
+
+// grad_l from the sums, a warp per l; grid (ceil((lmax + 1) / 8), B)
+__global__ void __launch_bounds__(kThreads) harmonic_grad(int lmax, int ne, const double* __restrict__ part,
+                                                          double* __restrict__ grad)
+{
+    const int b = blockIdx.y, l = blockIdx.x * (kThreads / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (l > lmax) return;
+    const size_t nh = (size_t)ne * TS;
+    const double* p = part + (size_t)b * kHarmSplit * 2 * nh;
+    double g = 0.0;
+    if (l >= 2)
+        for (int h = l * l - 4 + lane; h < (l + 1) * (l + 1) - 4; h += 32) {
+            double zz = 0.0, zy = 0.0;
+            for (int z = 0; z < kHarmSplit; ++z) {
+                zz += p[(size_t)(2 * z) * nh + h];
+                zy += p[(size_t)(2 * z + 1) * nh + h];
+            }
+            g += zz - zy * zy;
+        }
+    for (int o = 16; o > 0; o >>= 1) g += __shfl_down_sync(0xffffffffu, g, o);
+    if (lane == 0) grad[(size_t)b * (lmax + 1) + l] = g;
+}
+
 }  // namespace
 
 void fp64_packed_to_tiled(int n, int nt, const double* c, const double* f, const double* nz, double* A, cudaStream_t s)
@@ -619,43 +744,109 @@ void fp64_dot(int n, const double* a, const double* b, double* out, cudaStream_t
 void fp64_free(cg_ctx* ctx)
 {
     Fp64Work& w = ctx->w64;
-    cudaFree(w.A); cudaFree(w.M); cudaFree(w.Dinv); cudaFree(w.diag); cudaFree(w.clc);
-    cudaFree(w.dvec); cudaFree(w.alpha); cudaFree(w.gpart); cudaFree(w.st); cudaFree(w.ld);
+    cudaFree(w.A); cudaFree(w.E); cudaFree(w.dig); cudaFree(w.Yt); cudaFree(w.diag); cudaFree(w.dvec);
+    cudaFree(w.alpha); cudaFree(w.gpart); cudaFree(w.st); cudaFree(w.ld); cudaFree(w.err);
     w = Fp64Work();
 }
 
-// Device bytes of one batch element's FP64 workspace: the allocations of fp64_ensure, in its order
-size_t fp64_bytes_per_element(const cg_ctx* ctx)
+static int nharm_of(int lmax) { return (lmax + 1) * (lmax + 1) - 4; }  // l = 2..lmax
+
+// The factorisation's extra block rows (even): the map alone for a value, the harmonics and the map
+// for a gradient, the identity where the gradient goes through C^-1
+static int ext_blocks(const cg_ctx* ctx, bool grad)
 {
-    const size_t tiled = tiled_elems(ctx->nt);
-    const int ntile = ntiles_lower(ctx->nt);
-    return sizeof(double) * tiled * 2 + sizeof(double) * (size_t)ctx->nt * TILE_ELEMS +
-           sizeof(double) * (size_t)ctx->N * 3 + sizeof(double) * (size_t)ntile * (ctx->lmax + 1) + sizeof(int) +
-           sizeof(double);
+    if (grad && !ctx->harm) return ctx->nt;
+    const int rows = grad ? nharm_of(ctx->lmax) + 1 : 1;
+    return 2 * ((rows + 2 * TS - 1) / (2 * TS));
 }
 
-int fp64_ensure(cg_ctx* ctx, int B)
+static size_t ext_elems(const cg_ctx* ctx, bool grad)
+{
+    if (grad && !ctx->harm) return tiled_elems(ctx->nt);
+    return (size_t)ext_blocks(ctx, grad) * ctx->nt * TILE_ELEMS;
+}
+
+static size_t gpart_elems(const cg_ctx* ctx)
+{
+    return ctx->harm ? (size_t)kHarmSplit * 2 * ext_blocks(ctx, true) * TS
+                     : (size_t)ntiles_lower(ctx->nt) * (ctx->lmax + 1);
+}
+
+// The harmonics' route takes nh / 128 block-row pairs through every column of the factorisation, the
+// route through C^-1 about 2/3 of the matrix's own pairs and then (lmax - 1) FP64 recurrence steps per
+// pixel pair, 0.8 lmax pairs' worth of time.  The addition theorem needs unit directions (cg_pix2vec's
+// are; a caller's are taken as unit below 1e-14).
+bool fp64_harmonics_ok(int n, int nt, int lmax, const double* xyz)
+{
+    if ((double)nharm_of(lmax) / 128.0 > nt / 3.0 + 0.8 * lmax) return false;
+    if (xyz)
+        for (int i = 0; i < n; ++i) {
+            const double x = xyz[3 * (size_t)i], y = xyz[3 * (size_t)i + 1], z = xyz[3 * (size_t)i + 2];
+            if (!(fabs(x * x + y * y + z * z - 1.0) <= 1e-14)) return false;
+        }
+    return true;
+}
+
+// The allocations of fp64_ensure for gradient calls (value calls need less)
+void fp64_bytes(const cg_ctx* ctx, size_t* fixed, size_t* per_element)
+{
+    *fixed = sizeof(int) + (ctx->harm ? sizeof(double) * (ext_elems(ctx, true) + ylm_rows(ctx->lmax) * ctx->N) : 0);
+    *per_element = sizeof(double) * (tiled_elems(ctx->nt) + ext_elems(ctx, true) + 3 * (size_t)ctx->N +
+                                     gpart_elems(ctx) + 1) +
+                   sizeof(int) + digit_bytes(ctx->nt, ext_blocks(ctx, true));
+}
+
+static int fp64_ensure(cg_ctx* ctx, int B, bool grad, cudaStream_t s)
 {
     Fp64Work& w = ctx->w64;
-    if (w.cap >= B) return CG_OK;
-    fp64_free(ctx);
-    const size_t tiled = tiled_elems(ctx->nt);
-    const int ntile = ntiles_lower(ctx->nt);
     auto alloc = [&](void** p, size_t bytes) -> bool { return cudaMalloc(p, bytes) == cudaSuccess; };
-    bool ok = alloc((void**)&w.A, sizeof(double) * tiled * B) && alloc((void**)&w.M, sizeof(double) * tiled * B) &&
-              alloc((void**)&w.Dinv, sizeof(double) * (size_t)B * ctx->nt * TILE_ELEMS) &&
-              alloc((void**)&w.diag, sizeof(double) * (size_t)B * ctx->N) &&
-              alloc((void**)&w.dvec, sizeof(double) * (size_t)B * ctx->N) &&
-              alloc((void**)&w.alpha, sizeof(double) * (size_t)B * ctx->N) &&
-              alloc((void**)&w.gpart, sizeof(double) * (size_t)B * ntile * (ctx->lmax + 1)) &&
-              alloc((void**)&w.st, sizeof(int) * (size_t)B) && alloc((void**)&w.ld, sizeof(double) * (size_t)B);
-    if (!ok) {
+    auto fail = [&] {
         fp64_free(ctx);
         cudaGetLastError();
         ctx->err = "device allocation failed for the FP64 workspace";
         return CG_ERR_ALLOC;
+    };
+    const size_t elems = ext_elems(ctx, grad), dig = digit_bytes(ctx->nt, ext_blocks(ctx, grad));
+    if (w.cap < B || w.ext_elems < elems || w.dig_bytes < dig) {
+        const int cap = std::max(B, w.cap);
+        const size_t ee = std::max(elems, w.ext_elems), de = std::max(dig, w.dig_bytes);
+        fp64_free(ctx);
+        if (!(alloc((void**)&w.A, sizeof(double) * tiled_elems(ctx->nt) * cap) &&
+              alloc((void**)&w.E, sizeof(double) * ee * cap) && alloc((void**)&w.dig, de * cap) &&
+              alloc((void**)&w.diag, sizeof(double) * (size_t)cap * ctx->N) &&
+              alloc((void**)&w.dvec, sizeof(double) * (size_t)cap * ctx->N) &&
+              alloc((void**)&w.alpha, sizeof(double) * (size_t)cap * ctx->N) &&
+              alloc((void**)&w.gpart, sizeof(double) * (size_t)cap * gpart_elems(ctx)) &&
+              alloc((void**)&w.st, sizeof(int) * (size_t)cap) && alloc((void**)&w.ld, sizeof(double) * (size_t)cap) &&
+              alloc((void**)&w.err, sizeof(int))))
+            return fail();
+        w.cap = cap;
+        w.ext_elems = ee;
+        w.dig_bytes = de;
     }
-    w.cap = B;
+    if (grad && ctx->harm && !w.Yt) {  // once per workspace: the pixels do not change
+        const int ne = ext_blocks(ctx, true);
+        double* Y = nullptr;
+        if (!alloc((void**)&w.Yt, sizeof(double) * ext_elems(ctx, true)) ||
+            !alloc((void**)&Y, sizeof(double) * ylm_rows(ctx->lmax) * ctx->N)) {
+            cudaFree(Y);
+            return fail();
+        }
+        int rc = ylm_fill(ctx, Y, s);
+        if (!rc) harmonic_tiles<<<dim3(ctx->nt, ne), kThreads, 0, s>>>(ctx->N, ctx->nt, nharm_of(ctx->lmax), Y, w.Yt);
+        const cudaError_t e = cudaStreamSynchronize(s);
+        cudaFree(Y);
+        if (!rc && e != cudaSuccess) { ctx->err = cudaGetErrorString(e); rc = CG_ERR_CUDA; }
+        if (rc) { cudaFree(w.Yt); w.Yt = nullptr; return rc; }
+    }
+    return CG_OK;
+}
+
+int fp64_identity_rows(cg_ctx* ctx, int B, int nt, double* E, size_t strideE, cudaStream_t s)
+{
+    identity_rows<<<dim3(ntiles_lower(nt), B), kThreads, 0, s>>>(E, strideE);
+    count_launch(ctx);
+    CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;
 }
 
@@ -670,11 +861,6 @@ int fp64_build_tiled_into(cg_ctx* ctx, int B, const double* d_cl, bool add_noise
     count_launch(ctx);
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;
-}
-
-int fp64_build_tiled(cg_ctx* ctx, int B, const double* d_cl, bool add_noise, cudaStream_t s)
-{
-    return fp64_build_tiled_into(ctx, B, d_cl, add_noise, ctx->w64.A, s);
 }
 
 int fp64_build_packed(cg_ctx* ctx, int B, const double* d_cl, double* d_out, cudaStream_t s)
@@ -749,32 +935,45 @@ int fp64_noise_matrix(cg_ctx* ctx, int nsims, int n, const double* d_sims, doubl
 int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int d_stride, double* d_m2lnl,
                  double* d_chi2, double* d_logdet, double* d_grad, int* d_status, cudaStream_t s)
 {
-    int rc = fp64_ensure(ctx, B);
+    const bool grad = d_grad != nullptr;
+    int rc = fp64_ensure(ctx, B, grad, s);
     if (rc) return rc;
     Fp64Work& w = ctx->w64;
     const int nt = ctx->nt, N = ctx->N, n = ctx->n, lmax = ctx->lmax;
     const size_t strideA = tiled_elems(nt);
-    const int ntile = ntiles_lower(nt);
+    const int ntile = ntiles_lower(nt), ne = ext_blocks(ctx, grad);
+    const bool inverse = grad && !ctx->harm;
     stage_mark(ctx, ST_BUILD, s);
+    CG_CUDA_TRY(ctx, cudaMemsetAsync(w.err, 0, sizeof(int), s));
     check_inputs<<<(B + 127) / 128, 128, 0, s>>>(B, lmax, d_cl, w.st);
     count_launch(ctx);
-    if ((rc = fp64_build_tiled(ctx, B, d_cl, true, s))) return rc;
+    if ((rc = fp64_build_tiled_into(ctx, B, d_cl, true, w.A, s))) return rc;
+    const int drow = grad ? nharm_of(lmax) : 0;
+    if (inverse) {
+        if ((rc = fp64_identity_rows(ctx, B, nt, w.E, w.ext_elems, s))) return rc;
+    } else {
+        ext_rows<<<dim3(nt, ne, B), kThreads, 0, s>>>(n, nt, drow, grad ? w.Yt : nullptr, d_d, d_stride, w.E,
+                                                      w.ext_elems);
+        count_launch(ctx);
+    }
     stage_mark(ctx, ST_CHOL, s);
-    if ((rc = tiled_cholesky<double>(ctx, B, nt, w.A, w.Dinv, w.diag, w.st, strideA, s))) return rc;
-    logdet_reduce<<<B, kThreads, 0, s>>>(n, N, w.diag, w.ld);
-    count_launch(ctx);
-    stage_mark(ctx, ST_TRTRI, s);
-    if ((rc = tiled_trtri<double>(ctx, B, nt, w.A, w.Dinv, w.M, strideA, s))) return rc;
-    stage_mark(ctx, ST_LAUUM, s);
-    if ((rc = tiled_lauum<double>(ctx, B, nt, w.M, w.A, strideA, s))) return rc;
+    if ((rc = digit_factor(ctx, B, nt, ne, inverse ? DIGIT_EXT_IDENTITY : DIGIT_EXT_ROWS, w.A, strideA, w.E,
+                           w.ext_elems, w.diag, w.st, w.dig, w.err, s)))
+        return rc;
     stage_mark(ctx, ST_SOLVE, s);
-    pad_data<<<dim3((N + 255) / 256, B), 256, 0, s>>>(n, N, B, d_d, d_stride, w.dvec);
-    symv_tiled<double><<<dim3(nt, B), kThreads, 0, s>>>(nt, N, w.A, strideA, w.dvec, w.alpha);
-    chi2_finish<<<B, kThreads, 0, s>>>(n, N, w.dvec, w.alpha, w.ld, d_m2lnl, d_chi2);
-    count_launch(ctx, 3);
-    stage_mark(ctx, ST_ADJOINT, s);
+    logdet_reduce<<<B, kThreads, 0, s>>>(n, N, w.diag, w.ld);
+    if (inverse) {
+        pad_data<<<dim3((N + 255) / 256, B), 256, 0, s>>>(n, N, B, d_d, d_stride, w.dvec);
+        symv_tiled<double><<<dim3(nt, B), kThreads, 0, s>>>(nt, N, w.A, strideA, w.dvec, w.alpha);
+        chi2_finish<<<B, kThreads, 0, s>>>(n, N, w.dvec, w.alpha, w.ld, d_m2lnl, d_chi2);
+        count_launch(ctx, 4);
+    } else {
+        chi2_rows<<<B, kThreads, 0, s>>>(nt, drow, w.E, w.ext_elems, w.ld, w.alpha, d_m2lnl, d_chi2);
+        count_launch(ctx, 2);
+    }
     if (d_logdet) CG_CUDA_TRY(ctx, cudaMemcpyAsync(d_logdet, w.ld, sizeof(double) * B, cudaMemcpyDeviceToDevice, s));
-    if (d_grad) {
+    stage_mark(ctx, ST_ADJOINT, s);
+    if (inverse) {
         for (int l0 = 2; l0 <= lmax; l0 += kAdjChunk) {
             const int l1 = (l0 + kAdjChunk <= lmax + 1) ? l0 + kAdjChunk : lmax + 1;
             adjoint_tiles<<<dim3(ntile, B), kThreads, 0, s>>>(n, N, l0, l1, ctx->d_xyz, ctx->d_lega, ctx->d_legb, w.A,
@@ -783,8 +982,12 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
         }
         adjoint_finish<<<B, 64, 0, s>>>(lmax, ntile, w.gpart, ctx->d_beam, d_grad);
         count_launch(ctx);
+    } else if (grad) {
+        harmonic_sums<<<dim3(ne, kHarmSplit, B), kThreads, 0, s>>>(nt, ne, w.E, w.ext_elems, w.alpha, w.gpart);
+        harmonic_grad<<<dim3((lmax + 8) / 8, B), kThreads, 0, s>>>(lmax, ne, w.gpart, d_grad);
+        count_launch(ctx, 2);
     }
-    if (d_status) { copy_status<<<(B + 127) / 128, 128, 0, s>>>(B, w.st, d_status); count_launch(ctx); }
+    if (d_status) { copy_status<<<(B + 127) / 128, 128, 0, s>>>(B, w.st, w.err, d_status); count_launch(ctx); }
     stage_mark(ctx, ST_END, s);
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;

@@ -589,6 +589,17 @@ int dalloc(cg_ctx* ctx, T** p, size_t count)
 
 }  // namespace
 
+size_t ylm_rows(int lmax) { return (size_t)nharm_pad(lmax); }
+
+int ylm_fill(cg_ctx* ctx, double* Y, cudaStream_t s)
+{
+    const int N = ctx->N, lmax = ctx->lmax;
+    CG_CUDA_TRY(ctx, cudaMemsetAsync(Y, 0, sizeof(double) * ylm_rows(lmax) * N, s));
+    ylm_basis<<<dim3((N + 127) / 128, lmax + 1), 128, 0, s>>>(ctx->n, N, lmax, ctx->d_xyz, ctx->d_beam, Y);
+    CG_CUDA_TRY(ctx, cudaGetLastError());
+    return CG_OK;
+}
+
 void mixed_free(cg_ctx* ctx)
 {
     MixedWork& w = ctx->wmx;
@@ -705,8 +716,7 @@ int mixed_prepare_reference(cg_ctx* ctx, const double* cl_ref_host)
     // whitened harmonic basis and table
     const int nhp = nharm_pad(lmax);
     if (!rc) {
-        CG_CUDA_TRY(ctx, cudaMemsetAsync(w.Y, 0, sizeof(double) * (size_t)nhp * N, s));
-        ylm_basis<<<dim3((N + 127) / 128, lmax + 1), 128, 0, s>>>(n, N, lmax, ctx->d_xyz, ctx->d_beam, w.Y);
+        if ((rc = ylm_fill(ctx, w.Y, s))) { cudaFree(st); return rc; }
         const size_t smz = 2 * (size_t)TS * SmemLd<double>::v * sizeof(double);
         CG_CUDA_TRY(ctx, cudaFuncSetAttribute(whiten_basis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
         whiten_basis<<<dim3(nt, nhp / TS), 256, smz, s>>>(nt, N, w.Mref, w.Y, w.Z);

@@ -1,0 +1,129 @@
+"""The tensor-core FP64 factorisation (k_digit.cu) at the sizes where its tiling changes: one to a few
+64-column steps, the edges of 64-row blocks and of 128-row pairs, extra rows that fill, exceed or leave
+free the last pair, batches beyond one CTA wave, both gradient routes and the packed drop-in, against
+FP64 numpy.
+
+Tolerances: a backward-stable factorisation of C (condition number kappa) moves chi2 = d^T C^-1 d by at
+most about n eps kappa chi2, ln det by n eps kappa, and C^-1 by n eps kappa |C^-1|; the bars below
+are 8 times these, with the gradient's scale sum_ij |W_ij| |dC_ij/dC_l|."""
+import numpy as np
+import pytest
+
+import cosmopp_gb300 as cg
+from cosmopp_gb300 import workload as W
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(float).eps
+
+
+def _legendre(x, lmax):
+    p = [np.ones_like(x), x]
+    for l in range(2, lmax + 1):
+        p.append((2 - 1.0 / l) * x * p[-1] - (1 - 1.0 / l) * p[-2])
+    return p
+
+
+def _setup(n, lmax, seed, batch, norm=1.0):
+    rng = np.random.default_rng(seed)
+    v = rng.standard_normal((n, 3))
+    v /= np.linalg.norm(v, axis=1)[:, None]
+    cls = W.lognormal_batch(W.fiducial_cl(lmax), batch, seed + 1)
+    d = 20.0 * rng.standard_normal((batch, n))
+    return v * norm, cls, d
+
+
+def _reference(v, cls, d, beam, var):
+    n, lmax = len(v), cls.shape[1] - 1
+    x = np.clip(v @ v.T, -1, 1)
+    p = _legendre(x, lmax)
+    w = (2 * np.arange(lmax + 1) + 1) / (4 * np.pi) * beam ** 2
+    out = []
+    for c, m in zip(cls, d):
+        cov = sum(c[l] * w[l] * p[l] for l in range(2, lmax + 1)) + var * np.eye(n)
+        ev = np.linalg.eigvalsh(cov)
+        inv = np.linalg.inv(cov)
+        inv = (inv + inv.T) / 2
+        a = np.linalg.solve(cov, m)
+        g, s = np.zeros(lmax + 1), np.zeros(lmax + 1)
+        for l in range(2, lmax + 1):
+            g[l] = np.sum((inv - np.outer(a, a)) * p[l]) * w[l]
+            s[l] = np.sum(np.abs(inv) + np.abs(np.outer(a, a))) * w[l]
+        out.append((m @ a, np.linalg.slogdet(cov)[1], g, s, 8 * n * EPS * ev[-1] / ev[0]))
+    return out
+
+
+def _check(r, ref, grad=True):
+    assert np.all(r["status"] == 0), r["status"]
+    for b, (chi2, ld, g, s, tol) in enumerate(ref):
+        assert abs(r["chi2"][b] - chi2) <= tol * chi2, (b, r["chi2"][b], chi2)
+        assert abs(r["logdet"][b] - ld) <= tol, (b, r["logdet"][b], ld)
+        assert r["m2lnl"][b] == r["chi2"][b] + r["logdet"][b]
+        if grad:
+            assert np.all(np.abs(r["grad"][b] - g) <= tol * s + 1e-300), (b, np.abs(r["grad"][b] - g) / s.max(), tol)
+
+
+# pixels: below, at and above one block, one pair, several pairs.  lmax 2, 7, 10, 12, 14: 5, 60, 117,
+# 165, 221 harmonics, so that the map's row falls in the first, second, third or fourth block of E
+@pytest.mark.parametrize("n,lmax,batch", [(1, 2, 1), (5, 3, 2), (63, 7, 1), (64, 7, 3), (65, 10, 1), (127, 10, 2),
+                                          (128, 12, 1), (129, 14, 2), (192, 12, 1), (193, 7, 40), (321, 14, 3)])
+@pytest.mark.parametrize("norm", [1.0, 1.0 + 1e-13], ids=["harmonics", "inverse"])
+def test_value_and_gradient(n, lmax, batch, norm):
+    """norm 1: the gradient through the harmonics; directions off the unit sphere by 1e-13 (no effect on
+    the numbers at these bars) take the route through C^-1."""
+    v, cls, d = _setup(n, lmax, 17 * n + lmax, batch, norm)
+    beam = np.exp(-0.002 * np.arange(lmax + 1.0) ** 2)
+    ref = _reference(v, cls, d, beam, 4.0)
+    with cg.Context(lmax=lmax, fwhm_deg=1.0, dirs=v, beam=beam, noise_sigma=2.0, max_batch=batch) as ctx:
+        val = ctx.loglike(cls, d)                 # value first: its workspace then grows for the gradient
+        full = ctx.loglike(cls, d, grad=True)
+        again = ctx.loglike(cls, d)               # and a value call on the grown workspace
+        one = ctx.loglike(cls, d[0], grad=True)   # one map for every element
+    _check(val, ref, grad=False)
+    _check(full, ref)
+    for k in ("m2lnl", "chi2", "logdet"):
+        assert np.array_equal(val[k], again[k])
+        assert one[k][0] == full[k][0]
+    assert np.array_equal(one["grad"][0], full["grad"][0])
+
+
+@pytest.mark.parametrize("scale", [1e-120, 1e-9, 1e7, 1e110])
+def test_scale_of_the_map_and_of_the_covariance(scale):
+    """Powers of two in the rows: covariance scale^2, map scale, chi2 unchanged to rounding."""
+    v, cls, d = _setup(150, 9, 5, 1)
+    beam = np.exp(-0.002 * np.arange(10.0) ** 2)
+    chi2, _, _, _, tol = _reference(v, cls, d, beam, 4.0)[0]
+    with cg.Context(lmax=9, fwhm_deg=1.0, dirs=v, beam=beam, noise_sigma=2.0 * scale) as ctx:
+        r = ctx.loglike(cls[0] * scale ** 2, d[0] * scale, grad=True)
+        q = ctx.loglike(cls[0] * scale ** 2, d[0] * scale * 1e-30)
+    assert r["status"] == 0 and abs(r["chi2"] - chi2) <= 2 * tol * chi2
+    assert abs(q["chi2"] - chi2 * 1e-60) <= 2 * tol * chi2 * 1e-60
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_nonfinite_map_stays_visible(bad):
+    v, cls, d = _setup(130, 7, 6, 2)
+    d[1, 77] = bad
+    with cg.Context(lmax=7, fwhm_deg=1.0, dirs=v, noise_sigma=2.0, max_batch=2) as ctx:
+        r = ctx.loglike(cls, d, grad=True)
+    assert np.isfinite(r["m2lnl"][0]) and not np.isfinite(r["m2lnl"][1])
+    assert np.all(np.isfinite(r["grad"][0])) and not np.any(np.isfinite(r["grad"][1][2:]))
+
+
+@pytest.mark.parametrize("n", [1, 2, 64, 65, 128, 129, 300])
+def test_packed_likelihood(n):
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((n, n + 5))
+    c = a @ a.T / n
+    c = (c + c.T) / 2
+    t = rng.standard_normal(n)
+    full = c + 0.5 * np.eye(n)
+    ev = np.linalg.eigvalsh(full)
+    tol = 8 * n * EPS * ev[-1] / ev[0]
+    lik = cg.Likelihood(W.full_to_packed(c), None, W.full_to_packed(0.5 * np.eye(n)))
+    for m in (t, -3 * t[::-1]):
+        _, chi2, ld = lik.calculate(m)
+        want = m @ np.linalg.solve(full, m)
+        assert abs(chi2 - want) <= tol * want
+        assert abs(lik.logdet_raw - np.linalg.slogdet(full)[1]) <= tol
+    lik.close()
