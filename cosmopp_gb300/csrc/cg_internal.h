@@ -60,6 +60,8 @@ struct Fp64Work {
     double* dvec = nullptr;      // [cap][N] data maps (padded)
     double* alpha = nullptr;     // [cap][N] L^-1 d, or C^-1 d
     double* gpart = nullptr;     // [cap][gpart_elems] gradient partial sums
+    long long* wfix = nullptr;   // [cap][lmax+1] fixed-point weights of the Legendre sum
+    int* wexp = nullptr;         // [cap] their exponent
     int* st = nullptr;           // [cap] status
     double* ld = nullptr;        // [cap] ln det
     int* err = nullptr;          // [1] a bounded device wait gave up

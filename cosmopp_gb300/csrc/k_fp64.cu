@@ -71,8 +71,9 @@ __device__ __forceinline__ void load_consts(double* sa, double* sb, double* sc, 
     }
 }
 
-// C (+ noise on the diagonal, identity padding) into the tiled layout, grid (tiles, B)
-__global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax, const double* __restrict__ xyz,
+// C (+ noise on the diagonal, identity padding) into the tiled layout with the reference's operations, for
+// the mixed path's reference point (its FP32 table and factor keep their bits), grid (tiles, B)
+__global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, const double* __restrict__ xyz,
                                                           const double* __restrict__ noise,
                                                           const double* __restrict__ lega,
                                                           const double* __restrict__ legb,
@@ -115,6 +116,118 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
                 val = (i == j) ? 1.0 : 0.0;
             }
             tile[e[q]] = val;
+        }
+    }
+}
+
+// ---- covariance for the likelihood, in 64-bit fixed point ----------------------------------
+//
+// The FP64 pipe gives 2 operations per cycle and SM, the integer pipes about 50 times that, and every
+// quantity of the Legendre sum is bounded: |P_l| <= 1, |x| <= 1, and the weights w_l = C_l (2l+1)/(4 pi)
+// B_l^2 are scaled by a power of two above sum |w_l|.  So the sum runs in integers, P_l = p 2^-60:
+//     t = x P_{l-1},  P_l = 2 t - P_{l-2} - (t - P_{l-2}) / l,  S += w_l P_l,
+// one 64 x 64 -> high 64 product each.  Each step rounds at 2^-60 where FP64 rounds at 2^-53: the sum
+// is 10 to 50 times nearer to the exact value than the FP64 recurrence's (lmax 12 to 255), and is then
+// rounded to FP64 once.  The P_l are shared by NB batch elements.
+
+// status and fixed-point weights of every element: wfix[b][l] = w_l 2^(62 - e), wexp[b] = e with
+// sum |w_l| < 2^e; a non-finite weight gives e = kBadWeights and a NaN covariance.  grid B
+constexpr int kBadWeights = 1 << 20;
+__global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const double* __restrict__ beam,
+                                                             const double* __restrict__ cl,
+                                                             long long* __restrict__ wfix, int* __restrict__ wexp,
+                                                             int* __restrict__ status)
+{
+    __shared__ double part[kThreads / 32];
+    const int b = blockIdx.x, l = threadIdx.x, L1 = lmax + 1;
+    const double c = l <= lmax ? cl[(size_t)b * L1 + l] : 0.0;
+    // clCopy[l] = cl[l] * (2 l + 1) / (4 pi)   (c_matrix_generator.cpp:190-193)
+    double w = 0.0;
+    if (l >= 2 && l <= lmax)
+        w = __dmul_rn(__dmul_rn(__ddiv_rn(__dmul_rn(c, (double)(2 * l + 1)), 4.0 * kPi), beam[l]), beam[l]);
+    double s = fabs(w);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (l % 32 == 0) part[l / 32] = s;
+    const int bad = __syncthreads_or(!isfinite(c));
+    s = 0.0;
+    for (int k = 0; k < kThreads / 32; ++k) s += part[k];
+    const int e = isfinite(s) ? (s > 0.0 ? ilogb(s) + 1 : -1000) : kBadWeights;
+    if (l <= lmax) wfix[(size_t)b * L1 + l] = e == kBadWeights ? 0 : __double2ll_rn(scalbn(w, 62 - e));
+    if (l == 0) {
+        wexp[b] = e;
+        status[b] = bad ? CG_ERR_NONFINITE : CG_OK;
+    }
+}
+
+// C (+ noise on the diagonal, identity padding) into the tiled layout; grid (tiles, ceil(B / NB)),
+// 4 pairs per thread and pass
+template <int NB>
+__global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax, int B,
+                                                          const double* __restrict__ xyz,
+                                                          const double* __restrict__ noise,
+                                                          const long long* __restrict__ wfix,
+                                                          const int* __restrict__ wexp, double* __restrict__ A,
+                                                          size_t strideA)
+{
+    extern __shared__ long long sfix[];
+    const int L1 = lmax + 1, b0 = blockIdx.y * NB;
+    long long* sr = sfix;        // 2^63 / l
+    long long* sw = sfix + L1;   // [l][NB]
+    for (int l = threadIdx.x; l <= lmax; l += kThreads) {
+        sr[l] = l >= 2 ? (long long)((0x8000000000000000ull + l / 2) / (unsigned)l) : 0;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) sw[l * NB + q] = b0 + q < B ? wfix[(size_t)(b0 + q) * L1 + l] : 0;
+    }
+    __syncthreads();
+    int I, J;
+    tile_coords(blockIdx.x, I, J);
+    for (int g = 0; g < TILE_ELEMS / (kThreads * 4); ++g) {
+        long long x[4], p0[4], p1[4], acc[NB][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = threadIdx.x + kThreads * (4 * g + q), i = I * TS + e % TS, j = J * TS + e / TS;
+            const double v = (i < n && j < n) ? pair_dot(xyz, N, i, j) : 0.0;
+            x[q] = __double2ll_rn(v * 4611686018427387904.0);  // 2^62
+            p0[q] = 1ll << 60;
+            p1[q] = x[q] >> 2;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) acc[k][q] = 0;
+        }
+#pragma unroll 2
+        for (int l = 2; l <= lmax; ++l) {
+            const long long rl = sr[l];
+            long long w[NB];
+#pragma unroll
+            for (int k = 0; k < NB; ++k) w[k] = sw[l * NB + k];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const long long t = __mul64hi(x[q], p1[q] << 2), d = t - p0[q];
+                const long long p = t + d - __mul64hi(d << 1, rl);
+                p0[q] = p1[q];
+                p1[q] = p;
+#pragma unroll
+                for (int k = 0; k < NB; ++k) acc[k][q] += __mul64hi(p << 2, w[k]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            if (b0 + k >= B) break;
+            const int we = wexp[b0 + k];
+            double* tile = A + (size_t)(b0 + k) * strideA + (size_t)blockIdx.x * TILE_ELEMS;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int e = threadIdx.x + kThreads * (4 * g + q), i = I * TS + e % TS, j = J * TS + e / TS;
+                double val;
+                if (i < n && j < n) {
+                    val = we == kBadWeights ? __longlong_as_double(0x7ff8000000000000ll)
+                                            : scalbn(__ll2double_rn(acc[k][q]), we - 60);
+                    // cInv_(i,j) = c + fiducial(0) + noise  (source/likelihood.cpp:102-110)
+                    if (i == j) val = __dadd_rn(val, noise[i]);
+                } else {
+                    val = (i == j) ? 1.0 : 0.0;
+                }
+                tile[e] = val;
+            }
         }
     }
 }
@@ -359,17 +472,6 @@ __global__ void adjoint_finish(int lmax, int ntile, const double* __restrict__ g
             for (int t = 0; t < ntile; ++t) s += gpart[((size_t)b * ntile + t) * (lmax + 1) + l];
         grad[(size_t)b * (lmax + 1) + l] = (l < 2) ? 0.0 : s * ((2 * l + 1) / (4 * kPi)) * beam[l] * beam[l];
     }
-}
-
-// input check: non-finite C_l -> status NONFINITE, else OK
-__global__ void check_inputs(int B, int lmax, const double* __restrict__ cl, int* __restrict__ status)
-{
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    int st = CG_OK;
-    for (int l = 0; l <= lmax; ++l)
-        if (!isfinite(cl[(size_t)b * (lmax + 1) + l])) st = CG_ERR_NONFINITE;
-    status[b] = st;
 }
 
 // a bounded device wait that gave up (*err) marks every element of the batch
@@ -746,6 +848,7 @@ void fp64_free(cg_ctx* ctx)
     Fp64Work& w = ctx->w64;
     cudaFree(w.A); cudaFree(w.E); cudaFree(w.dig); cudaFree(w.Yt); cudaFree(w.diag); cudaFree(w.dvec);
     cudaFree(w.alpha); cudaFree(w.gpart); cudaFree(w.st); cudaFree(w.ld); cudaFree(w.err);
+    cudaFree(w.wfix); cudaFree(w.wexp);
     w = Fp64Work();
 }
 
@@ -793,7 +896,7 @@ void fp64_bytes(const cg_ctx* ctx, size_t* fixed, size_t* per_element)
     *fixed = sizeof(int) + (ctx->harm ? sizeof(double) * (ext_elems(ctx, true) + ylm_rows(ctx->lmax) * ctx->N) : 0);
     *per_element = sizeof(double) * (tiled_elems(ctx->nt) + ext_elems(ctx, true) + 3 * (size_t)ctx->N +
                                      gpart_elems(ctx) + 1) +
-                   sizeof(int) + digit_bytes(ctx->nt, ext_blocks(ctx, true));
+                   sizeof(long long) * ((size_t)ctx->lmax + 1) + 2 * sizeof(int) + digit_bytes(ctx->nt, ext_blocks(ctx, true));
 }
 
 static int fp64_ensure(cg_ctx* ctx, int B, bool grad, cudaStream_t s)
@@ -818,7 +921,8 @@ static int fp64_ensure(cg_ctx* ctx, int B, bool grad, cudaStream_t s)
               alloc((void**)&w.alpha, sizeof(double) * (size_t)cap * ctx->N) &&
               alloc((void**)&w.gpart, sizeof(double) * (size_t)cap * gpart_elems(ctx)) &&
               alloc((void**)&w.st, sizeof(int) * (size_t)cap) && alloc((void**)&w.ld, sizeof(double) * (size_t)cap) &&
-              alloc((void**)&w.err, sizeof(int))))
+              alloc((void**)&w.wfix, sizeof(long long) * (size_t)cap * (ctx->lmax + 1)) &&
+              alloc((void**)&w.wexp, sizeof(int) * (size_t)cap) && alloc((void**)&w.err, sizeof(int))))
             return fail();
         w.cap = cap;
         w.ext_elems = ee;
@@ -855,7 +959,7 @@ static size_t const_smem(int lmax) { return sizeof(double) * 4 * (size_t)(lmax +
 int fp64_build_tiled_into(cg_ctx* ctx, int B, const double* d_cl, bool add_noise, double* A, cudaStream_t s)
 {
     const int ntile = ntiles_lower(ctx->nt);
-    build_c_tiled<<<dim3(ntile, B), kThreads, const_smem(ctx->lmax), s>>>(
+    build_c_ref<<<dim3(ntile, B), kThreads, const_smem(ctx->lmax), s>>>(
         ctx->n, ctx->N, ctx->lmax, ctx->d_xyz, ctx->d_noise, ctx->d_lega, ctx->d_legb, ctx->d_beam, d_cl,
         add_noise ? 1 : 0, A, tiled_elems(ctx->nt));
     count_launch(ctx);
@@ -945,9 +1049,16 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
     const bool inverse = grad && !ctx->harm;
     stage_mark(ctx, ST_BUILD, s);
     CG_CUDA_TRY(ctx, cudaMemsetAsync(w.err, 0, sizeof(int), s));
-    check_inputs<<<(B + 127) / 128, 128, 0, s>>>(B, lmax, d_cl, w.st);
-    count_launch(ctx);
-    if ((rc = fp64_build_tiled_into(ctx, B, d_cl, true, w.A, s))) return rc;
+    legendre_weights<<<B, kThreads, 0, s>>>(lmax, ctx->d_beam, d_cl, w.wfix, w.wexp, w.st);
+    // one element per thread block below four: twice the blocks of the shared form, and a single
+    // element has nothing to share
+    if (B >= 4)
+        build_c_tiled<4><<<dim3(ntile, (B + 3) / 4), kThreads, sizeof(long long) * 5 * (lmax + 1), s>>>(
+            n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
+    else
+        build_c_tiled<1><<<dim3(ntile, B), kThreads, sizeof(long long) * 2 * (lmax + 1), s>>>(
+            n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
+    count_launch(ctx, 2);
     const int drow = grad ? nharm_of(lmax) : 0;
     if (inverse) {
         if ((rc = fp64_identity_rows(ctx, B, nt, w.E, w.ext_elems, s))) return rc;
