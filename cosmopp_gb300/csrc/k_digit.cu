@@ -207,92 +207,428 @@ __device__ __forceinline__ double* ext_tile(const Dig& g, int b, int eb, int k)
     return g.E + (size_t)b * g.strideE + t * TILE_ELEMS;
 }
 
-// L_kk and its inverse in one sweep.  Thread (tr, tc) holds rows tr + 16 a, columns tc + 16 b.  At
-// column c the trailing part is updated by the outer product of L's column c and the inverse's rows
-// below c by that column times the inverse's finished row c, so the whole lower triangle takes part in
-// every step and no second pass is needed.  All updates of an entry are summed apart (u) and
-// subtracted once, when its column is reached.  87 k FMAs at 2 per cycle are half of the kernel's
-// time; the rest is the chain of 64 pivots.
-__global__ void __launch_bounds__(kThreads) digit_diag(int k, Dig g, double* __restrict__ diag,
-                                                       int* __restrict__ status)
+// ---- diagonal block: L_kk in 64-bit fixed point, its inverse in FP64, one cluster per matrix ----
+//
+// The FP64 pipe takes a warp instruction every 64 cycles and SM partition, whatever its active lanes
+// (a lone rsqrt is 456 cycles), so the 64 dependent pivots and the 44 k FMAs of a 64 x 64 factorisation
+// in FP64 took 83 us with the inverse; this takes 44 (alone) or 47 us.  CTA 0 factors the block in integers instead: row r is scaled
+// by 2^-e_r, 2^(2 e_r) above S_rr, so that |S| and |L| are at most 1, held as 2^58 times their
+// value.  A product sum is three 32 x 32 -> 64 multiply-adds (64 per cycle) on L = h 2^29 + l: h h'
+// and h l' + l h', l l' (below 2^-56 of a product) left out; the sums cannot overflow, since rows of L
+// have norm at most 1 (sum h h' <= 2^58, sum of the cross terms <= 2^61).  All updates of an entry are
+// thus summed exactly but for the last bits and subtracted once, when its column is reached.
+//
+// Within CTA 0 one warp factors the 4 x 4 diagonal block of a panel of four columns (the chain of pivots),
+// two warps follow it with the panel's 64 rows, and sixteen warps hold the entries' sums and update
+// them, the next panel's columns first, while those go on.  The other CTAs of the cluster form 8 to 24
+// columns each of the inverse in FP64 as the factor's columns arrive in their shared memory.
+constexpr int kDiagOwners = 512, kBlockThread = kDiagOwners + TS, kDiagThreads = kBlockThread + 32;
+constexpr int kMaxHelpers = 7, kPanel = 4;
+constexpr int kFrac = 58, kLow = 29;
+constexpr int kDiagLd = TS + 1;
+
+struct DiagFactor {                     // CTA 0
+    long long t[TS * kDiagLd];          // scaled block, column-major
+    long long colv[2][kPanel][TS];      // a panel's columns with their updates
+    long long group[2][8][TS];          // eight columns of L
+    int2 lsp[2][kPanel][TS];            // a panel's columns of L, split (h, l)
+    longlong2 piv[kPanel];              // a pivot's inverse root: (c, a << 32 | m) of InvSqrt
+    long long pv[kPanel];               // the pivot
+    int2 sb[kPanel][kPanel];            // the diagonal block's columns of L, split
+};
+struct DiagInverse {                    // the other CTAs
+    long long lq[8][8][TS];             // L's columns as they arrive, 8 groups
+    double ld[2][8][TS];                // the current group in FP64, two buffers
+    double x[TS][24];                   // finished rows of this CTA's columns
+    int smax[kMaxHelpers + 1][TS];      // row exponents of each CTA's part
+};
+struct DiagShared {
+    union {
+        DiagFactor f;
+        DiagInverse v;
+    };
+    long long yq[TS];                   // 1 / L_cc as yq 2^(yk - 61)
+    int yk[TS];
+    int e[TS];                          // row scales
+    uint64_t full[8];
+    int bad;
+};
+
+// the CTA's shared-memory address p in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t mapa(const void* p, int rank)
 {
-    __shared__ double colv[TS], rowv[TS], lv[TS], gv[TS];
-    __shared__ double sx[TS][TS + 1];
-    __shared__ int smax[4][TS];
-    const int b = blockIdx.x, t = threadIdx.x, tr = t % 16, tc = t / 16;
-    const double* tile = g.A + (size_t)b * g.strideA + (size_t)tile_index(k, k) * TILE_ELEMS;
-    double s[4][4], u[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            s[a][q] = q <= a ? tile[tr + 16 * a + TS * (tc + 16 * q)] : 0.0;
-            u[a][q] = 0.0;
-        }
-    bool bad = false;
-#pragma unroll
-    for (int c1 = 0; c1 < 4; ++c1)
-        for (int c0 = 0; c0 < 16; ++c0) {
-            const int c = 16 * c1 + c0;
-            if (tc == c0) {
-#pragma unroll
-                for (int a = c1; a < 4; ++a) colv[tr + 16 * a] = s[a][c1] - u[a][c1];
-            }
-            if (tr == c0) {
-#pragma unroll
-                for (int q = 0; q <= c1; ++q) rowv[tc + 16 * q] = -u[c1][q];
-            }
-            __syncthreads();
-            if (t < 32) {
-                double v = colv[c];
-                if (!(v > 0.0)) {  // not positive definite (or NaN): flag, keep going on a benign value
-                    bad = true;
-                    v = 1.0;
-                }
-                const double inv = rsqrt(v);
-                if (t == 0) diag[(size_t)b * g.nt * TS + k * TS + c] = v * inv;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int r = t + 32 * h;
-                    const double l = (r > c ? colv[r] : rowv[r]) * inv;
-                    const double x = r == c ? inv : l;
-                    lv[r] = l;
-                    gv[r] = x;
-                    sx[c][r] = r <= c ? x : 0.0;
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int a = c1; a < 4; ++a) {
-                const int r = tr + 16 * a;
-                const double l = r > c ? lv[r] : 0.0;
-#pragma unroll
-                for (int q = 0; q <= a; ++q) {
-                    const int col = tc + 16 * q;
-                    u[a][q] = fma(l, gv[col], col == c && r > c ? 0.0 : u[a][q]);
-                }
-            }
-        }
-    __syncthreads();
-    if (t == 0 && bad && status[b] == CG_OK) status[b] = CG_ERR_NOT_PD;
-    // the inverse's rows in digits: thread (row r, columns 16 q .. 16 q + 15)
-    const int r = t % TS, q = t / TS;
-    int f = 0;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) f = max(f, exp_field(sx[r][16 * q + c]));
-    smax[q][r] = f;
-    __syncthreads();
-    const int e = row_exp(max(max(smax[0][r], smax[1][r]), max(smax[2][r], smax[3][r])));
-    if (q == 0) g.dex[(size_t)b * TS + r] = e;
-    unsigned char* out = g.dimg + (size_t)b * kDImg;
-#pragma unroll
-    for (int kc = 0; kc < 2; ++kc) {
-        unsigned long long w[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) w[c] = to_digits(to_fixed(sx[r][16 * q + 8 * kc + c], e));
-        unsigned char* o = out + (2 * q + kc) * kDCore + r * 16;
-        store_digits(w, [&](int i, uint4 v) { *reinterpret_cast<uint4*>(o + i * kDPlane) = v; });
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, long long v)
+{
+    asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, int v)
+{
+    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// what this thread has written or seen written is visible to the thread that sees the arrival
+__device__ __forceinline__ void arrive_cluster(uint64_t* bar, int rank)
+{
+    asm volatile("fence.acq_rel.cluster;\n\tmbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                     mapa(bar, rank))
+                 : "memory");
+}
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity)
+{
+    const uint32_t a = smem_u32(bar);
+    for (uint32_t it = 0; it < kWaits; ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (done) return true;
     }
+    return false;
+}
+
+// v 2^(kFrac - e) rounded to the nearest; false where |v| >= 2^e or v is not finite
+__device__ __forceinline__ bool to_scaled(double v, int e, long long& x)
+{
+    const long long bits = __double_as_longlong(v);
+    const int f = (int)((unsigned long long)bits >> 52) & 0x7ff, r = e - (f - 1022);
+    x = 0;
+    if (f == 0 || r > 60) return true;
+    if (r < 0 || f == 0x7ff) return false;
+    const unsigned long long m = ((unsigned long long)bits & 0xfffffffffffffull) | 0x10000000000000ull;
+    const long long y = (long long)(((m << (kFrac - 52) >> r) + 1) >> 1);
+    x = bits < 0 ? -y : y;
+    return true;
+}
+
+// 1 / sqrt(v) for v > 0 to about 2^-58: an FP32 estimate y0 = m 2^(a - 54), m of 24 bits (relative error
+// below 2^-21), and y0 (1 + c), c 2^-58 = h / 2 + 3 h^2 / 8, h = 1 - v y0^2 (the series of (1 - h)^(-1/2))
+struct InvSqrt {
+    unsigned m;
+    int a;
+    long long c;
+};
+__device__ __forceinline__ InvSqrt inv_sqrt(long long v)
+{
+    // v 2^-sh below 2^31 with at least 24 bits, sh even
+    const int sh = v >= (1ll << 52) ? 28 : 33 - ((__clzll(v) - 1) | 1);
+    float f;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"((float)(int)(sh >= 0 ? v >> sh : v << -sh)));
+    const unsigned bits = __float_as_uint(f);
+    InvSqrt y;
+    y.m = (bits & 0x7fffffu) | 0x800000u;
+    y.a = (int)(bits >> 23) - 127 - 23 + 54 - sh / 2;
+    // v 2^(2 a) m^2 is near 2^108: h = 1 - that, 2^58 times
+    const unsigned long long m2 = ((unsigned long long)y.m * y.m) << 14, n = (unsigned long long)v << (2 * y.a);
+    const unsigned ah = (unsigned)(n >> 31), al = (unsigned)n & 0x7fffffffu;
+    const unsigned bh = (unsigned)(m2 >> 31), bl = (unsigned)m2 & 0x7fffffffu;
+    const long long h = (1ll << 58) - (long long)(((unsigned long long)ah * bh >> 2) +
+                                                  (((unsigned long long)ah * bl + (unsigned long long)al * bh) >> 33));
+    const int hs = (int)(h >> 16);              // below 2^22
+    y.c = (h >> 1) + ((3 * (long long)hs * hs) >> 29);
+    return y;
+}
+
+// x y 2^(kFrac / 2) for |x| <= 2^(kFrac / 2) sqrt(v): an entry of L from the column's entry x
+__device__ __forceinline__ long long mul_inv_sqrt(long long x, const InvSqrt& y)
+{
+    const long long z = x << y.a;               // below 2^61
+    const int w = (int)(y.m << 7);
+    const long long l0 =
+        (long long)(int)(z >> 32) * w + (long long)(((unsigned long long)(unsigned)z * (unsigned)w) >> 32);
+    // + l0 c 2^-58, |c| < 2^38, in 29 + 29 and 22 + 16 bits
+    const int lh = (int)(l0 >> 29), ll = (int)(l0 & 0x1fffffff), ch = (int)(y.c >> 16), cl = (int)(y.c & 0xffff);
+    return l0 + (((long long)lh * ch >> 13) + (((long long)lh * cl + ((long long)ll * ch >> 13)) >> 29));
+}
+
+__device__ __forceinline__ int2 split_low(long long l)
+{
+    const int lo = (int)(((l + (1ll << (kLow - 1))) & ((1ll << kLow) - 1)) - (1ll << (kLow - 1)));
+    return make_int2((int)((l - lo) >> kLow), lo);
+}
+
+__device__ __forceinline__ void named_sync(int id, int threads)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// thread i < kDiagOwners: group g of L's columns and pivots into the shared memory of the other CTAs
+__device__ __forceinline__ void diag_publish(DiagShared& sh, int ctas, int g, int i)
+{
+    for (int rank = 1; rank < ctas; ++rank) {
+        st_cluster(mapa(&sh.v.lq[g][0][0] + i, rank), (&sh.f.group[g & 1][0][0])[i]);
+        if (i < 8) {
+            st_cluster(mapa(&sh.yq[8 * g + i], rank), sh.yq[8 * g + i]);
+            st_cluster(mapa(&sh.yk[8 * g + i], rank), sh.yk[8 * g + i]);
+        }
+    }
+}
+
+// named barriers of CTA 0: kPub + parity (the panel's columns are in colv: the two warps that hold them,
+// the row warps and the block warp), kFact + parity (L's columns are in lsp and group: every thread),
+// kCol + j (column j of the panel's diagonal block is in piv, pv, sb: the row warps and the block warp)
+constexpr int kPub = 1, kFact = 3, kCol = 5;
+constexpr int kPubThreads = 64 + TS + 32, kColThreads = TS + 32;
+
+// x - s q for split numbers of kFrac fraction bits
+__device__ __forceinline__ long long sub_product(long long x, int2 s, int2 q)
+{
+    return x - ((long long)s.x * q.x + (((long long)s.x * q.y + (long long)s.y * q.x) >> kLow));
+}
+
+// the diagonal block of panel p, columns 4 p .. 4 p + 3 (one warp, every lane the same)
+__device__ __forceinline__ bool diag_block(DiagShared& sh, int p)
+{
+    DiagFactor& f = sh.f;
+    const int buf = p & 1, c0 = kPanel * p, lane = threadIdx.x % 32;
+    bool bad = false;
+    long long d[kPanel][kPanel];
+#pragma unroll
+    for (int j = 0; j < kPanel; ++j)
+#pragma unroll
+        for (int i = j; i < kPanel; ++i) d[j][i] = f.colv[buf][j][c0 + i];
+#pragma unroll
+    for (int j = 0; j < kPanel; ++j) {
+        long long v = d[j][j];
+        if (v <= 0) {  // not positive definite: flag, keep going on a benign value
+            bad = true;
+            v = 1ll << kFrac;
+        }
+        const InvSqrt y = inv_sqrt(v);
+        int2 sb[kPanel];
+#pragma unroll
+        for (int i = j + 1; i < kPanel; ++i) sb[i] = split_low(mul_inv_sqrt(d[j][i], y));
+        if (lane == 0) {
+            f.piv[j] = make_longlong2(y.c, ((long long)y.a << 32) | y.m);
+            f.pv[j] = v;
+#pragma unroll
+            for (int i = j + 1; i < kPanel; ++i) f.sb[j][i] = sb[i];
+        }
+        __syncwarp();
+        named_arrive(kCol + j, kColThreads);
+#pragma unroll
+        for (int i = j + 1; i < kPanel; ++i)
+#pragma unroll
+            for (int q = i; q < kPanel; ++q) d[i][q] = sub_product(d[i][q], sb[i], sb[q]);
+    }
+    return bad;
+}
+
+// its rows: row r per thread
+__device__ __forceinline__ void diag_rows(DiagShared& sh, int p, int r)
+{
+    DiagFactor& f = sh.f;
+    const int buf = p & 1, c0 = kPanel * p;
+    long long x[kPanel];
+#pragma unroll
+    for (int j = 0; j < kPanel; ++j) x[j] = f.colv[buf][j][r];
+#pragma unroll
+    for (int j = 0; j < kPanel; ++j) {
+        named_sync(kCol + j, kColThreads);
+        const longlong2 w = f.piv[j];
+        InvSqrt y;
+        y.c = w.x;
+        y.m = (unsigned)w.y;
+        y.a = (int)(w.y >> 32);
+        if (r == c0 + j) x[j] = f.pv[j];
+        const long long l = r >= c0 + j ? mul_inv_sqrt(x[j], y) : 0;
+        const int2 s = split_low(l);
+#pragma unroll
+        for (int i = j + 1; i < kPanel; ++i) x[i] = sub_product(x[i], s, f.sb[j][i]);
+        f.group[(p >> 1) & 1][(p & 1) * kPanel + j][r] = l;
+        f.lsp[buf][j][r] = s;
+        if (r == c0 + j) {
+            sh.yq[r] = ((long long)y.m << 38) + (__mul64hi((long long)y.m << 38, y.c << 24) >> 18);
+            sh.yk[r] = y.a - 2;
+        }
+    }
+}
+
+__device__ __forceinline__ void diag_factor(DiagShared& sh, int ctas, const double* __restrict__ tile)
+{
+    DiagFactor& f = sh.f;
+    const int t = threadIdx.x, tr = t % 16, tc = t / 16;
+    bool bad = false;
+    for (int i = t; i < TILE_ELEMS; i += kDiagThreads) {
+        const int r = i % TS, c = i / TS;
+        long long x = 0;
+        if (r >= c) bad |= !to_scaled(tile[i], sh.e[r] + sh.e[c], x);
+        f.t[c * kDiagLd + r] = x;
+        if (c < kPanel) f.colv[0][c][r] = x;
+    }
+    if (bad) sh.bad = 1;
+    __syncthreads();
+    constexpr int np = TS / kPanel;
+    if (t >= kDiagOwners) {
+        bad = false;
+#pragma unroll 1
+        for (int p = 0; p < np; ++p) {
+            if (p > 0) named_sync(kPub + (p & 1), kPubThreads);
+            if (t >= kBlockThread) bad |= diag_block(sh, p);
+            else diag_rows(sh, p, t - kDiagOwners);
+            named_sync(kFact + (p & 1), kDiagThreads);
+        }
+        if (bad && t == kBlockThread) sh.bad = 1;
+    } else {
+        long long hh[4][2], hl[4][2];  // rows tr + 16 a, columns tc + 32 b
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) hh[a][b] = hl[a][b] = 0;
+        auto update = [&](int buf, int b) {  // columns tc + 32 b by the panel in buffer buf
+            int2 y[kPanel];
+#pragma unroll
+            for (int j = 0; j < kPanel; ++j) y[j] = f.lsp[buf][j][tc + 32 * b];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                // whole warps above the diagonal (a warp has two values of tc)
+                if ((tc & ~1) + 32 * b > 16 * a + 15) continue;
+#pragma unroll
+                for (int j = 0; j < kPanel; ++j) {
+                    const int2 x = f.lsp[buf][j][tr + 16 * a];
+                    hh[a][b] += (long long)x.x * y[j].x;
+                    hl[a][b] += (long long)x.x * y[j].y;
+                    hl[a][b] += (long long)x.y * y[j].x;
+                }
+            }
+        };
+        constexpr int per = 32 / kPanel;  // panels in 32 columns
+#pragma unroll 1
+        for (int p = 0; p < np; ++p) {
+            const int buf = p & 1;
+            named_sync(kFact + buf, kDiagThreads);
+            // the group published in the last step (every thread has passed its stores)
+            if (p > 0 && (p & 1) == 0 && t < ctas - 1) arrive_cluster(&sh.full[p / 2 - 1], 1 + t);
+            const bool mine = p + 1 < np && tc / kPanel == (p + 1) % per;  // columns of the next panel,
+            const int nb = (p + 1) / per;                                  // in the b = nb half
+            if (mine) {
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+                    if (b == nb) {
+                        update(buf, b);
+                        const int c = tc + 32 * b;
+#pragma unroll
+                        for (int a = 0; a < 4; ++a) {
+                            const int r = tr + 16 * a;
+                            f.colv[buf ^ 1][c % kPanel][r] =
+                                r >= c ? f.t[c * kDiagLd + r] - (hh[a][b] + (hl[a][b] >> kLow)) : 0;
+                        }
+                    }
+                named_arrive(kPub + (buf ^ 1), kPubThreads);
+            }
+            if (p & 1) diag_publish(sh, ctas, p / 2, t);
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+                if (tc / kPanel + per * b > p + 1) update(buf, b);
+        }
+    }
+    __syncthreads();
+    if (t < ctas - 1) arrive_cluster(&sh.full[7], 1 + t);
+}
+
+// a cluster of ctas CTAs (4 or 8) per matrix
+__global__ void __launch_bounds__(kDiagThreads, 1)
+    digit_diag(int k, int ctas, Dig g, double* __restrict__ diag, int* __restrict__ status)
+{
+    extern __shared__ __align__(128) unsigned char sm[];
+    DiagShared& sh = *reinterpret_cast<DiagShared*>(sm);
+    const int rank = blockIdx.x % ctas, b = blockIdx.x / ctas, t = threadIdx.x;
+    const double* tile = g.A + (size_t)b * g.strideA + (size_t)tile_index(k, k) * TILE_ELEMS;
+    if (t < 8) mbar_init(&sh.full[t], 1);
+    if (t == 0) sh.bad = 0;
+    fence_mbar_init();
+    if (t < TS) sh.e[t] = (exp_field(tile[t * (TS + 1)]) - 1022 + 1) >> 1;  // S_rr < 2^(2 e)
+    cluster_barrier();
+    if (rank == 0) {
+        diag_factor(sh, ctas, tile);
+        cluster_barrier();
+        if (t == 0 && sh.bad && status[b] == CG_OK) status[b] = CG_ERR_NOT_PD;
+        cluster_barrier();
+        return;
+    }
+    if (t >= kDiagOwners) {  // the panel's warps: nothing to do here
+        cluster_barrier();
+        cluster_barrier();
+        return;
+    }
+    DiagInverse& v = sh.v;
+    // columns q0 .. q0 + 8 nj - 1
+    const int q0 = ctas == 8 ? 8 * (rank - 1) : rank == 1 ? 0 : rank == 2 ? 16 : 40;
+    const int nj = ctas == 8 ? (rank == 7 ? 2 : 1) : rank == 1 ? 2 : 3;
+    const int r = t / 8, qi = t % 8;
+    double w[3] = {0.0, 0.0, 0.0};
+    bool ok = true;
+    for (int grp = 0; grp < 8; ++grp) {
+        ok = wait_cluster(&sh.full[grp], 0) && ok;
+        if (rank == 1 && t < 8) {  // L's diagonal
+            const int c = 8 * grp + t;
+            diag[(size_t)b * g.nt * TS + k * TS + c] = scaled(v.lq[grp][t][c], sh.e[c] - kFrac);
+        }
+        if (8 * grp + 7 < q0) continue;
+        v.ld[grp & 1][t / TS][t % TS] = scaled(v.lq[grp][t / TS][t % TS], -kFrac);
+        named_sync(1, kDiagOwners);
+        for (int c = 0; c < 8; ++c) {
+            const int m = 8 * grp + c;
+            if (r == m) {
+                const double inv = scaled(sh.yq[m], sh.yk[m] - 61);
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    if (j < nj) {
+                        const int q = q0 + qi + 8 * j;
+                        v.x[m][qi + 8 * j] = q == m ? inv : q < m ? -w[j] * inv : 0.0;
+                    }
+            }
+            named_sync(1, kDiagOwners);
+            if (4 * (t / 32) + 3 > m) {
+                const double l = r > m ? v.ld[grp & 1][c][r] : 0.0;
+#pragma unroll
+                for (int j = 0; j < 3; ++j)
+                    if (j < nj && q0 + 8 * j <= m) w[j] = fma(l, v.x[m][qi + 8 * j], w[j]);
+            }
+        }
+    }
+    if (!ok) atomicExch(g.err, 1);
+    named_sync(1, kDiagOwners);
+    // The inverse's rows in digits (columns scaled back by 2^-e), one exponent per row over all these CTAs:
+    // thread (row, 8 columns)
+    const int row = t % TS, part = t / TS;
+    if (t < TS) {
+        int f = -(1 << 28);
+        for (int q = 0; q < 8 * nj; ++q) {
+            const int x = exp_field(v.x[row][q]);
+            if (q0 + q <= row && x) f = max(f, x == 0x7ff ? kNonFinite : x - sh.e[q0 + q]);
+        }
+        for (int rk = 1; rk < ctas; ++rk) st_cluster(mapa(&v.smax[rank][row], rk), f);
+    }
+    cluster_barrier();
+    int e = v.smax[1][row];
+    for (int rk = 2; rk < ctas; ++rk) e = max(e, v.smax[rk][row]);
+    e = e > kNonFinite / 2 ? kNonFinite : e < -(1 << 27) ? -1022 : e - 1022;
+    if (rank == 1 && part == 0) g.dex[(size_t)b * TS + row] = e;
+    if (part < nj) {
+        unsigned long long d[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const int q = 8 * part + c;
+            d[c] = to_digits(q0 + q <= row ? to_fixed(v.x[row][q], e + sh.e[q0 + q]) : 0);
+        }
+        unsigned char* o = g.dimg + (size_t)b * kDImg + (q0 / 8 + part) * kDCore + row * 16;
+        store_digits(d, [&](int i, uint4 x) { *reinterpret_cast<uint4*>(o + i * kDPlane) = x; });
+    }
+    cluster_barrier();
 }
 
 // Panel of step k, one CTA per row pair: rows x (64 columns) times the inverted diagonal block, the
@@ -581,6 +917,26 @@ __global__ void __launch_bounds__(kThreads, 1) digit_update(int k, int njobs, in
 
 }  // namespace
 
+// Seven CTAs for the inverse keep up with the factor; three take a third longer, but beyond the clusters
+// of eight that the SMs hold at once a second wave would cost more.
+static int launch_diag(cg_ctx* ctx, int B, int k, const Dig& g, double* diag, int* status, cudaStream_t s)
+{
+    const int ctas = 8 * B <= ctx->sm_count ? 8 : 4;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas * B);
+    cfg.blockDim = dim3(kDiagThreads);
+    cfg.dynamicSmemBytes = sizeof(DiagShared);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CG_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, digit_diag, k, ctas, g, diag, status));
+    return CG_OK;
+}
+
 size_t digit_bytes(int nt, int ne)
 {
     const size_t pairs = (size_t)(nt + ne) / 2;
@@ -604,10 +960,11 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
     g.ex = reinterpret_cast<int*>(g.dimg + (size_t)B * kDImg);
     g.dex = g.ex + (size_t)B * pairs * 128;
     g.err = err;
+    CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DiagShared)));
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem));
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem));
     for (int k = 0; k < nt; ++k) {
-        digit_diag<<<B, kThreads, 0, s>>>(k, g, diag, status);
+        if (int rc = launch_diag(ctx, B, k, g, diag, status, s)) return rc;
         const int nq = nt / 2 - (k + 1) / 2;
         const int npe = ext == DIGIT_EXT_IDENTITY ? k / 2 + 1 : ne / 2;
         if (nq + npe == 0) { count_launch(ctx, 1); continue; }
