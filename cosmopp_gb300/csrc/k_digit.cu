@@ -68,14 +68,15 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
 }
 
 // the digit products of 16 columns (k-cores 2 kc, 2 kc + 1): digit i of A against runs of digits of B,
-// which land in consecutive 64-column accumulators i + j; the first column chunk initialises them
+// which land in consecutive accumulators i + j of NC columns; the first column chunk initialises them
+template <int NC>
 __device__ __forceinline__ void issue_products(uint32_t tmem, uint64_t a, uint64_t b, uint32_t a_plane,
                                                uint32_t b_plane, bool first)
 {
     const uint32_t acc = first ? 0u : 1u;
     auto run = [&](int i, int j, int cnt, uint32_t ac) {
-        mma_bf16(tmem + 64 * (i + j), a + (uint64_t)i * (a_plane >> 4), b + (uint64_t)j * (b_plane >> 4),
-                 idesc_bf16(128, 64 * cnt), ac);
+        mma_bf16(tmem + NC * (i + j), a + (uint64_t)i * (a_plane >> 4), b + (uint64_t)j * (b_plane >> 4),
+                 idesc_bf16(128, NC * cnt), ac);
     };
     run(0, 0, 4, acc);
     run(0, 4, 3, acc);
@@ -696,8 +697,8 @@ __global__ void __launch_bounds__(kThreads, 1) digit_panel(int k, Dig g)
         const uint64_t ad = smem_desc(smem_u32(sm + kPanelA), kCore, kGroupBytes);
         const uint64_t bd = smem_desc(smem_u32(sm + kPanelB), kDCore, kGroupBytes);
         for (int kc = 0; kc < 4; ++kc)
-            issue_products(tmem, ad + (uint64_t)kc * (2 * kCore >> 4), bd + (uint64_t)kc * (2 * kDCore >> 4), kPlane,
-                           kDPlane, kc == 0);
+            issue_products<TS>(tmem, ad + (uint64_t)kc * (2 * kCore >> 4), bd + (uint64_t)kc * (2 * kDCore >> 4),
+                               kPlane, kDPlane, kc == 0);
         mma_commit(&done);
     }
     __syncwarp();
@@ -757,11 +758,74 @@ __global__ void __launch_bounds__(kThreads, 1) digit_panel(int k, Dig g)
 }
 
 // Update of step k: persistent CTAs over (pair, pair) jobs of 128 x 128 outputs, K = 64.  Both images
-// (2 x 112 KB) fill the shared memory; the 64 columns of each half of the second pair are one pass, with
-// eight FP32 accumulators of 64 columns: all 512 tensor-memory columns.  The next job's images are
-// fetched while the last pass is joined and subtracted.
-constexpr int kUpB = kImg, kUpTail = 2 * kImg;
-constexpr int kUpSmem = kUpTail + 2 * 128 * 4;
+// (2 x 112 KB) fill the shared memory.  A job is four passes of 32 columns (8-column groups of one parity
+// of one half of the second pair), whose eight accumulators take 256 tensor-memory columns: two passes
+// are in flight (one 64-column pass after the other with 8 warps took 22 us a job, this 11.5 in a batch of
+// 16).  Warp 16 fetches the images, 16 columns at a time as the last pass of the job before is done
+// with them, and issues the products; warps 0 .. 15 join a pass's accumulators and add them to the FP64
+// matrix while the next pass runs.  Per job and SM the tensor cores need 8.7 k cycles, the FP64 pipe (one
+// addition per output, 64 cycles per warp and partition) 8.2 k, the integer work about 8 k.
+constexpr int kUpB = kImg, kUpSmem = 2 * kImg;
+constexpr int kUpWarps = 16, kUpThreads = (kUpWarps + 1) * 32, kPassCols = 32;
+
+// four columns of all eight accumulators (kPassCols columns apart), load and wait in one statement
+__device__ __forceinline__ void tmem_ld_acc4(uint32_t t, uint32_t (&r)[8][4])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4, %5, %6, %7}, [%33];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8, %9, %10, %11}, [%34];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%12, %13, %14, %15}, [%35];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16, %17, %18, %19}, [%36];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%20, %21, %22, %23}, [%37];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%24, %25, %26, %27}, [%38];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%28, %29, %30, %31}, [%39];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0][0]), "=r"(r[0][1]), "=r"(r[0][2]), "=r"(r[0][3]), "=r"(r[1][0]), "=r"(r[1][1]), "=r"(r[1][2]),
+          "=r"(r[1][3]), "=r"(r[2][0]), "=r"(r[2][1]), "=r"(r[2][2]), "=r"(r[2][3]), "=r"(r[3][0]), "=r"(r[3][1]),
+          "=r"(r[3][2]), "=r"(r[3][3]), "=r"(r[4][0]), "=r"(r[4][1]), "=r"(r[4][2]), "=r"(r[4][3]), "=r"(r[5][0]),
+          "=r"(r[5][1]), "=r"(r[5][2]), "=r"(r[5][3]), "=r"(r[6][0]), "=r"(r[6][1]), "=r"(r[6][2]), "=r"(r[6][3]),
+          "=r"(r[7][0]), "=r"(r[7][1]), "=r"(r[7][2]), "=r"(r[7][3])
+        : "r"(t), "r"(t + kPassCols), "r"(t + 2 * kPassCols), "r"(t + 3 * kPassCols), "r"(t + 4 * kPassCols),
+          "r"(t + 5 * kPassCols), "r"(t + 6 * kPassCols), "r"(t + 7 * kPassCols)
+        : "memory");
+}
+
+// The same sum as join_acc with the fewest operations: accumulators 0 .. 4 are at most 2^22 (64 columns of
+// at most 4 products of 2^14 beside the two with a top digit, which is at most 64), so adding 1.5 2^23
+// leaves the number in the low mantissa bits; pairs fit 32 bits.
+__device__ __forceinline__ long long join_acc4(const uint32_t (&r)[8][4], int q)
+{
+    constexpr unsigned kMagic = 0x4b400000u;  // 1.5 2^23
+    auto m = [&](int s) { return __float_as_uint(__uint_as_float(r[s][q]) + 12582912.0f); };
+    auto f = [&](int s) { return (unsigned)__float2int_rn(__uint_as_float(r[s][q])); };
+    const int v01 = (int)(m(0) * 256u + (m(1) - kMagic * 257u));
+    const int v23 = (int)(m(2) * 256u + (m(3) - kMagic * 257u));
+    const int v45 = (int)(m(4) * 256u + (f(5) - kMagic * 256u));
+    const int v67 = (int)(f(6) * 256u + (f(7) + 4096u));
+    long long x = (long long)v45 * 8 + (v67 >> 13);
+    x = (long long)v23 * 524288 + x;
+    return x + ((long long)v01 << 35);
+}
+
+// u 2^s in FP64, rounded to the nearest, its sign flipped by `flip` (0 or 0x80000000): __ll2double_rn is one
+// FP64-pipe instruction more per number, and that pipe is the scarcest
+__device__ __forceinline__ double scaled_int(long long u, int s, unsigned flip)
+{
+    const int hi = (int)(u >> 32), sg = hi >> 31;
+    const unsigned long long a = (unsigned long long)((u ^ sg) - sg);
+    const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
+    const int lz = __clz((int)ah);
+    const int e = 1085 - lz + s;  // exponent field less one
+    if (ah == 0 || (unsigned)(e - 1) > 2040u) {
+        const double x = scaled(u, s);
+        return __hiloint2double(__double2hiint(x) ^ (int)flip, __double2loint(x));
+    }
+    const unsigned nh = __funnelshift_l(al, ah, lz), nl = al << lz;
+    const unsigned long long m = (((unsigned long long)(nh >> 11) << 32) | __funnelshift_r(nl, nh, 11)) +
+                                 ((nl >> 10) & 1u) + ((unsigned long long)(unsigned)(e << 20) << 32);
+    return __hiloint2double((int)((unsigned)(m >> 32) | (((unsigned)sg ^ flip) & 0x80000000u)), (int)(unsigned)m);
+}
 
 struct UpJob {
     int b, kind, p, q;        // kind 0: A's trailing part, 1: E's rows, 2: V = M^T M; q: columns, p: rows
@@ -801,127 +865,142 @@ __device__ __forceinline__ UpJob up_job(const Dig& g, int k, int per, int npe, i
     return j;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) digit_update(int k, int njobs, int per, int npe, Dig g)
+// the passes of a job: halves [h0, h1) of the second pair, two parities each
+__device__ __forceinline__ void up_halves(const UpJob& j, int k, int& h0, int& h1)
+{
+    h0 = (j.kind != 2 && 2 * j.q <= k) ? 1 : 0;      // the half with column k is not part of the update
+    h1 = (j.kind == 2 && 2 * j.q + 1 > k) ? 1 : 2;
+}
+
+__global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, int per, int npe, Dig g)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    int* sex = reinterpret_cast<int*>(sm + kUpTail);  // [2][128] exponents of the column pair
-    __shared__ uint64_t full[4], done;
+    __shared__ uint64_t full[4], empty[4], tfull[2], tempty[2];
     __shared__ uint32_t tptr;
-    const int t = threadIdx.x, warp = t >> 5, m = t & 127, ch = t >> 7;
-    const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int pairs = dig_pairs(g);
     if (warp == 0) tmem_alloc(&tptr, 512);
-    auto fetch = [&](const UpJob& j) {  // thread 0: both images, 16 columns per barrier
-        const unsigned char* a = g.img + ((size_t)j.b * pairs + j.pa) * kImg;
-        const unsigned char* bb = g.img + ((size_t)j.b * pairs + j.pb) * kImg;
-        for (int kc = 0; kc < 4; ++kc) {
-            mbar_arrive_expect_tx(&full[kc], (j.pa == j.pb ? 2 : 4) * kCore);
-            bulk_g2s(smem_u32(sm + 2 * kc * kCore), a + 2 * kc * kCore, 2 * kCore, &full[kc]);
-            if (j.pa != j.pb)
-                bulk_g2s(smem_u32(sm + kUpB + 2 * kc * kCore), bb + 2 * kc * kCore, 2 * kCore, &full[kc]);
-        }
-    };
-    int job = blockIdx.x;
-    UpJob j = up_job(g, k, per, npe, job);
     if (t == 0) {
-        for (int kc = 0; kc < 4; ++kc) mbar_init(&full[kc], 1);
-        mbar_init(&done, 1);
+        for (int i = 0; i < 4; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&tfull[i], 1);
+            mbar_init(&tempty[i], kUpWarps);
+        }
         fence_mbar_init();
-        fetch(j);
     }
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = tptr;
-    uint32_t passes = 0, round = 0;
     bool ok = true;
-    for (; job < njobs; job += gridDim.x, ++round) {
-        // the half of the column pair that holds column k is not part of the update
-        const int h0 = (j.kind != 2 && 2 * j.q <= k) ? 1 : 0;
-        const int h1 = (j.kind == 2 && 2 * j.q + 1 > k) ? 1 : 2;
-        int* se = sex + 128 * (round & 1);
-        if (t < 128) se[t] = g.ex[((size_t)j.b * pairs + j.pb) * 128 + t];
-        const int ea = g.ex[((size_t)j.b * pairs + j.pa) * 128 + 64 * half + r];
-        const UpJob cur = j;
-        for (int h = h0; h < h1; ++h) {
-            if (t == 0) {
-                const uint64_t ad = smem_desc(smem_u32(sm), kCore, kGroupBytes);
-                const uint64_t bd = smem_desc(smem_u32(sm + (cur.pa == cur.pb ? 0 : kUpB) + h * kGroupBytes), kCore,
-                                              2 * kGroupBytes);
+    uint32_t pass = 0, round = 0;
+    if (warp == kUpWarps) {
+        if (lane == 0)
+            for (int job = blockIdx.x; job < njobs; job += gridDim.x, ++round) {
+                const UpJob j = up_job(g, k, per, npe, job);
+                const unsigned char* a = g.img + ((size_t)j.b * pairs + j.pa) * kImg;
+                const unsigned char* bb = g.img + ((size_t)j.b * pairs + j.pb) * kImg;
                 for (int kc = 0; kc < 4; ++kc) {
-                    if (h == h0) ok = mbar_wait(&full[kc], round & 1, kWaits, g.err) && ok;
-                    issue_products(tmem, ad + (uint64_t)kc * (2 * kCore >> 4), bd + (uint64_t)kc * (2 * kCore >> 4),
-                                   kPlane, kPlane, kc == 0);
+                    if (round > 0) ok = mbar_wait(&empty[kc], (round - 1) & 1, kWaits, g.err) && ok;
+                    mbar_arrive_expect_tx(&full[kc], (j.pa == j.pb ? 2 : 4) * kCore);
+                    bulk_g2s(smem_u32(sm + 2 * kc * kCore), a + 2 * kc * kCore, 2 * kCore, &full[kc]);
+                    if (j.pa != j.pb)
+                        bulk_g2s(smem_u32(sm + kUpB + 2 * kc * kCore), bb + 2 * kc * kCore, 2 * kCore, &full[kc]);
                 }
-                mma_commit(&done);
-            }
-            // where this row of the pass goes
-            const int rb = 2 * cur.p + half, cb = 2 * cur.q + h;
-            bool valid;
-            double* tile;
-            double* Ab = g.A + (size_t)cur.b * g.strideA;
-            if (cur.kind == 0) {
-                valid = rb > k && rb >= cb;
-                tile = Ab + (size_t)(valid ? tile_index(rb, cb) : 0) * TILE_ELEMS;
-            } else if (cur.kind == 1) {
-                valid = g.ext != DIGIT_EXT_IDENTITY || rb <= k;
-                tile = valid ? ext_tile(g, cur.b, rb, cb) : Ab;
-            } else {
-                valid = rb <= k && rb >= cb;
-                tile = Ab + (size_t)(valid ? tile_index(rb, cb) : 0) * TILE_ELEMS;
-            }
-            const bool fresh = cur.kind == 2 && rb == k;  // V's row k starts here
-            const bool read = valid && !fresh;
-            double* dst = tile + r + TS * 32 * ch;
-            double old[8], nxt[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) old[c] = read ? dst[TS * c] : 0.0;
-            __syncwarp();
-            ok = mbar_wait(&done, passes & 1, kWaits, g.err) && ok;
-            ++passes;
-            fence_after();
-            if (t == 0 && h == h1 - 1 && job + (int)gridDim.x < njobs) {
-                j = up_job(g, k, per, npe, job + gridDim.x);
-                fetch(j);
-            }
-            __syncthreads();  // the column exponents are in place
-#pragma unroll
-            for (int c8 = 0; c8 < 4; ++c8) {
-                if (c8 < 3) {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) nxt[c] = read ? dst[TS * (8 * (c8 + 1) + c)] : 0.0;
-                }
-                uint32_t acc[8][8];
-                tmem_ld_acc(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * ch + 8 * c8, acc);
-                if (valid) {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const double x = scaled(join_acc(acc, c), ea + se[64 * h + 32 * ch + 8 * c8 + c] - 55);
-                        dst[TS * (8 * c8 + c)] = cur.kind == 2 ? old[c] + x : old[c] - x;
+                int h0, h1;
+                up_halves(j, k, h0, h1);
+                for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
+                    const uint32_t buf = pass & 1;
+                    if (pass >= 2) ok = mbar_wait(&tempty[buf], ((pass >> 1) - 1) & 1, kWaits, g.err) && ok;
+                    fence_after();
+                    const uint64_t ad = smem_desc(smem_u32(sm), kCore, kGroupBytes);
+                    const uint64_t bd = smem_desc(smem_u32(sm + (j.pa == j.pb ? 0 : kUpB) + (i >> 1) * kGroupBytes +
+                                                           (i & 1) * 2 * kGroupBytes),
+                                                  kCore, 4 * kGroupBytes);
+                    for (int kc = 0; kc < 4; ++kc) {
+                        if (i == 2 * h0) ok = mbar_wait(&full[kc], round & 1, kWaits, g.err) && ok;
+                        issue_products<kPassCols>(tmem + 256 * buf, ad + (uint64_t)kc * (2 * kCore >> 4),
+                                                  bd + (uint64_t)kc * (2 * kCore >> 4), kPlane, kPlane, kc == 0);
+                        if (i == 2 * h1 - 1) mma_commit(&empty[kc]);
                     }
+                    mma_commit(&tfull[buf]);
                 }
-                __syncwarp();
-#pragma unroll
-                for (int c = 0; c < 8; ++c) old[c] = nxt[c];
             }
-            fence_before();
-            __syncthreads();
-            fence_after();
+        __syncwarp();
+    } else {
+        const int m = 32 * (warp & 3) + lane, c4 = warp >> 2;  // row of the pair image, 8-column group of the pass
+        const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
+        for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
+            const UpJob j = up_job(g, k, per, npe, job);
+            const int ea = g.ex[((size_t)j.b * pairs + j.pa) * 128 + 64 * half + r];
+            const int* eb = g.ex + ((size_t)j.b * pairs + j.pb) * 128;
+            double* Ab = g.A + (size_t)j.b * g.strideA;
+            const unsigned flip = j.kind == 2 ? 0u : 0x80000000u;
+            int h0, h1;
+            up_halves(j, k, h0, h1);
+            for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
+                const uint32_t buf = pass & 1;
+                const int rb = 2 * j.p + half, cb = 2 * j.q + (i >> 1), c0 = (2 * c4 + (i & 1)) * 8;
+                bool valid;
+                double* tile = Ab;
+                if (j.kind == 0) {
+                    valid = rb > k && rb >= cb;
+                    if (valid) tile = Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS;
+                } else if (j.kind == 1) {
+                    valid = g.ext != DIGIT_EXT_IDENTITY || rb <= k;
+                    if (valid) tile = ext_tile(g, j.b, rb, cb);
+                } else {
+                    valid = rb <= k && rb >= cb;
+                    if (valid) tile = Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS;
+                }
+                const bool read = valid && !(j.kind == 2 && rb == k);  // V's row k starts here
+                double* dst = tile + r + TS * c0;
+                double old[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) old[c] = read ? dst[TS * c] : 0.0;
+                const int4 e0 = *reinterpret_cast<const int4*>(eb + 64 * (i >> 1) + c0);
+                const int4 e1 = *reinterpret_cast<const int4*>(eb + 64 * (i >> 1) + c0 + 4);
+                const int se[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+                ok = mbar_wait(&tfull[buf], (pass >> 1) & 1, kWaits, g.err) && ok;
+                fence_after();
+                __syncwarp();
+                const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 256 * buf + 8 * c4;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    uint32_t acc[8][4];
+                    tmem_ld_acc4(ta + 4 * q, acc);
+                    if (q == 1) {
+                        fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&tempty[buf]);
+                    }
+                    if (valid) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            dst[TS * (4 * q + c)] =
+                                old[4 * q + c] + scaled_int(join_acc4(acc, c), ea + se[4 * q + c] - 55, flip);
+                    }
+                    __syncwarp();
+                }
+            }
         }
-        if (job + (int)gridDim.x < njobs) j = up_job(g, k, per, npe, job + gridDim.x);
     }
     if (!ok) atomicExch(g.err, 1);
+    fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace
 
-// Seven CTAs for the inverse keep up with the factor; three take a third longer, but beyond the clusters
-// of eight that the SMs hold at once a second wave would cost more.
+// Seven CTAs for the inverse keep up with the factor (44 us), three take a little longer (47 us); sixteen
+// clusters of eight do not fit the SMs at once (two waves, 87 us), so half the SMs are the limit.
 static int launch_diag(cg_ctx* ctx, int B, int k, const Dig& g, double* diag, int* status, cudaStream_t s)
 {
-    const int ctas = 8 * B <= ctx->sm_count ? 8 : 4;
+    const int ctas = 16 * B <= ctx->sm_count ? 8 : 4;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = ctas;
@@ -972,7 +1051,7 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
         const int per = nq * (nq + 1) / 2 + npe * nq + (ext == DIGIT_EXT_IDENTITY ? npe * (npe + 1) / 2 : 0);
         count_launch(ctx, per > 0 ? 3 : 2);
         if (per > 0)
-            digit_update<<<(unsigned)std::min<long long>((long long)per * B, ctx->sm_count), kThreads, kUpSmem, s>>>(
+            digit_update<<<(unsigned)std::min<long long>((long long)per * B, ctx->sm_count), kUpThreads, kUpSmem, s>>>(
                 k, per * B, per, npe, g);
     }
     CG_CUDA_TRY(ctx, cudaGetLastError());
