@@ -49,7 +49,6 @@ constexpr int kDPlane = 8 * kGroupBytes;    // the same for the 64 rows of an in
 constexpr int kDCore = kDig * kDPlane;
 constexpr int kDImg = 8 * kDCore;           // 57344 bytes
 constexpr int kNonFinite = 1 << 20;
-constexpr int kThreads = 256;
 constexpr uint32_t kWaits = 1u << 24;
 
 // M64 N: bf16 x bf16 -> fp32, both operands K-major
@@ -90,42 +89,6 @@ __device__ __forceinline__ void issue_products(uint32_t tmem, uint64_t a, uint64
     run(4, 0, 4, 1);
     run(5, 0, 3, 1);
     run(6, 0, 2, 1);
-}
-
-// eight columns of all eight accumulators (64 columns apart), load and wait in one statement
-__device__ __forceinline__ void tmem_ld_acc(uint32_t t, uint32_t (&r)[8][8])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%64];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%65];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%66];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%67];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%32, %33, %34, %35, %36, %37, %38, %39}, [%68];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%40, %41, %42, %43, %44, %45, %46, %47}, [%69];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%48, %49, %50, %51, %52, %53, %54, %55}, [%70];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%56, %57, %58, %59, %60, %61, %62, %63}, [%71];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0][0]), "=r"(r[0][1]), "=r"(r[0][2]), "=r"(r[0][3]), "=r"(r[0][4]), "=r"(r[0][5]), "=r"(r[0][6]),
-          "=r"(r[0][7]), "=r"(r[1][0]), "=r"(r[1][1]), "=r"(r[1][2]), "=r"(r[1][3]), "=r"(r[1][4]), "=r"(r[1][5]),
-          "=r"(r[1][6]), "=r"(r[1][7]), "=r"(r[2][0]), "=r"(r[2][1]), "=r"(r[2][2]), "=r"(r[2][3]), "=r"(r[2][4]),
-          "=r"(r[2][5]), "=r"(r[2][6]), "=r"(r[2][7]), "=r"(r[3][0]), "=r"(r[3][1]), "=r"(r[3][2]), "=r"(r[3][3]),
-          "=r"(r[3][4]), "=r"(r[3][5]), "=r"(r[3][6]), "=r"(r[3][7]), "=r"(r[4][0]), "=r"(r[4][1]), "=r"(r[4][2]),
-          "=r"(r[4][3]), "=r"(r[4][4]), "=r"(r[4][5]), "=r"(r[4][6]), "=r"(r[4][7]), "=r"(r[5][0]), "=r"(r[5][1]),
-          "=r"(r[5][2]), "=r"(r[5][3]), "=r"(r[5][4]), "=r"(r[5][5]), "=r"(r[5][6]), "=r"(r[5][7]), "=r"(r[6][0]),
-          "=r"(r[6][1]), "=r"(r[6][2]), "=r"(r[6][3]), "=r"(r[6][4]), "=r"(r[6][5]), "=r"(r[6][6]), "=r"(r[6][7]),
-          "=r"(r[7][0]), "=r"(r[7][1]), "=r"(r[7][2]), "=r"(r[7][3]), "=r"(r[7][4]), "=r"(r[7][5]), "=r"(r[7][6]),
-          "=r"(r[7][7])
-        : "r"(t), "r"(t + 64), "r"(t + 128), "r"(t + 192), "r"(t + 256), "r"(t + 320), "r"(t + 384), "r"(t + 448)
-        : "memory");
-}
-
-// the eight accumulators of one entry joined: units of 2^(ea + eb - 55), rounded to the nearest
-__device__ __forceinline__ long long join_acc(const uint32_t (&r)[8][8], int q)
-{
-    auto v = [&](int s) { return (long long)__float2int_rn(__uint_as_float(r[s][q])); };
-    const long long hi = v(0) * 16777216 + (v(1) * 65536 + (v(2) * 256 + v(3)));
-    const long long lo = v(4) * 16777216 + (v(5) * 65536 + (v(6) * 256 + (v(7) + 4096)));
-    return (hi << 19) + (lo >> 13);
 }
 
 // u 2^s in FP64 (one rounding; flushed to zero below the normal range)
@@ -632,143 +595,8 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     cluster_barrier();
 }
 
-// Panel of step k, one CTA per row pair: rows x (64 columns) times the inverted diagonal block, the
-// products formed as above, the result rounded row by row to digits without passing through FP64
-// (E's rows also to FP64, which the solve and the gradient read).
-constexpr int kPanelA = 0, kPanelB = kImg, kPanelTail = kImg + kDImg;
-constexpr int kPanelSmem = kPanelTail + 2 * 128 * 4 + TS * 4 + 64;
-
-__global__ void __launch_bounds__(kThreads, 1) digit_panel(int k, Dig g)
-{
-    extern __shared__ __align__(128) unsigned char sm[];
-    int* smax = reinterpret_cast<int*>(sm + kPanelTail);  // [2][128]
-    int* deb = smax + 256;                                // [64]
-    __shared__ uint64_t full, done;
-    __shared__ uint32_t tptr;
-    const int t = threadIdx.x, b = blockIdx.y, m = t & 127, ch = t >> 7, warp = t >> 5;
-    const int q0 = (k + 1) / 2, nq = g.nt / 2 - q0;
-    const bool isext = (int)blockIdx.x >= nq;
-    const int pair = isext ? g.nt / 2 + (int)blockIdx.x - nq : q0 + (int)blockIdx.x;
-    const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
-    const int blk = 2 * pair + half, eb = blk - g.nt;
-    const bool valid = isext ? (g.ext != DIGIT_EXT_IDENTITY || eb <= k) : blk > k;
-    if (warp == 0) tmem_alloc(&tptr, 512);
-    if (t == 0) {
-        mbar_init(&full, 1);
-        mbar_init(&done, 1);
-        fence_mbar_init();
-        mbar_arrive_expect_tx(&full, kDImg);
-        bulk_g2s(smem_u32(sm + kPanelB), g.dimg + (size_t)b * kDImg, kDImg, &full);
-    }
-    if (t < TS) deb[t] = g.dex[(size_t)b * TS + t];
-    double* tile = nullptr;
-    double v[32];
-    int f = 0;
-    if (valid) {
-        tile = isext ? ext_tile(g, b, eb, k)
-                     : g.A + (size_t)b * g.strideA + (size_t)tile_index(blk, k) * TILE_ELEMS;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = tile[r + TS * (32 * ch + c)];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) f = max(f, exp_field(v[c]));
-    } else {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = 0.0;
-    }
-    smax[128 * ch + m] = f;
-    __syncthreads();
-    const int ea = row_exp(max(smax[m], smax[128 + m]));
-#pragma unroll
-    for (int kc = 0; kc < 4; ++kc) {
-        unsigned long long w[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) w[c] = to_digits(to_fixed(v[8 * kc + c], ea));
-        unsigned char* o = sm + kPanelA + (4 * ch + kc) * kCore + m * 16;
-        store_digits(w, [&](int i, uint4 d) { *reinterpret_cast<uint4*>(o + i * kPlane) = d; });
-    }
-    fence_proxy_async();
-    fence_before();
-    __syncthreads();
-    fence_after();
-    const uint32_t tmem = tptr;
-    bool ok = true;
-    if (t == 0) {
-        ok = mbar_wait(&full, 0, kWaits, g.err);
-        const uint64_t ad = smem_desc(smem_u32(sm + kPanelA), kCore, kGroupBytes);
-        const uint64_t bd = smem_desc(smem_u32(sm + kPanelB), kDCore, kGroupBytes);
-        for (int kc = 0; kc < 4; ++kc)
-            issue_products<TS>(tmem, ad + (uint64_t)kc * (2 * kCore >> 4), bd + (uint64_t)kc * (2 * kDCore >> 4),
-                               kPlane, kDPlane, kc == 0);
-        mma_commit(&done);
-    }
-    __syncwarp();
-    ok = mbar_wait(&done, 0, kWaits, g.err) && ok;
-    if (!ok) atomicExch(g.err, 1);
-    fence_after();
-    __syncwarp();
-    // this thread's row, columns 32 ch .. 32 ch + 31, in units of 2^(ea + deb[c] - 55)
-    long long u[32];
-    int top = -(1 << 28);
-#pragma unroll
-    for (int c8 = 0; c8 < 4; ++c8) {
-        uint32_t acc[8][8];
-        tmem_ld_acc(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 32 * ch + 8 * c8, acc);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const long long x = join_acc(acc, c);
-            u[8 * c8 + c] = x;
-            const int e = deb[32 * ch + 8 * c8 + c];
-            if (x != 0 || e == kNonFinite) top = max(top, e + 64 - __clzll(x < 0 ? -x : x));
-        }
-    }
-    fence_before();
-    __syncthreads();  // smax is free again (its readers passed the barrier above the products)
-    if (warp == 0) tmem_dealloc(tmem, 512);
-    smax[128 * ch + m] = top;
-    __syncthreads();
-    top = max(smax[m], smax[128 + m]);
-    const bool nonfinite = ea == kNonFinite || top > kNonFinite / 2;
-    const int e = nonfinite ? kNonFinite : top < -(1 << 27) ? -1022 : top + ea - 55;
-    if (!valid) return;
-    if (ch == 0) g.ex[((size_t)b * dig_pairs(g) + pair) * 128 + 64 * half + r] = e;
-    unsigned char* out = g.img + ((size_t)b * dig_pairs(g) + pair) * kImg + (size_t)m * 16;
-#pragma unroll
-    for (int kc = 0; kc < 4; ++kc) {
-        unsigned long long w[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            // X = u 2^(deb - top + 54): |u| < 2^(top - deb), so |X| < 2^54
-            const int sh = deb[32 * ch + 8 * kc + c] - top + 54;
-            const long long x = u[8 * kc + c];
-            long long y = 0;
-            if (!nonfinite) {
-                if (sh >= 0) y = x << min(sh, 63);
-                else if (sh > -64) y = ((x >> (-sh - 1)) + 1) >> 1;
-            }
-            w[c] = to_digits(y);
-        }
-        unsigned char* o = out + (4 * ch + kc) * kCore;
-        store_digits(w, [&](int i, uint4 d) { *reinterpret_cast<uint4*>(o + i * kPlane) = d; });
-    }
-    if (isext && g.ext == DIGIT_EXT_ROWS) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-            tile[r + TS * (32 * ch + c)] = scaled(u[c], ea + deb[32 * ch + c] - 55);
-    }
-}
-
-// Update of step k: persistent CTAs over (pair, pair) jobs of 128 x 128 outputs, K = 64.  Both images
-// (2 x 112 KB) fill the shared memory.  A job is four passes of 32 columns (8-column groups of one parity
-// of one half of the second pair), whose eight accumulators take 256 tensor-memory columns: two passes
-// are in flight (one 64-column pass after the other with 8 warps took 22 us a job, this 11.5 in a batch of
-// 16).  Warp 16 fetches the images, 16 columns at a time as the last pass of the job before is done
-// with them, and issues the products; warps 0 .. 15 join a pass's accumulators and add them to the FP64
-// matrix while the next pass runs.  Per job and SM the tensor cores need 8.7 k cycles, the FP64 pipe (one
-// addition per output, 64 cycles per warp and partition) 8.2 k, the integer work about 8 k.
-constexpr int kUpB = kImg, kUpSmem = 2 * kImg;
-constexpr int kUpWarps = 16, kUpThreads = (kUpWarps + 1) * 32, kPassCols = 32;
-
-// four columns of all eight accumulators (kPassCols columns apart), load and wait in one statement
+// four columns of all eight accumulators (NC columns apart), load and wait in one statement
+template <int NC>
 __device__ __forceinline__ void tmem_ld_acc4(uint32_t t, uint32_t (&r)[8][4])
 {
     asm volatile(
@@ -786,14 +614,15 @@ __device__ __forceinline__ void tmem_ld_acc4(uint32_t t, uint32_t (&r)[8][4])
           "=r"(r[3][2]), "=r"(r[3][3]), "=r"(r[4][0]), "=r"(r[4][1]), "=r"(r[4][2]), "=r"(r[4][3]), "=r"(r[5][0]),
           "=r"(r[5][1]), "=r"(r[5][2]), "=r"(r[5][3]), "=r"(r[6][0]), "=r"(r[6][1]), "=r"(r[6][2]), "=r"(r[6][3]),
           "=r"(r[7][0]), "=r"(r[7][1]), "=r"(r[7][2]), "=r"(r[7][3])
-        : "r"(t), "r"(t + kPassCols), "r"(t + 2 * kPassCols), "r"(t + 3 * kPassCols), "r"(t + 4 * kPassCols),
-          "r"(t + 5 * kPassCols), "r"(t + 6 * kPassCols), "r"(t + 7 * kPassCols)
+        : "r"(t), "r"(t + NC), "r"(t + 2 * NC), "r"(t + 3 * NC), "r"(t + 4 * NC),
+          "r"(t + 5 * NC), "r"(t + 6 * NC), "r"(t + 7 * NC)
         : "memory");
 }
 
-// The same sum as join_acc with the fewest operations: accumulators 0 .. 4 are at most 2^22 (64 columns of
-// at most 4 products of 2^14 beside the two with a top digit, which is at most 64), so adding 1.5 2^23
-// leaves the number in the low mantissa bits; pairs fit 32 bits.
+// The eight accumulators of one entry joined, in units of 2^(ea + eb - 55), rounded to the nearest.
+// Accumulators 0 .. 4 are at most 2^22 (64 columns of at most 4 products of 2^14, the two with a top digit,
+// which is at most 64, counting half), so adding 1.5 2^23 leaves the number in the low mantissa bits;
+// pairs fit 32 bits.
 __device__ __forceinline__ long long join_acc4(const uint32_t (&r)[8][4], int q)
 {
     constexpr unsigned kMagic = 0x4b400000u;  // 1.5 2^23
@@ -826,6 +655,145 @@ __device__ __forceinline__ double scaled_int(long long u, int s, unsigned flip)
                                  ((nl >> 10) & 1u) + ((unsigned long long)(unsigned)(e << 20) << 32);
     return __hiloint2double((int)((unsigned)(m >> 32) | (((unsigned)sg ^ flip) & 0x80000000u)), (int)(unsigned)m);
 }
+
+// Panel of step k, one CTA per row pair: rows x (64 columns) times the inverted diagonal block, the
+// products formed as above, the result rounded row by row to digits without passing through FP64
+// (E's rows also to FP64, which the solve and the gradient read).  Thread (row m of the pair image,
+// columns 16 cq .. 16 cq + 15).  The chain of loads, row maximum, digits, products, row maximum, digits
+// bounds it; the loops over 8 columns stay rolled and read their input twice (the tile, the
+// accumulators), since the unrolled form spent a third of its 30 us waiting for instructions.
+constexpr int kPanelA = 0, kPanelB = kImg, kPanelTail = kImg + kDImg;
+constexpr int kPanelThreads = 512;
+constexpr int kPanelSmem = kPanelTail + 4 * 128 * 4 + TS * 4;
+
+__global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
+{
+    extern __shared__ __align__(128) unsigned char sm[];
+    int* smax = reinterpret_cast<int*>(sm + kPanelTail);  // [4][128]
+    int* deb = smax + 512;                                // [64]
+    __shared__ uint64_t full, done;
+    __shared__ uint32_t tptr;
+    const int t = threadIdx.x, b = blockIdx.y, m = t & 127, cq = t >> 7, warp = t >> 5;
+    const int q0 = (k + 1) / 2, nq = g.nt / 2 - q0;
+    const bool isext = (int)blockIdx.x >= nq;
+    const int pair = isext ? g.nt / 2 + (int)blockIdx.x - nq : q0 + (int)blockIdx.x;
+    const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
+    const int blk = 2 * pair + half, eb = blk - g.nt;
+    const bool valid = isext ? (g.ext != DIGIT_EXT_IDENTITY || eb <= k) : blk > k;
+    if (warp == 0) tmem_alloc(&tptr, 512);
+    if (t == 0) {
+        mbar_init(&full, 1);
+        mbar_init(&done, 1);
+        fence_mbar_init();
+        mbar_arrive_expect_tx(&full, kDImg);
+        bulk_g2s(smem_u32(sm + kPanelB), g.dimg + (size_t)b * kDImg, kDImg, &full);
+    }
+    if (t < TS) deb[t] = g.dex[(size_t)b * TS + t];
+    double* tile = nullptr;
+    int f = 0;
+    if (valid) {
+        tile = (isext ? ext_tile(g, b, eb, k)
+                      : g.A + (size_t)b * g.strideA + (size_t)tile_index(blk, k) * TILE_ELEMS) +
+               r + TS * 16 * cq;
+        double v[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) v[c] = tile[TS * c];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) f = max(f, exp_field(v[c]));
+    }
+    smax[128 * cq + m] = f;
+    __syncthreads();
+    const int ea = row_exp(max(max(smax[m], smax[128 + m]), max(smax[256 + m], smax[384 + m])));
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        unsigned long long w[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) w[c] = valid ? to_digits(to_fixed(tile[TS * (8 * h + c)], ea)) : 0;
+        unsigned char* o = sm + kPanelA + (2 * cq + h) * kCore + m * 16;
+        store_digits(w, [&](int i, uint4 d) { *reinterpret_cast<uint4*>(o + i * kPlane) = d; });
+    }
+    fence_proxy_async();
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = tptr;
+    bool ok = true;
+    if (t == 0) {
+        ok = mbar_wait(&full, 0, kWaits, g.err);
+        const uint64_t ad = smem_desc(smem_u32(sm + kPanelA), kCore, kGroupBytes);
+        const uint64_t bd = smem_desc(smem_u32(sm + kPanelB), kDCore, kGroupBytes);
+        for (int kc = 0; kc < 4; ++kc)
+            issue_products<TS>(tmem, ad + (uint64_t)kc * (2 * kCore >> 4), bd + (uint64_t)kc * (2 * kDCore >> 4),
+                               kPlane, kDPlane, kc == 0);
+        mma_commit(&done);
+    }
+    __syncwarp();
+    ok = mbar_wait(&done, 0, kWaits, g.err) && ok;
+    if (!ok) atomicExch(g.err, 1);
+    fence_after();
+    __syncwarp();
+    // this thread's entries in units of 2^(ea + deb[c] - 55), and the row's largest
+    const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 16 * cq;
+    int top = -(1 << 28);
+#pragma unroll 1
+    for (int h = 0; h < 4; ++h) {
+        uint32_t acc[8][4];
+        tmem_ld_acc4<TS>(ta + 4 * h, acc);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const long long x = join_acc4(acc, c);
+            const int e = deb[16 * cq + 4 * h + c];
+            if (x != 0 || e == kNonFinite) top = max(top, e + 64 - __clzll(x < 0 ? -x : x));
+        }
+    }
+    smax[128 * cq + m] = top;  // its readers passed the barrier above the products
+    __syncthreads();
+    top = max(max(smax[m], smax[128 + m]), max(smax[256 + m], smax[384 + m]));
+    const bool nonfinite = ea == kNonFinite || top > kNonFinite / 2;
+    const int e = nonfinite ? kNonFinite : top < -(1 << 27) ? -1022 : top + ea - 55;
+    const bool wide = isext && g.ext == DIGIT_EXT_ROWS;
+    if (valid && cq == 0) g.ex[((size_t)b * dig_pairs(g) + pair) * 128 + 64 * half + r] = e;
+    unsigned char* out = g.img + ((size_t)b * dig_pairs(g) + pair) * kImg + (size_t)m * 16;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        unsigned long long w[8];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            uint32_t acc[8][4];
+            tmem_ld_acc4<TS>(ta + 8 * h + 4 * q, acc);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int col = 8 * h + 4 * q + c, de = deb[16 * cq + col];
+                const long long x = join_acc4(acc, c);
+                // X = x 2^(de - top + 54): |x| < 2^(top - de), so |X| < 2^54
+                const int sh = de - top + 54;
+                long long y = 0;
+                if (!nonfinite) {
+                    if (sh >= 0) y = x << min(sh, 63);
+                    else if (sh > -64) y = ((x >> (-sh - 1)) + 1) >> 1;
+                }
+                w[4 * q + c] = to_digits(y);
+                if (wide) tile[TS * col] = scaled_int(x, ea + de - 55, 0);
+            }
+        }
+        unsigned char* o = out + (2 * cq + h) * kCore;
+        if (valid) store_digits(w, [&](int i, uint4 d) { *reinterpret_cast<uint4*>(o + i * kPlane) = d; });
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+// Update of step k: persistent CTAs over (pair, pair) jobs of 128 x 128 outputs, K = 64.  Both images
+// (2 x 112 KB) fill the shared memory.  A job is four passes of 32 columns (8-column groups of one parity
+// of one half of the second pair), whose eight accumulators take 256 tensor-memory columns: two passes
+// are in flight (one 64-column pass after the other with 8 warps took 22 us a job, this 11.5 in a batch of
+// 16).  Warp 16 fetches the images, 16 columns at a time as the last pass of the job before is done
+// with them, and issues the products; warps 0 .. 15 join a pass's accumulators and add them to the FP64
+// matrix while the next pass runs.  Per job and SM the tensor cores need 8.7 k cycles, the FP64 pipe (one
+// addition per output, 64 cycles per warp and partition) 8.2 k, the integer work about 8 k.
+constexpr int kUpB = kImg, kUpSmem = 2 * kImg;
+constexpr int kUpWarps = 16, kUpThreads = (kUpWarps + 1) * 32, kPassCols = 32;
 
 struct UpJob {
     int b, kind, p, q;        // kind 0: A's trailing part, 1: E's rows, 2: V = M^T M; q: columns, p: rows
@@ -971,7 +939,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     uint32_t acc[8][4];
-                    tmem_ld_acc4(ta + 4 * q, acc);
+                    tmem_ld_acc4<kPassCols>(ta + 4 * q, acc);
                     if (q == 1) {
                         fence_before();
                         __syncwarp();
@@ -1047,7 +1015,7 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
         const int nq = nt / 2 - (k + 1) / 2;
         const int npe = ext == DIGIT_EXT_IDENTITY ? k / 2 + 1 : ne / 2;
         if (nq + npe == 0) { count_launch(ctx, 1); continue; }
-        digit_panel<<<dim3(nq + npe, B), kThreads, kPanelSmem, s>>>(k, g);
+        digit_panel<<<dim3(nq + npe, B), kPanelThreads, kPanelSmem, s>>>(k, g);
         const int per = nq * (nq + 1) / 2 + npe * nq + (ext == DIGIT_EXT_IDENTITY ? npe * (npe + 1) / 2 : 0);
         count_launch(ctx, per > 0 ? 3 : 2);
         if (per > 0)
