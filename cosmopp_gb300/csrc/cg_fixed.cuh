@@ -1,0 +1,76 @@
+// FP64 numbers to and from 64-bit fixed point, and fixed-point products, for the integer pipes: the
+// FP64 pipe of sm_103a takes a warp instruction every 64 cycles and SM partition.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace cg {
+
+// exponent of a row with an infinity or a NaN: what it enters becomes NaN
+constexpr int kNonFinite = 1 << 20;
+
+// u 2^s in FP64 (one rounding; flushed to zero below the normal range)
+__device__ __forceinline__ double scaled(long long u, int s)
+{
+    const double x = __ll2double_rn(u);
+    const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) + s;
+    if (s > kNonFinite / 2) return __longlong_as_double(0x7ff8000000000000ll);
+    if (u == 0 || e <= 0) return 0.0;
+    if (e >= 0x7ff) return __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
+    return __hiloint2double(hi + (s << 20), __double2loint(x));
+}
+
+__device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+// the row's exponent from the largest exponent field of its entries: |v| < 2^e
+__device__ __forceinline__ int row_exp(int field) { return field == 0x7ff ? kNonFinite : field - 1022; }
+
+// v as 2^(e - FB) X, |v| < 2^e, X rounded to the nearest; FB <= 62
+template <int FB = 54>
+__device__ __forceinline__ long long to_fixed(double v, int e)
+{
+    const long long bits = __double_as_longlong(v);
+    const int f = (int)((unsigned long long)bits >> 52) & 0x7ff;
+    const unsigned long long m = ((unsigned long long)bits & 0xfffffffffffffull) | 0x10000000000000ull;
+    int r = e - (f - 1022);
+    if (f == 0 || r > FB + 1) return 0;
+    if (r < 0) r = 0;  // only with a non-finite entry, whose row is marked
+    const long long x = (long long)(((m << (FB - 52) >> r) + 1) >> 1);
+    return bits < 0 ? -x : x;
+}
+
+// u 2^s in FP64, rounded to the nearest, its sign flipped by `flip` (0 or 0x80000000): __ll2double_rn is one
+// FP64-pipe instruction more per number, and that pipe is the scarcest
+__device__ __forceinline__ double scaled_int(long long u, int s, unsigned flip)
+{
+    const int hi = (int)(u >> 32), sg = hi >> 31;
+    const unsigned long long a = (unsigned long long)((u ^ sg) - sg);
+    const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
+    const int lz = __clz((int)ah);
+    const int e = 1085 - lz + s;  // exponent field less one
+    if (ah == 0 || (unsigned)(e - 1) > 2040u) {
+        const double x = scaled(u, s);
+        return __hiloint2double(__double2hiint(x) ^ (int)flip, __double2loint(x));
+    }
+    const unsigned nh = __funnelshift_l(al, ah, lz), nl = al << lz;
+    const unsigned long long m = (((unsigned long long)(nh >> 11) << 32) | __funnelshift_r(nl, nh, 11)) +
+                                 ((nl >> 10) & 1u) + ((unsigned long long)(unsigned)(e << 20) << 32);
+    return __hiloint2double((int)((unsigned)(m >> 32) | (((unsigned)sg ^ flip) & 0x80000000u)), (int)(unsigned)m);
+}
+
+// ---- products of numbers with 61 fraction bits ----------------------------------------------
+
+// v = h 2^31 + l, 0 <= l < 2^31
+struct Split61 {
+    int h, l;
+};
+__device__ __forceinline__ Split61 split61(long long v) { return {(int)(v >> 31), (int)v & 0x7fffffff}; }
+
+// a b 2^-61 to about one unit: three 32 x 32 -> 64 multiply-adds.  l l' is left out; 2^30, its mean and
+// half a unit, stands for it
+__device__ __forceinline__ long long mul61(Split61 a, Split61 b)
+{
+    const long long c = (long long)a.l * b.h + ((long long)a.h * b.l + (1ll << 30));
+    return 2 * ((long long)a.h * b.h) + (c >> 30);
+}
+
+}  // namespace cg

@@ -31,6 +31,7 @@
 // A row with an infinity or a NaN gets the exponent kNonFinite, which makes everything it enters NaN.
 #include <algorithm>
 
+#include "cg_fixed.cuh"
 #include "cg_internal.h"
 #include "cg_tc.cuh"
 
@@ -48,7 +49,6 @@ constexpr int kImg = 8 * kCore;             // a pair image: 114688 bytes
 constexpr int kDPlane = 8 * kGroupBytes;    // the same for the 64 rows of an inverted diagonal block
 constexpr int kDCore = kDig * kDPlane;
 constexpr int kDImg = 8 * kDCore;           // 57344 bytes
-constexpr int kNonFinite = 1 << 20;
 constexpr uint32_t kWaits = 1u << 24;
 
 // M64 N: bf16 x bf16 -> fp32, both operands K-major
@@ -89,34 +89,6 @@ __device__ __forceinline__ void issue_products(uint32_t tmem, uint64_t a, uint64
     run(4, 0, 4, 1);
     run(5, 0, 3, 1);
     run(6, 0, 2, 1);
-}
-
-// u 2^s in FP64 (one rounding; flushed to zero below the normal range)
-__device__ __forceinline__ double scaled(long long u, int s)
-{
-    const double x = __ll2double_rn(u);
-    const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) + s;
-    if (s > kNonFinite / 2) return __longlong_as_double(0x7ff8000000000000ll);
-    if (u == 0 || e <= 0) return 0.0;
-    if (e >= 0x7ff) return __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
-    return __hiloint2double(hi + (s << 20), __double2loint(x));
-}
-
-__device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
-// the row's exponent from the largest exponent field of its entries: |v| < 2^e
-__device__ __forceinline__ int row_exp(int field) { return field == 0x7ff ? kNonFinite : field - 1022; }
-
-// v as 2^(e-54) X, |v| < 2^e, X rounded to the nearest
-__device__ __forceinline__ long long to_fixed(double v, int e)
-{
-    const long long bits = __double_as_longlong(v);
-    const int f = (int)((unsigned long long)bits >> 52) & 0x7ff;
-    unsigned long long m = ((unsigned long long)bits & 0xfffffffffffffull) | 0x10000000000000ull;
-    int r = e - (f - 1075) - 53;
-    if (f == 0 || r > 56) return 0;
-    if (r < 0) r = 0;  // only with a non-finite entry, whose row is marked
-    const long long x = (long long)(((m << 2 >> r) + 1) >> 1);
-    return bits < 0 ? -x : x;
 }
 
 // X as two's complement digits, byte p the digit of weight 256^p (bytes 0 .. 5 balanced, byte 6 the top)
@@ -635,25 +607,6 @@ __device__ __forceinline__ long long join_acc4(const uint32_t (&r)[8][4], int q)
     long long x = (long long)v45 * 8 + (v67 >> 13);
     x = (long long)v23 * 524288 + x;
     return x + ((long long)v01 << 35);
-}
-
-// u 2^s in FP64, rounded to the nearest, its sign flipped by `flip` (0 or 0x80000000): __ll2double_rn is one
-// FP64-pipe instruction more per number, and that pipe is the scarcest
-__device__ __forceinline__ double scaled_int(long long u, int s, unsigned flip)
-{
-    const int hi = (int)(u >> 32), sg = hi >> 31;
-    const unsigned long long a = (unsigned long long)((u ^ sg) - sg);
-    const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
-    const int lz = __clz((int)ah);
-    const int e = 1085 - lz + s;  // exponent field less one
-    if (ah == 0 || (unsigned)(e - 1) > 2040u) {
-        const double x = scaled(u, s);
-        return __hiloint2double(__double2hiint(x) ^ (int)flip, __double2loint(x));
-    }
-    const unsigned nh = __funnelshift_l(al, ah, lz), nl = al << lz;
-    const unsigned long long m = (((unsigned long long)(nh >> 11) << 32) | __funnelshift_r(nl, nh, 11)) +
-                                 ((nl >> 10) & 1u) + ((unsigned long long)(unsigned)(e << 20) << 32);
-    return __hiloint2double((int)((unsigned)(m >> 32) | (((unsigned)sg ^ flip) & 0x80000000u)), (int)(unsigned)m);
 }
 
 // Panel of step k, one CTA per row pair: rows x (64 columns) times the inverted diagonal block, the

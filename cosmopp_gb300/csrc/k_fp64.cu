@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "cg_fixed.cuh"
 #include "cg_internal.h"
 
 namespace cg {
@@ -122,17 +123,18 @@ __global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, 
 
 // ---- covariance for the likelihood, in 64-bit fixed point ----------------------------------
 //
-// The FP64 pipe gives 2 operations per cycle and SM, the integer pipes about 50 times that, and every
-// quantity of the Legendre sum is bounded: |P_l| <= 1, |x| <= 1, and the weights w_l = C_l (2l+1)/(4 pi)
-// B_l^2 are scaled by a power of two above sum |w_l|.  So the sum runs in integers, P_l = p 2^-60:
+// The FP64 pipe gives 2 operations per cycle and SM, the 32 x 32 -> 64 multiply-add 64, and every quantity of
+// the Legendre sum is bounded: |P_l| <= 1, |x| <= 1, and the weights w_l = C_l (2l+1)/(4 pi) B_l^2 are
+// scaled by a power of two above sum |w_l|.  So the sum runs in integers, P_l = p 2^-60, x, w_l and 1 / l
+// with 61 fraction bits:
 //     t = x P_{l-1},  P_l = 2 t - P_{l-2} - (t - P_{l-2}) / l,  S += w_l P_l,
-// one 64 x 64 -> high 64 product each.  Each step rounds at 2^-60 where FP64 rounds at 2^-53: the sum
-// is 10 to 50 times nearer to the exact value than the FP64 recurrence's (lmax 12 to 255), and is then
-// rounded to FP64 once.  The P_l are shared by NB batch elements.
+// three multiply-adds a product.  x itself is the dot product of the directions in fixed point, and the
+// sum becomes FP64 in integer operations.  Each step rounds at 2^-60 where FP64 rounds at 2^-53: the sum
+// is 10 to 30 times nearer to the exact value than the FP64 recurrence's (lmax 12 to 255).  The P_l are
+// shared by NB batch elements.
 
-// status and fixed-point weights of every element: wfix[b][l] = w_l 2^(62 - e), wexp[b] = e with
-// sum |w_l| < 2^e; a non-finite weight gives e = kBadWeights and a NaN covariance.  grid B
-constexpr int kBadWeights = 1 << 20;
+// status and fixed-point weights of every element: wfix[b][l] = w_l 2^(61 - e), wexp[b] = e with
+// sum |w_l| < 2^e; a non-finite weight gives e = kNonFinite and a NaN covariance.  grid B
 __global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const double* __restrict__ beam,
                                                              const double* __restrict__ cl,
                                                              long long* __restrict__ wfix, int* __restrict__ wexp,
@@ -151,8 +153,8 @@ __global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const dou
     const int bad = __syncthreads_or(!isfinite(c));
     s = 0.0;
     for (int k = 0; k < kThreads / 32; ++k) s += part[k];
-    const int e = isfinite(s) ? (s > 0.0 ? ilogb(s) + 1 : -1000) : kBadWeights;
-    if (l <= lmax) wfix[(size_t)b * L1 + l] = e == kBadWeights ? 0 : __double2ll_rn(scalbn(w, 62 - e));
+    const int e = isfinite(s) ? (s > 0.0 ? ilogb(s) + 1 : -1000) : kNonFinite;
+    if (l <= lmax) wfix[(size_t)b * L1 + l] = e == kNonFinite ? 0 : __double2ll_rn(scalbn(w, 61 - e));
     if (l == 0) {
         wexp[b] = e;
         status[b] = bad ? CG_ERR_NONFINITE : CG_OK;
@@ -160,7 +162,8 @@ __global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const dou
 }
 
 // C (+ noise on the diagonal, identity padding) into the tiled layout; grid (tiles, ceil(B / NB)),
-// 4 pairs per thread and pass
+// 4 pairs per thread and pass.  Directions with a component beyond 1 (a caller's, off the unit
+// sphere) take their dot product in FP64, with the reference's clamp.
 template <int NB>
 __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax, int B,
                                                           const double* __restrict__ xyz,
@@ -169,44 +172,61 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
                                                           const int* __restrict__ wexp, double* __restrict__ A,
                                                           size_t strideA)
 {
-    extern __shared__ long long sfix[];
+    extern __shared__ Split61 sfix[];
+    __shared__ Split61 dir[2][3][TS];
     const int L1 = lmax + 1, b0 = blockIdx.y * NB;
-    long long* sr = sfix;        // 2^63 / l
-    long long* sw = sfix + L1;   // [l][NB]
-    for (int l = threadIdx.x; l <= lmax; l += kThreads) {
-        sr[l] = l >= 2 ? (long long)((0x8000000000000000ull + l / 2) / (unsigned)l) : 0;
-#pragma unroll
-        for (int q = 0; q < NB; ++q) sw[l * NB + q] = b0 + q < B ? wfix[(size_t)(b0 + q) * L1 + l] : 0;
-    }
-    __syncthreads();
+    Split61* sr = sfix;        // 1 / l
+    Split61* sw = sfix + L1;   // [l][NB]
     int I, J;
     tile_coords(blockIdx.x, I, J);
+    for (int l = threadIdx.x; l <= lmax; l += kThreads) {
+        sr[l] = split61(l >= 2 ? (long long)(((1ull << 61) + l / 2) / (unsigned)l) : 0);
+#pragma unroll
+        for (int q = 0; q < NB; ++q) sw[l * NB + q] = split61(b0 + q < B ? wfix[(size_t)(b0 + q) * L1 + l] : 0);
+    }
+    bool beyond = false;
+    for (int e = threadIdx.x; e < 6 * TS; e += kThreads) {
+        const int s = e / (3 * TS), c = e / TS % 3, i = e % TS;
+        const double v = xyz[(size_t)c * N + (s ? J : I) * TS + i];
+        beyond |= !(fabs(v) <= 1.0);
+        dir[s][c][i] = split61(to_fixed<62>(v, 1));
+    }
+    beyond = __syncthreads_or(beyond);
     for (int g = 0; g < TILE_ELEMS / (kThreads * 4); ++g) {
-        long long x[4], p0[4], p1[4], acc[NB][4];
+        Split61 x[4];
+        long long p0[4], p1[4], acc[NB][4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int e = threadIdx.x + kThreads * (4 * g + q), i = I * TS + e % TS, j = J * TS + e / TS;
-            const double v = (i < n && j < n) ? pair_dot(xyz, N, i, j) : 0.0;
-            x[q] = __double2ll_rn(v * 4611686018427387904.0);  // 2^62
+            const int e = threadIdx.x + kThreads * (4 * g + q), i = e % TS, j = e / TS;
+            long long v = 0;
+            if (!beyond) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) v += mul61(dir[0][c][i], dir[1][c][j]);
+                v = min(max(v, -(1ll << 61)), 1ll << 61);
+            } else if (I * TS + i < n && J * TS + j < n) {
+                v = to_fixed<62>(pair_dot(xyz, N, I * TS + i, J * TS + j), 1);
+            }
+            x[q] = split61(v);
             p0[q] = 1ll << 60;
-            p1[q] = x[q] >> 2;
+            p1[q] = v >> 1;
 #pragma unroll
             for (int k = 0; k < NB; ++k) acc[k][q] = 0;
         }
 #pragma unroll 2
         for (int l = 2; l <= lmax; ++l) {
-            const long long rl = sr[l];
-            long long w[NB];
+            const Split61 rl = sr[l];
+            Split61 w[NB];
 #pragma unroll
             for (int k = 0; k < NB; ++k) w[k] = sw[l * NB + k];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const long long t = __mul64hi(x[q], p1[q] << 2), d = t - p0[q];
-                const long long p = t + d - __mul64hi(d << 1, rl);
+                const long long t = mul61(split61(p1[q]), x[q]), d = t - p0[q];
+                const long long p = t + d - mul61(split61(d), rl);
                 p0[q] = p1[q];
                 p1[q] = p;
+                const Split61 ps = split61(p);
 #pragma unroll
-                for (int k = 0; k < NB; ++k) acc[k][q] += __mul64hi(p << 2, w[k]);
+                for (int k = 0; k < NB; ++k) acc[k][q] += mul61(ps, w[k]);
             }
         }
 #pragma unroll
@@ -219,8 +239,8 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
                 const int e = threadIdx.x + kThreads * (4 * g + q), i = I * TS + e % TS, j = J * TS + e / TS;
                 double val;
                 if (i < n && j < n) {
-                    val = we == kBadWeights ? __longlong_as_double(0x7ff8000000000000ll)
-                                            : scalbn(__ll2double_rn(acc[k][q]), we - 60);
+                    // a non-finite weight's exponent gives NaN
+                    val = scaled_int(acc[k][q], we - 60, 0);
                     // cInv_(i,j) = c + fiducial(0) + noise  (source/likelihood.cpp:102-110)
                     if (i == j) val = __dadd_rn(val, noise[i]);
                 } else {
@@ -1053,10 +1073,10 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
     // one element per thread block below four: twice the blocks of the shared form, and a single
     // element has nothing to share
     if (B >= 4)
-        build_c_tiled<4><<<dim3(ntile, (B + 3) / 4), kThreads, sizeof(long long) * 5 * (lmax + 1), s>>>(
+        build_c_tiled<4><<<dim3(ntile, (B + 3) / 4), kThreads, sizeof(Split61) * 5 * (lmax + 1), s>>>(
             n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
     else
-        build_c_tiled<1><<<dim3(ntile, B), kThreads, sizeof(long long) * 2 * (lmax + 1), s>>>(
+        build_c_tiled<1><<<dim3(ntile, B), kThreads, sizeof(Split61) * 2 * (lmax + 1), s>>>(
             n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
     count_launch(ctx, 2);
     const int drow = grad ? nharm_of(lmax) : 0;
