@@ -90,6 +90,7 @@ extern "C" void cg_destroy(cg_ctx* ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (cg_ctx::Graph& gr : ctx->graphs)
         if (gr.exec) cudaGraphExecDestroy(gr.exec);
+    cg::digit_free(ctx);
     cg::fp64_free(ctx);
     cg::mixed_free(ctx);
     cudaFree(ctx->d_xyz); cudaFree(ctx->d_noise); cudaFree(ctx->d_lega); cudaFree(ctx->d_legb);
@@ -684,6 +685,7 @@ extern "C" void cg_likelihood_destroy(cg_lik* lik)
     if (!lik) return;
     cudaSetDevice(lik->ctx.device);
     if (lik->ctx.stream) cudaStreamSynchronize(lik->ctx.stream);
+    cg::digit_free(&lik->ctx);
     cudaFree(lik->A); cudaFree(lik->diag); cudaFree(lik->tmp); cudaFree(lik->st);
     cudaFree(lik->Ninv);
     if (lik->ctx.stream) cudaStreamDestroy(lik->ctx.stream);

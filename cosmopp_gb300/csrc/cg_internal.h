@@ -162,6 +162,9 @@ struct cg_ctx {
     // priority, and the events that fork it from the caller's stream, hand each column to trtri and join
     cudaStream_t hi = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_col = nullptr, ev_join = nullptr;
+    // the FP64 factorisation's second stream (k_digit.cu) and the events between the two
+    cudaStream_t aux = nullptr;
+    cudaEvent_t ev_chain[2] = {nullptr, nullptr};
     std::vector<double> xyz;     // [n][3]
     std::vector<double> noise;   // [n]
     cg::LegConsts leg;
@@ -261,6 +264,7 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
 // work: digit_bytes(nt, ne) per matrix, 16-byte aligned; *err is set if a bounded wait gives up.
 enum DigitExt { DIGIT_EXT_ROWS = 0, DIGIT_EXT_IDENTITY = 1 };
 size_t digit_bytes(int nt, int ne);
+void digit_free(cg_ctx* ctx);  // the context's second stream and its events
 int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t strideA, double* E,
                  size_t strideE, double* diag, int* status, unsigned char* work, int* err, cudaStream_t s);
 // generic tiled FP64 / FP32 factorisation entry points (k_chol.cu)

@@ -30,6 +30,7 @@
 //
 // A row with an infinity or a NaN gets the exponent kNonFinite, which makes everything it enters NaN.
 #include <algorithm>
+#include <cmath>
 
 #include "cg_fixed.cuh"
 #include "cg_internal.h"
@@ -121,6 +122,12 @@ __device__ __forceinline__ void store_digits(const unsigned long long (&w)[8], S
                             digit_pair(w[6], w[7], p)));
     }
 }
+
+// Programmatic dependent launch: the next kernel of the stream may take its place as soon as SMs are free
+// and does its set-up there; what it reads and writes comes after the wait for this one.  A kernel boundary
+// took 4 us without it.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 struct Dig {
     int nt, ne, ext;          // block rows of A and of E (both even); ext: DigitExt
@@ -486,6 +493,8 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     if (t < 8) mbar_init(&sh.full[t], 1);
     if (t == 0) sh.bad = 0;
     fence_mbar_init();
+    launch_dependents();
+    wait_prior();
     if (t < TS) sh.e[t] = (exp_field(tile[t * (TS + 1)]) - 1022 + 1) >> 1;  // S_rr < 2^(2 e)
     cluster_barrier();
     if (rank == 0) {
@@ -633,11 +642,16 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
     const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
     const int blk = 2 * pair + half, eb = blk - g.nt;
     const bool valid = isext ? (g.ext != DIGIT_EXT_IDENTITY || eb <= k) : blk > k;
+    launch_dependents();
     if (warp == 0) tmem_alloc(&tptr, 512);
     if (t == 0) {
         mbar_init(&full, 1);
         mbar_init(&done, 1);
         fence_mbar_init();
+    }
+    __syncwarp();
+    wait_prior();
+    if (t == 0) {
         mbar_arrive_expect_tx(&full, kDImg);
         bulk_g2s(smem_u32(sm + kPanelB), g.dimg + (size_t)b * kDImg, kDImg, &full);
     }
@@ -753,32 +767,52 @@ struct UpJob {
     int pa, pb;               // images
 };
 
-__device__ __forceinline__ UpJob up_job(const Dig& g, int k, int per, int npe, int job)
+// The jobs of a launch: column pairs [q0, q0 + ncol) of the trailing part (ncol = 1 or all that are left), E's
+// rows over the same columns, and with v the pairs of V
+struct UpRange {
+    int q0, ncol, npe, v;
+};
+__host__ __device__ inline int up_tri(const UpRange& u, int nq)
+{
+    const int m = nq - u.q0;
+    return u.ncol == 1 ? m : m * (m + 1) / 2;
+}
+__host__ __device__ inline int up_jobs(const UpRange& u, int nq)
+{
+    return (u.ncol > 0 ? up_tri(u, nq) + u.npe * u.ncol : 0) + (u.v ? u.npe * (u.npe + 1) / 2 : 0);
+}
+
+__device__ __forceinline__ UpJob up_job(const Dig& g, const UpRange& u, int per, int job)
 {
     UpJob j;
     j.b = job / per;
     int l = job % per;
-    const int nq = g.nt / 2, q0 = (k + 1) / 2, m = nq - q0, tri = m * (m + 1) / 2;
+    const int nq = g.nt / 2, tri = u.ncol > 0 ? up_tri(u, nq) : 0;
     if (l < tri) {
-        int I, J;
-        tile_coords(tri - 1 - l, I, J);  // columns in order, the next diagonal block's first
+        if (u.ncol == 1) {
+            j.q = u.q0;
+            j.p = u.q0 + l;
+        } else {
+            int I, J;
+            tile_coords(tri - 1 - l, I, J);
+            j.q = nq - 1 - I;
+            j.p = nq - 1 - J;
+        }
         j.kind = 0;
-        j.q = nq - 1 - I;
-        j.p = nq - 1 - J;
         j.pa = j.p;
         j.pb = j.q;
         return j;
     }
     l -= tri;
-    if (l < npe * m) {
+    if (l < u.npe * u.ncol) {
         j.kind = 1;
-        j.q = q0 + l / npe;
-        j.p = l % npe;
+        j.q = u.q0 + l / u.npe;
+        j.p = l % u.npe;
         j.pa = nq + j.p;
         j.pb = j.q;
         return j;
     }
-    l -= npe * m;
+    l -= u.npe * u.ncol;
     tile_coords(l, j.p, j.q);
     j.kind = 2;
     j.pa = nq + j.p;
@@ -793,13 +827,14 @@ __device__ __forceinline__ void up_halves(const UpJob& j, int k, int& h0, int& h
     h1 = (j.kind == 2 && 2 * j.q + 1 > k) ? 1 : 2;
 }
 
-__global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, int per, int npe, Dig g)
+__global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, int per, UpRange u, Dig g)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ uint64_t full[4], empty[4], tfull[2], tempty[2];
     __shared__ uint32_t tptr;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int pairs = dig_pairs(g);
+    launch_dependents();
     if (warp == 0) tmem_alloc(&tptr, 512);
     if (t == 0) {
         for (int i = 0; i < 4; ++i) {
@@ -816,12 +851,13 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
     __syncthreads();
     fence_after();
     const uint32_t tmem = tptr;
+    wait_prior();
     bool ok = true;
     uint32_t pass = 0, round = 0;
     if (warp == kUpWarps) {
         if (lane == 0)
             for (int job = blockIdx.x; job < njobs; job += gridDim.x, ++round) {
-                const UpJob j = up_job(g, k, per, npe, job);
+                const UpJob j = up_job(g, u, per, job);
                 const unsigned char* a = g.img + ((size_t)j.b * pairs + j.pa) * kImg;
                 const unsigned char* bb = g.img + ((size_t)j.b * pairs + j.pb) * kImg;
                 for (int kc = 0; kc < 4; ++kc) {
@@ -855,7 +891,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
         const int m = 32 * (warp & 3) + lane, c4 = warp >> 2;  // row of the pair image, 8-column group of the pass
         const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
         for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
-            const UpJob j = up_job(g, k, per, npe, job);
+            const UpJob j = up_job(g, u, per, job);
             const int ea = g.ex[((size_t)j.b * pairs + j.pa) * 128 + 64 * half + r];
             const int* eb = g.ex + ((size_t)j.b * pairs + j.pb) * 128;
             double* Ab = g.A + (size_t)j.b * g.strideA;
@@ -917,36 +953,108 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
 
 }  // namespace
 
-// Seven CTAs for the inverse keep up with the factor (44 us), three take a little longer (47 us); sixteen
-// clusters of eight do not fit the SMs at once (two waves, 87 us), so half the SMs are the limit.
-static int launch_diag(cg_ctx* ctx, int B, int k, const Dig& g, double* diag, int* status, cudaStream_t s)
+// a launch that may start beside the end of the kernel before it (launch_dependents, wait_prior), in clusters
+// of `cluster` CTAs
+template <typename... P, typename... A>
+static int launch(cg_ctx* ctx, void (*kernel)(P...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t s,
+                  A... args)
 {
-    const int ctas = 16 * B <= ctx->sm_count ? 8 : 4;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = ctas;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas * B);
-    cfg.blockDim = dim3(kDiagThreads);
-    cfg.dynamicSmemBytes = sizeof(DiagShared);
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CG_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, digit_diag, k, ctas, g, diag, status));
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    count_launch(ctx);
+    CG_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kernel, P(args)...));
     return CG_OK;
+}
+
+// Seven CTAs for the inverse keep up with the factor (44 us), three take a little longer (47 us); sixteen
+// clusters of eight do not fit the SMs at once (two waves, 87 us), so half the SMs are the limit.  Beside an
+// update a cluster of eight may wait 30 us for eight free SMs next to each other; four are found at once.
+static int launch_diag(cg_ctx* ctx, int B, int k, bool beside, const Dig& g, double* diag, int* status, cudaStream_t s)
+{
+    const int ctas = !beside && 16 * B <= ctx->sm_count ? 8 : 4;
+    return launch(ctx, digit_diag, dim3(ctas * B), kDiagThreads, sizeof(DiagShared), ctas, s, k, ctas, g, diag, status);
 }
 
 size_t digit_bytes(int nt, int ne)
 {
     const size_t pairs = (size_t)(nt + ne) / 2;
-    return pairs * kImg + pairs * 128 * sizeof(int) + kDImg + TS * sizeof(int);
+    return 2 * pairs * (kImg + 128 * sizeof(int)) + kDImg + TS * sizeof(int);
+}
+
+static int launch_update(cg_ctx* ctx, int B, int k, const UpRange& u, const Dig& g, int ctas, cudaStream_t s)
+{
+    const int per = up_jobs(u, g.nt / 2);
+    if (per <= 0) return CG_OK;
+    return launch(ctx, digit_update, dim3((unsigned)std::min<long long>((long long)per * B, ctas)), kUpThreads, kUpSmem, 1, s,
+                  k, per * B, per, u, g);
+}
+
+// The factorisation's chain (diagonal block, panel, the update of the next column pair) beside the rest of
+// the update of the step before, on a second stream and on all but `reserve` SMs: the reserve that makes the
+// longer of the two shortest, or 0 where one after the other is as fast.  Per SM a job takes about 11 us and a
+// panel's CTA 12, a diagonal step 45; a saving below 7 % is left (large batches and matrices, whose updates
+// fill the chip).  One factorisation at nside 16 with its harmonics: 3.94 ms one after the other, 3.16 beside.
+static int chain_reserve(const cg_ctx* ctx, int B, int nq, int npe, int v)
+{
+    const UpRange all = {0, nq, npe, v}, one = {0, 1, npe, 0};
+    const double sms = ctx->sm_count, col = (double)up_jobs(one, nq) * B, jobs = (double)up_jobs(all, nq) * B;
+    auto waves = [](double n, double s) { return std::max(1.0, std::ceil(n / s)); };
+    const double serial = 45 + 12 * waves(col, sms) + 11 * waves(jobs, sms) + 6;
+    double best = 0.93 * serial;
+    int reserve = 0;
+    for (int r = 8; r <= ctx->sm_count / 2; r += 8) {
+        const double chain = 45 * waves(4.0 * B, r) + 23 * waves(col, r) + 8;
+        const double t = std::max(chain, 11 * waves(jobs - col, sms - r) + 4);
+        if (t < best) {
+            best = t;
+            reserve = r;
+        }
+    }
+    return reserve;
+}
+
+static bool chain_streams(cg_ctx* ctx)
+{
+    if (!ctx->aux && cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking) != cudaSuccess) ctx->aux = nullptr;
+    bool ok = ctx->aux != nullptr;
+    for (cudaEvent_t& e : ctx->ev_chain)
+        if (ok && !e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            e = nullptr;
+            ok = false;
+        }
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
+void digit_free(cg_ctx* ctx)
+{
+    if (ctx->aux) {
+        cudaStreamSynchronize(ctx->aux);
+        cudaStreamDestroy(ctx->aux);
+        ctx->aux = nullptr;
+    }
+    for (cudaEvent_t& e : ctx->ev_chain) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
 }
 
 int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t strideA, double* E,
                  size_t strideE, double* diag, int* status, unsigned char* work, int* err, cudaStream_t s)
 {
     const size_t pairs = (size_t)(nt + ne) / 2;
+    const int nq = nt / 2, v = ext == DIGIT_EXT_IDENTITY ? 1 : 0;
     Dig g;
     g.nt = nt;
     g.ne = ne;
@@ -955,26 +1063,48 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
     g.E = E;
     g.strideA = strideA;
     g.strideE = strideE;
-    g.img = work;
-    g.dimg = g.img + (size_t)B * pairs * kImg;
-    g.ex = reinterpret_cast<int*>(g.dimg + (size_t)B * kDImg);
-    g.dex = g.ex + (size_t)B * pairs * 128;
+    // two sets of images, for the steps in turn where the update of one runs beside the panel of the next
+    unsigned char* const img[2] = {work, work + (size_t)B * pairs * kImg};
+    g.dimg = img[1] + (size_t)B * pairs * kImg;
+    int* const ex[2] = {reinterpret_cast<int*>(g.dimg + (size_t)B * kDImg),
+                        reinterpret_cast<int*>(g.dimg + (size_t)B * kDImg) + (size_t)B * pairs * 128};
+    g.dex = ex[1] + (size_t)B * pairs * 128;
     g.err = err;
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DiagShared)));
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem));
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem));
+    bool rest = false;  // an update on the second stream that the caller's stream has not waited for
     for (int k = 0; k < nt; ++k) {
-        if (int rc = launch_diag(ctx, B, k, g, diag, status, s)) return rc;
-        const int nq = nt / 2 - (k + 1) / 2;
-        const int npe = ext == DIGIT_EXT_IDENTITY ? k / 2 + 1 : ne / 2;
-        if (nq + npe == 0) { count_launch(ctx, 1); continue; }
-        digit_panel<<<dim3(nq + npe, B), kPanelThreads, kPanelSmem, s>>>(k, g);
-        const int per = nq * (nq + 1) / 2 + npe * nq + (ext == DIGIT_EXT_IDENTITY ? npe * (npe + 1) / 2 : 0);
-        count_launch(ctx, per > 0 ? 3 : 2);
-        if (per > 0)
-            digit_update<<<(unsigned)std::min<long long>((long long)per * B, ctx->sm_count), kUpThreads, kUpSmem, s>>>(
-                k, per * B, per, npe, g);
+        const int q0 = (k + 1) / 2, m = nq - q0, npe = v ? k / 2 + 1 : ne / 2;
+        g.img = img[0];
+        g.ex = ex[0];
+        if (int rc = launch_diag(ctx, B, k, rest, g, diag, status, s)) return rc;
+        if (m + npe == 0) continue;
+        const int reserve = m > 1 ? chain_reserve(ctx, B, m, npe, v) : 0;
+        const bool beside = reserve > 0 && chain_streams(ctx);
+        if (rest && !beside) {
+            CG_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain[1], 0));
+            rest = false;
+        }
+        if (beside || rest) {
+            g.img = img[k & 1];
+            g.ex = ex[k & 1];
+        }
+        if (int rc = launch(ctx, digit_panel, dim3(m + npe, B), kPanelThreads, kPanelSmem, 1, s, k, g)) return rc;
+        if (!beside) {
+            if (int rc = launch_update(ctx, B, k, {q0, m, npe, v}, g, ctx->sm_count, s)) return rc;
+            continue;
+        }
+        CG_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_chain[0], s));
+        CG_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->aux, ctx->ev_chain[0], 0));
+        // the next column pair needs the rest of the step before
+        if (rest) CG_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain[1], 0));
+        if (int rc = launch_update(ctx, B, k, {q0, 1, npe, 0}, g, ctx->sm_count, s)) return rc;
+        if (int rc = launch_update(ctx, B, k, {q0 + 1, m - 1, npe, v}, g, ctx->sm_count - reserve, ctx->aux)) return rc;
+        CG_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_chain[1], ctx->aux));
+        rest = true;
     }
+    if (rest) CG_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain[1], 0));
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;
 }
