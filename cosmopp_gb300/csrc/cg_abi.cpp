@@ -672,7 +672,7 @@ struct cg_lik {
     cg_ctx ctx;                  // device, sizes, stream and error text
     double* A = nullptr;         // tiled C + F + N, then C^-1
     double* diag = nullptr;
-    double* tmp = nullptr;       // [4][N] vectors + scalars
+    double* tmp = nullptr;       // [4][N] vectors, 8 scalars, 3 sums per tile
     int* st = nullptr;
     double logdet = 0;
     std::vector<double> fg;
@@ -718,7 +718,7 @@ extern "C" int cg_likelihood_create(cg_lik** out, int n, const double* c_packed,
     // the factorisation's scratch (M = L^-1 and the digit images) is given back when it is done
     auto free_scratch = [&] { cudaFree(dpk); cudaFree(M); cudaFree(work); };
     if (!dalloc(&lik->A, tiled) || !dalloc(&M, tiled) || !dalloc(&work, cg::digit_bytes(ctx.nt, ctx.nt)) ||
-        !dalloc(&lik->diag, (size_t)ctx.N) || !dalloc(&lik->tmp, 4 * (size_t)ctx.N + 8) || !dalloc(&lik->st, 2) ||
+        !dalloc(&lik->diag, (size_t)ctx.N) || !dalloc(&lik->tmp, 4 * (size_t)ctx.N + 8 + 3 * (size_t)cg::ntiles_lower(ctx.nt)) || !dalloc(&lik->st, 2) ||
         !dalloc(&dpk, 3 * np)) {
         free_scratch();
         g_create_error = "device allocation failed";
@@ -777,19 +777,12 @@ static int lik_finish(cg_lik* lik, double* chi2, double* logdet)
     const int n = ctx.n, N = ctx.N;
     cudaStream_t s = ctx.stream;
     double* tv = lik->tmp;          // padded t
-    double* ta = tv + N;            // C^-1 t
-    double* fv = ta + N;            // padded f
-    double* fa = fv + N;            // C^-1 f
-    double* sc = fa + N;            // scalars
-    cg::fp64_symv(1, ctx.nt, N, lik->A, tv, ta, s);
-    cg::fp64_dot(n, tv, ta, sc + 1, s);  // chi2 = t^T C^-1 t (Likelihood::vmv, source/likelihood.cpp:137-152)
+    double* fv = tv + 2 * (size_t)N; // padded f
+    double* sc = fv + 2 * (size_t)N; // scalars
     const bool fgm = !lik->fg.empty();
-    if (fgm) {
-        cudaMemcpyAsync(fv, lik->fg.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s);
-        cg::fp64_symv(1, ctx.nt, N, lik->A, fv, fa, s);
-        cg::fp64_dot(n, tv, fa, sc + 2, s);
-        cg::fp64_dot(n, fv, fa, sc + 3, s);
-    }
+    if (fgm) cudaMemcpyAsync(fv, lik->fg.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s);
+    // chi2 = t^T C^-1 t (Likelihood::vmv, source/likelihood.cpp:137-152), and t^T C^-1 f, f^T C^-1 f
+    cg::fp64_quad(ctx.nt, lik->A, tv, fgm ? fv : nullptr, sc + 8, sc + 1, s);
     double h[4] = {0, 0, 0, 0};
     cudaMemcpyAsync(h, sc, sizeof(double) * 4, cudaMemcpyDeviceToHost, s);
     CG_CUDA_TRY(&ctx, cudaStreamSynchronize(s));

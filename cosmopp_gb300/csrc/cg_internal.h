@@ -330,6 +330,8 @@ void fp64_free(cg_ctx* ctx);
 int fp64_identity_rows(cg_ctx* ctx, int B, int nt, double* E, size_t strideE, cudaStream_t s);
 void fp64_packed_to_tiled(int n, int nt, const double* c, const double* f, const double* nz, double* A, cudaStream_t s);
 void fp64_symv(int B, int nt, int N, const double* V, const double* dv, double* alpha, cudaStream_t s);
+// out[0] = t^T V t and, with f, out[1] = t^T V f, out[2] = f^T V f for V in lower tiles; part: 3 per tile
+void fp64_quad(int nt, const double* V, const double* tv, const double* fv, double* part, double* out, cudaStream_t s);
 void fp64_logdet(int B, int n, int N, const double* diag, double* out, cudaStream_t s);
 void fp64_dot(int n, const double* a, const double* b, double* out, cudaStream_t s);
 }  // namespace cg

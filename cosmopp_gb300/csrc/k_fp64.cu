@@ -350,16 +350,18 @@ __global__ void __launch_bounds__(kThreads) build_fid_packed(int n, int N, int l
 }
 
 // ln det = 2 sum_i ln L_ii over the n real pixels (source/matrix_impl.cpp:322-338), grid B
-__global__ void __launch_bounds__(kThreads) logdet_reduce(int n, int N, const double* __restrict__ diag,
-                                                          double* __restrict__ logdet)
+// (an FP64 logarithm is some 30 instructions of 64 cycles each and partition)
+constexpr int kLogThreads = 1024;
+__global__ void __launch_bounds__(kLogThreads) logdet_reduce(int n, int N, const double* __restrict__ diag,
+                                                             double* __restrict__ logdet)
 {
-    __shared__ double red[kThreads];
+    __shared__ double red[kLogThreads];
     const int b = blockIdx.x;
     double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += kThreads) s += log(fabs(diag[(size_t)b * N + i]));
+    for (int i = threadIdx.x; i < n; i += kLogThreads) s += log(fabs(diag[(size_t)b * N + i]));
     red[threadIdx.x] = s;
     __syncthreads();
-    for (int w = kThreads / 2; w > 0; w >>= 1) {
+    for (int w = kLogThreads / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
@@ -536,6 +538,61 @@ __global__ void dot_kernel(int n, const double* __restrict__ a, const double* __
         __syncthreads();
     }
     if (threadIdx.x == 0) *out = red[0];
+}
+
+// The quadratic forms of the packed Likelihood from its inverse's lower tiles: part[t][0] = t^T V t and, with a
+// foreground f, part[t][1] = t^T V f, part[t][2] = f^T V f over tile t and its mirror.  One CTA per tile: the
+// matrix is read once for both vectors and every SM takes part (a CTA per row block and vector left 40 SMs to
+// do it, 152 us a vector at 2469 pixels); a tile costs half the products of a matrix-vector product, whose
+// vector nobody needs.  grid tiles
+__global__ void __launch_bounds__(kThreads) quad_tiles(const double* __restrict__ V, const double* __restrict__ tv,
+                                                       const double* __restrict__ fv, double* __restrict__ part)
+{
+    __shared__ double red[2][4][TS];
+    __shared__ double sum[3][2];
+    int I, J;
+    tile_coords(blockIdx.x, I, J);
+    const double* tile = V + (size_t)blockIdx.x * TILE_ELEMS;
+    const int r = threadIdx.x % TS, q = threadIdx.x / TS;
+    double y = 0.0, z = 0.0;
+#pragma unroll
+    for (int c = q; c < TS; c += 4) {
+        const double v = tile[r + TS * c];
+        y = fma(v, tv[J * TS + c], y);
+        if (fv) z = fma(v, fv[J * TS + c], z);
+    }
+    red[0][q][r] = y;
+    red[1][q][r] = z;
+    __syncthreads();
+    if (threadIdx.x < TS) {
+        y = ((red[0][0][r] + red[0][1][r]) + red[0][2][r]) + red[0][3][r];
+        z = ((red[1][0][r] + red[1][1][r]) + red[1][2][r]) + red[1][3][r];
+        const double t = tv[I * TS + r], f = fv ? fv[I * TS + r] : 0.0, two = I == J ? 1.0 : 2.0;
+        double s[3] = {two * (t * y), I == J ? t * z : fma(t, z, f * y), two * (f * z)};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], o);
+            if (r % 32 == 0) sum[k][r / 32] = s[k];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) part[3 * (size_t)blockIdx.x + threadIdx.x] = sum[threadIdx.x][0] + sum[threadIdx.x][1];
+}
+
+// out[k] = sum over tiles of part[t][k]; grid 3
+__global__ void __launch_bounds__(kThreads) quad_sum(int ntile, const double* __restrict__ part,
+                                                     double* __restrict__ out)
+{
+    __shared__ double red[kThreads];
+    double s = 0.0;
+    for (int t = threadIdx.x; t < ntile; t += kThreads) s += part[3 * (size_t)t + blockIdx.x];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = kThreads / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
 }
 
 // Dense FP64 helpers of the polarisation likelihood's set-up (column-major, leading dimension
@@ -853,9 +910,15 @@ void fp64_symv(int B, int nt, int N, const double* V, const double* dv, double* 
     symv_tiled<double><<<dim3(nt, B), kThreads, 0, s>>>(nt, N, V, tiled_elems(nt), dv, alpha);
 }
 
+void fp64_quad(int nt, const double* V, const double* tv, const double* fv, double* part, double* out, cudaStream_t s)
+{
+    quad_tiles<<<ntiles_lower(nt), kThreads, 0, s>>>(V, tv, fv, part);
+    quad_sum<<<fv ? 3 : 1, kThreads, 0, s>>>(ntiles_lower(nt), part, out);
+}
+
 void fp64_logdet(int B, int n, int N, const double* diag, double* out, cudaStream_t s)
 {
-    logdet_reduce<<<B, kThreads, 0, s>>>(n, N, diag, out);
+    logdet_reduce<<<B, kLogThreads, 0, s>>>(n, N, diag, out);
 }
 
 void fp64_dot(int n, const double* a, const double* b, double* out, cudaStream_t s)
@@ -1092,7 +1155,7 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
                            w.ext_elems, w.diag, w.st, w.dig, w.err, s)))
         return rc;
     stage_mark(ctx, ST_SOLVE, s);
-    logdet_reduce<<<B, kThreads, 0, s>>>(n, N, w.diag, w.ld);
+    logdet_reduce<<<B, kLogThreads, 0, s>>>(n, N, w.diag, w.ld);
     if (inverse) {
         pad_data<<<dim3((N + 255) / 256, B), 256, 0, s>>>(n, N, B, d_d, d_stride, w.dvec);
         symv_tiled<double><<<dim3(nt, B), kThreads, 0, s>>>(nt, N, w.A, strideA, w.dvec, w.alpha);

@@ -127,3 +127,23 @@ def test_packed_likelihood(n):
         assert abs(chi2 - want) <= tol * want
         assert abs(lik.logdet_raw - np.linalg.slogdet(full)[1]) <= tol
     lik.close()
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 130, 257])
+def test_packed_likelihood_foreground(n):
+    """The marginalised foreground (source/likelihood.cpp:171-177) needs t^T C^-1 f and f^T C^-1 f: three
+    quadratic forms, each within the bar of one."""
+    rng = np.random.default_rng(1000 + n)
+    a = rng.standard_normal((n, n + 5))
+    c = a @ a.T / n
+    full = (c + c.T) / 2 + 0.5 * np.eye(n)
+    t, f = rng.standard_normal(n), 1.0 + rng.standard_normal(n)
+    ev = np.linalg.eigvalsh(full)
+    tol = 8 * n * EPS * ev[-1] / ev[0]
+    lik = cg.Likelihood(W.full_to_packed(full), None, np.zeros(n * (n + 1) // 2), foreground=f)
+    _, chi2, ld = lik.calculate(t)
+    at, af = np.linalg.solve(full, t), np.linalg.solve(full, f)
+    tt, tf, ff = t @ at, t @ af, f @ af
+    assert abs(chi2 - (tt - tf * tf / ff)) <= 3 * tol * tt
+    assert abs((ld - cg.DET_OFFSET) - (np.linalg.slogdet(full)[1] + np.log(ff / n))) <= 2 * tol + 8 * EPS * abs(ld)
+    lik.close()
