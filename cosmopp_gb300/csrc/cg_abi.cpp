@@ -672,7 +672,7 @@ struct cg_lik {
     cg_ctx ctx;                  // device, sizes, stream and error text
     double* A = nullptr;         // tiled C + F + N, then C^-1
     double* diag = nullptr;
-    double* tmp = nullptr;       // [4][N] vectors, 8 scalars, 3 sums per tile
+    double* tmp = nullptr;       // [4][N] vectors, 8 scalars, partial sums
     int* st = nullptr;
     double logdet = 0;
     std::vector<double> fg;
@@ -718,7 +718,7 @@ extern "C" int cg_likelihood_create(cg_lik** out, int n, const double* c_packed,
     // the factorisation's scratch (M = L^-1 and the digit images) is given back when it is done
     auto free_scratch = [&] { cudaFree(dpk); cudaFree(M); cudaFree(work); };
     if (!dalloc(&lik->A, tiled) || !dalloc(&M, tiled) || !dalloc(&work, cg::digit_bytes(ctx.nt, ctx.nt)) ||
-        !dalloc(&lik->diag, (size_t)ctx.N) || !dalloc(&lik->tmp, 4 * (size_t)ctx.N + 8 + 3 * (size_t)cg::ntiles_lower(ctx.nt)) || !dalloc(&lik->st, 2) ||
+        !dalloc(&lik->diag, (size_t)ctx.N) || !dalloc(&lik->tmp, 4 * (size_t)ctx.N + 8 + std::max(3 * (size_t)cg::ntiles_lower(ctx.nt), (size_t)cg::kResidualSplit * ctx.N)) || !dalloc(&lik->st, 2) ||
         !dalloc(&dpk, 3 * np)) {
         free_scratch();
         g_create_error = "device allocation failed";
@@ -824,7 +824,7 @@ extern "C" int cg_likelihood_pol_create(cg_lik** out, int npix, const int* good,
     for (int i = 0; i < ngood; ++i)
         if (good[i] < 0 || good[i] >= npix) { g_create_error = "good pixel index out of range"; return CG_ERR_BAD_ARG; }
     // source/likelihood.cpp:371-384: the Q and U rows and columns of the kept pixels
-    const int n = 2 * ngood, size = 2 * npix, ld = (n + 63) / 64 * 64;
+    const int n = 2 * ngood, size = 2 * npix, ld = (n + 127) / 128 * 128;
     auto full = [&](int k) { return k < ngood ? good[k] : npix + good[k - ngood]; };
     const size_t np = (size_t)n * (n + 1) / 2;
     std::vector<double> cg_packed(np), nd((size_t)ld * ld, 0.0);
@@ -849,8 +849,10 @@ extern "C" int cg_likelihood_pol_create(cg_lik** out, int npix, const int* good,
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) { g_create_error = "stream"; return CG_ERR_CUDA; }
     const size_t nel = (size_t)ld * ld;
     double *d_c = nullptr, *d_n = nullptr, *d_cd = nullptr, *d_t = nullptr, *d_m = nullptr, *d_mp = nullptr;
+    unsigned char* work = nullptr;
+    int *d_err = nullptr, err = 0;
     int rc = CG_OK;
-    if (!dalloc(&d_c, np) || !dalloc(&d_n, nel) || !dalloc(&d_cd, nel) || !dalloc(&d_t, nel) || !dalloc(&d_m, nel) ||
+    if (!dalloc(&work, cg::digit_gemm_bytes(ld / cg::TS)) || !dalloc(&d_err, 1) || !dalloc(&d_c, np) || !dalloc(&d_n, nel) || !dalloc(&d_cd, nel) || !dalloc(&d_t, nel) || !dalloc(&d_m, nel) ||
         !dalloc(&d_mp, np)) {
         g_create_error = "device allocation failed";
         rc = CG_ERR_ALLOC;
@@ -860,15 +862,18 @@ extern "C" int cg_likelihood_pol_create(cg_lik** out, int npix, const int* good,
         cudaMemcpyAsync(d_c, cg_packed.data(), sizeof(double) * np, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(d_n, nd.data(), sizeof(double) * nel, cudaMemcpyHostToDevice, s);
         // source/likelihood.cpp:386-387: cInv = N^-1 + N^-1 C N^-1
-        rc = cg::fp64_pol_matrix(&tmpctx, n, ld, d_c, d_n, d_cd, d_t, d_m, d_mp, s);
+        cudaMemsetAsync(d_err, 0, sizeof(int), s);
+        rc = cg::fp64_pol_matrix(&tmpctx, n, ld, d_c, d_n, d_cd, d_t, d_m, d_mp, work, d_err, s);
         if (rc == CG_OK) {
             cudaMemcpyAsync(m_packed.data(), d_mp, sizeof(double) * np, cudaMemcpyDeviceToHost, s);
+            cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
             if (cudaStreamSynchronize(s) != cudaSuccess) { g_create_error = "polarisation matrix build failed"; rc = CG_ERR_CUDA; }
+            else if (err) { g_create_error = "a device wait gave up"; rc = CG_ERR_TIMEOUT; }
         } else {
             g_create_error = tmpctx.err;
         }
     }
-    cudaFree(d_c); cudaFree(d_cd); cudaFree(d_t); cudaFree(d_m); cudaFree(d_mp);
+    cudaFree(d_c); cudaFree(d_cd); cudaFree(d_t); cudaFree(d_m); cudaFree(d_mp); cudaFree(work); cudaFree(d_err);
     cudaStreamDestroy(s);
     if (rc == CG_OK) rc = cg_likelihood_create(out, n, m_packed.data(), nullptr, zero.data(), nullptr, device);
     if (rc != CG_OK) {
@@ -898,7 +903,7 @@ extern "C" int cg_likelihood_pol_calculate(cg_lik* lik, const double* v, const d
     cudaMemcpyAsync(vv, v, sizeof(double) * n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(sv, subtract, sizeof(double) * n, cudaMemcpyHostToDevice, s);
     // source/likelihood.cpp:595-600: vCopy -= N^-1 subtractMap
-    int rc = cg::fp64_dense_residual(&ctx, n, lik->ld, lik->Ninv, vv, sv, w, s);
+    int rc = cg::fp64_dense_residual(&ctx, n, lik->ld, lik->Ninv, vv, sv, w, sv + 2 * (size_t)N + 8, s);
     if (rc) return rc;
     cudaMemsetAsync(vv, 0, sizeof(double) * 2 * N, s);
     return lik_finish(lik, chi2, logdet);   // chi2 = w^T cInv w (source/likelihood.cpp:602-609)

@@ -238,13 +238,15 @@ int ylm_fill(cg_ctx* ctx, double* Y, cudaStream_t s);
 void mixed_bytes(const cg_ctx* ctx, size_t* fixed, size_t* per_element);
 int fp64_build_tiled_into(cg_ctx* ctx, int B, const double* d_cl, bool add_noise, double* A, cudaStream_t s);
 int fp64_build_packed(cg_ctx* ctx, int B, const double* d_cl, double* d_out, cudaStream_t s);
-// polarisation likelihood set-up: M = N^-1 + N^-1 C N^-1 for packed C and dense N^-1 (ld x ld,
-// column-major, zero padded), packed into d_m_packed; d_cd, d_t, d_m are ld x ld scratch
+// polarisation likelihood set-up: M = N^-1 + N^-1 C N^-1 for packed C and dense N^-1 (ld x ld, column-major,
+// zero padded, ld a multiple of 128), packed into d_m_packed; d_cd, d_t, d_m are ld x ld scratch, work
+// digit_gemm_bytes(ld / 64), *err set if a bounded wait gives up
 int fp64_pol_matrix(cg_ctx* ctx, int n, int ld, const double* d_c_packed, const double* d_ninv, double* d_cd,
-                    double* d_t, double* d_m, double* d_m_packed, cudaStream_t s);
-// w = v - N^-1 s for the dense N^-1 above
+                    double* d_t, double* d_m, double* d_m_packed, unsigned char* work, int* err, cudaStream_t s);
+// w = v - N^-1 s for the dense N^-1 above; part: kResidualSplit n doubles
+constexpr int kResidualSplit = 8;
 int fp64_dense_residual(cg_ctx* ctx, int n, int ld, const double* d_ninv, const double* d_v, const double* d_s,
-                        double* d_w, cudaStream_t s);
+                        double* d_w, double* part, cudaStream_t s);
 // P_l(x_ij) for l0 <= l < l1 into d_out [(l1 - l0)][n(n+1)/2]; d_a, d_b = the recurrence
 // coefficients, at least l1 entries each (device pointers)
 int fp64_legendre_table(cg_ctx* ctx, int l0, int l1, const double* d_a, const double* d_b, double* d_out,
@@ -262,11 +264,17 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
 //   DIGIT_EXT_IDENTITY  ne = nt, E holds the identity, tile (eb, k >= eb) at tile_index(k, eb); it ends
 //                       as scratch and A as the inverse
 // work: digit_bytes(nt, ne) per matrix, 16-byte aligned; *err is set if a bounded wait gives up.
-enum DigitExt { DIGIT_EXT_ROWS = 0, DIGIT_EXT_IDENTITY = 1 };
+enum DigitExt { DIGIT_EXT_ROWS = 0, DIGIT_EXT_IDENTITY = 1, DIGIT_EXT_PRODUCT = 2 };
 size_t digit_bytes(int nt, int ne);
 void digit_free(cg_ctx* ctx);  // the context's second stream and its events
 int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t strideA, double* E,
                  size_t strideE, double* diag, int* status, unsigned char* work, int* err, cudaStream_t s);
+// out += A B for dense square matrices of nt (even) 64-blocks, the same digit products: A column-major; B
+// column-major (kindB = 1) or in out's layout (kindB = 2); out in tiles, (I, J) at I nt + J, element (r, c) at
+// r + 64 c.  work: digit_gemm_bytes(nt)
+size_t digit_gemm_bytes(int nt);
+int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* B, int kindB, double* out, unsigned char* work,
+               int* err, cudaStream_t s);
 // generic tiled FP64 / FP32 factorisation entry points (k_chol.cu)
 template <typename T>
 int tiled_cholesky(cg_ctx* ctx, int B, int nt, T* A, T* Dinv, T* diag, int* status, size_t strideA, cudaStream_t s);

@@ -136,6 +136,8 @@ struct Dig {
     size_t strideA, strideE;  // doubles
     unsigned char* img;       // [B][pairs][kImg]
     int* ex;                  // [B][pairs][128]
+    int nk;                   // sets of images that an update takes one after the other (1 in a factorisation)
+    size_t kimg, kex;         // their distances
     unsigned char* dimg;      // [B][kDImg]
     int* dex;                 // [B][64]
     int* err;
@@ -771,11 +773,12 @@ struct UpJob {
 // rows over the same columns, and with v the pairs of V
 struct UpRange {
     int q0, ncol, npe, v;
+    int a = 1;                // 0: E's rows alone
 };
 __host__ __device__ inline int up_tri(const UpRange& u, int nq)
 {
     const int m = nq - u.q0;
-    return u.ncol == 1 ? m : m * (m + 1) / 2;
+    return u.a == 0 ? 0 : u.ncol == 1 ? m : m * (m + 1) / 2;
 }
 __host__ __device__ inline int up_jobs(const UpRange& u, int nq)
 {
@@ -827,13 +830,15 @@ __device__ __forceinline__ void up_halves(const UpJob& j, int k, int& h0, int& h
     h1 = (j.kind == 2 && 2 * j.q + 1 > k) ? 1 : 2;
 }
 
+// SETS: several sets of images per job (a product); a factorisation's step has one
+template <bool SETS>
 __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, int per, UpRange u, Dig g)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ uint64_t full[4], empty[4], tfull[2], tempty[2];
     __shared__ uint32_t tptr;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int pairs = dig_pairs(g);
+    const int pairs = dig_pairs(g), nk = SETS ? g.nk : 1;
     launch_dependents();
     if (warp == 0) tmem_alloc(&tptr, 512);
     if (t == 0) {
@@ -856,34 +861,36 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
     uint32_t pass = 0, round = 0;
     if (warp == kUpWarps) {
         if (lane == 0)
-            for (int job = blockIdx.x; job < njobs; job += gridDim.x, ++round) {
+            for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
                 const UpJob j = up_job(g, u, per, job);
-                const unsigned char* a = g.img + ((size_t)j.b * pairs + j.pa) * kImg;
-                const unsigned char* bb = g.img + ((size_t)j.b * pairs + j.pb) * kImg;
-                for (int kc = 0; kc < 4; ++kc) {
-                    if (round > 0) ok = mbar_wait(&empty[kc], (round - 1) & 1, kWaits, g.err) && ok;
-                    mbar_arrive_expect_tx(&full[kc], (j.pa == j.pb ? 2 : 4) * kCore);
-                    bulk_g2s(smem_u32(sm + 2 * kc * kCore), a + 2 * kc * kCore, 2 * kCore, &full[kc]);
-                    if (j.pa != j.pb)
-                        bulk_g2s(smem_u32(sm + kUpB + 2 * kc * kCore), bb + 2 * kc * kCore, 2 * kCore, &full[kc]);
-                }
                 int h0, h1;
                 up_halves(j, k, h0, h1);
-                for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
-                    const uint32_t buf = pass & 1;
-                    if (pass >= 2) ok = mbar_wait(&tempty[buf], ((pass >> 1) - 1) & 1, kWaits, g.err) && ok;
-                    fence_after();
-                    const uint64_t ad = smem_desc(smem_u32(sm), kCore, kGroupBytes);
-                    const uint64_t bd = smem_desc(smem_u32(sm + (j.pa == j.pb ? 0 : kUpB) + (i >> 1) * kGroupBytes +
-                                                           (i & 1) * 2 * kGroupBytes),
-                                                  kCore, 4 * kGroupBytes);
+                for (int ks = 0; ks < nk; ++ks, ++round) {
+                    const unsigned char* a = g.img + ks * g.kimg + ((size_t)j.b * pairs + j.pa) * kImg;
+                    const unsigned char* bb = g.img + ks * g.kimg + ((size_t)j.b * pairs + j.pb) * kImg;
                     for (int kc = 0; kc < 4; ++kc) {
-                        if (i == 2 * h0) ok = mbar_wait(&full[kc], round & 1, kWaits, g.err) && ok;
-                        issue_products<kPassCols>(tmem + 256 * buf, ad + (uint64_t)kc * (2 * kCore >> 4),
-                                                  bd + (uint64_t)kc * (2 * kCore >> 4), kPlane, kPlane, kc == 0);
-                        if (i == 2 * h1 - 1) mma_commit(&empty[kc]);
+                        if (round > 0) ok = mbar_wait(&empty[kc], (round - 1) & 1, kWaits, g.err) && ok;
+                        mbar_arrive_expect_tx(&full[kc], (j.pa == j.pb ? 2 : 4) * kCore);
+                        bulk_g2s(smem_u32(sm + 2 * kc * kCore), a + 2 * kc * kCore, 2 * kCore, &full[kc]);
+                        if (j.pa != j.pb)
+                            bulk_g2s(smem_u32(sm + kUpB + 2 * kc * kCore), bb + 2 * kc * kCore, 2 * kCore, &full[kc]);
                     }
-                    mma_commit(&tfull[buf]);
+                    for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
+                        const uint32_t buf = pass & 1;
+                        if (pass >= 2) ok = mbar_wait(&tempty[buf], ((pass >> 1) - 1) & 1, kWaits, g.err) && ok;
+                        fence_after();
+                        const uint64_t ad = smem_desc(smem_u32(sm), kCore, kGroupBytes);
+                        const uint64_t bd = smem_desc(smem_u32(sm + (j.pa == j.pb ? 0 : kUpB) + (i >> 1) * kGroupBytes +
+                                                               (i & 1) * 2 * kGroupBytes),
+                                                      kCore, 4 * kGroupBytes);
+                        for (int kc = 0; kc < 4; ++kc) {
+                            if (i == 2 * h0) ok = mbar_wait(&full[kc], round & 1, kWaits, g.err) && ok;
+                            issue_products<kPassCols>(tmem + 256 * buf, ad + (uint64_t)kc * (2 * kCore >> 4),
+                                                      bd + (uint64_t)kc * (2 * kCore >> 4), kPlane, kPlane, kc == 0);
+                            if (i == 2 * h1 - 1) mma_commit(&empty[kc]);
+                        }
+                        mma_commit(&tfull[buf]);
+                    }
                 }
             }
         __syncwarp();
@@ -892,55 +899,57 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
         const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
         for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
             const UpJob j = up_job(g, u, per, job);
-            const int ea = g.ex[((size_t)j.b * pairs + j.pa) * 128 + 64 * half + r];
-            const int* eb = g.ex + ((size_t)j.b * pairs + j.pb) * 128;
             double* Ab = g.A + (size_t)j.b * g.strideA;
-            const unsigned flip = j.kind == 2 ? 0u : 0x80000000u;
+            const unsigned flip = j.kind == 2 || g.ext == DIGIT_EXT_PRODUCT ? 0u : 0x80000000u;
             int h0, h1;
             up_halves(j, k, h0, h1);
-            for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
-                const uint32_t buf = pass & 1;
-                const int rb = 2 * j.p + half, cb = 2 * j.q + (i >> 1), c0 = (2 * c4 + (i & 1)) * 8;
-                bool valid;
-                double* tile = Ab;
-                if (j.kind == 0) {
-                    valid = rb > k && rb >= cb;
-                    if (valid) tile = Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS;
-                } else if (j.kind == 1) {
-                    valid = g.ext != DIGIT_EXT_IDENTITY || rb <= k;
-                    if (valid) tile = ext_tile(g, j.b, rb, cb);
-                } else {
-                    valid = rb <= k && rb >= cb;
-                    if (valid) tile = Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS;
-                }
-                const bool read = valid && !(j.kind == 2 && rb == k);  // V's row k starts here
-                double* dst = tile + r + TS * c0;
-                double old[8];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) old[c] = read ? dst[TS * c] : 0.0;
-                const int4 e0 = *reinterpret_cast<const int4*>(eb + 64 * (i >> 1) + c0);
-                const int4 e1 = *reinterpret_cast<const int4*>(eb + 64 * (i >> 1) + c0 + 4);
-                const int se[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
-                ok = mbar_wait(&tfull[buf], (pass >> 1) & 1, kWaits, g.err) && ok;
-                fence_after();
-                __syncwarp();
-                const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 256 * buf + 8 * c4;
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    uint32_t acc[8][4];
-                    tmem_ld_acc4<kPassCols>(ta + 4 * q, acc);
-                    if (q == 1) {
-                        fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&tempty[buf]);
+            for (int ks = 0; ks < nk; ++ks) {
+                const int ea = g.ex[ks * g.kex + ((size_t)j.b * pairs + j.pa) * 128 + 64 * half + r];
+                const int* eb = g.ex + ks * g.kex + ((size_t)j.b * pairs + j.pb) * 128;
+                for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
+                    const uint32_t buf = pass & 1;
+                    const int rb = 2 * j.p + half, cb = 2 * j.q + (i >> 1), c0 = (2 * c4 + (i & 1)) * 8;
+                    bool valid;
+                    double* tile = Ab;
+                    if (j.kind == 0) {
+                        valid = rb > k && rb >= cb;
+                        if (valid) tile = Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS;
+                    } else if (j.kind == 1) {
+                        valid = g.ext != DIGIT_EXT_IDENTITY || rb <= k;
+                        if (valid) tile = ext_tile(g, j.b, rb, cb);
+                    } else {
+                        valid = rb <= k && rb >= cb;
+                        if (valid) tile = Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS;
                     }
-                    if (valid) {
+                    const bool read = valid && !(j.kind == 2 && rb == k);  // V's row k starts here
+                    double* dst = tile + r + TS * c0;
+                    double old[8];
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
-                            dst[TS * (4 * q + c)] =
-                                old[4 * q + c] + scaled_int(join_acc4(acc, c), ea + se[4 * q + c] - 55, flip);
-                    }
+                    for (int c = 0; c < 8; ++c) old[c] = read ? dst[TS * c] : 0.0;
+                    const int4 e0 = *reinterpret_cast<const int4*>(eb + 64 * (i >> 1) + c0);
+                    const int4 e1 = *reinterpret_cast<const int4*>(eb + 64 * (i >> 1) + c0 + 4);
+                    const int se[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+                    ok = mbar_wait(&tfull[buf], (pass >> 1) & 1, kWaits, g.err) && ok;
+                    fence_after();
                     __syncwarp();
+                    const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 256 * buf + 8 * c4;
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        uint32_t acc[8][4];
+                        tmem_ld_acc4<kPassCols>(ta + 4 * q, acc);
+                        if (q == 1) {
+                            fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&tempty[buf]);
+                        }
+                        if (valid) {
+#pragma unroll
+                            for (int c = 0; c < 4; ++c)
+                                dst[TS * (4 * q + c)] =
+                                    old[4 * q + c] + scaled_int(join_acc4(acc, c), ea + se[4 * q + c] - 55, flip);
+                        }
+                        __syncwarp();
+                    }
                 }
             }
         }
@@ -949,6 +958,40 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
     fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+// Images of a dense operand's row pairs for K blocks k0, k0 + 1, ..: grid (row pairs, K blocks).  Element
+// (row, k): kind 0 at k ld + row, kind 1 at row ld + k, kind 2 in 64 x 64 tiles (k / 64, row / 64) of nt to a
+// row, element (r, c) at r + 64 c.  Thread (row, 16 columns), as in the panel.
+__global__ void __launch_bounds__(kPanelThreads) digit_slice(int kind, int ld, int k0, int first, const double* __restrict__ src, Dig g)
+{
+    __shared__ int smax[4][128];
+    const int t = threadIdx.x, m = t & 127, cq = t >> 7, pair = blockIdx.x, nt = ld / TS;
+    const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7), row = 128 * pair + 64 * half + r;
+    const int kb = k0 + blockIdx.y;
+    auto at = [&](int c) {
+        const int k = TS * kb + c;
+        return kind == 0   ? src[(size_t)k * ld + row]
+               : kind == 1 ? src[(size_t)row * ld + k]
+                           : src[((size_t)kb * nt + row / TS) * TILE_ELEMS + c + TS * r];
+    };
+    int f = 0;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) f = max(f, exp_field(at(16 * cq + c)));
+    smax[cq][m] = f;
+    __syncthreads();
+    const int e = row_exp(max(max(smax[0][m], smax[1][m]), max(smax[2][m], smax[3][m])));
+    const size_t p = first + pair;
+    if (cq == 0) g.ex[blockIdx.y * g.kex + p * 128 + 64 * half + r] = e;
+    unsigned char* out = g.img + blockIdx.y * g.kimg + p * kImg + (size_t)m * 16;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        unsigned long long w[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) w[c] = to_digits(to_fixed(at(16 * cq + 8 * h + c), e));
+        unsigned char* o = out + (2 * cq + h) * kCore;
+        store_digits(w, [&](int i, uint4 d) { *reinterpret_cast<uint4*>(o + i * kPlane) = d; });
+    }
 }
 
 }  // namespace
@@ -996,7 +1039,7 @@ static int launch_update(cg_ctx* ctx, int B, int k, const UpRange& u, const Dig&
 {
     const int per = up_jobs(u, g.nt / 2);
     if (per <= 0) return CG_OK;
-    return launch(ctx, digit_update, dim3((unsigned)std::min<long long>((long long)per * B, ctas)), kUpThreads, kUpSmem, 1, s,
+    return launch(ctx, digit_update<false>, dim3((unsigned)std::min<long long>((long long)per * B, ctas)), kUpThreads, kUpSmem, 1, s,
                   k, per * B, per, u, g);
 }
 
@@ -1063,6 +1106,8 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
     g.E = E;
     g.strideA = strideA;
     g.strideE = strideE;
+    g.nk = 1;
+    g.kimg = g.kex = 0;
     // two sets of images, for the steps in turn where the update of one runs beside the panel of the next
     unsigned char* const img[2] = {work, work + (size_t)B * pairs * kImg};
     g.dimg = img[1] + (size_t)B * pairs * kImg;
@@ -1072,7 +1117,7 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
     g.err = err;
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DiagShared)));
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem));
-    CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem));
+    CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_update<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem));
     bool rest = false;  // an update on the second stream that the caller's stream has not waited for
     for (int k = 0; k < nt; ++k) {
         const int q0 = (k + 1) / 2, m = nq - q0, npe = v ? k / 2 + 1 : ne / 2;
@@ -1105,6 +1150,38 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
         rest = true;
     }
     if (rest) CG_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain[1], 0));
+    CG_CUDA_TRY(ctx, cudaGetLastError());
+    return CG_OK;
+}
+
+// K blocks whose images are held at once
+static int gemm_chunk(int nt) { return std::min(nt, 16); }
+
+size_t digit_gemm_bytes(int nt) { return (size_t)gemm_chunk(nt) * nt * (kImg + 128 * sizeof(int)); }
+
+int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, int kindB, double* out, unsigned char* work,
+               int* err, cudaStream_t s)
+{
+    const int nq = nt / 2, chunk = gemm_chunk(nt), ld = nt * TS;
+    Dig g = {};
+    g.nt = g.ne = nt;
+    g.ext = DIGIT_EXT_PRODUCT;
+    g.A = g.E = out;
+    g.kimg = (size_t)nt * kImg;
+    g.kex = (size_t)nt * 128;
+    g.img = work;
+    g.ex = reinterpret_cast<int*>(work + chunk * g.kimg);
+    g.err = err;
+    CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_update<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem));
+    const UpRange u = {0, nq, nq, 0, 0};
+    const int per = up_jobs(u, nq);
+    for (int k0 = 0; k0 < nt; k0 += chunk) {
+        g.nk = std::min(chunk, nt - k0);
+        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(kindB, ld, k0, 0, Bm, g);
+        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(0, ld, k0, nq, A, g);
+        digit_update<true><<<std::min(per, ctx->sm_count), kUpThreads, kUpSmem, s>>>(-1, per, per, u, g);
+        count_launch(ctx, 3);
+    }
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;
 }

@@ -596,50 +596,15 @@ __global__ void __launch_bounds__(kThreads) quad_sum(int ntile, const double* __
 }
 
 // Dense FP64 helpers of the polarisation likelihood's set-up (column-major, leading dimension
-// ld, a multiple of 64, zero padding beyond n).
-// out = add + A B: one 64 x 64 output tile per CTA, 16-deep K slices of A and B in shared memory,
-// 4 x 4 outputs per thread at rows tx + 16 p and columns ty + 16 q
-__global__ void __launch_bounds__(kThreads) dense_gemm64(int ld, const double* __restrict__ A,
-                                                         const double* __restrict__ Bm,
-                                                         const double* __restrict__ add, double* __restrict__ out)
+// ld, a multiple of 128, zero padding beyond n; the products run in k_digit.cu on 64 x 64 tiles).
+
+// column-major to tiles (I, J) at I nt + J, element (r, c) at r + 64 c; grid (nt, nt)
+__global__ void __launch_bounds__(kThreads) dense_to_tiles(int ld, const double* __restrict__ d, double* __restrict__ t)
 {
-    __shared__ double As[16][65], Bs[16][65];
-    const int bi = blockIdx.x * 64, bj = blockIdx.y * 64;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    double acc[4][4];
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[p][q] = 0.0;
-    for (int k0 = 0; k0 < ld; k0 += 16) {
-        for (int e = threadIdx.x; e < 1024; e += kThreads) {
-            const int r = e % 64, kk = e / 64;
-            As[kk][r] = A[(size_t)(k0 + kk) * ld + bi + r];
-            const int kb = e % 16, c = e / 16;
-            Bs[kb][c] = Bm[(size_t)(bj + c) * ld + k0 + kb];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            double a[4], b[4];
-#pragma unroll
-            for (int p = 0; p < 4; ++p) a[p] = As[kk][tx + 16 * p];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) b[q] = Bs[kk][ty + 16 * q];
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const size_t o = (size_t)(bj + ty + 16 * q) * ld + bi + tx + 16 * p;
-            out[o] = (add ? add[o] : 0.0) + acc[p][q];
-        }
+    const int I = blockIdx.x, J = blockIdx.y, nt = ld / TS;
+    double* tile = t + ((size_t)I * nt + J) * TILE_ELEMS;
+    for (int e = threadIdx.x; e < TILE_ELEMS; e += kThreads)
+        tile[e] = d[(size_t)(J * TS + e / TS) * ld + I * TS + e % TS];
 }
 
 // packed symmetric (i <= j at j(j+1)/2 + i) to dense, zero outside n x n; grid covers ld x ld
@@ -652,8 +617,8 @@ __global__ void packed_to_dense(int n, int ld, const double* __restrict__ pk, do
     d[e] = (j < n) ? pk[(size_t)j * (j + 1) / 2 + i] : 0.0;
 }
 
-// the upper triangle of a dense symmetric matrix, packed
-__global__ void dense_to_packed(int n, int ld, const double* __restrict__ d, double* __restrict__ pk)
+// the upper triangle of a symmetric matrix in tiles, packed
+__global__ void tiles_to_packed(int n, int nt, const double* __restrict__ t, double* __restrict__ pk)
 {
     const long np = (long)n * (n + 1) / 2;
     const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -662,17 +627,33 @@ __global__ void dense_to_packed(int n, int ld, const double* __restrict__ d, dou
     while (j * (j + 1) / 2 > k) --j;
     while ((j + 1) * (j + 2) / 2 <= k) ++j;
     const long i = k - j * (j + 1) / 2;
-    pk[k] = d[(size_t)j * ld + i];
+    pk[k] = t[((size_t)(i / TS) * nt + j / TS) * TILE_ELEMS + i % TS + TS * (j % TS)];
 }
 
-// w = v - N s for a dense symmetric N (row i read as column i, coalesced over i)
-__global__ void dense_residual(int n, int ld, const double* __restrict__ Nm, const double* __restrict__ v,
-                               const double* __restrict__ sv, double* __restrict__ w)
+// part[z][i] = sum of N_ij s_j over the columns of slice z, four partial sums per row; one CTA per 64 rows and
+// slice (one thread per row and all columns left five CTAs to do it, 287 us at 1228 rows);
+// grid (ceil(n / 64), kResidualSplit)
+__global__ void __launch_bounds__(kThreads) residual_parts(int n, int ld, const double* __restrict__ Nm,
+                                                           const double* __restrict__ sv, double* __restrict__ part)
+{
+    __shared__ double red[4][TS];
+    const int r = threadIdx.x % TS, q = threadIdx.x / TS, i = blockIdx.x * TS + r;
+    const int len = (n + kResidualSplit - 1) / kResidualSplit, j0 = blockIdx.y * len, j1 = min(n, j0 + len);
+    double acc = 0.0;
+    if (i < n)
+        for (int j = j0 + q; j < j1; j += 4) acc = fma(Nm[(size_t)j * ld + i], sv[j], acc);
+    red[q][r] = acc;
+    __syncthreads();
+    if (q == 0 && i < n) part[(size_t)blockIdx.y * n + i] = ((red[0][r] + red[1][r]) + red[2][r]) + red[3][r];
+}
+
+// w = v - N s from the slices
+__global__ void residual_sum(int n, const double* __restrict__ part, const double* __restrict__ v, double* __restrict__ w)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double acc = 0.0;
-    for (int j = 0; j < n; ++j) acc = fma(Nm[(size_t)j * ld + i], sv[j], acc);
+    for (int z = 0; z < kResidualSplit; ++z) acc += part[(size_t)z * n + i];
     w[i] = v[i] - acc;
 }
 
@@ -1074,25 +1055,29 @@ int fp64_build_fiducial(cg_ctx* ctx, int lo, int hi, const double* d_tab, double
 }
 
 int fp64_pol_matrix(cg_ctx* ctx, int n, int ld, const double* d_c_packed, const double* d_ninv, double* d_cd,
-                    double* d_t, double* d_m, double* d_m_packed, cudaStream_t s)
+                    double* d_t, double* d_m, double* d_m_packed, unsigned char* work, int* err, cudaStream_t s)
 {
     const size_t nel = (size_t)ld * ld;
+    const int nt = ld / TS;
     packed_to_dense<<<(unsigned)((nel + kThreads - 1) / kThreads), kThreads, 0, s>>>(n, ld, d_c_packed, d_cd);
-    const dim3 grid(ld / 64, ld / 64);
-    dense_gemm64<<<grid, kThreads, 0, s>>>(ld, d_cd, d_ninv, nullptr, d_t);   // T = C N^-1
-    dense_gemm64<<<grid, kThreads, 0, s>>>(ld, d_ninv, d_t, d_ninv, d_m);     // M = N^-1 + N^-1 T
+    CG_CUDA_TRY(ctx, cudaMemsetAsync(d_t, 0, sizeof(double) * nel, s));
+    dense_to_tiles<<<dim3(nt, nt), kThreads, 0, s>>>(ld, d_ninv, d_m);
+    int rc = digit_gemm(ctx, nt, d_cd, d_ninv, 1, d_t, work, err, s);      // T = C N^-1
+    if (!rc) rc = digit_gemm(ctx, nt, d_ninv, d_t, 2, d_m, work, err, s);  // M = N^-1 + N^-1 T
+    if (rc) return rc;
     const long np = (long)n * (n + 1) / 2;
-    dense_to_packed<<<(unsigned)((np + kThreads - 1) / kThreads), kThreads, 0, s>>>(n, ld, d_m, d_m_packed);
-    count_launch(ctx, 4);
+    tiles_to_packed<<<(unsigned)((np + kThreads - 1) / kThreads), kThreads, 0, s>>>(n, nt, d_m, d_m_packed);
+    count_launch(ctx, 3);
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;
 }
 
 int fp64_dense_residual(cg_ctx* ctx, int n, int ld, const double* d_ninv, const double* d_v, const double* d_s,
-                        double* d_w, cudaStream_t s)
+                        double* d_w, double* part, cudaStream_t s)
 {
-    dense_residual<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, ld, d_ninv, d_v, d_s, d_w);
-    count_launch(ctx);
+    residual_parts<<<dim3((n + TS - 1) / TS, kResidualSplit), kThreads, 0, s>>>(n, ld, d_ninv, d_s, part);
+    residual_sum<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, part, d_v, d_w);
+    count_launch(ctx, 2);
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;
 }

@@ -147,3 +147,34 @@ def test_packed_likelihood_foreground(n):
     assert abs(chi2 - (tt - tf * tf / ff)) <= 3 * tol * tt
     assert abs((ld - cg.DET_OFFSET) - (np.linalg.slogdet(full)[1] + np.log(ff / n))) <= 2 * tol + 8 * EPS * abs(ld)
     lik.close()
+
+
+@pytest.mark.parametrize("npix,ngood", [(1, 1), (40, 32), (40, 33), (100, 64), (100, 65), (600, 544)])
+def test_polarisation_products(npix, ngood):
+    """N^-1 + N^-1 C N^-1 at 2, 64, 66, 128, 130 and 1088 kept values: one pair of blocks, the edges of the next, and
+    more K blocks than are held at once (17 of 64).  A product of n terms is off by at most n eps |A| |B| per
+    entry; chi2 and ln det then carry the factorisation's bar."""
+    rng = np.random.default_rng(npix + ngood)
+    size = 2 * npix
+    a = rng.standard_normal((size, size)) / np.sqrt(size)
+    b = rng.standard_normal((size, size)) / np.sqrt(size)
+    c = a @ a.T + 0.5 * np.eye(size)
+    ninv = b @ b.T + 2.0 * np.eye(size)
+    good = np.sort(rng.permutation(npix)[:ngood]).astype(np.int32)
+    k = np.concatenate([good, npix + good])
+    n = len(k)
+    v, sub = rng.standard_normal(n), 0.3 * rng.standard_normal(n)
+    nk = ninv[np.ix_(k, k)]
+    m = nk + nk @ c[np.ix_(k, k)] @ nk
+    m = (m + m.T) / 2
+    ev = np.linalg.eigvalsh(m)
+    tol = 16 * n * EPS * ev[-1] / ev[0]
+    lik = cg.LikelihoodPolarization(W.full_to_packed(c), npix, good, np.ascontiguousarray(ninv))
+    _, chi2, _ = lik.calculate(v, sub)
+    w = v - nk @ sub
+    # chi2 = w^T cInv w, cInv the inverse of m (the factored matrix)
+    want = w @ np.linalg.solve(m, w)
+    scale = (np.abs(v) + np.abs(nk) @ np.abs(sub)) @ np.abs(np.linalg.solve(m, w))
+    assert abs(lik.logdet_raw - np.linalg.slogdet(m)[1]) <= tol
+    assert abs(chi2 - want) <= tol * max(scale, want)
+    lik.close()
