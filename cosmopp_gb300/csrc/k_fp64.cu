@@ -38,37 +38,53 @@ __device__ __forceinline__ double pair_dot(const double* __restrict__ xyz, int N
     return d;
 }
 
-// sum_{l=2}^{lmax} ((clc_l * P_l) * B_l) * B_l in the reference's order, 4 pairs at once
-__device__ __forceinline__ void cmat_sum4(const double x[4], double out[4], int lmax, const double* sa,
+// sum_{l=2}^{lmax} ((clc_l * P_l) * B_l) * B_l in the reference's order, 4 pairs of NB elements at once;
+// sc[l][NB].  Four of the eight FP64 operations per pair and l are the recurrence's, which the elements share.
+template <int NB>
+__device__ __forceinline__ void cmat_sum4(const double x[4], double (&acc)[NB][4], int lmax, const double* sa,
                                           const double* sb, const double* sc, const double* sbeam)
 {
-    double p0[4], p1[4], acc[4];
+    double p0[4], p1[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) { p0[q] = 1.0; p1[q] = x[q]; acc[q] = 0.0; }
+    for (int q = 0; q < 4; ++q) {
+        p0[q] = 1.0;
+        p1[q] = x[q];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) acc[k][q] = 0.0;
+    }
     for (int l = 2; l <= lmax; ++l) {
-        const double a = sa[l], b = sb[l], c = sc[l], bm = sbeam[l];
+        const double a = sa[l], b = sb[l], bm = sbeam[l];
+        double c[NB];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) c[k] = sc[l * NB + k];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const double p = __dsub_rn(__dmul_rn(__dmul_rn(a, x[q]), p1[q]), __dmul_rn(b, p0[q]));
-            acc[q] = __dadd_rn(acc[q], __dmul_rn(__dmul_rn(__dmul_rn(c, p), bm), bm));
+#pragma unroll
+            for (int k = 0; k < NB; ++k)
+                acc[k][q] = __dadd_rn(acc[k][q], __dmul_rn(__dmul_rn(__dmul_rn(c[k], p), bm), bm));
             p0[q] = p1[q];
             p1[q] = p;
         }
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) out[q] = acc[q];
 }
 
-__device__ __forceinline__ void load_consts(double* sa, double* sb, double* sc, double* sbeam, int lmax,
+// the tables of elements b0 .. b0 + NB - 1 of B: sc[l][NB]
+template <int NB>
+__device__ __forceinline__ void load_consts(double* sa, double* sb, double* sc, double* sbeam, int lmax, int b0, int B,
                                             const double* lega, const double* legb, const double* beam,
-                                            const double* cl_b)
+                                            const double* cl)
 {
     for (int l = threadIdx.x; l <= lmax; l += blockDim.x) {
         sa[l] = lega[l];
         sb[l] = legb[l];
         sbeam[l] = beam[l];
         // clCopy[l] = cl[l] * (2 l + 1) / (4 pi)   (c_matrix_generator.cpp:190-193)
-        sc[l] = (l >= 2) ? __ddiv_rn(__dmul_rn(cl_b[l], (double)(2 * l + 1)), 4.0 * kPi) : 0.0;
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+            sc[l * NB + k] = (l >= 2 && b0 + k < B)
+                                 ? __ddiv_rn(__dmul_rn(cl[(size_t)(b0 + k) * (lmax + 1) + l], (double)(2 * l + 1)), 4.0 * kPi)
+                                 : 0.0;
     }
 }
 
@@ -88,13 +104,13 @@ __global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, 
     double* sc = sb + (lmax + 1);
     double* sbeam = sc + (lmax + 1);
     const int b = blockIdx.y;
-    load_consts(sa, sb, sc, sbeam, lmax, lega, legb, beam, cl + (size_t)b * (lmax + 1));
+    load_consts<1>(sa, sb, sc, sbeam, lmax, b, b + 1, lega, legb, beam, cl);
     __syncthreads();
     int I, J;
     tile_coords(blockIdx.x, I, J);
     double* tile = A + (size_t)b * strideA + (size_t)blockIdx.x * TILE_ELEMS;
     for (int g = 0; g < TILE_ELEMS / (kThreads * 4); ++g) {
-        double x[4], v[4];
+        double x[4], v[1][4];
         int e[4];
         bool real[4];
 #pragma unroll
@@ -104,13 +120,13 @@ __global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, 
             real[q] = (i < n && j < n);
             x[q] = real[q] ? pair_dot(xyz, N, i, j) : 0.0;
         }
-        cmat_sum4(x, v, lmax, sa, sb, sc, sbeam);
+        cmat_sum4<1>(x, v, lmax, sa, sb, sc, sbeam);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int i = I * TS + e[q] % TS, j = J * TS + e[q] / TS;
             double val;
             if (real[q]) {
-                val = v[q];
+                val = v[0][q];
                 // cInv_(i,j) = c + fiducial(0) + noise  (source/likelihood.cpp:102-110)
                 if (add_noise && i == j) val = __dadd_rn(__dadd_rn(val, 0.0), noise[i]);
             } else {
@@ -252,8 +268,10 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
     }
 }
 
-// packed output (i <= j at j(j+1)/2 + i), one thread per entry, grid (ceil(np/256), B)
-__global__ void __launch_bounds__(kThreads) build_c_packed(int n, int N, int lmax, const double* __restrict__ xyz,
+// packed output (i <= j at j(j+1)/2 + i), four entries per thread of NB elements; the reference's operations
+// and rounding; grid (ceil(np / 1024), ceil(B / NB))
+template <int NB>
+__global__ void __launch_bounds__(kThreads) build_c_packed(int n, int N, int lmax, int B, const double* __restrict__ xyz,
                                                            const double* __restrict__ lega,
                                                            const double* __restrict__ legb,
                                                            const double* __restrict__ beam,
@@ -263,9 +281,9 @@ __global__ void __launch_bounds__(kThreads) build_c_packed(int n, int N, int lma
     double* sa = sconst;
     double* sb = sa + (lmax + 1);
     double* sc = sb + (lmax + 1);
-    double* sbeam = sc + (lmax + 1);
-    const int b = blockIdx.y;
-    load_consts(sa, sb, sc, sbeam, lmax, lega, legb, beam, cl + (size_t)b * (lmax + 1));
+    double* sbeam = sc + NB * (lmax + 1);
+    const int b0 = blockIdx.y * NB;
+    load_consts<NB>(sa, sb, sc, sbeam, lmax, b0, B, lega, legb, beam, cl);
     __syncthreads();
     const long np = (long)n * (n + 1) / 2;
     const long k0 = 4 * ((long)blockIdx.x * kThreads + threadIdx.x);
@@ -274,7 +292,7 @@ __global__ void __launch_bounds__(kThreads) build_c_packed(int n, int N, int lma
     while (j * (j + 1) / 2 > k0) --j;
     while ((j + 1) * (j + 2) / 2 <= k0) ++j;
     long i = k0 - j * (j + 1) / 2;
-    double x[4], v[4];
+    double x[4], v[NB][4];
     long kk[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {  // four consecutive packed entries: walk i, wrap to the next column
@@ -282,10 +300,13 @@ __global__ void __launch_bounds__(kThreads) build_c_packed(int n, int N, int lma
         x[q] = (kk[q] < np) ? pair_dot(xyz, N, (int)i, (int)j) : 0.0;
         if (++i > j) { ++j; i = 0; }
     }
-    cmat_sum4(x, v, lmax, sa, sb, sc, sbeam);
+    cmat_sum4<NB>(x, v, lmax, sa, sb, sc, sbeam);
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-        if (kk[q] < np) out[(size_t)b * np + kk[q]] = v[q];
+    for (int k = 0; k < NB; ++k)
+        if (b0 + k < B)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (kk[q] < np) out[(size_t)(b0 + k) * np + kk[q]] = v[k][q];
 }
 
 // CMatrixGenerator::getFiducialMatrix (source/c_matrix_generator.cpp:706-772), packed i <= j:
@@ -1034,8 +1055,17 @@ int fp64_build_tiled_into(cg_ctx* ctx, int B, const double* d_cl, bool add_noise
 int fp64_build_packed(cg_ctx* ctx, int B, const double* d_cl, double* d_out, cudaStream_t s)
 {
     const long np = (long)ctx->n * (ctx->n + 1) / 2;
-    build_c_packed<<<dim3((unsigned)((np + 4 * kThreads - 1) / (4 * kThreads)), B), kThreads, const_smem(ctx->lmax), s>>>(
-        ctx->n, ctx->N, ctx->lmax, ctx->d_xyz, ctx->d_lega, ctx->d_legb, ctx->d_beam, d_cl, d_out);
+    const unsigned gx = (unsigned)((np + 4 * kThreads - 1) / (4 * kThreads));
+    const int L1 = ctx->lmax + 1;
+    // 8 FP64 operations per pair, l and element alone, 6 for two that share the recurrence, 5 for four: the
+    // pipe is the bound (four matrices at nside 16: 8.79 ms alone, 5.5 ms shared)
+    auto run = [&](auto kernel, int nb) {
+        kernel<<<dim3(gx, (B + nb - 1) / nb), kThreads, sizeof(double) * (3 + nb) * L1, s>>>(
+            ctx->n, ctx->N, ctx->lmax, B, ctx->d_xyz, ctx->d_lega, ctx->d_legb, ctx->d_beam, d_cl, d_out);
+    };
+    if (B == 1) run(build_c_packed<1>, 1);
+    else if (B == 2) run(build_c_packed<2>, 2);
+    else run(build_c_packed<4>, 4);
     count_launch(ctx);
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;

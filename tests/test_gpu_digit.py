@@ -178,3 +178,14 @@ def test_polarisation_products(npix, ngood):
     assert abs(lik.logdet_raw - np.linalg.slogdet(m)[1]) <= tol
     assert abs(chi2 - want) <= tol * max(scale, want)
     lik.close()
+
+
+@pytest.mark.parametrize("batch", [1, 2, 3, 4, 5, 9])
+def test_packed_covariances_of_a_batch_are_those_of_each(batch):
+    """Elements that share the recurrence (two or four at a time, and what is left over) keep the bits of a call
+    of their own."""
+    v, cls, _ = _setup(70, 11, 3, batch)
+    with cg.Context(lmax=11, fwhm_deg=9.0, dirs=v, max_batch=batch) as ctx:
+        full = ctx.build_cmatrix(cls)
+        for b in range(batch):
+            assert np.array_equal(full[b], ctx.build_cmatrix(cls[b]))
