@@ -676,7 +676,7 @@ struct cg_lik {
     int* st = nullptr;
     double logdet = 0;
     std::vector<double> fg;
-    double* Ninv = nullptr;      // polarisation likelihood: dense N^-1 (ld x ld, column-major)
+    double* Ninv = nullptr;      // polarisation likelihood: dense N^-1 (ld x ld, row-major)
     int ld = 0;
 };
 
@@ -695,13 +695,10 @@ extern "C" void cg_likelihood_destroy(cg_lik* lik)
 extern "C" const char* cg_likelihood_last_error(const cg_lik* lik) { return lik ? lik->ctx.err.c_str() : g_create_error.c_str(); }
 extern "C" double cg_likelihood_logdet(const cg_lik* lik) { return lik ? lik->logdet : 0.0; }
 
-extern "C" int cg_likelihood_create(cg_lik** out, int n, const double* c_packed, const double* fid_packed,
-                                    const double* noise_packed, const double* foreground, int device)
+// a new cg_lik for n pixels: sizes and stream
+static int lik_new(std::unique_ptr<cg_lik>& lik, int n, int device)
 {
-    g_create_error.clear();
-    if (!out || n <= 0 || !c_packed || !noise_packed) { g_create_error = "bad arguments to cg_likelihood_create"; return CG_ERR_BAD_ARG; }
-    *out = nullptr;
-    std::unique_ptr<cg_lik> lik(new (std::nothrow) cg_lik());
+    lik.reset(new (std::nothrow) cg_lik());
     if (!lik) return CG_ERR_ALLOC;
     cg_ctx& ctx = lik->ctx;
     std::string why;
@@ -712,45 +709,46 @@ extern "C" int cg_likelihood_create(cg_lik** out, int n, const double* c_packed,
     ctx.N = ctx.nt * cg::TS;
     cudaSetDevice(device);
     if (cudaStreamCreateWithFlags(&ctx.stream, cudaStreamNonBlocking) != cudaSuccess) { g_create_error = "stream"; return CG_ERR_CUDA; }
-    const size_t np = (size_t)n * (n + 1) / 2, tiled = cg::tiled_elems(ctx.nt);
-    double *dpk = nullptr, *M = nullptr;
-    unsigned char* work = nullptr;
-    // the factorisation's scratch (M = L^-1 and the digit images) is given back when it is done
-    auto free_scratch = [&] { cudaFree(dpk); cudaFree(M); cudaFree(work); };
-    if (!dalloc(&lik->A, tiled) || !dalloc(&M, tiled) || !dalloc(&work, cg::digit_bytes(ctx.nt, ctx.nt)) ||
-        !dalloc(&lik->diag, (size_t)ctx.N) || !dalloc(&lik->tmp, 4 * (size_t)ctx.N + 8 + std::max(3 * (size_t)cg::ntiles_lower(ctx.nt), (size_t)cg::kResidualSplit * ctx.N)) || !dalloc(&lik->st, 2) ||
-        !dalloc(&dpk, 3 * np)) {
-        free_scratch();
-        g_create_error = "device allocation failed";
-        cg_likelihood_destroy(lik.release());
-        return CG_ERR_ALLOC;
-    }
-    for (size_t k = 0; k < np; ++k)
-        if (!std::isfinite(c_packed[k]) || !std::isfinite(noise_packed[k]) || (fid_packed && !std::isfinite(fid_packed[k]))) {
-            free_scratch();
-            g_create_error = "non-finite matrix entry";
-            cg_likelihood_destroy(lik.release());
-            return CG_ERR_NONFINITE;
-        }
+    return CG_OK;
+}
+
+// its ln det and inverse from the packed matrices c + f + nz on the device (f, nz nullable); on an error lik is
+// destroyed
+static int lik_factor(std::unique_ptr<cg_lik>& lik, const double* c, const double* f, const double* nz)
+{
+    cg_ctx& ctx = lik->ctx;
+    const size_t tiled = cg::tiled_elems(ctx.nt), N = ctx.N;
     cudaStream_t s = ctx.stream;
-    cudaMemcpyAsync(dpk, c_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
-    if (fid_packed) cudaMemcpyAsync(dpk + np, fid_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(dpk + 2 * np, noise_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
-    cudaMemsetAsync(lik->st, 0, 2 * sizeof(int), s);
-    cg::fp64_packed_to_tiled(n, ctx.nt, dpk, fid_packed ? dpk + np : nullptr, dpk + 2 * np, lik->A, s);
-    int rc = cg::fp64_identity_rows(&ctx, 1, ctx.nt, M, tiled, s);
+    double* M = nullptr;
+    unsigned char* work = nullptr;
+    int rc = CG_OK, st[3] = {0, 0, 0};
+    if (!dalloc(&lik->A, tiled) || !dalloc(&M, tiled) || !dalloc(&work, cg::digit_bytes(ctx.nt, ctx.nt)) ||
+        !dalloc(&lik->diag, N) || !dalloc(&lik->tmp, 4 * N + 8 + 3 * (size_t)cg::ntiles_lower(ctx.nt)) || !dalloc(&lik->st, 3)) {
+        ctx.err = "device allocation failed";
+        rc = CG_ERR_ALLOC;
+    }
+    if (!rc) {
+        cudaMemsetAsync(lik->st, 0, 3 * sizeof(int), s);
+        cg::fp64_packed_to_tiled(ctx.n, ctx.nt, c, f, nz, lik->A, lik->st + 2, s);
+        rc = cg::fp64_identity_rows(&ctx, 1, ctx.nt, M, tiled, s);
+    }
     if (!rc)
         rc = cg::digit_factor(&ctx, 1, ctx.nt, ctx.nt, cg::DIGIT_EXT_IDENTITY, lik->A, tiled, M, tiled, lik->diag,
                               lik->st, work, lik->st + 1, s);
-    if (!rc) cg::fp64_logdet(1, n, ctx.N, lik->diag, lik->tmp + 4 * (size_t)ctx.N, s);
-    int st[2] = {0, 0};
     if (!rc) {
-        cudaMemcpyAsync(&lik->logdet, lik->tmp + 4 * (size_t)ctx.N, sizeof(double), cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(st, lik->st, 2 * sizeof(int), cudaMemcpyDeviceToHost, s);
-        cudaError_t e = cudaStreamSynchronize(s);
+        cg::fp64_logdet(1, ctx.n, ctx.N, lik->diag, lik->tmp + 4 * N, s);
+        cudaMemcpyAsync(&lik->logdet, lik->tmp + 4 * N, sizeof(double), cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(st, lik->st, 3 * sizeof(int), cudaMemcpyDeviceToHost, s);
+        const cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) { ctx.err = cudaGetErrorString(e); rc = CG_ERR_CUDA; }
     }
-    free_scratch();
+    // the factorisation's scratch (M = L^-1 and the digit images) is given back when it is done
+    cudaFree(M);
+    cudaFree(work);
+    if (!rc && st[2]) {
+        ctx.err = "non-finite matrix entry";
+        rc = CG_ERR_NONFINITE;
+    }
     if (!rc && st[1]) {
         ctx.err = "a device wait gave up";
         rc = CG_ERR_TIMEOUT;
@@ -763,8 +761,33 @@ extern "C" int cg_likelihood_create(cg_lik** out, int n, const double* c_packed,
     if (rc) {
         g_create_error = ctx.err;
         cg_likelihood_destroy(lik.release());
-        return rc;
     }
+    return rc;
+}
+
+extern "C" int cg_likelihood_create(cg_lik** out, int n, const double* c_packed, const double* fid_packed,
+                                    const double* noise_packed, const double* foreground, int device)
+{
+    g_create_error.clear();
+    if (!out || n <= 0 || !c_packed || !noise_packed) { g_create_error = "bad arguments to cg_likelihood_create"; return CG_ERR_BAD_ARG; }
+    *out = nullptr;
+    std::unique_ptr<cg_lik> lik;
+    int rc = lik_new(lik, n, device);
+    if (rc) return rc;
+    const size_t np = (size_t)n * (n + 1) / 2;
+    cudaStream_t s = lik->ctx.stream;
+    double* dpk = nullptr;
+    if (!dalloc(&dpk, (fid_packed ? 3 : 2) * np)) {
+        g_create_error = "device allocation failed";
+        cg_likelihood_destroy(lik.release());
+        return CG_ERR_ALLOC;
+    }
+    cudaMemcpyAsync(dpk, c_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(dpk + np, noise_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
+    if (fid_packed) cudaMemcpyAsync(dpk + 2 * np, fid_packed, sizeof(double) * np, cudaMemcpyHostToDevice, s);
+    rc = lik_factor(lik, dpk, fid_packed ? dpk + 2 * np : nullptr, dpk + np);
+    cudaFree(dpk);
+    if (rc) return rc;
     if (foreground) lik->fg.assign(foreground, foreground + n);
     *out = lik.release();
     return CG_OK;
@@ -823,65 +846,73 @@ extern "C" int cg_likelihood_pol_create(cg_lik** out, int npix, const int* good,
     *out = nullptr;
     for (int i = 0; i < ngood; ++i)
         if (good[i] < 0 || good[i] >= npix) { g_create_error = "good pixel index out of range"; return CG_ERR_BAD_ARG; }
-    // source/likelihood.cpp:371-384: the Q and U rows and columns of the kept pixels
+    // source/likelihood.cpp:371-384: the Q and U rows and columns of the kept pixels; N^-1 row by row.  A
+    // non-finite value makes the sum of zeros NaN.
     const int n = 2 * ngood, size = 2 * npix, ld = (n + 127) / 128 * 128;
-    auto full = [&](int k) { return k < ngood ? good[k] : npix + good[k - ngood]; };
-    const size_t np = (size_t)n * (n + 1) / 2;
-    std::vector<double> cg_packed(np), nd((size_t)ld * ld, 0.0);
+    const size_t np = (size_t)n * (n + 1) / 2, nel = (size_t)ld * ld;
+    std::vector<int> full(n);
+    for (int k = 0; k < n; ++k) full[k] = k < ngood ? good[k] : npix + good[k - ngood];
+    std::unique_ptr<double[]> cp(new (std::nothrow) double[np]), nd(new (std::nothrow) double[(size_t)n * n]);
+    if (!cp || !nd) { g_create_error = "out of host memory"; return CG_ERR_ALLOC; }
+    double zero[4] = {0, 0, 0, 0};
     for (int j = 0; j < n; ++j) {
-        const long fj = full(j);
+        const long fj = full[j];
+        double* row = cp.get() + (size_t)j * (j + 1) / 2;
         for (int i = 0; i <= j; ++i) {
-            const long fi = full(i), a = std::min(fi, fj), b = std::max(fi, fj);
-            cg_packed[(size_t)j * (j + 1) / 2 + i] = c_packed[(size_t)b * (b + 1) / 2 + a];
+            const long fi = full[i], a = std::min(fi, fj), b = std::max(fi, fj);
+            row[i] = c_packed[(size_t)b * (b + 1) / 2 + a];
+            zero[i & 3] += row[i] * 0.0;
         }
-        for (int i = 0; i < n; ++i) nd[(size_t)j * ld + i] = ninv[(size_t)full(i) * size + fj];
+        const double* src = ninv + (size_t)fj * size;
+        row = nd.get() + (size_t)j * n;
+        for (int i = 0; i < n; ++i) {
+            row[i] = src[full[i]];
+            zero[i & 3] += row[i] * 0.0;
+        }
     }
-    for (double v : cg_packed)
-        if (!std::isfinite(v)) { g_create_error = "non-finite matrix entry"; return CG_ERR_NONFINITE; }
-    for (double v : nd)
-        if (!std::isfinite(v)) { g_create_error = "non-finite matrix entry"; return CG_ERR_NONFINITE; }
-    cg_ctx tmpctx;
-    std::string why;
-    if (!device_ok(device, &tmpctx.sm_count, why)) { g_create_error = why; return CG_ERR_NO_DEVICE; }
-    tmpctx.device = device;
-    cudaSetDevice(device);
-    cudaStream_t s = nullptr;
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) { g_create_error = "stream"; return CG_ERR_CUDA; }
-    const size_t nel = (size_t)ld * ld;
-    double *d_c = nullptr, *d_n = nullptr, *d_cd = nullptr, *d_t = nullptr, *d_m = nullptr, *d_mp = nullptr;
+    if (!(zero[0] + zero[1] + zero[2] + zero[3] == 0.0)) { g_create_error = "non-finite matrix entry"; return CG_ERR_NONFINITE; }
+    std::unique_ptr<cg_lik> lik;
+    int rc = lik_new(lik, n, device), err = 0;
+    if (rc) return rc;
+    cg_ctx& ctx = lik->ctx;
+    cudaStream_t s = ctx.stream;
+    double *d_c = nullptr, *d_n = nullptr, *d_cd = nullptr, *d_t = nullptr, *d_m = nullptr;
     unsigned char* work = nullptr;
-    int *d_err = nullptr, err = 0;
-    int rc = CG_OK;
-    if (!dalloc(&work, cg::digit_gemm_bytes(ld / cg::TS)) || !dalloc(&d_err, 1) || !dalloc(&d_c, np) || !dalloc(&d_n, nel) || !dalloc(&d_cd, nel) || !dalloc(&d_t, nel) || !dalloc(&d_m, nel) ||
-        !dalloc(&d_mp, np)) {
-        g_create_error = "device allocation failed";
+    int* d_err = nullptr;
+    if (!dalloc(&d_c, np) || !dalloc(&d_n, nel) || !dalloc(&d_cd, nel) || !dalloc(&d_t, nel) || !dalloc(&d_m, nel) ||
+        !dalloc(&work, cg::digit_gemm_bytes(ld / cg::TS)) || !dalloc(&d_err, 1)) {
+        ctx.err = "device allocation failed";
         rc = CG_ERR_ALLOC;
     }
-    std::vector<double> m_packed(np), zero(np, 0.0);
-    if (rc == CG_OK) {
-        cudaMemcpyAsync(d_c, cg_packed.data(), sizeof(double) * np, cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(d_n, nd.data(), sizeof(double) * nel, cudaMemcpyHostToDevice, s);
-        // source/likelihood.cpp:386-387: cInv = N^-1 + N^-1 C N^-1
+    if (!rc) {
         cudaMemsetAsync(d_err, 0, sizeof(int), s);
-        rc = cg::fp64_pol_matrix(&tmpctx, n, ld, d_c, d_n, d_cd, d_t, d_m, d_mp, work, d_err, s);
-        if (rc == CG_OK) {
-            cudaMemcpyAsync(m_packed.data(), d_mp, sizeof(double) * np, cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
-            if (cudaStreamSynchronize(s) != cudaSuccess) { g_create_error = "polarisation matrix build failed"; rc = CG_ERR_CUDA; }
-            else if (err) { g_create_error = "a device wait gave up"; rc = CG_ERR_TIMEOUT; }
-        } else {
-            g_create_error = tmpctx.err;
-        }
+        cudaMemsetAsync(d_n, 0, sizeof(double) * nel, s);
+        cudaMemcpyAsync(d_c, cp.get(), sizeof(double) * np, cudaMemcpyHostToDevice, s);
+        cudaMemcpy2DAsync(d_n, sizeof(double) * ld, nd.get(), sizeof(double) * n, sizeof(double) * n, n,
+                          cudaMemcpyHostToDevice, s);
+        // source/likelihood.cpp:386-387: cInv = N^-1 + N^-1 C N^-1, packed over C
+        rc = cg::fp64_pol_matrix(&ctx, n, ld, d_c, d_n, d_cd, d_t, d_m, d_c, work, d_err, s);
     }
-    cudaFree(d_c); cudaFree(d_cd); cudaFree(d_t); cudaFree(d_m); cudaFree(d_mp); cudaFree(work); cudaFree(d_err);
-    cudaStreamDestroy(s);
-    if (rc == CG_OK) rc = cg_likelihood_create(out, n, m_packed.data(), nullptr, zero.data(), nullptr, device);
-    if (rc != CG_OK) {
+    if (!rc) {
+        cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (cudaStreamSynchronize(s) != cudaSuccess) { ctx.err = "polarisation matrix build failed"; rc = CG_ERR_CUDA; }
+        else if (err) { ctx.err = "a device wait gave up"; rc = CG_ERR_TIMEOUT; }
+    }
+    cudaFree(d_cd); cudaFree(d_t); cudaFree(d_m); cudaFree(work); cudaFree(d_err);
+    if (rc) {
+        g_create_error = ctx.err;
+        cg_likelihood_destroy(lik.release());
+    } else {
+        rc = lik_factor(lik, d_c, nullptr, nullptr);
+    }
+    cudaFree(d_c);
+    if (rc) {
         cudaFree(d_n);
         return rc;
     }
-    (*out)->Ninv = d_n;
-    (*out)->ld = ld;
+    lik->Ninv = d_n;
+    lik->ld = ld;
+    *out = lik.release();
     return CG_OK;
 }
 
@@ -903,7 +934,7 @@ extern "C" int cg_likelihood_pol_calculate(cg_lik* lik, const double* v, const d
     cudaMemcpyAsync(vv, v, sizeof(double) * n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(sv, subtract, sizeof(double) * n, cudaMemcpyHostToDevice, s);
     // source/likelihood.cpp:595-600: vCopy -= N^-1 subtractMap
-    int rc = cg::fp64_dense_residual(&ctx, n, lik->ld, lik->Ninv, vv, sv, w, sv + 2 * (size_t)N + 8, s);
+    int rc = cg::fp64_dense_residual(&ctx, n, lik->ld, lik->Ninv, vv, sv, w, s);
     if (rc) return rc;
     cudaMemsetAsync(vv, 0, sizeof(double) * 2 * N, s);
     return lik_finish(lik, chi2, logdet);   // chi2 = w^T cInv w (source/likelihood.cpp:602-609)

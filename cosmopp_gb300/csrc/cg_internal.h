@@ -238,15 +238,14 @@ int ylm_fill(cg_ctx* ctx, double* Y, cudaStream_t s);
 void mixed_bytes(const cg_ctx* ctx, size_t* fixed, size_t* per_element);
 int fp64_build_tiled_into(cg_ctx* ctx, int B, const double* d_cl, bool add_noise, double* A, cudaStream_t s);
 int fp64_build_packed(cg_ctx* ctx, int B, const double* d_cl, double* d_out, cudaStream_t s);
-// polarisation likelihood set-up: M = N^-1 + N^-1 C N^-1 for packed C and dense N^-1 (ld x ld, column-major,
-// zero padded, ld a multiple of 128), packed into d_m_packed; d_cd, d_t, d_m are ld x ld scratch, work
-// digit_gemm_bytes(ld / 64), *err set if a bounded wait gives up
+// polarisation likelihood set-up: M = N^-1 + N^-1 C N^-1 for packed C and dense N^-1 (ld x ld, row-major, zero
+// padded, ld a multiple of 128), packed into d_m_packed (which may be C); d_cd, d_t, d_m are ld x ld scratch,
+// work digit_gemm_bytes(ld / 64), *err set if a bounded wait gives up
 int fp64_pol_matrix(cg_ctx* ctx, int n, int ld, const double* d_c_packed, const double* d_ninv, double* d_cd,
                     double* d_t, double* d_m, double* d_m_packed, unsigned char* work, int* err, cudaStream_t s);
-// w = v - N^-1 s for the dense N^-1 above; part: kResidualSplit n doubles
-constexpr int kResidualSplit = 8;
+// w = v - N^-1 s for the dense N^-1 above
 int fp64_dense_residual(cg_ctx* ctx, int n, int ld, const double* d_ninv, const double* d_v, const double* d_s,
-                        double* d_w, double* part, cudaStream_t s);
+                        double* d_w, cudaStream_t s);
 // P_l(x_ij) for l0 <= l < l1 into d_out [(l1 - l0)][n(n+1)/2]; d_a, d_b = the recurrence
 // coefficients, at least l1 entries each (device pointers)
 int fp64_legendre_table(cg_ctx* ctx, int l0, int l1, const double* d_a, const double* d_b, double* d_out,
@@ -269,11 +268,11 @@ size_t digit_bytes(int nt, int ne);
 void digit_free(cg_ctx* ctx);  // the context's second stream and its events
 int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t strideA, double* E,
                  size_t strideE, double* diag, int* status, unsigned char* work, int* err, cudaStream_t s);
-// out += A B for dense square matrices of nt (even) 64-blocks, the same digit products: A column-major; B
-// column-major (kindB = 1) or in out's layout (kindB = 2); out in tiles, (I, J) at I nt + J, element (r, c) at
+// out += A B for dense square matrices of nt (even) 64-blocks, the same digit products: A and B row-major, B in
+// out's layout with tilesB; out in tiles, (I, J) at I nt + J, element (r, c) at
 // r + 64 c.  work: digit_gemm_bytes(nt)
 size_t digit_gemm_bytes(int nt);
-int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* B, int kindB, double* out, unsigned char* work,
+int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* B, bool tilesB, double* out, unsigned char* work,
                int* err, cudaStream_t s);
 // generic tiled FP64 / FP32 factorisation entry points (k_chol.cu)
 template <typename T>
@@ -336,7 +335,9 @@ void fp64_free(cg_ctx* ctx);
 // small FP64 launchers used by the Likelihood drop-in (k_fp64.cu)
 // E = identity of DIGIT_EXT_IDENTITY (lower tiles of the batch)
 int fp64_identity_rows(cg_ctx* ctx, int B, int nt, double* E, size_t strideE, cudaStream_t s);
-void fp64_packed_to_tiled(int n, int nt, const double* c, const double* f, const double* nz, double* A, cudaStream_t s);
+// f, nz nullable; *bad (nullable) is set by a non-finite entry
+void fp64_packed_to_tiled(int n, int nt, const double* c, const double* f, const double* nz, double* A, int* bad,
+                          cudaStream_t s);
 void fp64_symv(int B, int nt, int N, const double* V, const double* dv, double* alpha, cudaStream_t s);
 // out[0] = t^T V t and, with f, out[1] = t^T V f, out[2] = f^T V f for V in lower tiles; part: 3 per tile
 void fp64_quad(int nt, const double* V, const double* tv, const double* fv, double* part, double* out, cudaStream_t s);

@@ -961,7 +961,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
 }
 
 // Images of a dense operand's row pairs for K blocks k0, k0 + 1, ..: grid (row pairs, K blocks).  Element
-// (row, k): kind 0 at k ld + row, kind 1 at row ld + k, kind 2 in 64 x 64 tiles (k / 64, row / 64) of nt to a
+// (row, k): kind 0 at k ld + row (B of a product, row-major), kind 1 at row ld + k (A), kind 2 in 64 x 64 tiles (k / 64, row / 64) of nt to a
 // row, element (r, c) at r + 64 c.  Thread (row, 16 columns), as in the panel.
 __global__ void __launch_bounds__(kPanelThreads) digit_slice(int kind, int ld, int k0, int first, const double* __restrict__ src, Dig g)
 {
@@ -1159,7 +1159,7 @@ static int gemm_chunk(int nt) { return std::min(nt, 16); }
 
 size_t digit_gemm_bytes(int nt) { return (size_t)gemm_chunk(nt) * nt * (kImg + 128 * sizeof(int)); }
 
-int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, int kindB, double* out, unsigned char* work,
+int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, bool tilesB, double* out, unsigned char* work,
                int* err, cudaStream_t s)
 {
     const int nq = nt / 2, chunk = gemm_chunk(nt), ld = nt * TS;
@@ -1177,8 +1177,8 @@ int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, int kindB
     const int per = up_jobs(u, nq);
     for (int k0 = 0; k0 < nt; k0 += chunk) {
         g.nk = std::min(chunk, nt - k0);
-        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(kindB, ld, k0, 0, Bm, g);
-        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(0, ld, k0, nq, A, g);
+        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(tilesB ? 2 : 0, ld, k0, 0, Bm, g);
+        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(1, ld, k0, nq, A, g);
         digit_update<true><<<std::min(per, ctx->sm_count), kUpThreads, kUpSmem, s>>>(-1, per, per, u, g);
         count_launch(ctx, 3);
     }

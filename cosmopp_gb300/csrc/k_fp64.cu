@@ -528,23 +528,28 @@ __global__ void copy_status(int B, const int* __restrict__ src, const int* __res
 // in the reference's summation order (source/likelihood.cpp:102-110); grid tiles
 __global__ void __launch_bounds__(kThreads) packed_sum_to_tiled(int n, const double* __restrict__ c,
                                                                 const double* __restrict__ f,
-                                                                const double* __restrict__ nz, double* __restrict__ A)
+                                                                const double* __restrict__ nz, double* __restrict__ A,
+                                                                int* __restrict__ bad)
 {
     int I, J;
     tile_coords(blockIdx.x, I, J);
     double* tile = A + (size_t)blockIdx.x * TILE_ELEMS;
+    bool nonfinite = false;
     for (int e = threadIdx.x; e < TILE_ELEMS; e += kThreads) {
         const int i = I * TS + e % TS, j = J * TS + e / TS;
         double v;
         if (i < n && j < n) {
             const int lo = i < j ? i : j, hi = i < j ? j : i;
             const size_t k = (size_t)hi * (hi + 1) / 2 + lo;
-            v = __dadd_rn(__dadd_rn(c[k], f ? f[k] : 0.0), nz[k]);
+            const double ck = c[k], fk = f ? f[k] : 0.0, nk = nz ? nz[k] : 0.0;
+            nonfinite |= !(isfinite(ck) && isfinite(fk) && isfinite(nk));
+            v = __dadd_rn(__dadd_rn(ck, fk), nk);
         } else {
             v = (i == j) ? 1.0 : 0.0;
         }
         tile[e] = v;
     }
+    if (nonfinite && bad) *bad = 1;
 }
 
 __global__ void dot_kernel(int n, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out)
@@ -616,16 +621,16 @@ __global__ void __launch_bounds__(kThreads) quad_sum(int ntile, const double* __
     if (threadIdx.x == 0) out[blockIdx.x] = red[0];
 }
 
-// Dense FP64 helpers of the polarisation likelihood's set-up (column-major, leading dimension
+// Dense FP64 helpers of the polarisation likelihood's set-up (row-major, leading dimension
 // ld, a multiple of 128, zero padding beyond n; the products run in k_digit.cu on 64 x 64 tiles).
 
-// column-major to tiles (I, J) at I nt + J, element (r, c) at r + 64 c; grid (nt, nt)
+// row-major to tiles (I, J) at I nt + J, element (r, c) at r + 64 c; grid (nt, nt)
 __global__ void __launch_bounds__(kThreads) dense_to_tiles(int ld, const double* __restrict__ d, double* __restrict__ t)
 {
     const int I = blockIdx.x, J = blockIdx.y, nt = ld / TS;
     double* tile = t + ((size_t)I * nt + J) * TILE_ELEMS;
     for (int e = threadIdx.x; e < TILE_ELEMS; e += kThreads)
-        tile[e] = d[(size_t)(J * TS + e / TS) * ld + I * TS + e % TS];
+        tile[e % TS * TS + e / TS] = d[(size_t)(I * TS + e / TS) * ld + J * TS + e % TS];
 }
 
 // packed symmetric (i <= j at j(j+1)/2 + i) to dense, zero outside n x n; grid covers ld x ld
@@ -651,31 +656,18 @@ __global__ void tiles_to_packed(int n, int nt, const double* __restrict__ t, dou
     pk[k] = t[((size_t)(i / TS) * nt + j / TS) * TILE_ELEMS + i % TS + TS * (j % TS)];
 }
 
-// part[z][i] = sum of N_ij s_j over the columns of slice z, four partial sums per row; one CTA per 64 rows and
-// slice (one thread per row and all columns left five CTAs to do it, 287 us at 1228 rows);
-// grid (ceil(n / 64), kResidualSplit)
-__global__ void __launch_bounds__(kThreads) residual_parts(int n, int ld, const double* __restrict__ Nm,
-                                                           const double* __restrict__ sv, double* __restrict__ part)
+// w = v - N s, a warp per row: 32 partial sums over its columns, then a tree (one thread per row left five CTAs
+// to do it, 287 us at 1228 rows)
+__global__ void __launch_bounds__(kThreads) dense_residual(int n, int ld, const double* __restrict__ Nm,
+                                                           const double* __restrict__ v, const double* __restrict__ sv,
+                                                           double* __restrict__ w)
 {
-    __shared__ double red[4][TS];
-    const int r = threadIdx.x % TS, q = threadIdx.x / TS, i = blockIdx.x * TS + r;
-    const int len = (n + kResidualSplit - 1) / kResidualSplit, j0 = blockIdx.y * len, j1 = min(n, j0 + len);
-    double acc = 0.0;
-    if (i < n)
-        for (int j = j0 + q; j < j1; j += 4) acc = fma(Nm[(size_t)j * ld + i], sv[j], acc);
-    red[q][r] = acc;
-    __syncthreads();
-    if (q == 0 && i < n) part[(size_t)blockIdx.y * n + i] = ((red[0][r] + red[1][r]) + red[2][r]) + red[3][r];
-}
-
-// w = v - N s from the slices
-__global__ void residual_sum(int n, const double* __restrict__ part, const double* __restrict__ v, double* __restrict__ w)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * (kThreads / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
     if (i >= n) return;
     double acc = 0.0;
-    for (int z = 0; z < kResidualSplit; ++z) acc += part[(size_t)z * n + i];
-    w[i] = v[i] - acc;
+    for (int j = lane; j < n; j += 32) acc = fma(Nm[(size_t)i * ld + j], sv[j], acc);
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) w[i] = v[i] - acc;
 }
 
 // LegendrePolynomialContainer's table (source/c_matrix_generator.cpp:30-76): P_l(x_ij) for
@@ -902,9 +894,10 @@ __global__ void __launch_bounds__(kThreads) harmonic_grad(int lmax, int ne, cons
 
 }  // namespace
 
-void fp64_packed_to_tiled(int n, int nt, const double* c, const double* f, const double* nz, double* A, cudaStream_t s)
+void fp64_packed_to_tiled(int n, int nt, const double* c, const double* f, const double* nz, double* A, int* bad,
+                          cudaStream_t s)
 {
-    packed_sum_to_tiled<<<ntiles_lower(nt), kThreads, 0, s>>>(n, c, f, nz, A);
+    packed_sum_to_tiled<<<ntiles_lower(nt), kThreads, 0, s>>>(n, c, f, nz, A, bad);
 }
 
 void fp64_symv(int B, int nt, int N, const double* V, const double* dv, double* alpha, cudaStream_t s)
@@ -1092,8 +1085,8 @@ int fp64_pol_matrix(cg_ctx* ctx, int n, int ld, const double* d_c_packed, const 
     packed_to_dense<<<(unsigned)((nel + kThreads - 1) / kThreads), kThreads, 0, s>>>(n, ld, d_c_packed, d_cd);
     CG_CUDA_TRY(ctx, cudaMemsetAsync(d_t, 0, sizeof(double) * nel, s));
     dense_to_tiles<<<dim3(nt, nt), kThreads, 0, s>>>(ld, d_ninv, d_m);
-    int rc = digit_gemm(ctx, nt, d_cd, d_ninv, 1, d_t, work, err, s);      // T = C N^-1
-    if (!rc) rc = digit_gemm(ctx, nt, d_ninv, d_t, 2, d_m, work, err, s);  // M = N^-1 + N^-1 T
+    int rc = digit_gemm(ctx, nt, d_cd, d_ninv, false, d_t, work, err, s);      // T = C N^-1
+    if (!rc) rc = digit_gemm(ctx, nt, d_ninv, d_t, true, d_m, work, err, s);  // M = N^-1 + N^-1 T
     if (rc) return rc;
     const long np = (long)n * (n + 1) / 2;
     tiles_to_packed<<<(unsigned)((np + kThreads - 1) / kThreads), kThreads, 0, s>>>(n, nt, d_m, d_m_packed);
@@ -1103,11 +1096,10 @@ int fp64_pol_matrix(cg_ctx* ctx, int n, int ld, const double* d_c_packed, const 
 }
 
 int fp64_dense_residual(cg_ctx* ctx, int n, int ld, const double* d_ninv, const double* d_v, const double* d_s,
-                        double* d_w, double* part, cudaStream_t s)
+                        double* d_w, cudaStream_t s)
 {
-    residual_parts<<<dim3((n + TS - 1) / TS, kResidualSplit), kThreads, 0, s>>>(n, ld, d_ninv, d_s, part);
-    residual_sum<<<(n + kThreads - 1) / kThreads, kThreads, 0, s>>>(n, part, d_v, d_w);
-    count_launch(ctx, 2);
+    dense_residual<<<(n + 7) / 8, kThreads, 0, s>>>(n, ld, d_ninv, d_v, d_s, d_w);
+    count_launch(ctx);
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;
 }

@@ -128,7 +128,7 @@ extern "C" int cg_likelihood_noalloc(int n, const double* d_c_packed, const doub
         cg::set_global_error("cg_likelihood_noalloc: cudaMemsetAsync / cudaMemcpyAsync failed");
         return CG_ERR_CUDA;
     }
-    cg::fp64_packed_to_tiled(n, ctx.nt, d_c_packed, d_fid_packed, d_noise_packed, A, s);
+    cg::fp64_packed_to_tiled(n, ctx.nt, d_c_packed, d_fid_packed, d_noise_packed, A, nullptr, s);
     rc = cg::tiled_cholesky<double>(&ctx, 1, ctx.nt, A, Dinv, diag, st, tiled, s);
     if (!rc) {
         cg::fp64_logdet(1, n, ctx.N, diag, sc, s);

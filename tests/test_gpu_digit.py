@@ -189,3 +189,31 @@ def test_packed_covariances_of_a_batch_are_those_of_each(batch):
         full = ctx.build_cmatrix(cls)
         for b in range(batch):
             assert np.array_equal(full[b], ctx.build_cmatrix(cls[b]))
+
+
+@pytest.mark.parametrize("which", ["c", "fid", "noise"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_nonfinite_packed_matrices_are_refused(which, bad):
+    n = 130
+    eye = W.full_to_packed(np.eye(n))
+    m = dict(c=eye.copy(), fid=0.0 * eye, noise=eye.copy())
+    m[which][len(eye) // 3] = bad
+    with pytest.raises(cg.CGError) as e:
+        cg.Likelihood(m["c"], m["fid"], m["noise"])
+    assert e.value.code == cg.CG_ERR_NONFINITE
+
+
+@pytest.mark.parametrize("pixel,refused", [(3, True), (4, False)])
+def test_nonfinite_polarisation_entries_count_where_they_are_kept(pixel, refused):
+    npix, good = 40, np.array([1, 3, 7, 39], dtype=np.int32)
+    c, ninv = np.eye(2 * npix), 2.0 * np.eye(2 * npix)
+    for k, m in enumerate((c, ninv)):
+        bad = [c.copy(), ninv.copy()]
+        bad[k][pixel, pixel] = np.nan
+        args = (W.full_to_packed(bad[0]), npix, good, bad[1])
+        if refused:
+            with pytest.raises(cg.CGError) as e:
+                cg.LikelihoodPolarization(*args)
+            assert e.value.code == cg.CG_ERR_NONFINITE
+        else:
+            cg.LikelihoodPolarization(*args).close()
