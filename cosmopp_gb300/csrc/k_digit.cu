@@ -156,7 +156,7 @@ __device__ __forceinline__ double* ext_tile(const Dig& g, int b, int eb, int k)
 //
 // The FP64 pipe takes a warp instruction every 64 cycles and SM partition, whatever its active lanes
 // (a lone rsqrt is 456 cycles), so the 64 dependent pivots and the 44 k FMAs of a 64 x 64 factorisation
-// in FP64 took 83 us with the inverse; this takes 44 (alone) or 47 us.  CTA 0 factors the block in integers instead: row r is scaled
+// in FP64 took 83 us with the inverse; this takes 37 us, 29 of them the chain of pivots.  CTA 0 factors the block in integers instead: row r is scaled
 // by 2^-e_r, 2^(2 e_r) above S_rr, so that |S| and |L| are at most 1, held as 2^58 times their
 // value.  A product sum is three 32 x 32 -> 64 multiply-adds (64 per cycle) on L = h 2^29 + l: h h'
 // and h l' + l h', l l' (below 2^-56 of a product) left out; the sums cannot overflow, since rows of L
@@ -165,10 +165,12 @@ __device__ __forceinline__ double* ext_tile(const Dig& g, int b, int eb, int k)
 //
 // Within CTA 0 one warp factors the 4 x 4 diagonal block of a panel of four columns (the chain of pivots),
 // two warps follow it with the panel's 64 rows, and sixteen warps hold the entries' sums and update
-// them, the next panel's columns first, while those go on.  The other CTAs of the cluster form 8 to 24
-// columns each of the inverse in FP64 as the factor's columns arrive in their shared memory.
+// them, the next panel's columns first, while those go on.  The other CTAs of the cluster form 16 to 24
+// columns each of the inverse in FP64 as the factor's columns arrive in their shared memory, eight rows at a
+// time: those eight by one warp per eight columns, then eight products for every row below.  (One row at a time
+// took 400 to 1000 cycles a row, which even seven CTAs of eight columns could not hide.)
 constexpr int kDiagOwners = 512, kBlockThread = kDiagOwners + TS, kDiagThreads = kBlockThread + 32;
-constexpr int kMaxHelpers = 7, kPanel = 4;
+constexpr int kDiagCtas = 4, kPanel = 4;
 constexpr int kFrac = 58, kLow = 29;
 constexpr int kDiagLd = TS + 1;
 
@@ -176,7 +178,7 @@ struct DiagFactor {                     // CTA 0
     long long t[TS * kDiagLd];          // scaled block, column-major
     long long colv[2][kPanel][TS];      // a panel's columns with their updates
     long long group[2][8][TS];          // eight columns of L
-    int2 lsp[2][kPanel][TS];            // a panel's columns of L, split (h, l)
+    int4 lsp[2][kPanel / 2][TS];        // a panel's columns of L, split (h, l), two columns side by side
     longlong2 piv[kPanel];              // a pivot's inverse root: (c, a << 32 | m) of InvSqrt
     long long pv[kPanel];               // the pivot
     int2 sb[kPanel][kPanel];            // the diagonal block's columns of L, split
@@ -184,8 +186,9 @@ struct DiagFactor {                     // CTA 0
 struct DiagInverse {                    // the other CTAs
     long long lq[8][8][TS];             // L's columns as they arrive, 8 groups
     double ld[2][8][TS];                // the current group in FP64, two buffers
-    double x[TS][24];                   // finished rows of this CTA's columns
-    int smax[kMaxHelpers + 1][TS];      // row exponents of each CTA's part
+    double x[TS][24];                   // rows of this CTA's columns: sums, then the inverse
+    double inv[2][8];                   // 1 / L_cc of the current group
+    int smax[kDiagCtas][TS];            // row exponents of each CTA's part
 };
 struct DiagShared {
     union {
@@ -216,6 +219,7 @@ __device__ __forceinline__ void st_cluster(uint32_t a, int v)
 }
 __device__ __forceinline__ void cluster_barrier()
 {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // what this thread has written or seen written is visible to the thread that sees the arrival
@@ -301,19 +305,23 @@ __device__ __forceinline__ int2 split_low(long long l)
     return make_int2((int)((l - lo) >> kLow), lo);
 }
 
+// (a warp arrives once: its lanes are brought together first)
 __device__ __forceinline__ void named_sync(int id, int threads)
 {
+    __syncwarp();
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 __device__ __forceinline__ void named_arrive(int id, int threads)
 {
+    __syncwarp();
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
 // thread i < kDiagOwners: group g of L's columns and pivots into the shared memory of the other CTAs
-__device__ __forceinline__ void diag_publish(DiagShared& sh, int ctas, int g, int i)
+__device__ __forceinline__ void diag_publish(DiagShared& sh, int g, int i)
 {
-    for (int rank = 1; rank < ctas; ++rank) {
+#pragma unroll
+    for (int rank = 1; rank < kDiagCtas; ++rank) {
         st_cluster(mapa(&sh.v.lq[g][0][0] + i, rank), (&sh.f.group[g & 1][0][0])[i]);
         if (i < 8) {
             st_cluster(mapa(&sh.yq[8 * g + i], rank), sh.yq[8 * g + i]);
@@ -338,7 +346,7 @@ __device__ __forceinline__ long long sub_product(long long x, int2 s, int2 q)
 __device__ __forceinline__ bool diag_block(DiagShared& sh, int p)
 {
     DiagFactor& f = sh.f;
-    const int buf = p & 1, c0 = kPanel * p, lane = threadIdx.x % 32;
+    const int buf = p & 1, c0 = kPanel * p;
     bool bad = false;
     long long d[kPanel][kPanel];
 #pragma unroll
@@ -356,13 +364,10 @@ __device__ __forceinline__ bool diag_block(DiagShared& sh, int p)
         int2 sb[kPanel];
 #pragma unroll
         for (int i = j + 1; i < kPanel; ++i) sb[i] = split_low(mul_inv_sqrt(d[j][i], y));
-        if (lane == 0) {
-            f.piv[j] = make_longlong2(y.c, ((long long)y.a << 32) | y.m);
-            f.pv[j] = v;
+        f.piv[j] = make_longlong2(y.c, ((long long)y.a << 32) | y.m);
+        f.pv[j] = v;
 #pragma unroll
-            for (int i = j + 1; i < kPanel; ++i) f.sb[j][i] = sb[i];
-        }
-        __syncwarp();
+        for (int i = j + 1; i < kPanel; ++i) f.sb[j][i] = sb[i];
         named_arrive(kCol + j, kColThreads);
 #pragma unroll
         for (int i = j + 1; i < kPanel; ++i)
@@ -394,7 +399,7 @@ __device__ __forceinline__ void diag_rows(DiagShared& sh, int p, int r)
 #pragma unroll
         for (int i = j + 1; i < kPanel; ++i) x[i] = sub_product(x[i], s, f.sb[j][i]);
         f.group[(p >> 1) & 1][(p & 1) * kPanel + j][r] = l;
-        f.lsp[buf][j][r] = s;
+        reinterpret_cast<int2*>(&f.lsp[buf][j / 2][r])[j & 1] = s;
         if (r == c0 + j) {
             sh.yq[r] = ((long long)y.m << 38) + (__mul64hi((long long)y.m << 38, y.c << 24) >> 18);
             sh.yk[r] = y.a - 2;
@@ -402,7 +407,7 @@ __device__ __forceinline__ void diag_rows(DiagShared& sh, int p, int r)
     }
 }
 
-__device__ __forceinline__ void diag_factor(DiagShared& sh, int ctas, const double* __restrict__ tile)
+__device__ __forceinline__ void diag_factor(DiagShared& sh, const double* __restrict__ tile)
 {
     DiagFactor& f = sh.f;
     const int t = threadIdx.x, tr = t % 16, tc = t / 16;
@@ -433,37 +438,45 @@ __device__ __forceinline__ void diag_factor(DiagShared& sh, int ctas, const doub
         for (int a = 0; a < 4; ++a)
 #pragma unroll
             for (int b = 0; b < 2; ++b) hh[a][b] = hl[a][b] = 0;
-        auto update = [&](int buf, int b) {  // columns tc + 32 b by the panel in buffer buf
-            int2 y[kPanel];
-#pragma unroll
-            for (int j = 0; j < kPanel; ++j) y[j] = f.lsp[buf][j][tc + 32 * b];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                // whole warps above the diagonal (a warp has two values of tc)
-                if ((tc & ~1) + 32 * b > 16 * a + 15) continue;
-#pragma unroll
-                for (int j = 0; j < kPanel; ++j) {
-                    const int2 x = f.lsp[buf][j][tr + 16 * a];
-                    hh[a][b] += (long long)x.x * y[j].x;
-                    hl[a][b] += (long long)x.x * y[j].y;
-                    hl[a][b] += (long long)x.y * y[j].x;
-                }
-            }
-        };
         constexpr int per = 32 / kPanel;  // panels in 32 columns
 #pragma unroll 1
         for (int p = 0; p < np; ++p) {
             const int buf = p & 1;
             named_sync(kFact + buf, kDiagThreads);
             // the group published in the last step (every thread has passed its stores)
-            if (p > 0 && (p & 1) == 0 && t < ctas - 1) arrive_cluster(&sh.full[p / 2 - 1], 1 + t);
+            if (p > 0 && (p & 1) == 0 && t < kDiagCtas - 1) arrive_cluster(&sh.full[p / 2 - 1], 1 + t);
+            int4 x[4][2];  // this thread's rows of the panel: 16-byte loads, once for both columns
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) x[a][j] = f.lsp[buf][j][tr + 16 * a];
+            auto update = [&](int b) {  // columns tc + 32 b
+                const int4 y0 = f.lsp[buf][0][tc + 32 * b], y1 = f.lsp[buf][1][tc + 32 * b];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    // whole warps above the diagonal (a warp has two values of tc) or past the last column
+                    if ((tc & ~1) + 32 * b > 16 * a + 15 || 16 * a + 15 < kPanel * (p + 1)) continue;
+                    hh[a][b] += (long long)x[a][0].x * y0.x;
+                    hl[a][b] += (long long)x[a][0].x * y0.y;
+                    hl[a][b] += (long long)x[a][0].y * y0.x;
+                    hh[a][b] += (long long)x[a][0].z * y0.z;
+                    hl[a][b] += (long long)x[a][0].z * y0.w;
+                    hl[a][b] += (long long)x[a][0].w * y0.z;
+                    hh[a][b] += (long long)x[a][1].x * y1.x;
+                    hl[a][b] += (long long)x[a][1].x * y1.y;
+                    hl[a][b] += (long long)x[a][1].y * y1.x;
+                    hh[a][b] += (long long)x[a][1].z * y1.z;
+                    hl[a][b] += (long long)x[a][1].z * y1.w;
+                    hl[a][b] += (long long)x[a][1].w * y1.z;
+                }
+            };
             const bool mine = p + 1 < np && tc / kPanel == (p + 1) % per;  // columns of the next panel,
             const int nb = (p + 1) / per;                                  // in the b = nb half
             if (mine) {
 #pragma unroll
                 for (int b = 0; b < 2; ++b)
                     if (b == nb) {
-                        update(buf, b);
+                        update(b);
                         const int c = tc + 32 * b;
 #pragma unroll
                         for (int a = 0; a < 4; ++a) {
@@ -474,23 +487,23 @@ __device__ __forceinline__ void diag_factor(DiagShared& sh, int ctas, const doub
                     }
                 named_arrive(kPub + (buf ^ 1), kPubThreads);
             }
-            if (p & 1) diag_publish(sh, ctas, p / 2, t);
+            if (p & 1) diag_publish(sh, p / 2, t);
 #pragma unroll
             for (int b = 0; b < 2; ++b)
-                if (tc / kPanel + per * b > p + 1) update(buf, b);
+                if (tc / kPanel + per * b > p + 1) update(b);
         }
     }
     __syncthreads();
-    if (t < ctas - 1) arrive_cluster(&sh.full[7], 1 + t);
+    if (t < kDiagCtas - 1) arrive_cluster(&sh.full[7], 1 + t);
 }
 
-// a cluster of ctas CTAs (4 or 8) per matrix
+// a cluster of kDiagCtas CTAs per matrix
 __global__ void __launch_bounds__(kDiagThreads, 1)
-    digit_diag(int k, int ctas, Dig g, double* __restrict__ diag, int* __restrict__ status)
+    digit_diag(int k, Dig g, double* __restrict__ diag, int* __restrict__ status)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     DiagShared& sh = *reinterpret_cast<DiagShared*>(sm);
-    const int rank = blockIdx.x % ctas, b = blockIdx.x / ctas, t = threadIdx.x;
+    const int rank = blockIdx.x % kDiagCtas, b = blockIdx.x / kDiagCtas, t = threadIdx.x;
     const double* tile = g.A + (size_t)b * g.strideA + (size_t)tile_index(k, k) * TILE_ELEMS;
     if (t < 8) mbar_init(&sh.full[t], 1);
     if (t == 0) sh.bad = 0;
@@ -500,7 +513,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     if (t < TS) sh.e[t] = (exp_field(tile[t * (TS + 1)]) - 1022 + 1) >> 1;  // S_rr < 2^(2 e)
     cluster_barrier();
     if (rank == 0) {
-        diag_factor(sh, ctas, tile);
+        diag_factor(sh, tile);
         cluster_barrier();
         if (t == 0 && sh.bad && status[b] == CG_OK) status[b] = CG_ERR_NOT_PD;
         cluster_barrier();
@@ -513,10 +526,9 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     }
     DiagInverse& v = sh.v;
     // columns q0 .. q0 + 8 nj - 1
-    const int q0 = ctas == 8 ? 8 * (rank - 1) : rank == 1 ? 0 : rank == 2 ? 16 : 40;
-    const int nj = ctas == 8 ? (rank == 7 ? 2 : 1) : rank == 1 ? 2 : 3;
+    const int q0 = rank == 1 ? 0 : rank == 2 ? 16 : 40, nj = rank == 1 ? 2 : 3;
     const int r = t / 8, qi = t % 8;
-    double w[3] = {0.0, 0.0, 0.0};
+    double w[3] = {0.0, 0.0, 0.0};  // row r's sums, columns q0 + qi + 8 j
     bool ok = true;
     for (int grp = 0; grp < 8; ++grp) {
         ok = wait_cluster(&sh.full[grp], 0) && ok;
@@ -525,25 +537,41 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
             diag[(size_t)b * g.nt * TS + k * TS + c] = scaled(v.lq[grp][t][c], sh.e[c] - kFrac);
         }
         if (8 * grp + 7 < q0) continue;
-        v.ld[grp & 1][t / TS][t % TS] = scaled(v.lq[grp][t / TS][t % TS], -kFrac);
+        double (&ld)[8][TS] = v.ld[grp & 1];
+        ld[t / TS][t % TS] = scaled(v.lq[grp][t / TS][t % TS], -kFrac);
+        if (t < 8) v.inv[grp & 1][t] = scaled(sh.yq[8 * grp + t], sh.yk[8 * grp + t] - 61);
+        // the group's eight rows: their sums to one warp per eight columns, which finishes them in order (lane:
+        // rows u and u + 4, one column), then eight products for every row below
+        if (r / 8 == grp) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                if (j < nj) v.x[r][qi + 8 * j] = w[j];
+        }
         named_sync(1, kDiagOwners);
-        for (int c = 0; c < 8; ++c) {
-            const int m = 8 * grp + c;
-            if (r == m) {
-                const double inv = scaled(sh.yq[m], sh.yk[m] - 61);
+        if (t / 32 < nj) {
+            const int u = (t % 32) / 8, q = 8 * (t / 32) + qi, m0 = 8 * grp;
+            double a0 = v.x[m0 + u][q], a1 = v.x[m0 + u + 4][q];
+            // X_mq = (delta - sum) / L_mm; a column beyond the row stays zero
+            a0 = (q0 + q == m0 + u ? 1.0 : 0.0) - a0;
+            a1 = (q0 + q == m0 + u + 4 ? 1.0 : 0.0) - a1;
 #pragma unroll
-                for (int j = 0; j < 3; ++j)
-                    if (j < nj) {
-                        const int q = q0 + qi + 8 * j;
-                        v.x[m][qi + 8 * j] = q == m ? inv : q < m ? -w[j] * inv : 0.0;
-                    }
+            for (int c = 0; c < 8; ++c) {
+                const double xm = __shfl_sync(0xffffffffu, (c < 4 ? a0 : a1) * v.inv[grp & 1][c], 8 * (c & 3) + qi);
+                if (u == (c & 3)) (c < 4 ? a0 : a1) = xm;
+                if (c < 4) a0 = u > c ? fma(-ld[c][m0 + u], xm, a0) : a0;
+                a1 = u + 4 > c ? fma(-ld[c][m0 + u + 4], xm, a1) : a1;
             }
-            named_sync(1, kDiagOwners);
-            if (4 * (t / 32) + 3 > m) {
-                const double l = r > m ? v.ld[grp & 1][c][r] : 0.0;
+            v.x[m0 + u][q] = a0;
+            v.x[m0 + u + 4][q] = a1;
+        }
+        named_sync(1, kDiagOwners);
+        if (r / 8 > grp) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const double l = ld[c][r];
 #pragma unroll
                 for (int j = 0; j < 3; ++j)
-                    if (j < nj && q0 + 8 * j <= m) w[j] = fma(l, v.x[m][qi + 8 * j], w[j]);
+                    if (j < nj && q0 + 8 * j < 8 * grp + 8) w[j] = fma(l, v.x[8 * grp + c][qi + 8 * j], w[j]);
             }
         }
     }
@@ -558,11 +586,10 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
             const int x = exp_field(v.x[row][q]);
             if (q0 + q <= row && x) f = max(f, x == 0x7ff ? kNonFinite : x - sh.e[q0 + q]);
         }
-        for (int rk = 1; rk < ctas; ++rk) st_cluster(mapa(&v.smax[rank][row], rk), f);
+        for (int rk = 1; rk < kDiagCtas; ++rk) st_cluster(mapa(&v.smax[rank][row], rk), f);
     }
     cluster_barrier();
-    int e = v.smax[1][row];
-    for (int rk = 2; rk < ctas; ++rk) e = max(e, v.smax[rk][row]);
+    int e = max(max(v.smax[1][row], v.smax[2][row]), v.smax[3][row]);
     e = e > kNonFinite / 2 ? kNonFinite : e < -(1 << 27) ? -1022 : e - 1022;
     if (rank == 1 && part == 0) g.dex[(size_t)b * TS + row] = e;
     if (part < nj) {
@@ -707,6 +734,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
 #pragma unroll 1
     for (int h = 0; h < 4; ++h) {
         uint32_t acc[8][4];
+        __syncwarp();
         tmem_ld_acc4<TS>(ta + 4 * h, acc);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -729,6 +757,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             uint32_t acc[8][4];
+            __syncwarp();
             tmem_ld_acc4<TS>(ta + 8 * h + 4 * q, acc);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -1020,15 +1049,6 @@ static int launch(cg_ctx* ctx, void (*kernel)(P...), dim3 grid, int threads, siz
     return CG_OK;
 }
 
-// Seven CTAs for the inverse keep up with the factor (44 us), three take a little longer (47 us); sixteen
-// clusters of eight do not fit the SMs at once (two waves, 87 us), so half the SMs are the limit.  Beside an
-// update a cluster of eight may wait 30 us for eight free SMs next to each other; four are found at once.
-static int launch_diag(cg_ctx* ctx, int B, int k, bool beside, const Dig& g, double* diag, int* status, cudaStream_t s)
-{
-    const int ctas = !beside && 16 * B <= ctx->sm_count ? 8 : 4;
-    return launch(ctx, digit_diag, dim3(ctas * B), kDiagThreads, sizeof(DiagShared), ctas, s, k, ctas, g, diag, status);
-}
-
 size_t digit_bytes(int nt, int ne)
 {
     const size_t pairs = (size_t)(nt + ne) / 2;
@@ -1046,18 +1066,18 @@ static int launch_update(cg_ctx* ctx, int B, int k, const UpRange& u, const Dig&
 // The factorisation's chain (diagonal block, panel, the update of the next column pair) beside the rest of
 // the update of the step before, on a second stream and on all but `reserve` SMs: the reserve that makes the
 // longer of the two shortest, or 0 where one after the other is as fast.  Per SM a job takes about 11 us and a
-// panel's CTA 12, a diagonal step 45; a saving below 7 % is left (large batches and matrices, whose updates
+// panel's CTA 12, a diagonal step 38; a saving below 7 % is left (large batches and matrices, whose updates
 // fill the chip).  One factorisation at nside 16 with its harmonics: 3.94 ms one after the other, 3.16 beside.
 static int chain_reserve(const cg_ctx* ctx, int B, int nq, int npe, int v)
 {
     const UpRange all = {0, nq, npe, v}, one = {0, 1, npe, 0};
     const double sms = ctx->sm_count, col = (double)up_jobs(one, nq) * B, jobs = (double)up_jobs(all, nq) * B;
     auto waves = [](double n, double s) { return std::max(1.0, std::ceil(n / s)); };
-    const double serial = 45 + 12 * waves(col, sms) + 11 * waves(jobs, sms) + 6;
+    const double serial = 38 + 12 * waves(col, sms) + 11 * waves(jobs, sms) + 6;
     double best = 0.93 * serial;
     int reserve = 0;
     for (int r = 8; r <= ctx->sm_count / 2; r += 8) {
-        const double chain = 45 * waves(4.0 * B, r) + 23 * waves(col, r) + 8;
+        const double chain = 38 * waves((double)kDiagCtas * B, r) + 23 * waves(col, r) + 8;
         const double t = std::max(chain, 11 * waves(jobs - col, sms - r) + 4);
         if (t < best) {
             best = t;
@@ -1123,7 +1143,8 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
         const int q0 = (k + 1) / 2, m = nq - q0, npe = v ? k / 2 + 1 : ne / 2;
         g.img = img[0];
         g.ex = ex[0];
-        if (int rc = launch_diag(ctx, B, k, rest, g, diag, status, s)) return rc;
+        if (int rc = launch(ctx, digit_diag, dim3(kDiagCtas * B), kDiagThreads, sizeof(DiagShared), kDiagCtas, s, k, g, diag, status))
+            return rc;
         if (m + npe == 0) continue;
         const int reserve = m > 1 ? chain_reserve(ctx, B, m, npe, v) : 0;
         const bool beside = reserve > 0 && chain_streams(ctx);
