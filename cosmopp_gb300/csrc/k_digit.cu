@@ -508,8 +508,8 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     if (t < 8) mbar_init(&sh.full[t], 1);
     if (t == 0) sh.bad = 0;
     fence_mbar_init();
-    launch_dependents();
     wait_prior();
+    launch_dependents();  // not before: the panel reads column k ahead of its own wait
     if (t < TS) sh.e[t] = (exp_field(tile[t * (TS + 1)]) - 1022 + 1) >> 1;  // S_rr < 2^(2 e)
     cluster_barrier();
     if (rank == 0) {
@@ -678,13 +678,9 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
         mbar_init(&done, 1);
         fence_mbar_init();
     }
-    __syncwarp();
-    wait_prior();
-    if (t == 0) {
-        mbar_arrive_expect_tx(&full, kDImg);
-        bulk_g2s(smem_u32(sm + kPanelB), g.dimg + (size_t)b * kDImg, kDImg, &full);
-    }
-    if (t < TS) deb[t] = g.dex[(size_t)b * TS + t];
+    // The rows' column k is final before the diagonal block starts (its kernel waits for the update before it, and
+    // this one starts after that wait), so their digits are made beside it (read from L2, where that update left
+    // them); the inverted block comes after the wait.
     double* tile = nullptr;
     int f = 0;
     if (valid) {
@@ -693,7 +689,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
                r + TS * 16 * cq;
         double v[16];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) v[c] = tile[TS * c];
+        for (int c = 0; c < 16; ++c) v[c] = __ldcg(&tile[TS * c]);
 #pragma unroll
         for (int c = 0; c < 16; ++c) f = max(f, exp_field(v[c]));
     }
@@ -704,11 +700,17 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
     for (int h = 0; h < 2; ++h) {
         unsigned long long w[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) w[c] = valid ? to_digits(to_fixed(tile[TS * (8 * h + c)], ea)) : 0;
+        for (int c = 0; c < 8; ++c) w[c] = valid ? to_digits(to_fixed(__ldcg(&tile[TS * (8 * h + c)]), ea)) : 0;
         unsigned char* o = sm + kPanelA + (2 * cq + h) * kCore + m * 16;
         store_digits(w, [&](int i, uint4 d) { *reinterpret_cast<uint4*>(o + i * kPlane) = d; });
     }
     fence_proxy_async();
+    wait_prior();
+    if (t == 0) {
+        mbar_arrive_expect_tx(&full, kDImg);
+        bulk_g2s(smem_u32(sm + kPanelB), g.dimg + (size_t)b * kDImg, kDImg, &full);
+    }
+    if (t < TS) deb[t] = g.dex[(size_t)b * TS + t];
     fence_before();
     __syncthreads();
     fence_after();
