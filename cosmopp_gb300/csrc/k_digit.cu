@@ -78,18 +78,18 @@ __device__ __forceinline__ void issue_products(uint32_t tmem, uint64_t a, uint64
         mma_bf16(tmem + NC * (i + j), a + (uint64_t)i * (a_plane >> 4), b + (uint64_t)j * (b_plane >> 4),
                  idesc_bf16(128, NC * cnt), ac);
     };
-    run(0, 0, 4, acc);
-    run(0, 4, 3, acc);
-    run(1, 6, 1, acc);  // accumulator 7 starts here
-    run(1, 0, 4, 1);
-    run(1, 4, 2, 1);
-    run(2, 0, 4, 1);
-    run(2, 4, 2, 1);
-    run(3, 0, 4, 1);
-    run(3, 4, 1, 1);
-    run(4, 0, 4, 1);
-    run(5, 0, 3, 1);
-    run(6, 0, 2, 1);
+    // N is at most 256: 4 digits of 64 columns, all 7 of 32.  Fewer, wider instructions matter: each reads
+    // A's digit again (with 4 digits of 32 columns at a time the operand reads held the tensor pipe for 65 % of
+    // the update, its arithmetic for 37 %).
+    constexpr int most = 256 / NC < kDig ? 256 / NC : kDig;
+    if (first) run(1, 6, 1, 0u);  // accumulator 7 starts here
+#pragma unroll
+    for (int i = 0; i < kDig; ++i) {
+        const int n = i == 0 ? kDig : i == 1 && first ? kDig - 1 : kDig + 1 - i;
+#pragma unroll
+        for (int j = 0; j < kDig; j += most)
+            if (j < n) run(i, j, n - j < most ? n - j : most, i == 0 ? acc : 1u);
+    }
 }
 
 // X as two's complement digits, byte p the digit of weight 256^p (bytes 0 .. 5 balanced, byte 6 the top)
@@ -138,6 +138,7 @@ struct Dig {
     int* ex;                  // [B][pairs][128]
     int nk;                   // sets of images that an update takes one after the other (1 in a factorisation)
     size_t kimg, kex;         // their distances
+    int prefetch;             // the matrices exceed L2: an update fetches the next job's tiles ahead
     unsigned char* dimg;      // [B][kDImg]
     int* dex;                 // [B][64]
     int* err;
@@ -861,6 +862,15 @@ __device__ __forceinline__ void up_halves(const UpJob& j, int k, int& h0, int& h
     h1 = (j.kind == 2 && 2 * j.q + 1 > k) ? 1 : 2;
 }
 
+// a job's tile of the FP64 matrix, row block rb and column block cb (nullptr where the job does not touch it)
+__device__ __forceinline__ double* up_tile(const Dig& g, const UpJob& j, int k, int rb, int cb)
+{
+    double* Ab = g.A + (size_t)j.b * g.strideA;
+    if (j.kind == 0) return rb > k && rb >= cb ? Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS : nullptr;
+    if (j.kind == 1) return g.ext != DIGIT_EXT_IDENTITY || rb <= k ? ext_tile(g, j.b, rb, cb) : nullptr;
+    return rb <= k && rb >= cb ? Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS : nullptr;
+}
+
 // SETS: several sets of images per job (a product); a factorisation's step has one
 template <bool SETS>
 __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, int per, UpRange u, Dig g)
@@ -896,6 +906,19 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
                 const UpJob j = up_job(g, u, per, job);
                 int h0, h1;
                 up_halves(j, k, h0, h1);
+                if (g.prefetch && job + (int)gridDim.x < njobs) {  // the next job's tiles on their way from DRAM
+                    const UpJob n = up_job(g, u, per, job + gridDim.x);
+                    int n0, n1;
+                    up_halves(n, k, n0, n1);
+                    for (int i = 0; i < 4; ++i) {
+                        const double* tile = (i >> 1) >= n0 && (i >> 1) < n1
+                                                 ? up_tile(g, n, k, 2 * n.p + (i & 1), 2 * n.q + (i >> 1)) : nullptr;
+                        if (tile)
+                            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(tile),
+                                         "r"((uint32_t)(TILE_ELEMS * sizeof(double)))
+                                         : "memory");
+                    }
+                }
                 for (int ks = 0; ks < nk; ++ks, ++round) {
                     const unsigned char* a = g.img + ks * g.kimg + ((size_t)j.b * pairs + j.pa) * kImg;
                     const unsigned char* bb = g.img + ks * g.kimg + ((size_t)j.b * pairs + j.pb) * kImg;
@@ -930,7 +953,6 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
         const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
         for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
             const UpJob j = up_job(g, u, per, job);
-            double* Ab = g.A + (size_t)j.b * g.strideA;
             const unsigned flip = j.kind == 2 || g.ext == DIGIT_EXT_PRODUCT ? 0u : 0x80000000u;
             int h0, h1;
             up_halves(j, k, h0, h1);
@@ -940,18 +962,8 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
                 for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
                     const uint32_t buf = pass & 1;
                     const int rb = 2 * j.p + half, cb = 2 * j.q + (i >> 1), c0 = (2 * c4 + (i & 1)) * 8;
-                    bool valid;
-                    double* tile = Ab;
-                    if (j.kind == 0) {
-                        valid = rb > k && rb >= cb;
-                        if (valid) tile = Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS;
-                    } else if (j.kind == 1) {
-                        valid = g.ext != DIGIT_EXT_IDENTITY || rb <= k;
-                        if (valid) tile = ext_tile(g, j.b, rb, cb);
-                    } else {
-                        valid = rb <= k && rb >= cb;
-                        if (valid) tile = Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS;
-                    }
+                    double* const tile = up_tile(g, j, k, rb, cb);
+                    const bool valid = tile != nullptr;
                     const bool read = valid && !(j.kind == 2 && rb == k);  // V's row k starts here
                     double* dst = tile + r + TS * c0;
                     double old[8];
@@ -1130,6 +1142,8 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
     g.strideE = strideE;
     g.nk = 1;
     g.kimg = g.kex = 0;
+    // 2 to 5 % of a factorisation that exceeds L2 (129 MB); 1 % lost on one that does not
+    g.prefetch = sizeof(double) * B * (strideA + strideE) > ((size_t)100 << 20);
     // two sets of images, for the steps in turn where the update of one runs beside the panel of the next
     unsigned char* const img[2] = {work, work + (size_t)B * pairs * kImg};
     g.dimg = img[1] + (size_t)B * pairs * kImg;
