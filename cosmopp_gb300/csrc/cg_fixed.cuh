@@ -38,23 +38,45 @@ __device__ __forceinline__ long long to_fixed(double v, int e)
     return bits < 0 ? -x : x;
 }
 
-// u 2^s in FP64, rounded to the nearest, its sign flipped by `flip` (0 or 0x80000000): __ll2double_rn is one
-// FP64-pipe instruction more per number, and that pipe is the scarcest
+// u 2^s in FP64, rounded to the nearest, the signs flipped by `flip` (0 or 0x80000000): __ll2double_rn is one
+// FP64-pipe instruction more per number, and that pipe is the scarcest (with one, two, three of four numbers
+// through it the update of a factorisation took 1, 4, 10 % longer).  Numbers below 2^32 and results that may
+// not be normal take one branch for all N, so that the N chains of the usual case interleave.
+template <int N>
+__device__ __forceinline__ void scaled_ints(const long long (&u)[N], const int (&s)[N], unsigned flip, double (&x)[N])
+{
+    unsigned low = 0xffffffffu;
+    int smin = s[0], smax = s[0];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int hi = (int)(u[i] >> 32), sg = hi >> 31;
+        const unsigned long long a = (unsigned long long)((u[i] ^ sg) - sg);
+        const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
+        const int lz = __clz((int)ah);
+        low = min(low, ah);
+        smin = min(smin, s[i]);
+        smax = max(smax, s[i]);
+        const unsigned nh = __funnelshift_l(al, ah, lz), nl = al << (lz & 31);
+        const unsigned long long m = (((unsigned long long)(nh >> 11) << 32) | __funnelshift_r(nl, nh, 11)) +
+                                     ((nl >> 10) & 1u) +  // 1085 - lz + s: the exponent field less one
+                                     ((unsigned long long)((unsigned)(1085 + s[i] - lz) << 20) << 32);
+        x[i] = __hiloint2double((int)((unsigned)(m >> 32) | (((unsigned)sg ^ flip) & 0x80000000u)), (int)(unsigned)m);
+    }
+    if (low == 0 || smin < -1021 || smax > 959) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const double y = scaled(u[i], s[i]);
+            x[i] = __hiloint2double(__double2hiint(y) ^ (int)flip, __double2loint(y));
+        }
+    }
+}
 __device__ __forceinline__ double scaled_int(long long u, int s, unsigned flip)
 {
-    const int hi = (int)(u >> 32), sg = hi >> 31;
-    const unsigned long long a = (unsigned long long)((u ^ sg) - sg);
-    const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a;
-    const int lz = __clz((int)ah);
-    const int e = 1085 - lz + s;  // exponent field less one
-    if (ah == 0 || (unsigned)(e - 1) > 2040u) {
-        const double x = scaled(u, s);
-        return __hiloint2double(__double2hiint(x) ^ (int)flip, __double2loint(x));
-    }
-    const unsigned nh = __funnelshift_l(al, ah, lz), nl = al << lz;
-    const unsigned long long m = (((unsigned long long)(nh >> 11) << 32) | __funnelshift_r(nl, nh, 11)) +
-                                 ((nl >> 10) & 1u) + ((unsigned long long)(unsigned)(e << 20) << 32);
-    return __hiloint2double((int)((unsigned)(m >> 32) | (((unsigned)sg ^ flip) & 0x80000000u)), (int)(unsigned)m);
+    const long long v[1] = {u};
+    const int t[1] = {s};
+    double x[1];
+    scaled_ints<1>(v, t, flip, x);
+    return x[0];
 }
 
 // ---- products of numbers with 61 fraction bits ----------------------------------------------

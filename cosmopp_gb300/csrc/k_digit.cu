@@ -24,11 +24,13 @@
 //   digit_update  S_ij -= L_ik L_jk^T over the trailing trapezoid, V_ij += M_ki^T M_kj
 //
 // Rows are kept in pairs of 64-row blocks; a pair's digits of the current column form one image,
-// [8 k-cores][7 digits][8 row groups][2 blocks][8 rows][16 bytes], which serves as the A operand (128
-// rows: groups 128 bytes apart) and, one block at a time, as the B operand (64 rows of four digits as
-// N = 256: groups 256 bytes apart).
+// [8 k-cores][7 digits][16 row groups][8 rows][16 bytes], which is the A operand as it stands (128 rows) and,
+// 32 rows at a time, taken out by a tensor copy as [8][7][4][8][16 bytes], the B operand (the 7 digits of 32
+// rows as N = 224, groups 128 bytes apart).
 //
 // A row with an infinity or a NaN gets the exponent kNonFinite, which makes everything it enters NaN.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 
@@ -47,6 +49,9 @@ constexpr int kGroupBytes = 128;            // 8 rows x 16 bytes
 constexpr int kPlane = 16 * kGroupBytes;    // one digit of 128 rows, 8 columns
 constexpr int kCore = kDig * kPlane;        // 8 columns of a pair image
 constexpr int kImg = 8 * kCore;             // a pair image: 114688 bytes
+constexpr int kPieceRow = 4 * kGroupBytes;  // a digit of the 32 rows of a piece
+constexpr int kPieceCore = kDig * kPieceRow;
+constexpr int kPiece = 8 * kPieceCore;      // 28672 bytes
 constexpr int kDPlane = 8 * kGroupBytes;    // the same for the 64 rows of an inverted diagonal block
 constexpr int kDCore = kDig * kDPlane;
 constexpr int kDImg = 8 * kDCore;           // 57344 bytes
@@ -138,6 +143,7 @@ struct Dig {
     int* ex;                  // [B][pairs][128]
     int nk;                   // sets of images that an update takes one after the other (1 in a factorisation)
     size_t kimg, kex;         // their distances
+    int im0, kim;             // img and kimg as numbers of images from the start of the tensor map
     int prefetch;             // the matrices exceed L2: an update fetches the next job's tiles ahead
     unsigned char* dimg;      // [B][kDImg]
     int* dex;                 // [B][64]
@@ -669,7 +675,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
     const int q0 = (k + 1) / 2, nq = g.nt / 2 - q0;
     const bool isext = (int)blockIdx.x >= nq;
     const int pair = isext ? g.nt / 2 + (int)blockIdx.x - nq : q0 + (int)blockIdx.x;
-    const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
+    const int half = m >> 6, r = m & 63;
     const int blk = 2 * pair + half, eb = blk - g.nt;
     const bool valid = isext ? (g.ext != DIGIT_EXT_IDENTITY || eb <= k) : blk > k;
     launch_dependents();
@@ -752,7 +758,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
     const bool nonfinite = ea == kNonFinite || top > kNonFinite / 2;
     const int e = nonfinite ? kNonFinite : top < -(1 << 27) ? -1022 : top + ea - 55;
     const bool wide = isext && g.ext == DIGIT_EXT_ROWS;
-    if (valid && cq == 0) g.ex[((size_t)b * dig_pairs(g) + pair) * 128 + 64 * half + r] = e;
+    if (valid && cq == 0) g.ex[((size_t)b * dig_pairs(g) + pair) * 128 + m] = e;
     unsigned char* out = g.img + ((size_t)b * dig_pairs(g) + pair) * kImg + (size_t)m * 16;
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
@@ -785,16 +791,39 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
     if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-// Update of step k: persistent CTAs over (pair, pair) jobs of 128 x 128 outputs, K = 64.  Both images
-// (2 x 112 KB) fill the shared memory.  A job is four passes of 32 columns (8-column groups of one parity
-// of one half of the second pair), whose eight accumulators take 256 tensor-memory columns: two passes
-// are in flight (one 64-column pass after the other with 8 warps took 22 us a job, this 11.5 in a batch of
-// 16).  Warp 16 fetches the images, 16 columns at a time as the last pass of the job before is done
-// with them, and issues the products; warps 0 .. 15 join a pass's accumulators and add them to the FP64
-// matrix while the next pass runs.  Per job and SM the tensor cores need 8.7 k cycles, the FP64 pipe (one
-// addition per output, 64 cycles per warp and partition) 8.2 k, the integer work about 8 k.
-constexpr int kUpB = kImg, kUpSmem = 2 * kImg;
-constexpr int kUpWarps = 16, kUpThreads = (kUpWarps + 1) * 32, kPassCols = 32;
+// Update of step k: persistent CTAs over (pair, pair) jobs of 128 x 128 outputs, K = 64.  A job is four
+// passes of 32 columns, whose eight accumulators take 256 tensor-memory columns: two passes are in flight (one
+// 64-column pass after the other with 8 warps took 22 us a job).  Warp 17 works out the jobs and fetches, warp
+// 16 issues the products, warps 0 .. 15 join a pass's accumulators and add them to the FP64 matrix while the
+// next pass runs.
+//
+// A CTA takes its jobs in runs of up to kRun that share the first pair: its image stays in shared memory, and
+// the second pair's comes in four pieces, each fetched as soon as the pass that used it is done, three passes
+// ahead of the next (both images again for every job, and every warp working out the job: 11.1 us a job in a
+// batch of 16 at nside 16, this 9.9).  Per job and SM the tensor cores need 8.7 k cycles, the FP64 pipe (one
+// addition per output, 64 cycles per warp and partition) 8.2 k, the issue slots (about 70 instructions per
+// output and thread, 20 to join, 25 to convert) 9 k; the matrix takes 256 KB of DRAM traffic, 5.4 of the 6.8 TB/s.
+constexpr int kUpB = kImg, kUpSmem = 2 * kImg, kRun = 8;
+constexpr int kUpWarps = 16, kUpThreads = (kUpWarps + 2) * 32, kPassCols = 32;
+
+// job s of this CTA: whole rounds of kRun jobs per CTA, then the rest in equal runs; -1 past the last
+__device__ __forceinline__ int up_at(int s, int njobs)
+{
+    const int G = gridDim.x, base = s / kRun * kRun * G, rest = njobs - base;
+    if (rest <= 0) return -1;
+    const int run = min(kRun, (rest + G - 1) / G), i = s % kRun, job = base + (int)blockIdx.x * run + i;
+    return i < run && job < njobs ? job : -1;
+}
+
+// box of a piece: 32 rows of all digits and columns of one image
+__device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap* map, int piece, int image, uint64_t* bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+        "[%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(piece), "r"(8 * kDig * image), "r"(smem_u32(bar))
+        : "memory");
+}
 
 struct UpJob {
     int b, kind, p, q;        // kind 0: A's trailing part, 1: E's rows, 2: V = M^T M; q: columns, p: rows
@@ -829,9 +858,9 @@ __device__ __forceinline__ UpJob up_job(const Dig& g, const UpRange& u, int per,
             j.p = u.q0 + l;
         } else {
             int I, J;
-            tile_coords(tri - 1 - l, I, J);
-            j.q = nq - 1 - I;
-            j.p = nq - 1 - J;
+            tile_coords(l, I, J);
+            j.q = u.q0 + J;
+            j.p = u.q0 + I;
         }
         j.kind = 0;
         j.pa = j.p;
@@ -841,8 +870,8 @@ __device__ __forceinline__ UpJob up_job(const Dig& g, const UpRange& u, int per,
     l -= tri;
     if (l < u.npe * u.ncol) {
         j.kind = 1;
-        j.q = u.q0 + l / u.npe;
-        j.p = l % u.npe;
+        j.q = u.q0 + l % u.ncol;
+        j.p = l / u.ncol;
         j.pa = nq + j.p;
         j.pb = j.q;
         return j;
@@ -871,25 +900,65 @@ __device__ __forceinline__ double* up_tile(const Dig& g, const UpJob& j, int k, 
     return rb <= k && rb >= cb ? Ab + (size_t)tile_index(rb, cb) * TILE_ELEMS : nullptr;
 }
 
+// what a job's warps need, from the one thread that works it out (with a division or two and a root per job,
+// 18 warps each for themselves took a tenth of the issue slots)
+struct UpDesc {
+    double* tile[2][2];       // by row block and column block; nullptr: not part of the job
+    const int *ea, *eb;       // row exponents of the two pairs
+    int i0, i1;               // passes; none: past the last job
+    unsigned flip;            // sign of the products
+    bool fresh;               // another first image than the job before
+    bool start[2];            // by row block: V's row k starts here
+};
+constexpr int kUpDescs = 4;
+
+__device__ __forceinline__ void up_desc(const Dig& g, const UpJob& j, int k, bool fresh, UpDesc& d)
+{
+    const int pairs = dig_pairs(g);
+    int h0, h1;
+    up_halves(j, k, h0, h1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int a = i & 1, b = i >> 1;
+        d.tile[a][b] = b >= h0 && b < h1 ? up_tile(g, j, k, 2 * j.p + a, 2 * j.q + b) : nullptr;
+    }
+    d.ea = g.ex + ((size_t)j.b * pairs + j.pa) * 128;
+    d.eb = g.ex + ((size_t)j.b * pairs + j.pb) * 128;
+    d.i0 = 2 * h0;
+    d.i1 = 2 * h1;
+    d.flip = j.kind == 2 || g.ext == DIGIT_EXT_PRODUCT ? 0u : 0x80000000u;
+    d.fresh = fresh;
+    d.start[0] = j.kind == 2 && 2 * j.p == k;
+    d.start[1] = j.kind == 2 && 2 * j.p + 1 == k;
+}
+
 // SETS: several sets of images per job (a product); a factorisation's step has one
 template <bool SETS>
-__global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, int per, UpRange u, Dig g)
+__global__ void __launch_bounds__(kUpThreads, 1)
+    digit_update(int k, int njobs, int per, UpRange u, Dig g, const __grid_constant__ CUtensorMap map)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    __shared__ uint64_t full[4], empty[4], tfull[2], tempty[2];
+    __shared__ uint64_t afull[4], aempty[4], bfull[4], bempty[4], tfull[2], tempty[2], dfull[kUpDescs], dempty[kUpDescs];
+    __shared__ UpDesc desc[kUpDescs];
     __shared__ uint32_t tptr;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int pairs = dig_pairs(g), nk = SETS ? g.nk : 1;
+    const int nk = SETS ? g.nk : 1;
     launch_dependents();
     if (warp == 0) tmem_alloc(&tptr, 512);
     if (t == 0) {
         for (int i = 0; i < 4; ++i) {
-            mbar_init(&full[i], 1);
-            mbar_init(&empty[i], 1);
+            mbar_init(&afull[i], 1);
+            mbar_init(&aempty[i], 1);
+            mbar_init(&bfull[i], 1);
+            mbar_init(&bempty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&tfull[i], 1);
             mbar_init(&tempty[i], kUpWarps);
+        }
+        for (int i = 0; i < kUpDescs; ++i) {
+            mbar_init(&dfull[i], 1);
+            mbar_init(&dempty[i], kUpWarps + 1);
         }
         fence_mbar_init();
     }
@@ -899,101 +968,189 @@ __global__ void __launch_bounds__(kUpThreads, 1) digit_update(int k, int njobs, 
     const uint32_t tmem = tptr;
     wait_prior();
     bool ok = true;
-    uint32_t pass = 0, round = 0;
-    if (warp == kUpWarps) {
-        if (lane == 0)
-            for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
-                const UpJob j = up_job(g, u, per, job);
-                int h0, h1;
-                up_halves(j, k, h0, h1);
-                if (g.prefetch && job + (int)gridDim.x < njobs) {  // the next job's tiles on their way from DRAM
-                    const UpJob n = up_job(g, u, per, job + gridDim.x);
-                    int n0, n1;
-                    up_halves(n, k, n0, n1);
-                    for (int i = 0; i < 4; ++i) {
-                        const double* tile = (i >> 1) >= n0 && (i >> 1) < n1
-                                                 ? up_tile(g, n, k, 2 * n.p + (i & 1), 2 * n.q + (i >> 1)) : nullptr;
-                        if (tile)
-                            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(tile),
+    if (warp == kUpWarps + 1) {
+        if (lane == 0) {
+            uint32_t aphase = 0, bphase = 0;  // uses so far, mod 2: of A, of piece i in bit i
+            // job s into its slot (i1 = 0 past the last)
+            auto put = [&](int s, int job, const UpJob& j, bool fresh) {
+                UpDesc& d = desc[s % kUpDescs];
+                ok = mbar_wait(&dempty[s % kUpDescs], ((s / kUpDescs) & 1) ^ 1, kWaits, g.err) && ok;
+                if (job >= 0) up_desc(g, j, k, fresh, d);
+                else d.i0 = d.i1 = 0;
+                mbar_arrive(&dfull[s % kUpDescs]);
+            };
+            int job = up_at(0, njobs);
+            UpJob j = up_job(g, u, per, max(job, 0));
+            const int pairs = dig_pairs(g);
+            bool fresh = true;
+            put(0, job, j, true);
+            for (int s = 0; job >= 0; ++s) {
+                const int next = up_at(s + 1, njobs);
+                const UpJob n = up_job(g, u, per, max(next, 0));
+                const bool same = nk == 1 && next >= 0 && n.b == j.b && n.pa == j.pa;
+                put(s + 1, next, n, !same);
+                if (g.prefetch && next >= 0) {  // the next job's tiles on their way from DRAM
+                    const UpDesc& d = desc[(s + 1) % kUpDescs];
+#pragma unroll 1
+                    for (int i = 0; i < 4; ++i)
+                        if (d.tile[i & 1][i >> 1])
+                            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(d.tile[i & 1][i >> 1]),
                                          "r"((uint32_t)(TILE_ELEMS * sizeof(double)))
                                          : "memory");
-                    }
                 }
-                for (int ks = 0; ks < nk; ++ks, ++round) {
-                    const unsigned char* a = g.img + ks * g.kimg + ((size_t)j.b * pairs + j.pa) * kImg;
-                    const unsigned char* bb = g.img + ks * g.kimg + ((size_t)j.b * pairs + j.pb) * kImg;
-                    for (int kc = 0; kc < 4; ++kc) {
-                        if (round > 0) ok = mbar_wait(&empty[kc], (round - 1) & 1, kWaits, g.err) && ok;
-                        mbar_arrive_expect_tx(&full[kc], (j.pa == j.pb ? 2 : 4) * kCore);
-                        bulk_g2s(smem_u32(sm + 2 * kc * kCore), a + 2 * kc * kCore, 2 * kCore, &full[kc]);
-                        if (j.pa != j.pb)
-                            bulk_g2s(smem_u32(sm + kUpB + 2 * kc * kCore), bb + 2 * kc * kCore, 2 * kCore, &full[kc]);
-                    }
-                    for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
+                int h0, h1;
+                up_halves(j, k, h0, h1);
+                for (int ks = 0; ks < nk; ++ks) {
+                    const int ia = ks * g.kim + j.b * pairs + j.pa, ib = g.im0 + ks * g.kim + j.b * pairs + j.pb;
+                    auto piece = [&](int i) {
+                        ok = mbar_wait(&bempty[i], ((bphase >> i) & 1) ^ 1, kWaits, g.err) && ok;
+                        bphase ^= 1u << i;
+                        mbar_arrive_expect_tx(&bfull[i], kPiece);
+                        tensor_g2s(smem_u32(sm + kUpB + i * kPiece), &map, i, ib, &bfull[i]);
+                    };
+                    auto rows = [&]() {
+                        const unsigned char* a = g.img + (size_t)ia * kImg;
+                        for (int kc = 0; kc < 4; ++kc) {
+                            ok = mbar_wait(&aempty[kc], aphase ^ 1, kWaits, g.err) && ok;
+                            mbar_arrive_expect_tx(&afull[kc], 2 * kCore);
+                            bulk_g2s(smem_u32(sm + 2 * kc * kCore), a + 2 * kc * kCore, 2 * kCore, &afull[kc]);
+                        }
+                        aphase ^= 1;
+                    };
+                    // in the order in which the places become free
+                    const bool first = s == 0 && ks == 0;
+                    piece(2 * h0);
+                    if (first) rows();
+                    for (int i = 2 * h0 + 1; i < 2 * h1 - 1; ++i) piece(i);
+                    if (!first && fresh) rows();
+                    piece(2 * h1 - 1);
+                }
+                job = next;
+                j = n;
+                fresh = !same;
+            }
+        }
+        __syncwarp();
+    } else if (warp == kUpWarps) {
+        if (lane == 0) {
+            uint32_t aphase = 0, bphase = 0, pass = 0;
+            for (int s = 0;; ++s) {
+                const UpDesc& d = desc[s % kUpDescs];
+                ok = mbar_wait(&dfull[s % kUpDescs], (s / kUpDescs) & 1, kWaits, g.err) && ok;
+                const int i0 = d.i0, i1 = ok ? d.i1 : 0;
+                if (i1 == 0) break;
+                const bool fresh = d.fresh;
+                const UpDesc& n = desc[(s + 1) % kUpDescs];  // put there before this job's images were fetched
+                ok = mbar_wait(&dfull[(s + 1) % kUpDescs], ((s + 1) / kUpDescs) & 1, kWaits, g.err) && ok;
+                const bool last = n.i1 == 0 || n.fresh;
+                for (int ks = 0; ks < nk; ++ks) {
+                    for (int i = i0; i < i1; ++i, ++pass) {
                         const uint32_t buf = pass & 1;
-                        if (pass >= 2) ok = mbar_wait(&tempty[buf], ((pass >> 1) - 1) & 1, kWaits, g.err) && ok;
+                        ok = mbar_wait(&tempty[buf], ((pass >> 1) & 1) ^ 1, kWaits, g.err) && ok;
+                        ok = mbar_wait(&bfull[i], (bphase >> i) & 1, kWaits, g.err) && ok;
+                        bphase ^= 1u << i;
                         fence_after();
                         const uint64_t ad = smem_desc(smem_u32(sm), kCore, kGroupBytes);
-                        const uint64_t bd = smem_desc(smem_u32(sm + (j.pa == j.pb ? 0 : kUpB) + (i >> 1) * kGroupBytes +
-                                                               (i & 1) * 2 * kGroupBytes),
-                                                      kCore, 4 * kGroupBytes);
+                        const uint64_t bd = smem_desc(smem_u32(sm + kUpB + i * kPiece), kPieceCore, kGroupBytes);
                         for (int kc = 0; kc < 4; ++kc) {
-                            if (i == 2 * h0) ok = mbar_wait(&full[kc], round & 1, kWaits, g.err) && ok;
+                            if (fresh && i == i0) ok = mbar_wait(&afull[kc], aphase, kWaits, g.err) && ok;
                             issue_products<kPassCols>(tmem + 256 * buf, ad + (uint64_t)kc * (2 * kCore >> 4),
-                                                      bd + (uint64_t)kc * (2 * kCore >> 4), kPlane, kPlane, kc == 0);
-                            if (i == 2 * h1 - 1) mma_commit(&empty[kc]);
+                                                      bd + (uint64_t)kc * (2 * kPieceCore >> 4), kPlane, kPieceRow,
+                                                      kc == 0);
+                            if (last && i == i1 - 1) mma_commit(&aempty[kc]);
                         }
+                        mma_commit(&bempty[i]);
                         mma_commit(&tfull[buf]);
                     }
+                    if (fresh) aphase ^= 1;
                 }
+                mbar_arrive(&dempty[s % kUpDescs]);
             }
+        }
         __syncwarp();
     } else {
         const int m = 32 * (warp & 3) + lane, c4 = warp >> 2;  // row of the pair image, 8-column group of the pass
-        const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7);
-        for (int job = blockIdx.x; job < njobs; job += gridDim.x) {
-            const UpJob j = up_job(g, u, per, job);
-            const unsigned flip = j.kind == 2 || g.ext == DIGIT_EXT_PRODUCT ? 0u : 0x80000000u;
-            int h0, h1;
-            up_halves(j, k, h0, h1);
-            for (int ks = 0; ks < nk; ++ks) {
-                const int ea = g.ex[ks * g.kex + ((size_t)j.b * pairs + j.pa) * 128 + 64 * half + r];
-                const int* eb = g.ex + ks * g.kex + ((size_t)j.b * pairs + j.pb) * 128;
-                for (int i = 2 * h0; i < 2 * h1; ++i, ++pass) {
-                    const uint32_t buf = pass & 1;
-                    const int rb = 2 * j.p + half, cb = 2 * j.q + (i >> 1), c0 = (2 * c4 + (i & 1)) * 8;
-                    double* const tile = up_tile(g, j, k, rb, cb);
-                    const bool valid = tile != nullptr;
-                    const bool read = valid && !(j.kind == 2 && rb == k);  // V's row k starts here
-                    double* dst = tile + r + TS * c0;
-                    double old[8];
+        const int half = m >> 6, r = m & 63;
+        int s = 0, i = 0, i0 = 0, i1 = 0, ks = 0;
+        const int *ea = nullptr, *eb = nullptr;  // of this thread's row, of the job's columns
+        // A pass's entries of the matrix (the thread's eight columns from dst on; nullptr: not part of it) are
+        // loaded four at a time as soon as the pass before is done with the registers.
+        double* dst = nullptr;
+        double old[8];
+        auto open_job = [&]() {  // false: no more jobs
+            ok = mbar_wait(&dfull[s % kUpDescs], (s / kUpDescs) & 1, kWaits, g.err) && ok;
+            const UpDesc& d = desc[s % kUpDescs];
+            i0 = d.i0;
+            i1 = ok ? d.i1 : 0;
+            ea = d.ea + m;
+            eb = d.eb + 8 * c4;
+            i = i0;
+            ks = 0;
+            return i1 != 0;
+        };
+        auto open_pass = [&]() {
+            dst = desc[s % kUpDescs].tile[half][i >> 1];
+            if (dst != nullptr) dst += r + TS * (32 * (i & 1) + 8 * c4);
+        };
+        bool more = open_job();
+        if (more) {
+            open_pass();
+            const bool read = dst != nullptr && !desc[s % kUpDescs].start[half];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) old[c] = read ? dst[TS * c] : 0.0;
-                    const int4 e0 = *reinterpret_cast<const int4*>(eb + 64 * (i >> 1) + c0);
-                    const int4 e1 = *reinterpret_cast<const int4*>(eb + 64 * (i >> 1) + c0 + 4);
-                    const int se[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
-                    ok = mbar_wait(&tfull[buf], (pass >> 1) & 1, kWaits, g.err) && ok;
-                    fence_after();
+            for (int c = 0; c < 8; ++c) old[c] = read ? dst[TS * c] : 0.0;
+        }
+        for (uint32_t pass = 0; more; ++pass) {
+            const uint32_t buf = pass & 1;
+            const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 256 * buf + 8 * c4;
+            double* const out = dst;
+            const unsigned flip = desc[s % kUpDescs].flip;
+            const int e = ea[ks * g.kex] - 55;
+            const int4* const ec = reinterpret_cast<const int4*>(eb + ks * g.kex + 32 * i);
+            const int4 e0 = ec[0], e1 = ec[1];
+            const int se[8] = {e + e0.x, e + e0.y, e + e0.z, e + e0.w, e + e1.x, e + e1.y, e + e1.z, e + e1.w};
+            if (++i == i1) {
+                if (SETS && ++ks < nk) {
+                    i = i0;
+                } else {
                     __syncwarp();
-                    const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 256 * buf + 8 * c4;
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        uint32_t acc[8][4];
-                        tmem_ld_acc4<kPassCols>(ta + 4 * q, acc);
-                        if (q == 1) {
-                            fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&tempty[buf]);
-                        }
-                        if (valid) {
-#pragma unroll
-                            for (int c = 0; c < 4; ++c)
-                                dst[TS * (4 * q + c)] =
-                                    old[4 * q + c] + scaled_int(join_acc4(acc, c), ea + se[4 * q + c] - 55, flip);
-                        }
-                        __syncwarp();
-                    }
+                    if (lane == 0) mbar_arrive(&dempty[s % kUpDescs]);
+                    ++s;
+                    more = open_job();
                 }
+            }
+            bool read = false;
+            if (more) {
+                open_pass();
+                read = dst != nullptr && !desc[s % kUpDescs].start[half];
+            }
+            ok = mbar_wait(&tfull[buf], (pass >> 1) & 1, kWaits, g.err) && ok;
+            fence_after();
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                uint32_t acc[8][4];
+                tmem_ld_acc4<kPassCols>(ta + 4 * q, acc);
+                if (q == 1) {
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty[buf]);
+                }
+                if (out != nullptr) {
+                    long long x[4];
+                    int sx[4];
+                    double d[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        x[c] = join_acc4(acc, c);
+                        sx[c] = se[4 * q + c];
+                    }
+                    scaled_ints<4>(x, sx, flip, d);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) out[TS * (4 * q + c)] = old[4 * q + c] + d[c];
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) old[4 * q + c] = read ? dst[TS * (4 * q + c)] : 0.0;
+                __syncwarp();
             }
         }
     }
@@ -1010,13 +1167,13 @@ __global__ void __launch_bounds__(kPanelThreads) digit_slice(int kind, int ld, i
 {
     __shared__ int smax[4][128];
     const int t = threadIdx.x, m = t & 127, cq = t >> 7, pair = blockIdx.x, nt = ld / TS;
-    const int half = (m >> 3) & 1, r = (m >> 4) * 8 + (m & 7), row = 128 * pair + 64 * half + r;
+    const int row = 128 * pair + m;
     const int kb = k0 + blockIdx.y;
     auto at = [&](int c) {
         const int k = TS * kb + c;
         return kind == 0   ? src[(size_t)k * ld + row]
                : kind == 1 ? src[(size_t)row * ld + k]
-                           : src[((size_t)kb * nt + row / TS) * TILE_ELEMS + c + TS * r];
+                           : src[((size_t)kb * nt + row / TS) * TILE_ELEMS + c + TS * (m % TS)];
     };
     int f = 0;
 #pragma unroll
@@ -1025,7 +1182,7 @@ __global__ void __launch_bounds__(kPanelThreads) digit_slice(int kind, int ld, i
     __syncthreads();
     const int e = row_exp(max(max(smax[0][m], smax[1][m]), max(smax[2][m], smax[3][m])));
     const size_t p = first + pair;
-    if (cq == 0) g.ex[blockIdx.y * g.kex + p * 128 + 64 * half + r] = e;
+    if (cq == 0) g.ex[blockIdx.y * g.kex + p * 128 + m] = e;
     unsigned char* out = g.img + blockIdx.y * g.kimg + p * kImg + (size_t)m * 16;
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
@@ -1063,18 +1220,42 @@ static int launch(cg_ctx* ctx, void (*kernel)(P...), dim3 grid, int threads, siz
     return CG_OK;
 }
 
+// the images at base for tensor copies of their pieces: (512 bytes, 4 pieces, 56 digits of 8 columns per image)
+static int image_map(cg_ctx* ctx, CUtensorMap* map, void* base, size_t images)
+{
+    static const auto encode = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(f);
+    }();
+    const cuuint64_t dims[3] = {kPieceRow / 8, 4, (cuuint64_t)images * 8 * kDig}, strides[2] = {kPieceRow, kPlane};
+    const cuuint32_t box[3] = {kPieceRow / 8, 1, 8 * kDig}, step[3] = {1, 1, 1};
+    if (!encode || encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, base, dims, strides, box, step,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        ctx->err = "cuTensorMapEncodeTiled: no tensor map for the digit images";
+        return CG_ERR_CUDA;
+    }
+    return CG_OK;
+}
+
 size_t digit_bytes(int nt, int ne)
 {
     const size_t pairs = (size_t)(nt + ne) / 2;
     return 2 * pairs * (kImg + 128 * sizeof(int)) + kDImg + TS * sizeof(int);
 }
 
-static int launch_update(cg_ctx* ctx, int B, int k, const UpRange& u, const Dig& g, int ctas, cudaStream_t s)
+static int launch_update(cg_ctx* ctx, int B, int k, const UpRange& u, const Dig& g, const CUtensorMap& map, int ctas,
+                         cudaStream_t s)
 {
     const int per = up_jobs(u, g.nt / 2);
     if (per <= 0) return CG_OK;
     return launch(ctx, digit_update<false>, dim3((unsigned)std::min<long long>((long long)per * B, ctas)), kUpThreads, kUpSmem, 1, s,
-                  k, per * B, per, u, g);
+                  k, per * B, per, u, g, map);
 }
 
 // The factorisation's chain (diagonal block, panel, the update of the next column pair) beside the rest of
@@ -1142,10 +1323,13 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
     g.strideE = strideE;
     g.nk = 1;
     g.kimg = g.kex = 0;
+    g.kim = 0;
     // 2 to 5 % of a factorisation that exceeds L2 (129 MB); 1 % lost on one that does not
     g.prefetch = sizeof(double) * B * (strideA + strideE) > ((size_t)100 << 20);
     // two sets of images, for the steps in turn where the update of one runs beside the panel of the next
     unsigned char* const img[2] = {work, work + (size_t)B * pairs * kImg};
+    CUtensorMap map;
+    if (int rc = image_map(ctx, &map, work, 2 * B * pairs)) return rc;
     g.dimg = img[1] + (size_t)B * pairs * kImg;
     int* const ex[2] = {reinterpret_cast<int*>(g.dimg + (size_t)B * kDImg),
                         reinterpret_cast<int*>(g.dimg + (size_t)B * kDImg) + (size_t)B * pairs * 128};
@@ -1159,6 +1343,7 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
         const int q0 = (k + 1) / 2, m = nq - q0, npe = v ? k / 2 + 1 : ne / 2;
         g.img = img[0];
         g.ex = ex[0];
+        g.im0 = 0;
         if (int rc = launch(ctx, digit_diag, dim3(kDiagCtas * B), kDiagThreads, sizeof(DiagShared), kDiagCtas, s, k, g, diag, status))
             return rc;
         if (m + npe == 0) continue;
@@ -1171,18 +1356,19 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
         if (beside || rest) {
             g.img = img[k & 1];
             g.ex = ex[k & 1];
+            g.im0 = (k & 1) * B * (int)pairs;
         }
         if (int rc = launch(ctx, digit_panel, dim3(m + npe, B), kPanelThreads, kPanelSmem, 1, s, k, g)) return rc;
         if (!beside) {
-            if (int rc = launch_update(ctx, B, k, {q0, m, npe, v}, g, ctx->sm_count, s)) return rc;
+            if (int rc = launch_update(ctx, B, k, {q0, m, npe, v}, g, map, ctx->sm_count, s)) return rc;
             continue;
         }
         CG_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_chain[0], s));
         CG_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->aux, ctx->ev_chain[0], 0));
         // the next column pair needs the rest of the step before
         if (rest) CG_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain[1], 0));
-        if (int rc = launch_update(ctx, B, k, {q0, 1, npe, 0}, g, ctx->sm_count, s)) return rc;
-        if (int rc = launch_update(ctx, B, k, {q0 + 1, m - 1, npe, v}, g, ctx->sm_count - reserve, ctx->aux)) return rc;
+        if (int rc = launch_update(ctx, B, k, {q0, 1, npe, 0}, g, map, ctx->sm_count, s)) return rc;
+        if (int rc = launch_update(ctx, B, k, {q0 + 1, m - 1, npe, v}, g, map, ctx->sm_count - reserve, ctx->aux)) return rc;
         CG_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_chain[1], ctx->aux));
         rest = true;
     }
@@ -1206,17 +1392,20 @@ int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, bool tile
     g.A = g.E = out;
     g.kimg = (size_t)nt * kImg;
     g.kex = (size_t)nt * 128;
+    g.kim = nt;
     g.img = work;
     g.ex = reinterpret_cast<int*>(work + chunk * g.kimg);
     g.err = err;
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_update<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem));
+    CUtensorMap map;
+    if (int rc = image_map(ctx, &map, work, (size_t)chunk * nt)) return rc;
     const UpRange u = {0, nq, nq, 0, 0};
     const int per = up_jobs(u, nq);
     for (int k0 = 0; k0 < nt; k0 += chunk) {
         g.nk = std::min(chunk, nt - k0);
         digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(tilesB ? 2 : 0, ld, k0, 0, Bm, g);
         digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(1, ld, k0, nq, A, g);
-        digit_update<true><<<std::min(per, ctx->sm_count), kUpThreads, kUpSmem, s>>>(-1, per, per, u, g);
+        digit_update<true><<<std::min(per, ctx->sm_count), kUpThreads, kUpSmem, s>>>(-1, per, per, u, g, map);
         count_launch(ctx, 3);
     }
     CG_CUDA_TRY(ctx, cudaGetLastError());
