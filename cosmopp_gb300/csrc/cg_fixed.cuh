@@ -79,6 +79,34 @@ __device__ __forceinline__ double scaled_int(long long u, int s, unsigned flip)
     return x[0];
 }
 
+// ---- FP64 multiplication in integers, to the bit ----------------------------------------------
+
+// the 53-bit significand of a normal number, its top bit at bit 63
+__device__ __forceinline__ unsigned long long significand(double v)
+{
+    return (((unsigned long long)__double_as_longlong(v) & 0xfffffffffffffull) | 0x10000000000000ull) << 11;
+}
+
+// The product of two significands, rounded to the nearest (even) as an FP64 multiplication rounds: `shift`
+// counts the products below 2, and the top bit of `valid` goes where rounding carried past the top (such a
+// product is left to the caller).
+__device__ __forceinline__ unsigned long long mul_significand(unsigned long long a, unsigned long long b, unsigned& shift,
+                                                              unsigned& valid)
+{
+    const unsigned al = (unsigned)a, ah = (unsigned)(a >> 32), bl = (unsigned)b, bh = (unsigned)(b >> 32);
+    const unsigned long long t0 = (unsigned long long)al * bl, t1 = (unsigned long long)al * bh + (t0 >> 32),
+                             t2 = (unsigned long long)ah * bl + (unsigned)t1,
+                             hi = (unsigned long long)ah * bh + (t1 >> 32) + (t2 >> 32);
+    const unsigned hh = (unsigned)(hi >> 32), hl = (unsigned)hi, lh = (unsigned)t2, ll = (unsigned)t0;
+    const unsigned sh = ~hh >> 31;
+    unsigned long long h = ((unsigned long long)__funnelshift_l(hl, hh, sh) << 32) | __funnelshift_l(lh, hl, sh);
+    const unsigned rest = (lh << sh) | ll;
+    h += 0x3ff + (rest != 0 ? 1u : ((unsigned)h >> 11) & 1u);
+    shift += sh;
+    valid &= (unsigned)(h >> 32);
+    return h & ~0x7ffull;
+}
+
 // ---- products of numbers with 61 fraction bits ----------------------------------------------
 
 // v = h 2^31 + l, 0 <= l < 2^31

@@ -38,10 +38,8 @@ __device__ __forceinline__ double pair_dot(const double* __restrict__ xyz, int N
     return d;
 }
 
-// sum_{l=2}^{lmax} ((clc_l * P_l) * B_l) * B_l in the reference's order, 4 pairs of NB elements at once;
-// sc[l][NB].  Four of the eight FP64 operations per pair and l are the recurrence's, which the elements share.
-template <int NB>
-__device__ __forceinline__ void cmat_sum4(const double x[4], double (&acc)[NB][4], int lmax, const double* sa,
+// sum_{l=2}^{lmax} ((clc_l * P_l) * B_l) * B_l in the reference's order, 4 pairs at once
+__device__ __forceinline__ void cmat_sum4(const double x[4], double (&acc)[4], int lmax, const double* sa,
                                           const double* sb, const double* sc, const double* sbeam)
 {
     double p0[4], p1[4];
@@ -49,29 +47,21 @@ __device__ __forceinline__ void cmat_sum4(const double x[4], double (&acc)[NB][4
     for (int q = 0; q < 4; ++q) {
         p0[q] = 1.0;
         p1[q] = x[q];
-#pragma unroll
-        for (int k = 0; k < NB; ++k) acc[k][q] = 0.0;
+        acc[q] = 0.0;
     }
     for (int l = 2; l <= lmax; ++l) {
-        const double a = sa[l], b = sb[l], bm = sbeam[l];
-        double c[NB];
-#pragma unroll
-        for (int k = 0; k < NB; ++k) c[k] = sc[l * NB + k];
+        const double a = sa[l], b = sb[l], c = sc[l], bm = sbeam[l];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const double p = __dsub_rn(__dmul_rn(__dmul_rn(a, x[q]), p1[q]), __dmul_rn(b, p0[q]));
-#pragma unroll
-            for (int k = 0; k < NB; ++k)
-                acc[k][q] = __dadd_rn(acc[k][q], __dmul_rn(__dmul_rn(__dmul_rn(c[k], p), bm), bm));
+            acc[q] = __dadd_rn(acc[q], __dmul_rn(__dmul_rn(__dmul_rn(c, p), bm), bm));
             p0[q] = p1[q];
             p1[q] = p;
         }
     }
 }
 
-// the tables of elements b0 .. b0 + NB - 1 of B: sc[l][NB]
-template <int NB>
-__device__ __forceinline__ void load_consts(double* sa, double* sb, double* sc, double* sbeam, int lmax, int b0, int B,
+__device__ __forceinline__ void load_consts(double* sa, double* sb, double* sc, double* sbeam, int lmax,
                                             const double* lega, const double* legb, const double* beam,
                                             const double* cl)
 {
@@ -80,11 +70,7 @@ __device__ __forceinline__ void load_consts(double* sa, double* sb, double* sc, 
         sb[l] = legb[l];
         sbeam[l] = beam[l];
         // clCopy[l] = cl[l] * (2 l + 1) / (4 pi)   (c_matrix_generator.cpp:190-193)
-#pragma unroll
-        for (int k = 0; k < NB; ++k)
-            sc[l * NB + k] = (l >= 2 && b0 + k < B)
-                                 ? __ddiv_rn(__dmul_rn(cl[(size_t)(b0 + k) * (lmax + 1) + l], (double)(2 * l + 1)), 4.0 * kPi)
-                                 : 0.0;
+        sc[l] = (l >= 2) ? __ddiv_rn(__dmul_rn(cl[l], (double)(2 * l + 1)), 4.0 * kPi) : 0.0;
     }
 }
 
@@ -104,13 +90,13 @@ __global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, 
     double* sc = sb + (lmax + 1);
     double* sbeam = sc + (lmax + 1);
     const int b = blockIdx.y;
-    load_consts<1>(sa, sb, sc, sbeam, lmax, b, b + 1, lega, legb, beam, cl);
+    load_consts(sa, sb, sc, sbeam, lmax, lega, legb, beam, cl + (size_t)b * (lmax + 1));
     __syncthreads();
     int I, J;
     tile_coords(blockIdx.x, I, J);
     double* tile = A + (size_t)b * strideA + (size_t)blockIdx.x * TILE_ELEMS;
     for (int g = 0; g < TILE_ELEMS / (kThreads * 4); ++g) {
-        double x[4], v[1][4];
+        double x[4], v[4];
         int e[4];
         bool real[4];
 #pragma unroll
@@ -120,13 +106,13 @@ __global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, 
             real[q] = (i < n && j < n);
             x[q] = real[q] ? pair_dot(xyz, N, i, j) : 0.0;
         }
-        cmat_sum4<1>(x, v, lmax, sa, sb, sc, sbeam);
+        cmat_sum4(x, v, lmax, sa, sb, sc, sbeam);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int i = I * TS + e[q] % TS, j = J * TS + e[q] / TS;
             double val;
             if (real[q]) {
-                val = v[0][q];
+                val = v[q];
                 // cInv_(i,j) = c + fiducial(0) + noise  (source/likelihood.cpp:102-110)
                 if (add_noise && i == j) val = __dadd_rn(__dadd_rn(val, 0.0), noise[i]);
             } else {
@@ -268,8 +254,30 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
     }
 }
 
-// packed output (i <= j at j(j+1)/2 + i), four entries per thread of NB elements; the reference's operations
-// and rounding; grid (ceil(np / 1024), ceil(B / NB))
+// Packed output (i <= j at j(j+1)/2 + i) with the reference's operations and rounding, kPairs entries per thread
+// of NB elements; grid (ceil(np / (kPairs kThreads)), ceil(B / NB)).
+//
+// Of the FP64 operations per pair and l, four are the recurrence's, which the elements share, and four each
+// element's: ((c P_l) B_l) B_l and the addition.  The FP64 pipe takes a warp instruction every 64 cycles and
+// partition, so the three products are formed in integers with the same rounding (some 22 instructions each), the
+// final exponents added up beside them.  What is not plainly normal (P_l zero or below 2^-200, a C_l or B_l of 0 or
+// an exponent beyond 300 and 150, a product that rounds up to a power of two) goes through the FP64 pipe.
+// Four matrices at nside 16: 5.5 ms with all products in the FP64 pipe, 2.4 ms here, that pipe still 81 % busy (B_l's
+// partner in the recurrence, b P_(l-2), in integers too: no faster).
+constexpr int kPairs = 2;
+
+struct PackedTerm {          // the constants of one l and element
+    unsigned long long m;    // significand of c
+    double c;
+    unsigned k;              // sign and exponent of the product but for P_l's
+    int pad;
+};
+struct PackedL {
+    double a, b, bm;
+    unsigned long long m;    // significand of bm
+    int normal, pad;         // the integer products may be used
+};
+
 template <int NB>
 __global__ void __launch_bounds__(kThreads) build_c_packed(int n, int N, int lmax, int B, const double* __restrict__ xyz,
                                                            const double* __restrict__ lega,
@@ -278,35 +286,76 @@ __global__ void __launch_bounds__(kThreads) build_c_packed(int n, int N, int lma
                                                            const double* __restrict__ cl, double* __restrict__ out)
 {
     extern __shared__ double sconst[];
-    double* sa = sconst;
-    double* sb = sa + (lmax + 1);
-    double* sc = sb + (lmax + 1);
-    double* sbeam = sc + NB * (lmax + 1);
+    PackedL* sl = reinterpret_cast<PackedL*>(sconst);
+    PackedTerm* st = reinterpret_cast<PackedTerm*>(sl + lmax + 1);  // [l][NB]
     const int b0 = blockIdx.y * NB;
-    load_consts<NB>(sa, sb, sc, sbeam, lmax, b0, B, lega, legb, beam, cl);
+    auto field = [](double v) { return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu); };
+    for (int l = threadIdx.x; l <= lmax; l += kThreads) {
+        const double bm = beam[l];
+        bool normal = abs(field(bm) - 1023) <= 150;
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            // clCopy[l] = cl[l] * (2 l + 1) / (4 pi)   (c_matrix_generator.cpp:190-193); past B, the last again
+            const double c = __ddiv_rn(__dmul_rn(cl[(size_t)min(b0 + k, B - 1) * (lmax + 1) + l], (double)(2 * l + 1)), 4.0 * kPi);
+            PackedTerm& t = st[l * NB + k];
+            t.c = c;
+            t.m = significand(c);
+            t.k = ((unsigned)(field(c) + 2 * field(bm) - 3 * 1022 - 1) << 20) + ((unsigned)__double2hiint(c) & 0x80000000u);
+            normal = normal && abs(field(c) - 1023) <= 300;
+        }
+        sl[l] = {lega[l], legb[l], bm, significand(bm), normal, 0};
+    }
     __syncthreads();
     const long np = (long)n * (n + 1) / 2;
-    const long k0 = 4 * ((long)blockIdx.x * kThreads + threadIdx.x);
+    const long k0 = kPairs * ((long)blockIdx.x * kThreads + threadIdx.x);
     if (k0 >= np) return;
     long j = (long)((sqrt(8.0 * (double)k0 + 1.0) - 1.0) * 0.5);
     while (j * (j + 1) / 2 > k0) --j;
     while ((j + 1) * (j + 2) / 2 <= k0) ++j;
     long i = k0 - j * (j + 1) / 2;
-    double x[4], v[NB][4];
-    long kk[4];
+    double x[kPairs], p0[kPairs], p1[kPairs], acc[NB][kPairs];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {  // four consecutive packed entries: walk i, wrap to the next column
-        kk[q] = k0 + q;
-        x[q] = (kk[q] < np) ? pair_dot(xyz, N, (int)i, (int)j) : 0.0;
+    for (int q = 0; q < kPairs; ++q) {  // consecutive packed entries: walk i, wrap to the next column
+        x[q] = (k0 + q < np) ? pair_dot(xyz, N, (int)i, (int)j) : 0.0;
         if (++i > j) { ++j; i = 0; }
+        p0[q] = 1.0;
+        p1[q] = x[q];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) acc[k][q] = 0.0;
     }
-    cmat_sum4<NB>(x, v, lmax, sa, sb, sc, sbeam);
+    for (int l = 2; l <= lmax; ++l) {
+        const PackedL c = sl[l];
+#pragma unroll
+        for (int q = 0; q < kPairs; ++q) {
+            const double p = __dsub_rn(__dmul_rn(__dmul_rn(c.a, x[q]), p1[q]), __dmul_rn(c.b, p0[q]));
+            p0[q] = p1[q];
+            p1[q] = p;
+            const unsigned ph = (unsigned)__double2hiint(p);
+            const unsigned long long pm = significand(p);
+            double v[NB];
+            unsigned valid = 0xffffffffu;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
+                const PackedTerm& t = st[l * NB + k];
+                unsigned shift = 0;
+                const unsigned long long m =
+                    mul_significand(mul_significand(mul_significand(pm, t.m, shift, valid), c.m, shift, valid), c.m, shift, valid);
+                v[k] = __hiloint2double((int)((unsigned)(m >> 43) + (ph & 0xfff00000u) + t.k - (shift << 20)), (int)(unsigned)(m >> 11));
+            }
+            if (!c.normal || (int)valid >= 0 || (ph & 0x7ff00000u) - (823u << 20) > (201u << 20)) {
+#pragma unroll
+                for (int k = 0; k < NB; ++k) v[k] = __dmul_rn(__dmul_rn(__dmul_rn(st[l * NB + k].c, p), c.bm), c.bm);
+            }
+#pragma unroll
+            for (int k = 0; k < NB; ++k) acc[k][q] = __dadd_rn(acc[k][q], v[k]);
+        }
+    }
 #pragma unroll
     for (int k = 0; k < NB; ++k)
         if (b0 + k < B)
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (kk[q] < np) out[(size_t)(b0 + k) * np + kk[q]] = v[k][q];
+            for (int q = 0; q < kPairs; ++q)
+                if (k0 + q < np) out[(size_t)(b0 + k) * np + k0 + q] = acc[k][q];
 }
 
 // CMatrixGenerator::getFiducialMatrix (source/c_matrix_generator.cpp:706-772), packed i <= j:
@@ -1048,12 +1097,10 @@ int fp64_build_tiled_into(cg_ctx* ctx, int B, const double* d_cl, bool add_noise
 int fp64_build_packed(cg_ctx* ctx, int B, const double* d_cl, double* d_out, cudaStream_t s)
 {
     const long np = (long)ctx->n * (ctx->n + 1) / 2;
-    const unsigned gx = (unsigned)((np + 4 * kThreads - 1) / (4 * kThreads));
+    const unsigned gx = (unsigned)((np + kPairs * kThreads - 1) / (kPairs * kThreads));
     const int L1 = ctx->lmax + 1;
-    // 8 FP64 operations per pair, l and element alone, 6 for two that share the recurrence, 5 for four: the
-    // pipe is the bound (four matrices at nside 16: 8.79 ms alone, 5.5 ms shared)
     auto run = [&](auto kernel, int nb) {
-        kernel<<<dim3(gx, (B + nb - 1) / nb), kThreads, sizeof(double) * (3 + nb) * L1, s>>>(
+        kernel<<<dim3(gx, (B + nb - 1) / nb), kThreads, (sizeof(PackedL) + nb * sizeof(PackedTerm)) * L1, s>>>(
             ctx->n, ctx->N, ctx->lmax, B, ctx->d_xyz, ctx->d_lega, ctx->d_legb, ctx->d_beam, d_cl, d_out);
     };
     if (B == 1) run(build_c_packed<1>, 1);

@@ -217,3 +217,41 @@ def test_nonfinite_polarisation_entries_count_where_they_are_kept(pixel, refused
             assert e.value.code == cg.CG_ERR_NONFINITE
         else:
             cg.LikelihoodPolarization(*args).close()
+
+
+@pytest.mark.parametrize("batch", [1, 2, 4])
+@pytest.mark.parametrize("case", ["plain", "exact ties", "zeros", "tiny beam", "range of exponents", "negative"])
+def test_packed_covariance_rounds_every_operation(case, batch):
+    """The integer products of the packed covariance keep the bits of the FP64 operations in order, and what is
+    outside their range (zero terms and polynomials, exponents far from 1) takes those operations themselves."""
+    rng = np.random.default_rng(5)
+    lmax = 21
+    v = rng.standard_normal((40, 3))
+    v /= np.linalg.norm(v, axis=1)[:, None]
+    v = np.concatenate([v, np.eye(3), -np.eye(3), [[0.5, 0.5, 0.5], [0.75, 0.25, 0.0]]])  # x = 0, 1, -1, short x
+    cls = np.abs(rng.standard_normal((batch, lmax + 1))) + 0.1
+    beam = np.exp(-0.01 * np.arange(lmax + 1.0) ** 2)
+    if case == "exact ties":
+        cls = 4 * np.pi * 2.0 ** rng.integers(-3, 4, cls.shape)
+        beam = 1.0 + 2.0 ** -rng.integers(20, 53, lmax + 1)
+    elif case == "zeros":
+        cls[:, 2::3] = 0.0
+        cls[0, 4] = 0.0
+        beam[9] = 0.0
+    elif case == "tiny beam":
+        beam = np.exp(-0.8 * np.arange(lmax + 1.0) ** 2)
+    elif case == "range of exponents":
+        cls *= 10.0 ** rng.integers(-120, 121, cls.shape)
+    elif case == "negative":
+        cls *= rng.choice([-1.0, 1.0], cls.shape)
+    x = (v[:, None, 0] * v[None, :, 0] + v[:, None, 1] * v[None, :, 1]) + v[:, None, 2] * v[None, :, 2]
+    p = [np.ones_like(x), np.clip(x, -1, 1)]
+    for l in range(2, lmax + 1):
+        p.append(((2 - 1.0 / l) * p[1]) * p[-1] - (1 - 1.0 / l) * p[-2])
+    with cg.Context(lmax=lmax, fwhm_deg=0.0, beam=beam, dirs=v, max_batch=batch) as ctx:
+        got = ctx.build_cmatrix(cls).reshape(batch, -1)
+    for b in range(batch):
+        want = np.zeros_like(x)
+        for l in range(2, lmax + 1):
+            want += ((((cls[b, l] * (2 * l + 1)) / (4 * np.pi)) * p[l]) * beam[l]) * beam[l]
+        assert np.array_equal(got[b], W.full_to_packed(want))
