@@ -33,6 +33,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "cg_fixed.cuh"
 #include "cg_internal.h"
@@ -163,32 +164,32 @@ __device__ __forceinline__ double* ext_tile(const Dig& g, int b, int eb, int k)
 //
 // The FP64 pipe takes a warp instruction every 64 cycles and SM partition, whatever its active lanes
 // (a lone rsqrt is 456 cycles), so the 64 dependent pivots and the 44 k FMAs of a 64 x 64 factorisation
-// in FP64 took 83 us with the inverse; this takes 37 us, 29 of them the chain of pivots.  CTA 0 factors the block in integers instead: row r is scaled
-// by 2^-e_r, 2^(2 e_r) above S_rr, so that |S| and |L| are at most 1, held as 2^58 times their
-// value.  A product sum is three 32 x 32 -> 64 multiply-adds (64 per cycle) on L = h 2^29 + l: h h'
+// in FP64 took 83 us with the inverse; this takes 34 us, 25 of them the chain of pivots.  CTA 0 factors the block in
+// integers instead: row r is scaled by 2^-e_r, 2^(2 e_r) above S_rr, so that |S| and |L| are at most 1, held as 2^58
+// times their value.  A product sum is three 32 x 32 -> 64 multiply-adds (64 per cycle) on L = h 2^29 + l: h h'
 // and h l' + l h', l l' (below 2^-56 of a product) left out; the sums cannot overflow, since rows of L
 // have norm at most 1 (sum h h' <= 2^58, sum of the cross terms <= 2^61).  All updates of an entry are
 // thus summed exactly but for the last bits and subtracted once, when its column is reached.
 //
-// Within CTA 0 one warp factors the 4 x 4 diagonal block of a panel of four columns (the chain of pivots),
-// two warps follow it with the panel's 64 rows, and sixteen warps hold the entries' sums and update
-// them, the next panel's columns first, while those go on.  The other CTAs of the cluster form 16 to 24
-// columns each of the inverse in FP64 as the factor's columns arrive in their shared memory, eight rows at a
+// Within CTA 0 one warp factors the 4 x 4 diagonal block of a panel of four columns (the chain of pivots), two warps
+// follow it with the panel's 64 rows and add the panel's products to the next panel's columns, the four rows of its
+// diagonal block first; sixteen warps add them to the columns after that meanwhile.  (With the owners' sums in the
+// chain a panel took 3.5 k cycles; this 3.0 k, 2.1 k of them the four pivots.)  The other CTAs of the cluster form 16
+// to 24 columns each of the inverse in FP64 as the factor's columns arrive in their shared memory, eight rows at a
 // time: those eight by one warp per eight columns, then eight products for every row below.  (One row at a time
 // took 400 to 1000 cycles a row, which even seven CTAs of eight columns could not hide.)
 constexpr int kDiagOwners = 512, kBlockThread = kDiagOwners + TS, kDiagThreads = kBlockThread + 32;
 constexpr int kDiagCtas = 4, kPanel = 4;
 constexpr int kFrac = 58, kLow = 29;
-constexpr int kDiagLd = TS + 1;
 
 struct DiagFactor {                     // CTA 0
-    long long t[TS * kDiagLd];          // scaled block, column-major
-    long long colv[2][kPanel][TS];      // a panel's columns with their updates
+    longlong2 acc[TS][TS];              // column by column: an entry less its updates' high parts, their low parts
     long long group[2][8][TS];          // eight columns of L
     int4 lsp[2][kPanel / 2][TS];        // a panel's columns of L, split (h, l), two columns side by side
-    longlong2 piv[kPanel];              // a pivot's inverse root: (c, a << 32 | m) of InvSqrt
-    long long pv[kPanel];               // the pivot
-    int2 sb[kPanel][kPanel];            // the diagonal block's columns of L, split
+    longlong2 piv[2][kPanel];           // a pivot's inverse root: (c, a << 32 | m) of InvSqrt
+    long long pv[2][kPanel];            // the pivot
+    int2 sb[2][kPanel][2 * kPanel];     // the diagonal block's columns of L, split (rows past its last are not used)
+    long long next[kPanel][kPanel];     // the next diagonal block
 };
 struct DiagInverse {                    // the other CTAs
     long long lq[8][8][TS];             // L's columns as they arrive, 8 groups
@@ -337,11 +338,13 @@ __device__ __forceinline__ void diag_publish(DiagShared& sh, int g, int i)
     }
 }
 
-// named barriers of CTA 0: kPub + parity (the panel's columns are in colv: the two warps that hold them,
-// the row warps and the block warp), kFact + parity (L's columns are in lsp and group: every thread),
-// kCol + j (column j of the panel's diagonal block is in piv, pv, sb: the row warps and the block warp)
-constexpr int kPub = 1, kFact = 3, kCol = 5;
-constexpr int kPubThreads = 64 + TS + 32, kColThreads = TS + 32;
+// Named barriers of CTA 0.  With the panel's parity: kFact (L's columns are in lsp and group, 1 / L_cc in yq, and the
+// owners are done with the panel before: every thread; the block warp only arrives), kCol + 2 j (column j of the panel's diagonal block is in piv,
+// pv, sb: the row warps and the block warp, which may be a panel ahead of one of them).  kBase: the next panel's
+// diagonal block lacks this panel only (the owners' warp and the row warp that have it); kNext: it is complete, in
+// next (that row warp and the block warp).
+constexpr int kFact = 1, kNext = 3, kBase = 4, kCol = 5;
+constexpr int kColThreads = TS + 32, kNextThreads = 64;
 
 // x - s q for split numbers of kFrac fraction bits
 __device__ __forceinline__ long long sub_product(long long x, int2 s, int2 q)
@@ -349,67 +352,133 @@ __device__ __forceinline__ long long sub_product(long long x, int2 s, int2 q)
     return x - ((long long)s.x * q.x + (((long long)s.x * q.y + (long long)s.y * q.x) >> kLow));
 }
 
-// the diagonal block of panel p, columns 4 p .. 4 p + 3 (one warp, every lane the same)
-__device__ __forceinline__ bool diag_block(DiagShared& sh, int p)
+__device__ __forceinline__ long long shfl(long long v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+__device__ __forceinline__ int2 shfl(int2 v, int lane)
 {
+    return make_int2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+
+__device__ __forceinline__ long long joined(longlong2 a) { return a.x - (a.y >> kLow); }
+
+// an entry less the products of its row and column over a panel
+__device__ __forceinline__ longlong2 less_product(longlong2 o, int4 x0, int4 x1, int4 y0, int4 y1)
+{
+    long long h = (long long)x0.x * y0.x, l = (long long)x0.x * y0.y, k = (long long)x1.x * y1.y;
+    l += (long long)x0.y * y0.x;
+    k += (long long)x1.y * y1.x;
+    h += (long long)x0.z * y0.z;
+    l += (long long)x0.z * y0.w;
+    k += (long long)x1.z * y1.w;
+    l += (long long)x0.w * y0.z;
+    k += (long long)x1.w * y1.z;
+    h += (long long)x1.x * y1.x;
+    h += (long long)x1.z * y1.z;
+    return make_longlong2(o.x - h, o.y + (l + k));
+}
+
+// The owners' loop stays rolled: their sums in registers, 96 multiply-adds unrolled, ran at 8 cycles an instruction,
+// which each warp fetched anew for every panel.
+
+// The diagonal blocks of all panels, one warp, row lane % 4 each; panel p has columns 4 p .. 4 p + 3.  Returns whether
+// a pivot was not positive.
+__device__ __forceinline__ bool diag_blocks(DiagShared& sh)
+{
+    constexpr int np = TS / kPanel;
     DiagFactor& f = sh.f;
-    const int buf = p & 1, c0 = kPanel * p;
+    const int lane = threadIdx.x & 31, q = lane & (kPanel - 1);
     bool bad = false;
-    long long d[kPanel][kPanel];
+    long long x[kPanel];  // the row's entries from the current column on
 #pragma unroll
-    for (int j = 0; j < kPanel; ++j)
+    for (int j = 0; j < kPanel; ++j) x[j] = f.acc[j][q].x;
+#pragma unroll 1
+    for (int p = 0; p < np; ++p) {
+        const int buf = p & 1;
+        long long next = x[0];
 #pragma unroll
-        for (int i = j; i < kPanel; ++i) d[j][i] = f.colv[buf][j][c0 + i];
+        for (int j = 0; j < kPanel; ++j) {
+            long long v = shfl(next, j);
+            if (v <= 0) {  // not positive definite: flag, keep going on a benign value
+                bad = true;
+                v = 1ll << kFrac;
+            }
+            const InvSqrt y = inv_sqrt(v);
+            const int2 s = split_low(mul_inv_sqrt(x[0], y));
+            next = sub_product(x[1], s, s);  // in lane j + 1: the next pivot
+            if (lane == 0) {
+                f.piv[buf][j] = make_longlong2(y.c, ((long long)y.a << 32) | y.m);
+                f.pv[buf][j] = v;
+            }
+            if (lane > j && lane < kPanel) f.sb[buf][j][lane] = s;
+            named_arrive(kCol + 2 * j + buf, kColThreads);
 #pragma unroll
-    for (int j = 0; j < kPanel; ++j) {
-        long long v = d[j][j];
-        if (v <= 0) {  // not positive definite: flag, keep going on a benign value
-            bad = true;
-            v = 1ll << kFrac;
+            for (int i = 0; i + 1 < kPanel - j; ++i) x[i] = sub_product(x[i + 1], s, shfl(s, j + 1 + i));
         }
-        const InvSqrt y = inv_sqrt(v);
-        int2 sb[kPanel];
+        __syncwarp();
+        if (lane < kPanel) {  // 1 / L_cc
+            const longlong2 w = f.piv[buf][lane];
+            const long long m = (long long)(unsigned)w.y << 38;
+            sh.yq[kPanel * p + lane] = m + (__mul64hi(m, w.x << 24) >> 18);
+            sh.yk[kPanel * p + lane] = (int)(w.y >> 32) - 2;
+        }
+        named_arrive(kFact + buf, kDiagThreads);
+        if (p + 1 < np) {
+            named_sync(kNext, kNextThreads);
 #pragma unroll
-        for (int i = j + 1; i < kPanel; ++i) sb[i] = split_low(mul_inv_sqrt(d[j][i], y));
-        f.piv[j] = make_longlong2(y.c, ((long long)y.a << 32) | y.m);
-        f.pv[j] = v;
-#pragma unroll
-        for (int i = j + 1; i < kPanel; ++i) f.sb[j][i] = sb[i];
-        named_arrive(kCol + j, kColThreads);
-#pragma unroll
-        for (int i = j + 1; i < kPanel; ++i)
-#pragma unroll
-            for (int q = i; q < kPanel; ++q) d[i][q] = sub_product(d[i][q], sb[i], sb[q]);
+            for (int j = 0; j < kPanel; ++j) x[j] = f.next[q][j];
+        }
     }
     return bad;
 }
 
-// its rows: row r per thread
-__device__ __forceinline__ void diag_rows(DiagShared& sh, int p, int r)
+// The rows, row r per thread.  The owners' sums of a panel's columns lack the panel just before it, whose products the
+// rows add themselves (of them the block warp gets the diagonal block): so the owners have a panel's time for theirs,
+// and the chain of pivots passes through the rows only.
+__device__ __forceinline__ void diag_rows(DiagShared& sh, int r)
 {
+    constexpr int np = TS / kPanel;
     DiagFactor& f = sh.f;
-    const int buf = p & 1, c0 = kPanel * p;
-    long long x[kPanel];
+    const int lane = r & 31, er = (lane >> 2) & 3, ec = lane & 3;
+    long long x[kPanel];  // the row's entries from the current column on
 #pragma unroll
-    for (int j = 0; j < kPanel; ++j) x[j] = f.colv[buf][j][r];
+    for (int j = 0; j < kPanel; ++j) x[j] = f.acc[j][r].x;
+#pragma unroll 1
+    for (int p = 0; p < np; ++p) {
+        const int buf = p & 1, c0 = kPanel * p, from = (c0 + kPanel) & 31;
+        const bool completes = p + 1 < np && (c0 + kPanel) / 32 == r / 32;
+        long long dh = 0, dl = 0;
 #pragma unroll
-    for (int j = 0; j < kPanel; ++j) {
-        named_sync(kCol + j, kColThreads);
-        const longlong2 w = f.piv[j];
-        InvSqrt y;
-        y.c = w.x;
-        y.m = (unsigned)w.y;
-        y.a = (int)(w.y >> 32);
-        if (r == c0 + j) x[j] = f.pv[j];
-        const long long l = r >= c0 + j ? mul_inv_sqrt(x[j], y) : 0;
-        const int2 s = split_low(l);
+        for (int j = 0; j < kPanel; ++j) {
+            named_sync(kCol + 2 * j + buf, kColThreads);
+            const longlong2 w = f.piv[buf][j];
+            InvSqrt y;
+            y.c = w.x;
+            y.m = (unsigned)w.y;
+            y.a = (int)(w.y >> 32);
+            if (r == c0 + j) x[0] = f.pv[buf][j];
+            const long long l = r >= c0 + j ? mul_inv_sqrt(x[0], y) : 0;
+            const int2 s = split_low(l);
+            const int2 a = shfl(s, from + er), b = shfl(s, from + ec);
+            dh += (long long)a.x * b.x;
+            dl += (long long)a.x * b.y;
+            dl += (long long)a.y * b.x;
 #pragma unroll
-        for (int i = j + 1; i < kPanel; ++i) x[i] = sub_product(x[i], s, f.sb[j][i]);
-        f.group[(p >> 1) & 1][(p & 1) * kPanel + j][r] = l;
-        reinterpret_cast<int2*>(&f.lsp[buf][j / 2][r])[j & 1] = s;
-        if (r == c0 + j) {
-            sh.yq[r] = ((long long)y.m << 38) + (__mul64hi((long long)y.m << 38, y.c << 24) >> 18);
-            sh.yk[r] = y.a - 2;
+            for (int i = 0; i + 1 < kPanel; ++i) x[i] = sub_product(x[i + 1], s, f.sb[buf][j][j + 1 + i]);
+            f.group[(p >> 1) & 1][(p & 1) * kPanel + j][r] = l;
+            reinterpret_cast<int2*>(&f.lsp[buf][j / 2][r])[j & 1] = s;
+        }
+        if (completes) {
+            if (p > 0) named_sync(kBase, kNextThreads);
+            const longlong2 o = f.acc[c0 + kPanel + ec][c0 + kPanel + er];
+            if (lane < 16) f.next[er][ec] = joined(make_longlong2(o.x - dh, o.y + dl));
+            named_arrive(kNext, kNextThreads);
+        }
+        named_sync(kFact + buf, kDiagThreads);
+        if (p + 1 == np) break;
+        const int4 x0 = f.lsp[buf][0][r], x1 = f.lsp[buf][1][r];
+#pragma unroll
+        for (int j = 0; j < kPanel; ++j) {
+            const int c = c0 + kPanel + j;
+            x[j] = joined(less_product(f.acc[c][r], x0, x1, f.lsp[buf][0][c], f.lsp[buf][1][c]));
         }
     }
 }
@@ -417,87 +486,40 @@ __device__ __forceinline__ void diag_rows(DiagShared& sh, int p, int r)
 __device__ __forceinline__ void diag_factor(DiagShared& sh, const double* __restrict__ tile)
 {
     DiagFactor& f = sh.f;
-    const int t = threadIdx.x, tr = t % 16, tc = t / 16;
+    const int t = threadIdx.x;
     bool bad = false;
     for (int i = t; i < TILE_ELEMS; i += kDiagThreads) {
         const int r = i % TS, c = i / TS;
         long long x = 0;
         if (r >= c) bad |= !to_scaled(tile[i], sh.e[r] + sh.e[c], x);
-        f.t[c * kDiagLd + r] = x;
-        if (c < kPanel) f.colv[0][c][r] = x;
+        f.acc[c][r] = make_longlong2(x, 0);
     }
     if (bad) sh.bad = 1;
     __syncthreads();
     constexpr int np = TS / kPanel;
     if (t >= kDiagOwners) {
-        bad = false;
-#pragma unroll 1
-        for (int p = 0; p < np; ++p) {
-            if (p > 0) named_sync(kPub + (p & 1), kPubThreads);
-            if (t >= kBlockThread) bad |= diag_block(sh, p);
-            else diag_rows(sh, p, t - kDiagOwners);
-            named_sync(kFact + (p & 1), kDiagThreads);
+        if (t >= kBlockThread) {
+            if (diag_blocks(sh) && t == kBlockThread) sh.bad = 1;
+        } else {
+            diag_rows(sh, t - kDiagOwners);
         }
-        if (bad && t == kBlockThread) sh.bad = 1;
     } else {
-        long long hh[4][2], hl[4][2];  // rows tr + 16 a, columns tc + 32 b
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) hh[a][b] = hl[a][b] = 0;
-        constexpr int per = 32 / kPanel;  // panels in 32 columns
+        // warp w has the columns of panel w: this thread column c, rows tr + 8 a
+        const int w = t / 32, tr = t % 8, c = t / 8;
 #pragma unroll 1
         for (int p = 0; p < np; ++p) {
             const int buf = p & 1;
             named_sync(kFact + buf, kDiagThreads);
             // the group published in the last step (every thread has passed its stores)
             if (p > 0 && (p & 1) == 0 && t < kDiagCtas - 1) arrive_cluster(&sh.full[p / 2 - 1], 1 + t);
-            int4 x[4][2];  // this thread's rows of the panel: 16-byte loads, once for both columns
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) x[a][j] = f.lsp[buf][j][tr + 16 * a];
-            auto update = [&](int b) {  // columns tc + 32 b
-                const int4 y0 = f.lsp[buf][0][tc + 32 * b], y1 = f.lsp[buf][1][tc + 32 * b];
-#pragma unroll
-                for (int a = 0; a < 4; ++a) {
-                    // whole warps above the diagonal (a warp has two values of tc) or past the last column
-                    if ((tc & ~1) + 32 * b > 16 * a + 15 || 16 * a + 15 < kPanel * (p + 1)) continue;
-                    hh[a][b] += (long long)x[a][0].x * y0.x;
-                    hl[a][b] += (long long)x[a][0].x * y0.y;
-                    hl[a][b] += (long long)x[a][0].y * y0.x;
-                    hh[a][b] += (long long)x[a][0].z * y0.z;
-                    hl[a][b] += (long long)x[a][0].z * y0.w;
-                    hl[a][b] += (long long)x[a][0].w * y0.z;
-                    hh[a][b] += (long long)x[a][1].x * y1.x;
-                    hl[a][b] += (long long)x[a][1].x * y1.y;
-                    hl[a][b] += (long long)x[a][1].y * y1.x;
-                    hh[a][b] += (long long)x[a][1].z * y1.z;
-                    hl[a][b] += (long long)x[a][1].z * y1.w;
-                    hl[a][b] += (long long)x[a][1].w * y1.z;
-                }
-            };
-            const bool mine = p + 1 < np && tc / kPanel == (p + 1) % per;  // columns of the next panel,
-            const int nb = (p + 1) / per;                                  // in the b = nb half
-            if (mine) {
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-                    if (b == nb) {
-                        update(b);
-                        const int c = tc + 32 * b;
-#pragma unroll
-                        for (int a = 0; a < 4; ++a) {
-                            const int r = tr + 16 * a;
-                            f.colv[buf ^ 1][c % kPanel][r] =
-                                r >= c ? f.t[c * kDiagLd + r] - (hh[a][b] + (hl[a][b] >> kLow)) : 0;
-                        }
-                    }
-                named_arrive(kPub + (buf ^ 1), kPubThreads);
+            if (w > p + 1) {
+                const int4 y0 = f.lsp[buf][0][c], y1 = f.lsp[buf][1][c];
+#pragma unroll 2
+                for (int r = tr + kPanel * (w & ~1); r < TS; r += 8)
+                    f.acc[c][r] = less_product(f.acc[c][r], f.lsp[buf][0][r], f.lsp[buf][1][r], y0, y1);
+                if (w == p + 2) named_arrive(kBase, kNextThreads);
             }
             if (p & 1) diag_publish(sh, p / 2, t);
-#pragma unroll
-            for (int b = 0; b < 2; ++b)
-                if (tc / kPanel + per * b > p + 1) update(b);
         }
     }
     __syncthreads();
