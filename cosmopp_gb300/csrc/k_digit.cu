@@ -857,6 +857,7 @@ struct UpJob {
 struct UpRange {
     int q0, ncol, npe, v;
     int a = 1;                // 0: E's rows alone
+    int part = 0;             // of column pair q0, 1: the first half alone, 2: the second alone
 };
 __host__ __device__ inline int up_tri(const UpRange& u, int nq)
 {
@@ -907,10 +908,14 @@ __device__ __forceinline__ UpJob up_job(const Dig& g, const UpRange& u, int per,
 }
 
 // the passes of a job: halves [h0, h1) of the second pair, two parities each
-__device__ __forceinline__ void up_halves(const UpJob& j, int k, int& h0, int& h1)
+__device__ __forceinline__ void up_halves(const UpRange& u, const UpJob& j, int k, int& h0, int& h1)
 {
     h0 = (j.kind != 2 && 2 * j.q <= k) ? 1 : 0;      // the half with column k is not part of the update
     h1 = (j.kind == 2 && 2 * j.q + 1 > k) ? 1 : 2;
+    if (j.kind != 2 && j.q == u.q0) {
+        if (u.part == 1) h1 = 1;
+        if (u.part == 2) h0 = 1;
+    }
 }
 
 // a job's tile of the FP64 matrix, row block rb and column block cb (nullptr where the job does not touch it)
@@ -934,11 +939,11 @@ struct UpDesc {
 };
 constexpr int kUpDescs = 4;
 
-__device__ __forceinline__ void up_desc(const Dig& g, const UpJob& j, int k, bool fresh, UpDesc& d)
+__device__ __forceinline__ void up_desc(const Dig& g, const UpRange& u, const UpJob& j, int k, bool fresh, UpDesc& d)
 {
     const int pairs = dig_pairs(g);
     int h0, h1;
-    up_halves(j, k, h0, h1);
+    up_halves(u, j, k, h0, h1);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int a = i & 1, b = i >> 1;
@@ -997,7 +1002,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
             auto put = [&](int s, int job, const UpJob& j, bool fresh) {
                 UpDesc& d = desc[s % kUpDescs];
                 ok = mbar_wait(&dempty[s % kUpDescs], ((s / kUpDescs) & 1) ^ 1, kWaits, g.err) && ok;
-                if (job >= 0) up_desc(g, j, k, fresh, d);
+                if (job >= 0) up_desc(g, u, j, k, fresh, d);
                 else d.i0 = d.i1 = 0;
                 mbar_arrive(&dfull[s % kUpDescs]);
             };
@@ -1021,7 +1026,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                                          : "memory");
                 }
                 int h0, h1;
-                up_halves(j, k, h0, h1);
+                up_halves(u, j, k, h0, h1);
                 for (int ks = 0; ks < nk; ++ks) {
                     const int ia = ks * g.kim + j.b * pairs + j.pa, ib = g.im0 + ks * g.kim + j.b * pairs + j.pb;
                     auto piece = [&](int i) {
@@ -1282,20 +1287,21 @@ static int launch_update(cg_ctx* ctx, int B, int k, const UpRange& u, const Dig&
 
 // The factorisation's chain (diagonal block, panel, the update of the next column pair) beside the rest of
 // the update of the step before, on a second stream and on all but `reserve` SMs: the reserve that makes the
-// longer of the two shortest, or 0 where one after the other is as fast.  Per SM a job takes about 11 us and a
-// panel's CTA 12, a diagonal step 38; a saving below 7 % is left (large batches and matrices, whose updates
-// fill the chip).  One factorisation at nside 16 with its harmonics: 3.94 ms one after the other, 3.16 beside.
+// longer of the two shortest, or 0 where one after the other is as fast.  Per SM a job takes about 10 us and a
+// panel's CTA 12, the update of one pair 8, a diagonal step 34; a saving below 3 % is left.  One factorisation at
+// nside 16 with its harmonics: 3.94 ms one after the other, 3.16 beside when this came in, 2.48 now; sixteen of them
+// 14.94 -> 14.43 ms with the line at 3 % instead of 7 (14.10 at 2 %, but eight without harmonics 3.57 -> 3.63).
 static int chain_reserve(const cg_ctx* ctx, int B, int nq, int npe, int v)
 {
     const UpRange all = {0, nq, npe, v}, one = {0, 1, npe, 0};
     const double sms = ctx->sm_count, col = (double)up_jobs(one, nq) * B, jobs = (double)up_jobs(all, nq) * B;
     auto waves = [](double n, double s) { return std::max(1.0, std::ceil(n / s)); };
-    const double serial = 38 + 12 * waves(col, sms) + 11 * waves(jobs, sms) + 6;
-    double best = 0.93 * serial;
+    const double serial = 34 + 12 * waves(col, sms) + 10 * waves(jobs, sms) + 6;
+    double best = 0.97 * serial;
     int reserve = 0;
     for (int r = 8; r <= ctx->sm_count / 2; r += 8) {
-        const double chain = 38 * waves((double)kDiagCtas * B, r) + 23 * waves(col, r) + 8;
-        const double t = std::max(chain, 11 * waves(jobs - col, sms - r) + 4);
+        const double chain = 34 * waves((double)kDiagCtas * B, r) + 20 * waves(col, r) + 8;
+        const double t = std::max(chain, 10 * waves(jobs - col, sms - r) + 4);
         if (t < best) {
             best = t;
             reserve = r;
@@ -1389,8 +1395,12 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
         CG_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->aux, ctx->ev_chain[0], 0));
         // the next column pair needs the rest of the step before
         if (rest) CG_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain[1], 0));
-        if (int rc = launch_update(ctx, B, k, {q0, 1, npe, 0}, g, map, ctx->sm_count, s)) return rc;
-        if (int rc = launch_update(ctx, B, k, {q0 + 1, m - 1, npe, v}, g, map, ctx->sm_count - reserve, ctx->aux)) return rc;
+        // Step k + 1 needs column k + 1 alone.  Where that is the first half of the pair, the second goes with the rest:
+        // the update in the chain is two passes in every step (one factorisation at nside 16: 2545 -> 2495 us)
+        const bool split = k % 2 == 1;
+        if (int rc = launch_update(ctx, B, k, {q0, 1, npe, 0, 1, split ? 1 : 0}, g, map, ctx->sm_count, s)) return rc;
+        const UpRange left = split ? UpRange{q0, m, npe, v, 1, 2} : UpRange{q0 + 1, m - 1, npe, v};
+        if (int rc = launch_update(ctx, B, k, left, g, map, ctx->sm_count - reserve, ctx->aux)) return rc;
         CG_CUDA_TRY(ctx, cudaEventRecord(ctx->ev_chain[1], ctx->aux));
         rest = true;
     }
