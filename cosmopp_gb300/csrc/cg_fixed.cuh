@@ -107,20 +107,25 @@ __device__ __forceinline__ unsigned long long mul_significand(unsigned long long
     return h & ~0x7ffull;
 }
 
-// ---- products of numbers with 61 fraction bits ----------------------------------------------
+// ---- products of 64-bit fixed-point numbers ---------------------------------------------------
 
-// v = h 2^31 + l, 0 <= l < 2^31
-struct Split61 {
+// v = h 2^32 + l, both signed (|v| < 2^63 - 2^31)
+struct Split64 {
     int h, l;
 };
-__device__ __forceinline__ Split61 split61(long long v) { return {(int)(v >> 31), (int)v & 0x7fffffff}; }
-
-// a b 2^-61 to about one unit: three 32 x 32 -> 64 multiply-adds.  l l' is left out; 2^30, its mean and
-// half a unit, stands for it
-__device__ __forceinline__ long long mul61(Split61 a, Split61 b)
+__device__ __forceinline__ Split64 split64(long long v)
 {
-    const long long c = (long long)a.l * b.h + ((long long)a.h * b.l + (1ll << 30));
-    return 2 * ((long long)a.h * b.h) + (c >> 30);
+    const int l = (int)v;
+    return {(int)(v >> 32) + (int)((unsigned)l >> 31), l};
+}
+
+// a b 2^-64 to about one unit: three 32 x 32 -> 64 multiply-adds, the cross terms' high word as it stands in its
+// register.  l l' (a quarter of a unit, of either sign) is left out; |h l'| + |h' l| < 2^63.  (Halves of 31 bits need
+// shifts for the cross terms and for the result.)
+__device__ __forceinline__ long long mul64(Split64 a, Split64 b)
+{
+    const long long c = (long long)a.l * b.h + ((long long)a.h * b.l + (1ll << 31));
+    return (long long)a.h * b.h + (c >> 32);
 }
 
 }  // namespace cg

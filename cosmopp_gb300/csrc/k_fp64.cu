@@ -127,15 +127,16 @@ __global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, 
 //
 // The FP64 pipe gives 2 operations per cycle and SM, the 32 x 32 -> 64 multiply-add 64, and every quantity of
 // the Legendre sum is bounded: |P_l| <= 1, |x| <= 1, and the weights w_l = C_l (2l+1)/(4 pi) B_l^2 are
-// scaled by a power of two above sum |w_l|.  So the sum runs in integers, P_l = p 2^-60, x, w_l and 1 / l
-// with 61 fraction bits:
+// scaled by a power of two above sum |w_l|.  So the sum runs in integers, x, P_l and w_l with 62 fraction bits, 1 / l
+// with 64 (a product drops 64):
 //     t = x P_{l-1},  P_l = 2 t - P_{l-2} - (t - P_{l-2}) / l,  S += w_l P_l,
 // three multiply-adds a product.  x itself is the dot product of the directions in fixed point, and the
-// sum becomes FP64 in integer operations.  Each step rounds at 2^-60 where FP64 rounds at 2^-53: the sum
-// is 10 to 30 times nearer to the exact value than the FP64 recurrence's (lmax 12 to 255).  The P_l are
-// shared by NB batch elements.
+// sum becomes FP64 in integer operations.  The sum is 50 to 200 times nearer to the exact value than the FP64
+// recurrence's (lmax 12 to 255).  The P_l are shared by NB batch elements.  The integer pipes bound it (47
+// instructions per pair and l with one element, 57 % of the issue slots, 64 % of the multiply-add pipe): one matrix at
+// nside 16 2650 us in FP64, 418 with halves of 31 bits, 355 here; sixteen 42 ms, 2.9, 2.3.
 
-// status and fixed-point weights of every element: wfix[b][l] = w_l 2^(61 - e), wexp[b] = e with
+// status and fixed-point weights of every element: wfix[b][l] = w_l 2^(62 - e), wexp[b] = e with
 // sum |w_l| < 2^e; a non-finite weight gives e = kNonFinite and a NaN covariance.  grid B
 __global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const double* __restrict__ beam,
                                                              const double* __restrict__ cl,
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const dou
     s = 0.0;
     for (int k = 0; k < kThreads / 32; ++k) s += part[k];
     const int e = isfinite(s) ? (s > 0.0 ? ilogb(s) + 1 : -1000) : kNonFinite;
-    if (l <= lmax) wfix[(size_t)b * L1 + l] = e == kNonFinite ? 0 : __double2ll_rn(scalbn(w, 61 - e));
+    if (l <= lmax) wfix[(size_t)b * L1 + l] = e == kNonFinite ? 0 : __double2ll_rn(scalbn(w, 62 - e));
     if (l == 0) {
         wexp[b] = e;
         status[b] = bad ? CG_ERR_NONFINITE : CG_OK;
@@ -174,61 +175,64 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
                                                           const int* __restrict__ wexp, double* __restrict__ A,
                                                           size_t strideA)
 {
-    extern __shared__ Split61 sfix[];
-    __shared__ Split61 dir[2][3][TS];
+    extern __shared__ Split64 sfix[];
+    __shared__ Split64 dir[2][3][TS];
     const int L1 = lmax + 1, b0 = blockIdx.y * NB;
-    Split61* sr = sfix;        // 1 / l
-    Split61* sw = sfix + L1;   // [l][NB]
+    Split64* sr = sfix;        // 1 / l, l > 2
+    Split64* sw = sfix + L1;   // [l][NB]
     int I, J;
     tile_coords(blockIdx.x, I, J);
     for (int l = threadIdx.x; l <= lmax; l += kThreads) {
-        sr[l] = split61(l >= 2 ? (long long)(((1ull << 61) + l / 2) / (unsigned)l) : 0);
+        sr[l] = split64(l > 2 ? (long long)((0ull - (unsigned)l) / (unsigned)l + 1) : 0);  // 2^64 / l
 #pragma unroll
-        for (int q = 0; q < NB; ++q) sw[l * NB + q] = split61(b0 + q < B ? wfix[(size_t)(b0 + q) * L1 + l] : 0);
+        for (int q = 0; q < NB; ++q) sw[l * NB + q] = split64(b0 + q < B ? wfix[(size_t)(b0 + q) * L1 + l] : 0);
     }
     bool beyond = false;
     for (int e = threadIdx.x; e < 6 * TS; e += kThreads) {
         const int s = e / (3 * TS), c = e / TS % 3, i = e % TS;
         const double v = xyz[(size_t)c * N + (s ? J : I) * TS + i];
         beyond |= !(fabs(v) <= 1.0);
-        dir[s][c][i] = split61(to_fixed<62>(v, 1));
+        dir[s][c][i] = split64(2 * to_fixed<62>(v, 1));
     }
     beyond = __syncthreads_or(beyond);
     for (int g = 0; g < TILE_ELEMS / (kThreads * 4); ++g) {
-        Split61 x[4];
+        Split64 x[4];
         long long p0[4], p1[4], acc[NB][4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int e = threadIdx.x + kThreads * (4 * g + q), i = e % TS, j = e / TS;
-            long long v = 0;
+            long long v = 0;  // with 60 fraction bits
             if (!beyond) {
 #pragma unroll
-                for (int c = 0; c < 3; ++c) v += mul61(dir[0][c][i], dir[1][c][j]);
-                v = min(max(v, -(1ll << 61)), 1ll << 61);
+                for (int c = 0; c < 3; ++c) v += mul64(dir[0][c][i], dir[1][c][j]);
+                v = 4 * min(max(v, -(1ll << 60)), 1ll << 60);
             } else if (I * TS + i < n && J * TS + j < n) {
-                v = to_fixed<62>(pair_dot(xyz, N, I * TS + i, J * TS + j), 1);
+                v = 2 * to_fixed<62>(pair_dot(xyz, N, I * TS + i, J * TS + j), 1);
             }
-            x[q] = split61(v);
-            p0[q] = 1ll << 60;
-            p1[q] = v >> 1;
+            // P_2 = 2 t - 1 - (t - 1) / 2, t = x^2
+            x[q] = split64(v);
+            const long long d = 4 * mul64(x[q], x[q]) - (1ll << 62), p = d + (d >> 1) + (1ll << 62);
+            p0[q] = v;
+            p1[q] = p;
+            const Split64 ps = split64(p);
 #pragma unroll
-            for (int k = 0; k < NB; ++k) acc[k][q] = 0;
+            for (int k = 0; k < NB; ++k) acc[k][q] = mul64(ps, sw[2 * NB + k]);
         }
 #pragma unroll 2
-        for (int l = 2; l <= lmax; ++l) {
-            const Split61 rl = sr[l];
-            Split61 w[NB];
+        for (int l = 3; l <= lmax; ++l) {
+            const Split64 rl = sr[l];
+            Split64 w[NB];
 #pragma unroll
             for (int k = 0; k < NB; ++k) w[k] = sw[l * NB + k];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const long long t = mul61(split61(p1[q]), x[q]), d = t - p0[q];
-                const long long p = t + d - mul61(split61(d), rl);
+                const long long t = 4 * mul64(split64(p1[q]), x[q]), d = t - p0[q];
+                const long long p = t + d - mul64(split64(d), rl);
                 p0[q] = p1[q];
                 p1[q] = p;
-                const Split61 ps = split61(p);
+                const Split64 ps = split64(p);
 #pragma unroll
-                for (int k = 0; k < NB; ++k) acc[k][q] += mul61(ps, w[k]);
+                for (int k = 0; k < NB; ++k) acc[k][q] += mul64(ps, w[k]);
             }
         }
 #pragma unroll
@@ -1190,10 +1194,10 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
     // one element per thread block below four: twice the blocks of the shared form, and a single
     // element has nothing to share
     if (B >= 4)
-        build_c_tiled<4><<<dim3(ntile, (B + 3) / 4), kThreads, sizeof(Split61) * 5 * (lmax + 1), s>>>(
+        build_c_tiled<4><<<dim3(ntile, (B + 3) / 4), kThreads, sizeof(Split64) * 5 * (lmax + 1), s>>>(
             n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
     else
-        build_c_tiled<1><<<dim3(ntile, B), kThreads, sizeof(Split61) * 2 * (lmax + 1), s>>>(
+        build_c_tiled<1><<<dim3(ntile, B), kThreads, sizeof(Split64) * 2 * (lmax + 1), s>>>(
             n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
     count_launch(ctx, 2);
     const int drow = grad ? nharm_of(lmax) : 0;
