@@ -164,7 +164,7 @@ __device__ __forceinline__ double* ext_tile(const Dig& g, int b, int eb, int k)
 //
 // The FP64 pipe takes a warp instruction every 64 cycles and SM partition, whatever its active lanes
 // (a lone rsqrt is 456 cycles), so the 64 dependent pivots and the 44 k FMAs of a 64 x 64 factorisation
-// in FP64 took 83 us with the inverse; this takes 34 us, 25 of them the chain of pivots.  CTA 0 factors the block in
+// in FP64 took 83 us with the inverse; this takes 30 us, 23 of them the chain of pivots.  CTA 0 factors the block in
 // integers instead: row r is scaled by 2^-e_r, 2^(2 e_r) above S_rr, so that |S| and |L| are at most 1, held as 2^58
 // times their value.  A product sum is three 32 x 32 -> 64 multiply-adds (64 per cycle) on L = h 2^29 + l: h h'
 // and h l' + l h', l l' (below 2^-56 of a product) left out; the sums cannot overflow, since rows of L
@@ -194,9 +194,9 @@ struct DiagFactor {                     // CTA 0
 struct DiagInverse {                    // the other CTAs
     long long lq[8][8][TS];             // L's columns as they arrive, 8 groups
     double ld[2][8][TS];                // the current group in FP64, two buffers
-    double x[TS][24];                   // rows of this CTA's columns: sums, then the inverse
+    double x[TS][25];                   // rows of this CTA's columns: sums, then the inverse (and one against conflicts)
     double inv[2][8];                   // 1 / L_cc of the current group
-    int smax[kDiagCtas][TS];            // row exponents of each CTA's part
+    int smax[kDiagCtas][TS];            // row exponents of each CTA's part (0: this one's)
 };
 struct DiagShared {
     union {
@@ -526,6 +526,14 @@ __device__ __forceinline__ void diag_factor(DiagShared& sh, const double* __rest
     if (t < kDiagCtas - 1) arrive_cluster(&sh.full[7], 1 + t);
 }
 
+// The blocks of eight columns of the inverse that CTA `rank` forms: block q takes (7 - q)(8 - q) / 2 products of 8 x 8,
+// so 0, 6, 7 | 1, 4, 5 | 2, 3 (28, 30, 25 in all; in order, 0, 1 | 2, 3, 4 | 5, 6, 7, they were 49, 31, 4 and the first
+// CTA ended 7 us after the factor).
+__device__ __forceinline__ int diag_block_of(int rank, int j)
+{
+    return rank == 1 ? (j == 0 ? 0 : 5 + j) : rank == 2 ? (j == 0 ? 1 : 3 + j) : 2 + j;
+}
+
 // a cluster of kDiagCtas CTAs per matrix
 __global__ void __launch_bounds__(kDiagThreads, 1)
     digit_diag(int k, Dig g, double* __restrict__ diag, int* __restrict__ status)
@@ -545,19 +553,18 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
         diag_factor(sh, tile);
         cluster_barrier();
         if (t == 0 && sh.bad && status[b] == CG_OK) status[b] = CG_ERR_NOT_PD;
-        cluster_barrier();
         return;
     }
     if (t >= kDiagOwners) {  // the panel's warps: nothing to do here
         cluster_barrier();
-        cluster_barrier();
         return;
     }
     DiagInverse& v = sh.v;
-    // columns q0 .. q0 + 8 nj - 1
-    const int q0 = rank == 1 ? 0 : rank == 2 ? 16 : 40, nj = rank == 1 ? 2 : 3;
+    const int nj = rank == 3 ? 2 : 3, first = rank - 1;
+    auto block = [&](int j) { return diag_block_of(rank, j); };  // columns 8 block(j) .. 8 block(j) + 7
+    if (t < TS) v.smax[0][t] = -(1 << 28);
     const int r = t / 8, qi = t % 8;
-    double w[3] = {0.0, 0.0, 0.0};  // row r's sums, columns q0 + qi + 8 j
+    double w[3] = {0.0, 0.0, 0.0};  // row r's sums, columns 8 block(j) + qi
     bool ok = true;
     for (int grp = 0; grp < 8; ++grp) {
         ok = wait_cluster(&sh.full[grp], 0) && ok;
@@ -565,7 +572,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
             const int c = 8 * grp + t;
             diag[(size_t)b * g.nt * TS + k * TS + c] = scaled(v.lq[grp][t][c], sh.e[c] - kFrac);
         }
-        if (8 * grp + 7 < q0) continue;
+        if (grp < first) continue;
         double (&ld)[8][TS] = v.ld[grp & 1];
         ld[t / TS][t % TS] = scaled(v.lq[grp][t / TS][t % TS], -kFrac);
         if (t < 8) v.inv[grp & 1][t] = scaled(sh.yq[8 * grp + t], sh.yk[8 * grp + t] - 61);
@@ -581,8 +588,9 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
             const int u = (t % 32) / 8, q = 8 * (t / 32) + qi, m0 = 8 * grp;
             double a0 = v.x[m0 + u][q], a1 = v.x[m0 + u + 4][q];
             // X_mq = (delta - sum) / L_mm; a column beyond the row stays zero
-            a0 = (q0 + q == m0 + u ? 1.0 : 0.0) - a0;
-            a1 = (q0 + q == m0 + u + 4 ? 1.0 : 0.0) - a1;
+            const int col = 8 * block(t / 32) + qi;
+            a0 = (col == m0 + u ? 1.0 : 0.0) - a0;
+            a1 = (col == m0 + u + 4 ? 1.0 : 0.0) - a1;
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const double xm = __shfl_sync(0xffffffffu, (c < 4 ? a0 : a1) * v.inv[grp & 1][c], 8 * (c & 3) + qi);
@@ -595,13 +603,15 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
         }
         named_sync(1, kDiagOwners);
         if (r / 8 > grp) {
+            // (a branch per block: as a condition on each product the pipe took them all)
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const double l = ld[c][r];
+            for (int j = 0; j < 3; ++j)
+                if (j < nj && block(j) <= grp) {
+                    double sum = w[j];
 #pragma unroll
-                for (int j = 0; j < 3; ++j)
-                    if (j < nj && q0 + 8 * j < 8 * grp + 8) w[j] = fma(l, v.x[8 * grp + c][qi + 8 * j], w[j]);
-            }
+                    for (int c = 0; c < 8; ++c) sum = fma(ld[c][r], v.x[8 * grp + c][qi + 8 * j], sum);
+                    w[j] = sum;
+                }
         }
     }
     if (!ok) atomicExch(g.err, 1);
@@ -609,15 +619,20 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     // The inverse's rows in digits (columns scaled back by 2^-e), one exponent per row over all these CTAs:
     // thread (row, 8 columns)
     const int row = t % TS, part = t / TS;
+    int f = -(1 << 28);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int q = 3 * part + c, col = 8 * block(q / 8) + q % 8;
+        const int x = q < 8 * nj ? exp_field(v.x[row][q]) : 0;
+        if (x && col <= row) f = max(f, x == 0x7ff ? kNonFinite : x - sh.e[col]);
+    }
+    atomicMax(&v.smax[0][row], f);
+    named_sync(1, kDiagOwners);
     if (t < TS) {
-        int f = -(1 << 28);
-        for (int q = 0; q < 8 * nj; ++q) {
-            const int x = exp_field(v.x[row][q]);
-            if (q0 + q <= row && x) f = max(f, x == 0x7ff ? kNonFinite : x - sh.e[q0 + q]);
-        }
+        f = v.smax[0][row];
         for (int rk = 1; rk < kDiagCtas; ++rk) st_cluster(mapa(&v.smax[rank][row], rk), f);
     }
-    cluster_barrier();
+    cluster_barrier();  // the last access to another CTA's shared memory
     int e = max(max(v.smax[1][row], v.smax[2][row]), v.smax[3][row]);
     e = e > kNonFinite / 2 ? kNonFinite : e < -(1 << 27) ? -1022 : e - 1022;
     if (rank == 1 && part == 0) g.dex[(size_t)b * TS + row] = e;
@@ -625,13 +640,12 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
         unsigned long long d[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            const int q = 8 * part + c;
-            d[c] = to_digits(q0 + q <= row ? to_fixed(v.x[row][q], e + sh.e[q0 + q]) : 0);
+            const int q = 8 * part + c, col = 8 * block(part) + c;
+            d[c] = to_digits(col <= row ? to_fixed(v.x[row][q], e + sh.e[col]) : 0);
         }
-        unsigned char* o = g.dimg + (size_t)b * kDImg + (q0 / 8 + part) * kDCore + row * 16;
+        unsigned char* o = g.dimg + (size_t)b * kDImg + block(part) * kDCore + row * 16;
         store_digits(d, [&](int i, uint4 x) { *reinterpret_cast<uint4*>(o + i * kDPlane) = x; });
     }
-    cluster_barrier();
 }
 
 // four columns of all eight accumulators (NC columns apart), load and wait in one statement
@@ -1288,19 +1302,19 @@ static int launch_update(cg_ctx* ctx, int B, int k, const UpRange& u, const Dig&
 // The factorisation's chain (diagonal block, panel, the update of the next column pair) beside the rest of
 // the update of the step before, on a second stream and on all but `reserve` SMs: the reserve that makes the
 // longer of the two shortest, or 0 where one after the other is as fast.  Per SM a job takes about 10 us and a
-// panel's CTA 12, the update of one pair 8, a diagonal step 34; a saving below 3 % is left.  One factorisation at
-// nside 16 with its harmonics: 3.94 ms one after the other, 3.16 beside when this came in, 2.48 now; sixteen of them
+// panel's CTA 12, the update of one pair 8, a diagonal step 30; a saving below 3 % is left.  One factorisation at
+// nside 16 with its harmonics: 3.94 ms one after the other, 3.16 beside when this came in, 2.26 now; sixteen of them
 // 14.94 -> 14.43 ms with the line at 3 % instead of 7 (14.10 at 2 %, but eight without harmonics 3.57 -> 3.63).
 static int chain_reserve(const cg_ctx* ctx, int B, int nq, int npe, int v)
 {
     const UpRange all = {0, nq, npe, v}, one = {0, 1, npe, 0};
     const double sms = ctx->sm_count, col = (double)up_jobs(one, nq) * B, jobs = (double)up_jobs(all, nq) * B;
     auto waves = [](double n, double s) { return std::max(1.0, std::ceil(n / s)); };
-    const double serial = 34 + 12 * waves(col, sms) + 10 * waves(jobs, sms) + 6;
+    const double serial = 30 + 12 * waves(col, sms) + 10 * waves(jobs, sms) + 6;
     double best = 0.97 * serial;
     int reserve = 0;
     for (int r = 8; r <= ctx->sm_count / 2; r += 8) {
-        const double chain = 34 * waves((double)kDiagCtas * B, r) + 20 * waves(col, r) + 8;
+        const double chain = 30 * waves((double)kDiagCtas * B, r) + 20 * waves(col, r) + 8;
         const double t = std::max(chain, 10 * waves(jobs - col, sms - r) + 4);
         if (t < best) {
             best = t;
