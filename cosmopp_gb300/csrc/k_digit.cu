@@ -695,7 +695,7 @@ __device__ __forceinline__ long long join_acc4(const uint32_t (&r)[8][4], int q)
 // (E's rows also to FP64, which the solve and the gradient read).  Thread (row m of the pair image,
 // columns 16 cq .. 16 cq + 15).  The chain of loads, row maximum, digits, products, row maximum, digits
 // bounds it; the loops over 8 columns stay rolled and read their input twice (the tile, the
-// accumulators), since the unrolled form spent a third of its 30 us waiting for instructions.
+// joined accumulators), since the unrolled form spent a third of its 30 us waiting for instructions.
 constexpr int kPanelA = 0, kPanelB = kImg, kPanelTail = kImg + kDImg;
 constexpr int kPanelThreads = 512;
 constexpr int kPanelSmem = kPanelTail + 4 * 128 * 4 + TS * 4;
@@ -773,7 +773,8 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
     if (!ok) atomicExch(g.err, 1);
     fence_after();
     __syncwarp();
-    // this thread's entries in units of 2^(ea + deb[c] - 55), and the row's largest
+    // this thread's entries in units of 2^(ea + deb[c] - 55), into the place of the rows' digits, and the row's largest
+    long long* const mine = reinterpret_cast<long long*>(sm + kPanelA) + t;
     const uint32_t ta = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + 16 * cq;
     int top = -(1 << 28);
 #pragma unroll 1
@@ -784,6 +785,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const long long x = join_acc4(acc, c);
+            mine[kPanelThreads * (4 * h + c)] = x;
             const int e = deb[16 * cq + 4 * h + c];
             if (x != 0 || e == kNonFinite) top = max(top, e + 64 - __clzll(x < 0 ? -x : x));
         }
@@ -801,22 +803,27 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
         unsigned long long w[8];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            uint32_t acc[8][4];
-            __syncwarp();
-            tmem_ld_acc4<TS>(ta + 8 * h + 4 * q, acc);
+            long long x[4];
+            int sx[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int col = 8 * h + 4 * q + c, de = deb[16 * cq + col];
-                const long long x = join_acc4(acc, c);
+                x[c] = mine[kPanelThreads * col];
+                sx[c] = ea + de - 55;
                 // X = x 2^(de - top + 54): |x| < 2^(top - de), so |X| < 2^54
                 const int sh = de - top + 54;
                 long long y = 0;
                 if (!nonfinite) {
-                    if (sh >= 0) y = x << min(sh, 63);
-                    else if (sh > -64) y = ((x >> (-sh - 1)) + 1) >> 1;
+                    if (sh >= 0) y = x[c] << min(sh, 63);
+                    else if (sh > -64) y = ((x[c] >> (-sh - 1)) + 1) >> 1;
                 }
                 w[4 * q + c] = to_digits(y);
-                if (wide) tile[TS * col] = scaled_int(x, ea + de - 55, 0);
+            }
+            if (wide) {
+                double d[4];
+                scaled_ints<4>(x, sx, 0, d);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tile[TS * (8 * h + 4 * q + c)] = d[c];
             }
         }
         unsigned char* o = out + (2 * cq + h) * kCore;
