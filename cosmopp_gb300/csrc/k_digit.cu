@@ -19,7 +19,7 @@
 // likelihood: y = L^-1 d, Z = L^-1 Y.  With E = identity it is M^T, M = L^-1, and the same update
 // kernel also sums V = M^T M = A^-1.  Per step k (64 columns):
 //
-//   digit_diag    L_kk and its inverse (FP64, one CTA per matrix), the inverse in digits
+//   digit_diag    L_kk (fixed point) and its inverse (FP64), four CTAs per matrix, the inverse in digits
 //   digit_panel   L_ik = S_ik L_kk^-T for the rows below and E's rows, left in digits
 //   digit_update  S_ij -= L_ik L_jk^T over the trailing trapezoid, V_ij += M_ki^T M_kj
 //

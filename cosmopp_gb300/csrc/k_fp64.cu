@@ -1,18 +1,19 @@
 // Plain FP64 path: covariance build, likelihood and adjoint gradient.
 //
-// build_c_tiled / build_c_packed replace CMatrixGenerator::clToCMatrix
+// build_c_packed and build_c_ref replace CMatrixGenerator::clToCMatrix
 // (source/c_matrix_generator.cpp:164-232).  Each thread runs the Bonnet
 // recurrence once per pixel pair in registers; the reference restarts it for
 // every l (include/legendre.hpp:26-37) but produces the same P_l values bit for
 // bit, and the element sum keeps the reference's operation order
 //   element += ((clCopy_l * P_l) * B_l) * B_l
 // with explicitly rounded (non-fused) FP64 operations, so C is bit-identical
-// to the reference's.
+// to the reference's.  build_c_tiled, inside the likelihood, forms the same sum in
+// 64-bit fixed point, nearer to the exact value.
 //
 // The likelihood follows Likelihood::construct / calculate
-// (source/likelihood.cpp:69-180): C + N, Cholesky (k_chol.cu), ln det from
-// the factor's diagonal, explicit inverse, chi2 = d^T C^-1 d.  The adjoint
-// gradient (no reference counterpart) is
+// (source/likelihood.cpp:69-180): C + N, Cholesky of [C; harmonics, map] (k_digit.cu), ln det
+// from the factor's diagonal, chi2 = |L^-1 d|^2; the packed likelihoods keep C^-1 instead.  The
+// adjoint gradient (no reference counterpart) is
 //   d(-2lnL)/dC_l = sum_ij (C^-1 - a a^T)_ij (2l+1)/(4pi) B_l^2 P_l(x_ij),  a = C^-1 d.
 #include <algorithm>
 #include <cmath>
