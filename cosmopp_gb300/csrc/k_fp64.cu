@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, 
 // sum becomes FP64 in integer operations.  The sum is 50 to 200 times nearer to the exact value than the FP64
 // recurrence's (lmax 12 to 255).  The P_l are shared by NB batch elements.  The integer pipes bound it (47
 // instructions per pair and l with one element, 57 % of the issue slots, 64 % of the multiply-add pipe): one matrix at
-// nside 16 2650 us in FP64, 418 with halves of 31 bits, 355 here; sixteen 42 ms, 2.9, 2.3.
+// nside 16 2650 us in FP64, 418 with halves of 31 bits, 322 here; sixteen 42 ms, 2.9, 2.3.
 
 // status and fixed-point weights of every element: wfix[b][l] = w_l 2^(62 - e), wexp[b] = e with
 // sum |w_l| < 2^e; a non-finite weight gives e = kNonFinite and a NaN covariance.  grid B
@@ -165,9 +165,12 @@ __global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const dou
     }
 }
 
-// C (+ noise on the diagonal, identity padding) into the tiled layout; grid (tiles, ceil(B / NB)),
-// 4 pairs per thread and pass.  Directions with a component beyond 1 (a caller's, off the unit
+// C (+ noise on the diagonal, identity padding) into the tiled layout; grid (tiles * kBuildParts, ceil(B / NB)), a CTA
+// per quarter of a tile, 4 pairs per thread (a CTA per tile left SMs idle: the 55 tiles of nside 8 took 41 us, now 23
+// less; the 820 of nside 16, 1.3 waves, 355, now 322).  Directions with a component beyond 1 (a caller's, off the unit
 // sphere) take their dot product in FP64, with the reference's clamp.
+constexpr int kBuildParts = TILE_ELEMS / (kThreads * 4);
+
 template <int NB>
 __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax, int B,
                                                           const double* __restrict__ xyz,
@@ -181,8 +184,9 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
     const int L1 = lmax + 1, b0 = blockIdx.y * NB;
     Split64* sr = sfix;        // 1 / l, l > 2
     Split64* sw = sfix + L1;   // [l][NB]
+    const int tix = blockIdx.x / kBuildParts, g = blockIdx.x % kBuildParts;
     int I, J;
-    tile_coords(blockIdx.x, I, J);
+    tile_coords(tix, I, J);
     for (int l = threadIdx.x; l <= lmax; l += kThreads) {
         sr[l] = split64(l > 2 ? (long long)((0ull - (unsigned)l) / (unsigned)l + 1) : 0);  // 2^64 / l
 #pragma unroll
@@ -196,65 +200,63 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
         dir[s][c][i] = split64(2 * to_fixed<62>(v, 1));
     }
     beyond = __syncthreads_or(beyond);
-    for (int g = 0; g < TILE_ELEMS / (kThreads * 4); ++g) {
-        Split64 x[4];
-        long long p0[4], p1[4], acc[NB][4];
+    Split64 x[4];
+    long long p0[4], p1[4], acc[NB][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int e = threadIdx.x + kThreads * (4 * g + q), i = e % TS, j = e / TS;
+        long long v = 0;  // with 60 fraction bits
+        if (!beyond) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v += mul64(dir[0][c][i], dir[1][c][j]);
+            v = 4 * min(max(v, -(1ll << 60)), 1ll << 60);
+        } else if (I * TS + i < n && J * TS + j < n) {
+            v = 2 * to_fixed<62>(pair_dot(xyz, N, I * TS + i, J * TS + j), 1);
+        }
+        // P_2 = 2 t - 1 - (t - 1) / 2, t = x^2
+        x[q] = split64(v);
+        const long long d = 4 * mul64(x[q], x[q]) - (1ll << 62), p = d + (d >> 1) + (1ll << 62);
+        p0[q] = v;
+        p1[q] = p;
+        const Split64 ps = split64(p);
+#pragma unroll
+        for (int k = 0; k < NB; ++k) acc[k][q] = mul64(ps, sw[2 * NB + k]);
+    }
+#pragma unroll 2
+    for (int l = 3; l <= lmax; ++l) {
+        const Split64 rl = sr[l];
+        Split64 w[NB];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) w[k] = sw[l * NB + k];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int e = threadIdx.x + kThreads * (4 * g + q), i = e % TS, j = e / TS;
-            long long v = 0;  // with 60 fraction bits
-            if (!beyond) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) v += mul64(dir[0][c][i], dir[1][c][j]);
-                v = 4 * min(max(v, -(1ll << 60)), 1ll << 60);
-            } else if (I * TS + i < n && J * TS + j < n) {
-                v = 2 * to_fixed<62>(pair_dot(xyz, N, I * TS + i, J * TS + j), 1);
-            }
-            // P_2 = 2 t - 1 - (t - 1) / 2, t = x^2
-            x[q] = split64(v);
-            const long long d = 4 * mul64(x[q], x[q]) - (1ll << 62), p = d + (d >> 1) + (1ll << 62);
-            p0[q] = v;
+            const long long t = 4 * mul64(split64(p1[q]), x[q]), d = t - p0[q];
+            const long long p = t + d - mul64(split64(d), rl);
+            p0[q] = p1[q];
             p1[q] = p;
             const Split64 ps = split64(p);
 #pragma unroll
-            for (int k = 0; k < NB; ++k) acc[k][q] = mul64(ps, sw[2 * NB + k]);
+            for (int k = 0; k < NB; ++k) acc[k][q] += mul64(ps, w[k]);
         }
-#pragma unroll 2
-        for (int l = 3; l <= lmax; ++l) {
-            const Split64 rl = sr[l];
-            Split64 w[NB];
+    }
 #pragma unroll
-            for (int k = 0; k < NB; ++k) w[k] = sw[l * NB + k];
+    for (int k = 0; k < NB; ++k) {
+        if (b0 + k >= B) break;
+        const int we = wexp[b0 + k];
+        double* tile = A + (size_t)(b0 + k) * strideA + (size_t)tix * TILE_ELEMS;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const long long t = 4 * mul64(split64(p1[q]), x[q]), d = t - p0[q];
-                const long long p = t + d - mul64(split64(d), rl);
-                p0[q] = p1[q];
-                p1[q] = p;
-                const Split64 ps = split64(p);
-#pragma unroll
-                for (int k = 0; k < NB; ++k) acc[k][q] += mul64(ps, w[k]);
+        for (int q = 0; q < 4; ++q) {
+            const int e = threadIdx.x + kThreads * (4 * g + q), i = I * TS + e % TS, j = J * TS + e / TS;
+            double val;
+            if (i < n && j < n) {
+                // a non-finite weight's exponent gives NaN
+                val = scaled_int(acc[k][q], we - 60, 0);
+                // cInv_(i,j) = c + fiducial(0) + noise  (source/likelihood.cpp:102-110)
+                if (i == j) val = __dadd_rn(val, noise[i]);
+            } else {
+                val = (i == j) ? 1.0 : 0.0;
             }
-        }
-#pragma unroll
-        for (int k = 0; k < NB; ++k) {
-            if (b0 + k >= B) break;
-            const int we = wexp[b0 + k];
-            double* tile = A + (size_t)(b0 + k) * strideA + (size_t)blockIdx.x * TILE_ELEMS;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int e = threadIdx.x + kThreads * (4 * g + q), i = I * TS + e % TS, j = J * TS + e / TS;
-                double val;
-                if (i < n && j < n) {
-                    // a non-finite weight's exponent gives NaN
-                    val = scaled_int(acc[k][q], we - 60, 0);
-                    // cInv_(i,j) = c + fiducial(0) + noise  (source/likelihood.cpp:102-110)
-                    if (i == j) val = __dadd_rn(val, noise[i]);
-                } else {
-                    val = (i == j) ? 1.0 : 0.0;
-                }
-                tile[e] = val;
-            }
+            tile[e] = val;
         }
     }
 }
@@ -1195,10 +1197,10 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
     // one element per thread block below four: twice the blocks of the shared form, and a single
     // element has nothing to share
     if (B >= 4)
-        build_c_tiled<4><<<dim3(ntile, (B + 3) / 4), kThreads, sizeof(Split64) * 5 * (lmax + 1), s>>>(
+        build_c_tiled<4><<<dim3(ntile * kBuildParts, (B + 3) / 4), kThreads, sizeof(Split64) * 5 * (lmax + 1), s>>>(
             n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
     else
-        build_c_tiled<1><<<dim3(ntile, B), kThreads, sizeof(Split64) * 2 * (lmax + 1), s>>>(
+        build_c_tiled<1><<<dim3(ntile * kBuildParts, B), kThreads, sizeof(Split64) * 2 * (lmax + 1), s>>>(
             n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
     count_launch(ctx, 2);
     const int drow = grad ? nharm_of(lmax) : 0;
