@@ -20,6 +20,7 @@
 
 #include "cg_fixed.cuh"
 #include "cg_internal.h"
+#include "cg_launch.cuh"
 
 namespace cg {
 
@@ -137,14 +138,15 @@ __global__ void __launch_bounds__(kThreads) build_c_ref(int n, int N, int lmax, 
 // instructions per pair and l with one element, 57 % of the issue slots, 64 % of the multiply-add pipe): one matrix at
 // nside 16 2650 us in FP64, 418 with halves of 31 bits, 322 here; sixteen 42 ms, 2.9, 2.3.
 
-// status and fixed-point weights of every element: wfix[b][l] = w_l 2^(62 - e), wexp[b] = e with
+// status, the waits' error flag and fixed-point weights of every element: wfix[b][l] = w_l 2^(62 - e), wexp[b] = e with
 // sum |w_l| < 2^e; a non-finite weight gives e = kNonFinite and a NaN covariance.  grid B
 __global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const double* __restrict__ beam,
                                                              const double* __restrict__ cl,
                                                              long long* __restrict__ wfix, int* __restrict__ wexp,
-                                                             int* __restrict__ status)
+                                                             int* __restrict__ status, int* __restrict__ err)
 {
     __shared__ double part[kThreads / 32];
+    launch_dependents();
     const int b = blockIdx.x, l = threadIdx.x, L1 = lmax + 1;
     const double c = l <= lmax ? cl[(size_t)b * L1 + l] : 0.0;
     // clCopy[l] = cl[l] * (2 l + 1) / (4 pi)   (c_matrix_generator.cpp:190-193)
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(kThreads) legendre_weights(int lmax, const dou
     if (l == 0) {
         wexp[b] = e;
         status[b] = bad ? CG_ERR_NONFINITE : CG_OK;
+        if (b == 0) *err = 0;
     }
 }
 
@@ -182,6 +185,8 @@ __global__ void __launch_bounds__(kThreads) build_c_tiled(int n, int N, int lmax
     extern __shared__ Split64 sfix[];
     __shared__ Split64 dir[2][3][TS];
     const int L1 = lmax + 1, b0 = blockIdx.y * NB;
+    wait_prior();
+    launch_dependents();       // not before: ext_rows runs beside this without waiting for it
     Split64* sr = sfix;        // 1 / l, l > 2
     Split64* sw = sfix + L1;   // [l][NB]
     const int tix = blockIdx.x / kBuildParts, g = blockIdx.x % kBuildParts;
@@ -432,6 +437,8 @@ constexpr int kLogThreads = 1024;
 __global__ void __launch_bounds__(kLogThreads) logdet_reduce(int n, int N, const double* __restrict__ diag,
                                                              double* __restrict__ logdet)
 {
+    launch_dependents();
+    wait_prior();
     __shared__ double red[kLogThreads];
     const int b = blockIdx.x;
     double s = 0.0;
@@ -576,6 +583,8 @@ __global__ void adjoint_finish(int lmax, int ntile, const double* __restrict__ g
 // a bounded device wait that gave up (*err) marks every element of the batch
 __global__ void copy_status(int B, const int* __restrict__ src, const int* __restrict__ err, int* __restrict__ dst)
 {
+    launch_dependents();
+    wait_prior();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < B) dst[b] = *err ? CG_ERR_TIMEOUT : src[b];
 }
@@ -856,6 +865,7 @@ __global__ void __launch_bounds__(kThreads) ext_rows(int n, int nt, int drow, co
                                                      const double* __restrict__ d, int d_stride,
                                                      double* __restrict__ E, size_t strideE)
 {
+    launch_dependents();
     const int k = blockIdx.x, eb = blockIdx.y, b = blockIdx.z;
     const size_t off = ((size_t)eb * nt + k) * TILE_ELEMS;
     double* tile = E + (size_t)b * strideE + off;
@@ -868,13 +878,17 @@ __global__ void __launch_bounds__(kThreads) ext_rows(int n, int nt, int drow, co
         }
         tile[e] = v;
     }
+    wait_prior();  // the covariance, for the kernels after this one
 }
 
 // y = L^-1 d from E's row drow, chi2 = y . y, m2lnl = chi2 + logdet; grid B
 __global__ void __launch_bounds__(kThreads) chi2_rows(int nt, int drow, const double* __restrict__ E, size_t strideE,
                                                       const double* __restrict__ logdet, double* __restrict__ y,
-                                                      double* __restrict__ m2lnl, double* __restrict__ chi2)
+                                                      double* __restrict__ m2lnl, double* __restrict__ chi2,
+                                                      double* __restrict__ logdet_out)
 {
+    launch_dependents();
+    wait_prior();
     __shared__ double red[kThreads];
     const int b = blockIdx.x, N = nt * TS;
     const double* Eb = E + (size_t)b * strideE + (size_t)(drow / TS) * nt * TILE_ELEMS + drow % TS;
@@ -892,6 +906,7 @@ __global__ void __launch_bounds__(kThreads) chi2_rows(int nt, int drow, const do
     }
     if (threadIdx.x == 0) {
         if (chi2) chi2[b] = red[0];
+        if (logdet_out) logdet_out[b] = logdet[b];
         m2lnl[b] = red[0] + logdet[b];
     }
 }
@@ -904,6 +919,8 @@ constexpr int kHarmSplit = 8;
 __global__ void __launch_bounds__(kThreads) harmonic_sums(int nt, int ne, const double* __restrict__ E, size_t strideE,
                                                           const double* __restrict__ y, double* __restrict__ part)
 {
+    launch_dependents();
+    wait_prior();
     __shared__ double red[2][4][TS];
     const int eb = blockIdx.x, z = blockIdx.y, b = blockIdx.z, r = threadIdx.x % TS, q = threadIdx.x / TS;
     const double* Eb = E + (size_t)b * strideE + (size_t)eb * nt * TILE_ELEMS;
@@ -930,6 +947,8 @@ __global__ void __launch_bounds__(kThreads) harmonic_sums(int nt, int ne, const 
 __global__ void __launch_bounds__(kThreads) harmonic_grad(int lmax, int ne, const double* __restrict__ part,
                                                           double* __restrict__ grad)
 {
+    launch_dependents();
+    wait_prior();
     const int b = blockIdx.y, l = blockIdx.x * (kThreads / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
     if (l > lmax) return;
     const size_t nh = (size_t)ne * TS;
@@ -1192,41 +1211,41 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
     const int ntile = ntiles_lower(nt), ne = ext_blocks(ctx, grad);
     const bool inverse = grad && !ctx->harm;
     stage_mark(ctx, ST_BUILD, s);
-    CG_CUDA_TRY(ctx, cudaMemsetAsync(w.err, 0, sizeof(int), s));
-    legendre_weights<<<B, kThreads, 0, s>>>(lmax, ctx->d_beam, d_cl, w.wfix, w.wexp, w.st);
+    // The small kernels on either side of the factorisation overlap each other's ends, and ext_rows runs beside the
+    // build (one value at nside 4 318 -> 304 us, a gradient at nside 8 691 -> 671).
+    legendre_weights<<<B, kThreads, 0, s>>>(lmax, ctx->d_beam, d_cl, w.wfix, w.wexp, w.st, w.err);
+    count_launch(ctx);
     // one element per thread block below four: twice the blocks of the shared form, and a single
     // element has nothing to share
-    if (B >= 4)
-        build_c_tiled<4><<<dim3(ntile * kBuildParts, (B + 3) / 4), kThreads, sizeof(Split64) * 5 * (lmax + 1), s>>>(
-            n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
-    else
-        build_c_tiled<1><<<dim3(ntile * kBuildParts, B), kThreads, sizeof(Split64) * 2 * (lmax + 1), s>>>(
-            n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix, w.wexp, w.A, strideA);
-    count_launch(ctx, 2);
+    const int nb = B >= 4 ? 4 : 1;
+    if ((rc = launch(ctx, nb == 4 ? build_c_tiled<4> : build_c_tiled<1>, dim3(ntile * kBuildParts, (B + nb - 1) / nb), kThreads,
+                     sizeof(Split64) * (nb + 1) * (lmax + 1), 1, s, n, N, lmax, B, ctx->d_xyz, ctx->d_noise, w.wfix,
+                     w.wexp, w.A, strideA)))
+        return rc;
     const int drow = grad ? nharm_of(lmax) : 0;
     if (inverse) {
         if ((rc = fp64_identity_rows(ctx, B, nt, w.E, w.ext_elems, s))) return rc;
     } else {
-        ext_rows<<<dim3(nt, ne, B), kThreads, 0, s>>>(n, nt, drow, grad ? w.Yt : nullptr, d_d, d_stride, w.E,
-                                                      w.ext_elems);
-        count_launch(ctx);
+        if ((rc = launch(ctx, ext_rows, dim3(nt, ne, B), kThreads, 0, 1, s, n, nt, drow, grad ? w.Yt : nullptr, d_d, d_stride,
+                         w.E, w.ext_elems)))
+            return rc;
     }
     stage_mark(ctx, ST_CHOL, s);
     if ((rc = digit_factor(ctx, B, nt, ne, inverse ? DIGIT_EXT_IDENTITY : DIGIT_EXT_ROWS, w.A, strideA, w.E,
                            w.ext_elems, w.diag, w.st, w.dig, w.err, s)))
         return rc;
     stage_mark(ctx, ST_SOLVE, s);
-    logdet_reduce<<<B, kLogThreads, 0, s>>>(n, N, w.diag, w.ld);
+    if ((rc = launch(ctx, logdet_reduce, dim3(B), kLogThreads, 0, 1, s, n, N, w.diag, w.ld))) return rc;
     if (inverse) {
         pad_data<<<dim3((N + 255) / 256, B), 256, 0, s>>>(n, N, B, d_d, d_stride, w.dvec);
         symv_tiled<double><<<dim3(nt, B), kThreads, 0, s>>>(nt, N, w.A, strideA, w.dvec, w.alpha);
         chi2_finish<<<B, kThreads, 0, s>>>(n, N, w.dvec, w.alpha, w.ld, d_m2lnl, d_chi2);
-        count_launch(ctx, 4);
-    } else {
-        chi2_rows<<<B, kThreads, 0, s>>>(nt, drow, w.E, w.ext_elems, w.ld, w.alpha, d_m2lnl, d_chi2);
-        count_launch(ctx, 2);
+        count_launch(ctx, 3);
+        if (d_logdet) CG_CUDA_TRY(ctx, cudaMemcpyAsync(d_logdet, w.ld, sizeof(double) * B, cudaMemcpyDeviceToDevice, s));
+    } else if ((rc = launch(ctx, chi2_rows, dim3(B), kThreads, 0, 1, s, nt, drow, w.E, w.ext_elems, w.ld, w.alpha, d_m2lnl,
+                            d_chi2, d_logdet))) {
+        return rc;
     }
-    if (d_logdet) CG_CUDA_TRY(ctx, cudaMemcpyAsync(d_logdet, w.ld, sizeof(double) * B, cudaMemcpyDeviceToDevice, s));
     stage_mark(ctx, ST_ADJOINT, s);
     if (inverse) {
         for (int l0 = 2; l0 <= lmax; l0 += kAdjChunk) {
@@ -1238,11 +1257,12 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
         adjoint_finish<<<B, 64, 0, s>>>(lmax, ntile, w.gpart, ctx->d_beam, d_grad);
         count_launch(ctx);
     } else if (grad) {
-        harmonic_sums<<<dim3(ne, kHarmSplit, B), kThreads, 0, s>>>(nt, ne, w.E, w.ext_elems, w.alpha, w.gpart);
-        harmonic_grad<<<dim3((lmax + 8) / 8, B), kThreads, 0, s>>>(lmax, ne, w.gpart, d_grad);
-        count_launch(ctx, 2);
+        if ((rc = launch(ctx, harmonic_sums, dim3(ne, kHarmSplit, B), kThreads, 0, 1, s, nt, ne, w.E, w.ext_elems, w.alpha,
+                         w.gpart)) ||
+            (rc = launch(ctx, harmonic_grad, dim3((lmax + 8) / 8, B), kThreads, 0, 1, s, lmax, ne, w.gpart, d_grad)))
+            return rc;
     }
-    if (d_status) { copy_status<<<(B + 127) / 128, 128, 0, s>>>(B, w.st, w.err, d_status); count_launch(ctx); }
+    if (d_status && (rc = launch(ctx, copy_status, dim3((B + 127) / 128), 128, 0, 1, s, B, w.st, w.err, d_status))) return rc;
     stage_mark(ctx, ST_END, s);
     CG_CUDA_TRY(ctx, cudaGetLastError());
     return CG_OK;
