@@ -1009,8 +1009,8 @@ __global__ void __launch_bounds__(kUpThreads, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = tptr;
-    wait_prior();
     bool ok = true;
+    // (the jobs are worked out before the wait for the kernel before this one, which precedes every access to memory)
     if (warp == kUpWarps + 1) {
         if (lane == 0) {
             uint32_t aphase = 0, bphase = 0;  // uses so far, mod 2: of A, of piece i in bit i
@@ -1022,16 +1022,20 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                 else d.i0 = d.i1 = 0;
                 mbar_arrive(&dfull[s % kUpDescs]);
             };
-            int job = up_at(0, njobs);
-            UpJob j = up_job(g, u, per, max(job, 0));
+            int job = up_at(0, njobs), next = -1;
+            UpJob j = up_job(g, u, per, max(job, 0)), n = j;
             const int pairs = dig_pairs(g);
-            bool fresh = true;
+            bool fresh = true, same = false;
             put(0, job, j, true);
+            auto ahead = [&](int s) {  // the job after this one, s, into its slot
+                next = up_at(s, njobs);
+                n = up_job(g, u, per, max(next, 0));
+                same = nk == 1 && next >= 0 && n.b == j.b && n.pa == j.pa;
+                put(s, next, n, !same);
+            };
+            if (job >= 0) ahead(1);
+            wait_prior();
             for (int s = 0; job >= 0; ++s) {
-                const int next = up_at(s + 1, njobs);
-                const UpJob n = up_job(g, u, per, max(next, 0));
-                const bool same = nk == 1 && next >= 0 && n.b == j.b && n.pa == j.pa;
-                put(s + 1, next, n, !same);
                 if (g.prefetch && next >= 0) {  // the next job's tiles on their way from DRAM
                     const UpDesc& d = desc[(s + 1) % kUpDescs];
 #pragma unroll 1
@@ -1071,6 +1075,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                 job = next;
                 j = n;
                 fresh = !same;
+                if (job >= 0) ahead(s + 2);
             }
         }
         __syncwarp();
@@ -1112,6 +1117,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
         }
         __syncwarp();
     } else {
+        wait_prior();
         const int m = 32 * (warp & 3) + lane, c4 = warp >> 2;  // row of the pair image, 8-column group of the pass
         const int half = m >> 6, r = m & 63;
         int s = 0, i = 0, i0 = 0, i1 = 0, ks = 0;
