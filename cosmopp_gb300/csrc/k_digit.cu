@@ -1287,7 +1287,7 @@ static int launch_update(cg_ctx* ctx, int B, int k, const UpRange& u, const Dig&
 // the update of the step before, on a second stream and on all but `reserve` SMs: the reserve that makes the
 // longer of the two shortest, or 0 where one after the other is as fast.  Per SM a job takes about 10 us and a
 // panel's CTA 12, the update of one pair 8, a diagonal step 30; a saving below 3 % is left.  One factorisation at
-// nside 16 with its harmonics: 3.94 ms one after the other, 3.16 beside when this came in, 2.26 now; sixteen of them
+// nside 16 with its harmonics: 3.94 ms one after the other, 3.16 beside when this came in, 2.16 now; sixteen of them
 // 14.94 -> 14.43 ms with the line at 3 % instead of 7 (14.10 at 2 %, but eight without harmonics 3.57 -> 3.63).
 static int chain_reserve(const cg_ctx* ctx, int B, int nq, int npe, int v)
 {

@@ -255,3 +255,17 @@ def test_packed_covariance_rounds_every_operation(case, batch):
         for l in range(2, lmax + 1):
             want += ((((cls[b, l] * (2 * l + 1)) / (4 * np.pi)) * p[l]) * beam[l]) * beam[l]
         assert np.array_equal(got[b], W.full_to_packed(want))
+
+
+@pytest.mark.parametrize("n,lmax,batch", [(450, 11, 100), (700, 14, 40), (1300, 20, 12), (200, 20, 150)])
+def test_elements_of_a_batch_keep_the_bits_of_a_call_of_their_own(n, lmax, batch):
+    """A CTA's runs of jobs over several rounds and a remainder, the chain beside the rest of an update or before it,
+    and the split of a column pair between them order the work differently, never an element's operations."""
+    v, cls, d = _setup(n, lmax, 17, batch)
+    with cg.Context(lmax=lmax, fwhm_deg=9.0, dirs=v, noise_sigma=1.0, max_batch=batch) as ctx:
+        full = ctx.loglike(cls, d[0], grad=True)
+        assert np.all(full["status"] == cg.CG_OK)
+        for b in (0, batch // 2, batch - 1):
+            one = ctx.loglike(cls[b:b + 1], d[0], grad=True)
+            for name in ("m2lnl", "chi2", "logdet", "grad"):
+                assert np.array_equal(full[name][b], one[name][0]), (name, b)
