@@ -7,7 +7,10 @@
 //
 //   * each row of an operand block (64 columns) gets a power of two 2^e above its largest entry and
 //     is rounded to a 55-bit fixed-point number x = 2^(e-54) X, X written in seven signed base-256
-//     digits d_0 .. d_6 (|d| <= 128), each exact in BF16;
+//     digits d_0 .. d_6 (|d| <= 128), each exact in BF16.  An entry far below its row's largest thus keeps
+//     fewer bits than in FP64, so the columns of an operand are brought to one scale first where the other
+//     operand has the opposite one: S_ik = L_ik L_kk^T by the diagonal block's scales (diag_scale).
+//     L's own columns need none: row i of L has norm sqrt(A_ii);
 //   * the digit products i + j <= 7 run on the tensor cores, summed over the 64 columns in eight FP32
 //     accumulators, one per i + j.  Every partial sum is a whole number below 2^23 (64 columns, at
 //     most 6 pairs of 2^14), so FP32 accumulation is exact;
@@ -153,6 +156,22 @@ __device__ __forceinline__ double* ext_tile(const Dig& g, int b, int eb, int k)
 {
     const size_t t = g.ext == DIGIT_EXT_IDENTITY ? (size_t)tile_index(k, eb) : (size_t)eb * g.nt + k;
     return g.E + (size_t)b * g.strideE + t * TILE_ELEMS;
+}
+
+// e with S_rr < 2^(2 e) for an entry of the diagonal: row r of the factor is below 2^e, and column r of what the
+// panel multiplies by the inverse is scaled by 2^-e.  (With one exponent for a row of S and no scales, pixels of
+// sigma 1 and 1e9 side by side left chi2 with a relative error of 1e-9 where the FP64 factorisation has 1e-15.)
+__device__ __forceinline__ int diag_scale(double s) { return (exp_field(s) - 1022 + 1) >> 1; }
+
+// a row's exponent from the largest of its entries' scaled_field: |v 2^-e| < 2^(row exponent)
+__device__ __forceinline__ int scaled_field(double v, int e)
+{
+    const int f = exp_field(v);
+    return f == 0x7ff ? kNonFinite : f == 0 ? -(1 << 28) : f - e;
+}
+__device__ __forceinline__ int scaled_row_exp(int field)
+{
+    return field > kNonFinite / 2 ? kNonFinite : field < -(1 << 27) ? -1022 : field - 1022;
 }
 
 // ---- diagonal block: L_kk in 64-bit fixed point, its inverse in FP64, one cluster per matrix ----
@@ -542,7 +561,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     fence_mbar_init();
     wait_prior();
     launch_dependents();  // not before: the panel reads column k ahead of its own wait
-    if (t < TS) sh.e[t] = (exp_field(tile[t * (TS + 1)]) - 1022 + 1) >> 1;  // S_rr < 2^(2 e)
+    if (t < TS) sh.e[t] = diag_scale(tile[t * (TS + 1)]);
     cluster_barrier();
     if (rank == 0) {
         diag_factor(sh, tile);
@@ -611,15 +630,14 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     }
     if (!ok) atomicExch(g.err, 1);
     named_sync(1, kDiagOwners);
-    // The inverse's rows in digits (columns scaled back by 2^-e), one exponent per row over all these CTAs:
-    // thread (row, 8 columns)
+    // The rows of the scaled factor's inverse in digits, one exponent per row over all these CTAs: thread (row, 8
+    // columns).  The panel's rows carry the scales.
     const int row = t % TS, part = t / TS;
     int f = -(1 << 28);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const int q = 3 * part + c, col = 8 * block(q / 8) + q % 8;
-        const int x = q < 8 * nj ? exp_field(v.x[row][q]) : 0;
-        if (x && col <= row) f = max(f, x == 0x7ff ? kNonFinite : x - sh.e[col]);
+        if (q < 8 * nj && col <= row) f = max(f, scaled_field(v.x[row][q], 0));
     }
     atomicMax(&v.smax[0][row], f);
     named_sync(1, kDiagOwners);
@@ -628,15 +646,14 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
         for (int rk = 1; rk < kDiagCtas; ++rk) st_cluster(mapa(&v.smax[rank][row], rk), f);
     }
     cluster_barrier();  // the last access to another CTA's shared memory
-    int e = max(max(v.smax[1][row], v.smax[2][row]), v.smax[3][row]);
-    e = e > kNonFinite / 2 ? kNonFinite : e < -(1 << 27) ? -1022 : e - 1022;
+    const int e = scaled_row_exp(max(max(v.smax[1][row], v.smax[2][row]), v.smax[3][row]));
     if (rank == 1 && part == 0) g.dex[(size_t)b * TS + row] = e;
     if (part < nj) {
         unsigned long long d[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             const int q = 8 * part + c, col = 8 * block(part) + c;
-            d[c] = to_digits(col <= row ? to_fixed(v.x[row][q], e + sh.e[col]) : 0);
+            d[c] = to_digits(col <= row ? to_fixed(v.x[row][q], e) : 0);
         }
         unsigned char* o = g.dimg + (size_t)b * kDImg + block(part) * kDCore + row * 16;
         store_digits(d, [&](int i, uint4 x) { *reinterpret_cast<uint4*>(o + i * kDPlane) = x; });
@@ -685,7 +702,8 @@ __device__ __forceinline__ long long join_acc4(const uint32_t (&r)[8][4], int q)
     return x + ((long long)v01 << 35);
 }
 
-// Panel of step k, one CTA per row pair: rows x (64 columns) times the inverted diagonal block, the
+// Panel of step k, one CTA per row pair: rows x (64 columns) times the inverted diagonal block, S_ik 2^-e by
+// (2^-e L_kk)^-T with the diagonal's scales e, the
 // products formed as above, the result rounded row by row to digits without passing through FP64
 // (E's rows also to FP64, which the solve and the gradient read).  Thread (row m of the pair image,
 // columns 16 cq .. 16 cq + 15).  The chain of loads, row maximum, digits, products, row maximum, digits
@@ -693,13 +711,14 @@ __device__ __forceinline__ long long join_acc4(const uint32_t (&r)[8][4], int q)
 // joined accumulators), since the unrolled form spent a third of its 30 us waiting for instructions.
 constexpr int kPanelA = 0, kPanelB = kImg, kPanelTail = kImg + kDImg;
 constexpr int kPanelThreads = 512;
-constexpr int kPanelSmem = kPanelTail + 4 * 128 * 4 + TS * 4;
+constexpr int kPanelSmem = kPanelTail + 4 * 128 * 4 + 2 * TS * 4;
 
 __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     int* smax = reinterpret_cast<int*>(sm + kPanelTail);  // [4][128]
-    int* deb = smax + 512;                                // [64]
+    int* deb = smax + 512;                                // [64] exponents of the inverse's rows
+    int* scale = deb + TS;                                // [64] diag_scale of the columns
     __shared__ uint64_t full, done;
     __shared__ uint32_t tptr;
     const int t = threadIdx.x, b = blockIdx.y, m = t & 127, cq = t >> 7, warp = t >> 5;
@@ -720,25 +739,32 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
     // this one starts after that wait), so their digits are made beside it (read from L2, where that update left
     // them); the inverted block comes after the wait.
     double* tile = nullptr;
-    int f = 0;
+    double v[16];
+    if (t < TS)
+        scale[t] = diag_scale(__ldcg(g.A + (size_t)b * g.strideA + (size_t)tile_index(k, k) * TILE_ELEMS + t * (TS + 1)));
     if (valid) {
         tile = (isext ? ext_tile(g, b, eb, k)
                       : g.A + (size_t)b * g.strideA + (size_t)tile_index(blk, k) * TILE_ELEMS) +
                r + TS * 16 * cq;
-        double v[16];
 #pragma unroll
         for (int c = 0; c < 16; ++c) v[c] = __ldcg(&tile[TS * c]);
-#pragma unroll
-        for (int c = 0; c < 16; ++c) f = max(f, exp_field(v[c]));
     }
+    __syncthreads();
+    int f = -(1 << 28);
+    if (valid)
+#pragma unroll
+        for (int c = 0; c < 16; ++c) f = max(f, scaled_field(v[c], scale[16 * cq + c]));
     smax[128 * cq + m] = f;
     __syncthreads();
-    const int ea = row_exp(max(max(smax[m], smax[128 + m]), max(smax[256 + m], smax[384 + m])));
+    const int ea = scaled_row_exp(max(max(smax[m], smax[128 + m]), max(smax[256 + m], smax[384 + m])));
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
         unsigned long long w[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) w[c] = valid ? to_digits(to_fixed(__ldcg(&tile[TS * (8 * h + c)]), ea)) : 0;
+        for (int c = 0; c < 8; ++c) {
+            const int col = 8 * h + c;
+            w[c] = valid ? to_digits(to_fixed(__ldcg(&tile[TS * col]), ea + scale[16 * cq + col])) : 0;
+        }
         unsigned char* o = sm + kPanelA + (2 * cq + h) * kCore + m * 16;
         store_digits(w, [&](int i, uint4 d) { *reinterpret_cast<uint4*>(o + i * kPlane) = d; });
     }
