@@ -878,9 +878,9 @@ extern "C" int cg_likelihood_pol_create(cg_lik** out, int npix, const int* good,
     cudaStream_t s = ctx.stream;
     double *d_c = nullptr, *d_n = nullptr, *d_cd = nullptr, *d_t = nullptr, *d_m = nullptr;
     unsigned char* work = nullptr;
-    int* d_err = nullptr;
+    int* d_err = nullptr;  // the waits' flag, then the products' scales
     if (!dalloc(&d_c, np) || !dalloc(&d_n, nel) || !dalloc(&d_cd, nel) || !dalloc(&d_t, nel) || !dalloc(&d_m, nel) ||
-        !dalloc(&work, cg::digit_gemm_bytes(ld / cg::TS)) || !dalloc(&d_err, 1)) {
+        !dalloc(&work, cg::digit_gemm_bytes(ld / cg::TS)) || !dalloc(&d_err, 1 + 2 * (size_t)ld)) {
         ctx.err = "device allocation failed";
         rc = CG_ERR_ALLOC;
     }
@@ -891,7 +891,7 @@ extern "C" int cg_likelihood_pol_create(cg_lik** out, int npix, const int* good,
         cudaMemcpy2DAsync(d_n, sizeof(double) * ld, nd.get(), sizeof(double) * n, sizeof(double) * n, n,
                           cudaMemcpyHostToDevice, s);
         // source/likelihood.cpp:386-387: cInv = N^-1 + N^-1 C N^-1, packed over C
-        rc = cg::fp64_pol_matrix(&ctx, n, ld, d_c, d_n, d_cd, d_t, d_m, d_c, work, d_err, s);
+        rc = cg::fp64_pol_matrix(&ctx, n, ld, d_c, d_n, d_cd, d_t, d_m, d_c, work, d_err + 1, d_err, s);
     }
     if (!rc) {
         cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s);

@@ -21,8 +21,6 @@ __device__ __forceinline__ double scaled(long long u, int s)
 }
 
 __device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
-// the row's exponent from the largest exponent field of its entries: |v| < 2^e
-__device__ __forceinline__ int row_exp(int field) { return field == 0x7ff ? kNonFinite : field - 1022; }
 
 // v as 2^(e - FB) X, |v| < 2^e, X rounded to the nearest; FB <= 62
 template <int FB = 54>

@@ -240,9 +240,10 @@ int fp64_build_tiled_into(cg_ctx* ctx, int B, const double* d_cl, bool add_noise
 int fp64_build_packed(cg_ctx* ctx, int B, const double* d_cl, double* d_out, cudaStream_t s);
 // polarisation likelihood set-up: M = N^-1 + N^-1 C N^-1 for packed C and dense N^-1 (ld x ld, row-major, zero
 // padded, ld a multiple of 128), packed into d_m_packed (which may be C); d_cd, d_t, d_m are ld x ld scratch,
-// work digit_gemm_bytes(ld / 64), *err set if a bounded wait gives up
+// work digit_gemm_bytes(ld / 64), scale 2 ld ints of scratch, *err set if a bounded wait gives up
 int fp64_pol_matrix(cg_ctx* ctx, int n, int ld, const double* d_c_packed, const double* d_ninv, double* d_cd,
-                    double* d_t, double* d_m, double* d_m_packed, unsigned char* work, int* err, cudaStream_t s);
+                    double* d_t, double* d_m, double* d_m_packed, unsigned char* work, int* scale, int* err,
+                    cudaStream_t s);
 // w = v - N^-1 s for the dense N^-1 above
 int fp64_dense_residual(cg_ctx* ctx, int n, int ld, const double* d_ninv, const double* d_v, const double* d_s,
                         double* d_w, cudaStream_t s);
@@ -270,10 +271,13 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
                  size_t strideE, double* diag, int* status, unsigned char* work, int* err, cudaStream_t s);
 // out += A B for dense square matrices of nt (even) 64-blocks, the same digit products: A and B row-major, B in
 // out's layout with tilesB; out in tiles, (I, J) at I nt + J, element (r, c) at
-// r + 64 c.  work: digit_gemm_bytes(nt)
+// r + 64 c.  A's columns are taken times 2^(-sign scale), B's rows times 2^(sign scale) (digit_scales), so that neither
+// has entries of many scales side by side.  work: digit_gemm_bytes(nt)
 size_t digit_gemm_bytes(int nt);
-int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* B, bool tilesB, double* out, unsigned char* work,
-               int* err, cudaStream_t s);
+int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* B, bool tilesB, double* out, const int* scale, int sign,
+               unsigned char* work, int* err, cudaStream_t s);
+// scale[ld]: powers of two of the columns of a symmetric ld x ld matrix (2 ld ints, the second half scratch)
+int digit_scales(cg_ctx* ctx, int ld, const double* C, int* scale, cudaStream_t s);
 // generic tiled FP64 / FP32 factorisation entry points (k_chol.cu)
 template <typename T>
 int tiled_cholesky(cg_ctx* ctx, int B, int nt, T* A, T* Dinv, T* diag, int* status, size_t strideA, cudaStream_t s);

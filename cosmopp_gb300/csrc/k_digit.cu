@@ -9,8 +9,8 @@
 //     is rounded to a 55-bit fixed-point number x = 2^(e-54) X, X written in seven signed base-256
 //     digits d_0 .. d_6 (|d| <= 128), each exact in BF16.  An entry far below its row's largest thus keeps
 //     fewer bits than in FP64, so the columns of an operand are brought to one scale first where the other
-//     operand has the opposite one: S_ik = L_ik L_kk^T by the diagonal block's scales (diag_scale).
-//     L's own columns need none: row i of L has norm sqrt(A_ii);
+//     operand has the opposite one: S_ik = L_ik L_kk^T by the diagonal block's scales (diag_scale), the
+//     products of digit_gemm by those of digit_scales.  L's own columns need none: row i of L has norm sqrt(A_ii);
 //   * the digit products i + j <= 7 run on the tensor cores, summed over the 64 columns in eight FP32
 //     accumulators, one per i + j.  Every partial sum is a whole number below 2^23 (64 columns, at
 //     most 6 pairs of 2^14), so FP32 accumulation is exact;
@@ -1237,8 +1237,9 @@ __global__ void __launch_bounds__(kUpThreads, 1)
 
 // Images of a dense operand's row pairs for K blocks k0, k0 + 1, ..: grid (row pairs, K blocks).  Element
 // (row, k): kind 0 at k ld + row (B of a product, row-major), kind 1 at row ld + k (A), kind 2 in 64 x 64 tiles (k / 64, row / 64) of nt to a
-// row, element (r, c) at r + 64 c.  Thread (row, 16 columns), as in the panel.
-__global__ void __launch_bounds__(kPanelThreads) digit_slice(int kind, int ld, int k0, int first, const double* __restrict__ src, Dig g)
+// row, element (r, c) at r + 64 c.  Column k is scaled by 2^(-sign scale[k]).  Thread (row, 16 columns), as in the panel.
+__global__ void __launch_bounds__(kPanelThreads) digit_slice(int kind, int ld, int k0, int first, const double* __restrict__ src,
+                                                             const int* __restrict__ scale, int sign, Dig g)
 {
     __shared__ int smax[4][128];
     const int t = threadIdx.x, m = t & 127, cq = t >> 7, pair = blockIdx.x, nt = ld / TS;
@@ -1250,12 +1251,13 @@ __global__ void __launch_bounds__(kPanelThreads) digit_slice(int kind, int ld, i
                : kind == 1 ? src[(size_t)row * ld + k]
                            : src[((size_t)kb * nt + row / TS) * TILE_ELEMS + c + TS * (m % TS)];
     };
-    int f = 0;
+    auto shift = [&](int c) { return sign * scale[TS * kb + c]; };
+    int f = -(1 << 28);
 #pragma unroll
-    for (int c = 0; c < 16; ++c) f = max(f, exp_field(at(16 * cq + c)));
+    for (int c = 0; c < 16; ++c) f = max(f, scaled_field(at(16 * cq + c), shift(16 * cq + c)));
     smax[cq][m] = f;
     __syncthreads();
-    const int e = row_exp(max(max(smax[0][m], smax[1][m]), max(smax[2][m], smax[3][m])));
+    const int e = scaled_row_exp(max(max(smax[0][m], smax[1][m]), max(smax[2][m], smax[3][m])));
     const size_t p = first + pair;
     if (cq == 0) g.ex[blockIdx.y * g.kex + p * 128 + m] = e;
     unsigned char* out = g.img + blockIdx.y * g.kimg + p * kImg + (size_t)m * 16;
@@ -1263,10 +1265,53 @@ __global__ void __launch_bounds__(kPanelThreads) digit_slice(int kind, int ld, i
     for (int h = 0; h < 2; ++h) {
         unsigned long long w[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) w[c] = to_digits(to_fixed(at(16 * cq + 8 * h + c), e));
+        for (int c = 0; c < 8; ++c) {
+            const int col = 16 * cq + 8 * h + c;
+            w[c] = to_digits(to_fixed(at(col), e + shift(col)));
+        }
         unsigned char* o = out + (2 * cq + h) * kCore;
         store_digits(w, [&](int i, uint4 d) { *reinterpret_cast<uint4*>(o + i * kPlane) = d; });
     }
+}
+
+// Scales of the columns of a symmetric matrix C (ld x ld): C_ik 2^-(half[i] + scale[k]) is at most 1.  half[i] is the
+// diagonal's (of a row without one, its largest entry's), and scale[k] = max_i of what the entries need, half[k] but
+// for a rounding where C is positive semidefinite.  A column of zeros gets kNoScale, which puts what it meets below
+// every other entry.  One CTA per row.
+constexpr int kNoScale = -(1 << 14);
+
+__device__ __forceinline__ int cta_max(int v)
+{
+    __shared__ int red[kPanelThreads / 32];
+    v = __reduce_max_sync(0xffffffffu, v);
+    if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = v;
+    __syncthreads();
+    return __reduce_max_sync(0xffffffffu, red[threadIdx.x % (kPanelThreads / 32)]);
+}
+
+__global__ void __launch_bounds__(kPanelThreads) half_scales(int ld, const double* __restrict__ C, int* __restrict__ half)
+{
+    const double* row = C + (size_t)blockIdx.x * ld;
+    double d = row[blockIdx.x];
+    if (exp_field(d) == 0) {  // (the same for every thread)
+        int f = 0;
+        for (int i = threadIdx.x; i < ld; i += kPanelThreads) f = max(f, exp_field(row[i]));
+        d = __hiloint2double(cta_max(f) << 20, 0);
+    }
+    if (threadIdx.x == 0) half[blockIdx.x] = diag_scale(d);
+}
+
+__global__ void __launch_bounds__(kPanelThreads) column_scales(int ld, const double* __restrict__ C, const int* __restrict__ half,
+                                                              int* __restrict__ scale)
+{
+    const double* row = C + (size_t)blockIdx.x * ld;
+    int f = kNoScale;
+    for (int i = threadIdx.x; i < ld; i += kPanelThreads) {
+        const int x = exp_field(row[i]);
+        if (x) f = max(f, x - 1022 - half[i]);
+    }
+    f = cta_max(f);
+    if (threadIdx.x == 0) scale[blockIdx.x] = f;
 }
 
 }  // namespace
@@ -1438,8 +1483,17 @@ static int gemm_chunk(int nt) { return std::min(nt, 16); }
 
 size_t digit_gemm_bytes(int nt) { return (size_t)gemm_chunk(nt) * nt * (kImg + 128 * sizeof(int)); }
 
-int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, bool tilesB, double* out, unsigned char* work,
-               int* err, cudaStream_t s)
+int digit_scales(cg_ctx* ctx, int ld, const double* C, int* scale, cudaStream_t s)
+{
+    half_scales<<<ld, kPanelThreads, 0, s>>>(ld, C, scale + ld);
+    column_scales<<<ld, kPanelThreads, 0, s>>>(ld, C, scale + ld, scale);
+    count_launch(ctx, 2);
+    CG_CUDA_TRY(ctx, cudaGetLastError());
+    return CG_OK;
+}
+
+int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, bool tilesB, double* out, const int* scale, int sign,
+               unsigned char* work, int* err, cudaStream_t s)
 {
     const int nq = nt / 2, chunk = gemm_chunk(nt), ld = nt * TS;
     Dig g = {};
@@ -1459,8 +1513,8 @@ int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, bool tile
     const int per = up_jobs(u, nq);
     for (int k0 = 0; k0 < nt; k0 += chunk) {
         g.nk = std::min(chunk, nt - k0);
-        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(tilesB ? 2 : 0, ld, k0, 0, Bm, g);
-        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(1, ld, k0, nq, A, g);
+        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(tilesB ? 2 : 0, ld, k0, 0, Bm, scale, -sign, g);
+        digit_slice<<<dim3(nq, g.nk), kPanelThreads, 0, s>>>(1, ld, k0, nq, A, scale, sign, g);
         digit_update<true><<<std::min(per, ctx->sm_count), kUpThreads, kUpSmem, s>>>(-1, per, per, u, g, map);
         count_launch(ctx, 3);
     }

@@ -1151,15 +1151,19 @@ int fp64_build_fiducial(cg_ctx* ctx, int lo, int hi, const double* d_tab, double
 }
 
 int fp64_pol_matrix(cg_ctx* ctx, int n, int ld, const double* d_c_packed, const double* d_ninv, double* d_cd,
-                    double* d_t, double* d_m, double* d_m_packed, unsigned char* work, int* err, cudaStream_t s)
+                    double* d_t, double* d_m, double* d_m_packed, unsigned char* work, int* scale, int* err,
+                    cudaStream_t s)
 {
     const size_t nel = (size_t)ld * ld;
     const int nt = ld / TS;
     packed_to_dense<<<(unsigned)((nel + kThreads - 1) / kThreads), kThreads, 0, s>>>(n, ld, d_c_packed, d_cd);
     CG_CUDA_TRY(ctx, cudaMemsetAsync(d_t, 0, sizeof(double) * nel, s));
     dense_to_tiles<<<dim3(nt, nt), kThreads, 0, s>>>(ld, d_ninv, d_m);
-    int rc = digit_gemm(ctx, nt, d_cd, d_ninv, false, d_t, work, err, s);      // T = C N^-1
-    if (!rc) rc = digit_gemm(ctx, nt, d_ninv, d_t, true, d_m, work, err, s);  // M = N^-1 + N^-1 T
+    // C's scales: C in the units of its diagonal has entries of one size, and so has T = C N^-1; N^-1 keeps only what
+    // its own correlations give it (a scale taken from N^-1 would instead spread C over the noise's range)
+    int rc = digit_scales(ctx, ld, d_cd, scale, s);
+    if (!rc) rc = digit_gemm(ctx, nt, d_cd, d_ninv, false, d_t, scale, 1, work, err, s);      // T = C N^-1
+    if (!rc) rc = digit_gemm(ctx, nt, d_ninv, d_t, true, d_m, scale, -1, work, err, s);  // M = N^-1 + N^-1 T
     if (rc) return rc;
     const long np = (long)n * (n + 1) / 2;
     tiles_to_packed<<<(unsigned)((np + kThreads - 1) / kThreads), kThreads, 0, s>>>(n, nt, d_m, d_m_packed);
