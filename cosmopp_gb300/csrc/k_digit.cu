@@ -309,6 +309,14 @@ __device__ __forceinline__ InvSqrt inv_sqrt(long long v)
     return y;
 }
 
+// An entry of L beyond 1, which no positive definite matrix has and its numbers have no place for (mul_inv_sqrt wraps
+// from |x| 2^a = 2^63 on, the sums from |L| = 4 on): xh the high word of the column's entry x, lh of what mul_inv_sqrt
+// made of it.  |x| < 2^(62 - a), or 2^32 for a = 31, where its numbers are right, and |L| < 1 + 2^-26.
+__device__ __forceinline__ bool beyond_one(int xh, int lh, int a)
+{
+    return (xh ^ (xh >> 31)) >> max(30 - a, 0) != 0 || (lh ^ (lh >> 31)) > 1 << (kFrac - 32);
+}
+
 // x y 2^(kFrac / 2) for |x| <= 2^(kFrac / 2) sqrt(v): an entry of L from the column's entry x
 __device__ __forceinline__ long long mul_inv_sqrt(long long x, const InvSqrt& y)
 {
@@ -446,12 +454,13 @@ __device__ __forceinline__ bool diag_blocks(DiagShared& sh)
 
 // The rows, row r per thread.  The owners' sums of a panel's columns lack the panel just before it, whose products the
 // rows add themselves (of them the block warp gets the diagonal block): so the owners have a panel's time for theirs,
-// and the chain of pivots passes through the rows only.
-__device__ __forceinline__ void diag_rows(DiagShared& sh, int r)
+// and the chain of pivots passes through the rows only.  Returns whether an entry of L is beyond 1.
+__device__ __forceinline__ bool diag_rows(DiagShared& sh, int r)
 {
     constexpr int np = TS / kPanel;
     DiagFactor& f = sh.f;
     const int lane = r & 31, er = (lane >> 2) & 3, ec = lane & 3;
+    bool beyond = false;
     long long x[kPanel];  // the row's entries from the current column on
 #pragma unroll
     for (int j = 0; j < kPanel; ++j) x[j] = f.acc[j][r].x;
@@ -460,6 +469,7 @@ __device__ __forceinline__ void diag_rows(DiagShared& sh, int r)
         const int buf = p & 1, c0 = kPanel * p, from = (c0 + kPanel) & 31;
         const bool completes = p + 1 < np && (c0 + kPanel) / 32 == r / 32;
         long long dh = 0, dl = 0;
+        int xh[kPanel], lh[kPanel], ya[kPanel];
 #pragma unroll
         for (int j = 0; j < kPanel; ++j) {
             named_sync(kCol + 2 * j + buf, kColThreads);
@@ -469,8 +479,12 @@ __device__ __forceinline__ void diag_rows(DiagShared& sh, int r)
             y.m = (unsigned)w.y;
             y.a = (int)(w.y >> 32);
             if (r == c0 + j) x[0] = f.pv[buf][j];
-            const long long l = r >= c0 + j ? mul_inv_sqrt(x[0], y) : 0;
+            if (r < c0 + j) x[0] = 0;
+            const long long l = mul_inv_sqrt(x[0], y);
             const int2 s = split_low(l);
+            xh[j] = (int)(x[0] >> 32);
+            lh[j] = (int)(l >> 32);
+            ya[j] = y.a;
             const int2 a = shfl(s, from + er), b = shfl(s, from + ec);
             dh += (long long)a.x * b.x;
             dl += (long long)a.x * b.y;
@@ -486,6 +500,9 @@ __device__ __forceinline__ void diag_rows(DiagShared& sh, int r)
             if (lane < 16) f.next[er][ec] = joined(make_longlong2(o.x - dh, o.y + dl));
             named_arrive(kNext, kNextThreads);
         }
+        // (here, where the block warp does not wait for the rows)
+#pragma unroll
+        for (int j = 0; j < kPanel; ++j) beyond |= beyond_one(xh[j], lh[j], ya[j]);
         named_sync(kFact + buf, kDiagThreads);
         if (p + 1 == np) break;
         const int4 x0 = f.lsp[buf][0][r], x1 = f.lsp[buf][1][r];
@@ -495,6 +512,7 @@ __device__ __forceinline__ void diag_rows(DiagShared& sh, int r)
             x[j] = joined(less_product(f.acc[c][r], x0, x1, f.lsp[buf][0][c], f.lsp[buf][1][c]));
         }
     }
+    return beyond;
 }
 
 __device__ __forceinline__ void diag_factor(DiagShared& sh, const double* __restrict__ tile)
@@ -515,7 +533,7 @@ __device__ __forceinline__ void diag_factor(DiagShared& sh, const double* __rest
         if (t >= kBlockThread) {
             if (diag_blocks(sh) && t == kBlockThread) sh.bad = 1;
         } else {
-            diag_rows(sh, t - kDiagOwners);
+            if (diag_rows(sh, t - kDiagOwners)) sh.bad = 1;
         }
     } else {
         // warp w has the columns of panel w: this thread column c, rows tr + 8 a
