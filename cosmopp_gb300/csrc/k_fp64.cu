@@ -431,10 +431,19 @@ __global__ void __launch_bounds__(kThreads) build_fid_packed(int n, int N, int l
             out[kk[q]] = __dadd_rn(acc[q], __dmul_rn(__dmul_rn(__dmul_rn(m0, __dadd_rn(1.0, x[q])), b2), b2));
 }
 
+// An element without a number: a C_l that is none, whose covariance the factorisation puts benign values in place of,
+// or a bounded wait that gave up.  Its outputs are NaN, asked for its status or not.  (status, err nullable)
+__device__ __forceinline__ bool no_number(const int* __restrict__ status, const int* __restrict__ err, int b)
+{
+    return status && (status[b] == CG_ERR_NONFINITE || *err);
+}
+__device__ __forceinline__ double nan_value() { return __longlong_as_double(0x7ff8000000000000ll); }
+
 // ln det = 2 sum_i ln L_ii over the n real pixels (source/matrix_impl.cpp:322-338), grid B
 // (an FP64 logarithm is some 30 instructions of 64 cycles each and partition)
 constexpr int kLogThreads = 1024;
 __global__ void __launch_bounds__(kLogThreads) logdet_reduce(int n, int N, const double* __restrict__ diag,
+                                                             const int* __restrict__ status, const int* __restrict__ err,
                                                              double* __restrict__ logdet)
 {
     launch_dependents();
@@ -449,7 +458,7 @@ __global__ void __launch_bounds__(kLogThreads) logdet_reduce(int n, int N, const
         if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) logdet[b] = 2.0 * red[0];
+    if (threadIdx.x == 0) logdet[b] = no_number(status, err, b) ? nan_value() : 2.0 * red[0];
 }
 
 // padded copy of the data maps into dvec[b][N]
@@ -489,7 +498,8 @@ __global__ void __launch_bounds__(kThreads) symv_tiled(int nt, int N, const T* _
 // chi2 = d . alpha, m2lnl = chi2 + logdet; grid B
 __global__ void __launch_bounds__(kThreads) chi2_finish(int n, int N, const double* __restrict__ dv,
                                                         const double* __restrict__ alpha,
-                                                        const double* __restrict__ logdet, double* __restrict__ m2lnl,
+                                                        const double* __restrict__ logdet, const int* __restrict__ status,
+                                                        const int* __restrict__ err, double* __restrict__ m2lnl,
                                                         double* __restrict__ chi2)
 {
     __shared__ double red[kThreads];
@@ -503,8 +513,9 @@ __global__ void __launch_bounds__(kThreads) chi2_finish(int n, int N, const doub
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        if (chi2) chi2[b] = red[0];
-        m2lnl[b] = red[0] + logdet[b];
+        const double x = no_number(status, err, b) ? nan_value() : red[0];
+        if (chi2) chi2[b] = x;
+        m2lnl[b] = x + logdet[b];
     }
 }
 
@@ -569,14 +580,15 @@ __global__ void __launch_bounds__(kThreads) adjoint_tiles(int n, int N, int l0, 
 
 // grad_l = (sum over tiles) * ((2l+1)/(4 pi)) * B_l * B_l; grid B
 __global__ void adjoint_finish(int lmax, int ntile, const double* __restrict__ gpart, const double* __restrict__ beam,
-                               double* __restrict__ grad)
+                               const int* __restrict__ status, const int* __restrict__ err, double* __restrict__ grad)
 {
     const int b = blockIdx.x;
+    const bool none = no_number(status, err, b);
     for (int l = threadIdx.x; l <= lmax; l += blockDim.x) {
         double s = 0.0;
         if (l >= 2)
             for (int t = 0; t < ntile; ++t) s += gpart[((size_t)b * ntile + t) * (lmax + 1) + l];
-        grad[(size_t)b * (lmax + 1) + l] = (l < 2) ? 0.0 : s * ((2 * l + 1) / (4 * kPi)) * beam[l] * beam[l];
+        grad[(size_t)b * (lmax + 1) + l] = (l < 2) ? 0.0 : none ? nan_value() : s * ((2 * l + 1) / (4 * kPi)) * beam[l] * beam[l];
     }
 }
 
@@ -883,7 +895,8 @@ __global__ void __launch_bounds__(kThreads) ext_rows(int n, int nt, int drow, co
 
 // y = L^-1 d from E's row drow, chi2 = y . y, m2lnl = chi2 + logdet; grid B
 __global__ void __launch_bounds__(kThreads) chi2_rows(int nt, int drow, const double* __restrict__ E, size_t strideE,
-                                                      const double* __restrict__ logdet, double* __restrict__ y,
+                                                      const double* __restrict__ logdet, const int* __restrict__ status,
+                                                      const int* __restrict__ err, double* __restrict__ y,
                                                       double* __restrict__ m2lnl, double* __restrict__ chi2,
                                                       double* __restrict__ logdet_out)
 {
@@ -905,9 +918,10 @@ __global__ void __launch_bounds__(kThreads) chi2_rows(int nt, int drow, const do
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        if (chi2) chi2[b] = red[0];
+        const double x = no_number(status, err, b) ? nan_value() : red[0];
+        if (chi2) chi2[b] = x;
         if (logdet_out) logdet_out[b] = logdet[b];
-        m2lnl[b] = red[0] + logdet[b];
+        m2lnl[b] = x + logdet[b];
     }
 }
 
@@ -945,6 +959,7 @@ __global__ void __launch_bounds__(kThreads) harmonic_sums(int nt, int ne, const 
 
 // grad_l from the sums, a warp per l; grid (ceil((lmax + 1) / 8), B)
 __global__ void __launch_bounds__(kThreads) harmonic_grad(int lmax, int ne, const double* __restrict__ part,
+                                                          const int* __restrict__ status, const int* __restrict__ err,
                                                           double* __restrict__ grad)
 {
     launch_dependents();
@@ -964,7 +979,7 @@ __global__ void __launch_bounds__(kThreads) harmonic_grad(int lmax, int ne, cons
             g += zz - zy * zy;
         }
     for (int o = 16; o > 0; o >>= 1) g += __shfl_down_sync(0xffffffffu, g, o);
-    if (lane == 0) grad[(size_t)b * (lmax + 1) + l] = g;
+    if (lane == 0) grad[(size_t)b * (lmax + 1) + l] = l >= 2 && no_number(status, err, b) ? nan_value() : g;
 }
 
 }  // namespace
@@ -988,7 +1003,7 @@ void fp64_quad(int nt, const double* V, const double* tv, const double* fv, doub
 
 void fp64_logdet(int B, int n, int N, const double* diag, double* out, cudaStream_t s)
 {
-    logdet_reduce<<<B, kLogThreads, 0, s>>>(n, N, diag, out);
+    logdet_reduce<<<B, kLogThreads, 0, s>>>(n, N, diag, nullptr, nullptr, out);
 }
 
 void fp64_dot(int n, const double* a, const double* b, double* out, cudaStream_t s)
@@ -1239,15 +1254,15 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
                            w.ext_elems, w.diag, w.st, w.dig, w.err, s)))
         return rc;
     stage_mark(ctx, ST_SOLVE, s);
-    if ((rc = launch(ctx, logdet_reduce, dim3(B), kLogThreads, 0, 1, s, n, N, w.diag, w.ld))) return rc;
+    if ((rc = launch(ctx, logdet_reduce, dim3(B), kLogThreads, 0, 1, s, n, N, w.diag, w.st, w.err, w.ld))) return rc;
     if (inverse) {
         pad_data<<<dim3((N + 255) / 256, B), 256, 0, s>>>(n, N, B, d_d, d_stride, w.dvec);
         symv_tiled<double><<<dim3(nt, B), kThreads, 0, s>>>(nt, N, w.A, strideA, w.dvec, w.alpha);
-        chi2_finish<<<B, kThreads, 0, s>>>(n, N, w.dvec, w.alpha, w.ld, d_m2lnl, d_chi2);
+        chi2_finish<<<B, kThreads, 0, s>>>(n, N, w.dvec, w.alpha, w.ld, w.st, w.err, d_m2lnl, d_chi2);
         count_launch(ctx, 3);
         if (d_logdet) CG_CUDA_TRY(ctx, cudaMemcpyAsync(d_logdet, w.ld, sizeof(double) * B, cudaMemcpyDeviceToDevice, s));
-    } else if ((rc = launch(ctx, chi2_rows, dim3(B), kThreads, 0, 1, s, nt, drow, w.E, w.ext_elems, w.ld, w.alpha, d_m2lnl,
-                            d_chi2, d_logdet))) {
+    } else if ((rc = launch(ctx, chi2_rows, dim3(B), kThreads, 0, 1, s, nt, drow, w.E, w.ext_elems, w.ld, w.st, w.err, w.alpha,
+                            d_m2lnl, d_chi2, d_logdet))) {
         return rc;
     }
     stage_mark(ctx, ST_ADJOINT, s);
@@ -1258,12 +1273,13 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
                                                               strideA, w.alpha, w.gpart, ntile, lmax + 1);
             count_launch(ctx);
         }
-        adjoint_finish<<<B, 64, 0, s>>>(lmax, ntile, w.gpart, ctx->d_beam, d_grad);
+        adjoint_finish<<<B, 64, 0, s>>>(lmax, ntile, w.gpart, ctx->d_beam, w.st, w.err, d_grad);
         count_launch(ctx);
     } else if (grad) {
         if ((rc = launch(ctx, harmonic_sums, dim3(ne, kHarmSplit, B), kThreads, 0, 1, s, nt, ne, w.E, w.ext_elems, w.alpha,
                          w.gpart)) ||
-            (rc = launch(ctx, harmonic_grad, dim3((lmax + 8) / 8, B), kThreads, 0, 1, s, lmax, ne, w.gpart, d_grad)))
+            (rc = launch(ctx, harmonic_grad, dim3((lmax + 8) / 8, B), kThreads, 0, 1, s, lmax, ne, w.gpart, w.st, w.err,
+                         d_grad)))
             return rc;
     }
     if (d_status && (rc = launch(ctx, copy_status, dim3((B + 127) / 128), 128, 0, 1, s, B, w.st, w.err, d_status))) return rc;

@@ -144,7 +144,8 @@ int cg_noise_matrix_from_sims(cg_ctx* ctx, int nsims, int n, const double* sims,
    d: one map (d_stride = 0) or B maps at stride d_stride (>= n).
    grad (nullable): [B][lmax+1] d(-2lnL)/dC_l (l < 2 are 0) -- new, no reference counterpart.
    chi2 / logdet / status nullable; status[b] = CG_OK or CG_ERR_NOT_PD / CG_ERR_NONFINITE, or
-   (mixed path) CG_ERR_TIMEOUT when a bounded tensor-core wait gave up during the call.
+   CG_ERR_TIMEOUT when a bounded device wait gave up during the call.  On the FP64 path every
+   output of an element with CG_ERR_NONFINITE or CG_ERR_TIMEOUT is NaN (grad from l = 2 on).
    Returns CG_OK when the call ran, even if some elements carry a bad status. */
 int cg_loglike(cg_ctx* ctx, int B, const double* cl, const double* d, int d_stride,
                double* m2lnl, double* chi2, double* logdet, double* grad, int* status);
