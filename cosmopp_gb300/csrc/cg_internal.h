@@ -54,8 +54,8 @@ struct Fp64Work {
     double* E = nullptr;         // [cap][ext_elems] the factorisation's extra rows (k_digit.cu)
     size_t ext_elems = 0;        // doubles of E per element
     unsigned char* dig = nullptr;  // digit images, digit_bytes per element
-    size_t dig_bytes = 0;        // per element
     double* Yt = nullptr;        // [ext tiles] harmonics x B_l of the pixels, shared by every element
+    bool have_yt = false;        // Yt is filled
     double* diag = nullptr;      // [cap][N] diagonal of L
     double* dvec = nullptr;      // [cap][N] data maps (padded)
     double* alpha = nullptr;     // [cap][N] L^-1 d, or C^-1 d
@@ -266,7 +266,8 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
 // work: digit_bytes(nt, ne) per matrix, 16-byte aligned; *err is set if a bounded wait gives up.
 enum DigitExt { DIGIT_EXT_ROWS = 0, DIGIT_EXT_IDENTITY = 1, DIGIT_EXT_PRODUCT = 2 };
 size_t digit_bytes(int nt, int ne);
-void digit_free(cg_ctx* ctx);  // the context's second stream and its events
+bool digit_streams(cg_ctx* ctx);  // the context's second stream and its events, where they are not there yet
+void digit_free(cg_ctx* ctx);
 int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t strideA, double* E,
                  size_t strideE, double* diag, int* status, unsigned char* work, int* err, cudaStream_t s);
 // out += A B for dense square matrices of nt (even) 64-blocks, the same digit products: A and B row-major, B in

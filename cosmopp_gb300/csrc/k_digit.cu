@@ -1397,7 +1397,7 @@ static int chain_reserve(const cg_ctx* ctx, int B, int nq, int npe, int v)
     return reserve;
 }
 
-static bool chain_streams(cg_ctx* ctx)
+bool digit_streams(cg_ctx* ctx)
 {
     if (!ctx->aux && cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking) != cudaSuccess) ctx->aux = nullptr;
     bool ok = ctx->aux != nullptr;
@@ -1463,7 +1463,7 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
             return rc;
         if (m + npe == 0) continue;
         const int reserve = m > 1 ? chain_reserve(ctx, B, m, npe, v) : 0;
-        const bool beside = reserve > 0 && chain_streams(ctx);
+        const bool beside = reserve > 0 && digit_streams(ctx);
         if (rest && !beside) {
             CG_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain[1], 0));
             rest = false;

@@ -1031,10 +1031,12 @@ static int ext_blocks(const cg_ctx* ctx, bool grad)
     return 2 * ((rows + 2 * TS - 1) / (2 * TS));
 }
 
-static size_t ext_elems(const cg_ctx* ctx, bool grad)
+// Doubles of E per element, for the larger of a value's and a gradient's rows (the identity of two block rows is three
+// tiles, the map's 128 rows four)
+static size_t ext_elems(const cg_ctx* ctx)
 {
-    if (grad && !ctx->harm) return tiled_elems(ctx->nt);
-    return (size_t)ext_blocks(ctx, grad) * ctx->nt * TILE_ELEMS;
+    auto rows = [&](bool grad) { return (size_t)ext_blocks(ctx, grad) * ctx->nt * TILE_ELEMS; };
+    return ctx->harm ? rows(true) : std::max(rows(false), tiled_elems(ctx->nt));
 }
 
 static size_t gpart_elems(const cg_ctx* ctx)
@@ -1058,59 +1060,52 @@ bool fp64_harmonics_ok(int n, int nt, int lmax, const double* xyz)
     return true;
 }
 
-// The allocations of fp64_ensure for gradient calls (value calls need less)
+// The allocations of fp64_ensure
 void fp64_bytes(const cg_ctx* ctx, size_t* fixed, size_t* per_element)
 {
-    *fixed = sizeof(int) + (ctx->harm ? sizeof(double) * (ext_elems(ctx, true) + ylm_rows(ctx->lmax) * ctx->N) : 0);
-    *per_element = sizeof(double) * (tiled_elems(ctx->nt) + ext_elems(ctx, true) + 3 * (size_t)ctx->N +
+    *fixed = sizeof(int) + (ctx->harm ? sizeof(double) * ext_elems(ctx) : 0);
+    *per_element = sizeof(double) * (tiled_elems(ctx->nt) + ext_elems(ctx) + 3 * (size_t)ctx->N +
                                      gpart_elems(ctx) + 1) +
                    sizeof(long long) * ((size_t)ctx->lmax + 1) + 2 * sizeof(int) + digit_bytes(ctx->nt, ext_blocks(ctx, true));
 }
 
-static int fp64_ensure(cg_ctx* ctx, int B, bool grad, cudaStream_t s)
+// The workspace of B elements, for values and gradients alike, so that it moves only when B grows: a call may be
+// captured after any call of as many elements, and a captured one stays valid through every later call of no more.
+static int fp64_ensure(cg_ctx* ctx, int B)
 {
     Fp64Work& w = ctx->w64;
-    auto alloc = [&](void** p, size_t bytes) -> bool { return cudaMalloc(p, bytes) == cudaSuccess; };
-    auto fail = [&] {
+    if (w.cap >= B) return CG_OK;
+    const size_t n = B;
+    fp64_free(ctx);
+    auto alloc = [](auto** p, size_t count) { return cudaMalloc((void**)p, sizeof(**p) * count) == cudaSuccess; };
+    w.ext_elems = ext_elems(ctx);
+    if (!(alloc(&w.A, tiled_elems(ctx->nt) * n) && alloc(&w.E, w.ext_elems * n) &&
+          alloc(&w.dig, digit_bytes(ctx->nt, ext_blocks(ctx, true)) * n) && alloc(&w.diag, ctx->N * n) &&
+          alloc(&w.dvec, ctx->N * n) && alloc(&w.alpha, ctx->N * n) && alloc(&w.gpart, gpart_elems(ctx) * n) &&
+          alloc(&w.st, n) && alloc(&w.ld, n) && alloc(&w.wfix, (ctx->lmax + 1) * n) && alloc(&w.wexp, n) &&
+          alloc(&w.err, 1) && (!ctx->harm || alloc(&w.Yt, w.ext_elems)))) {
         fp64_free(ctx);
         cudaGetLastError();
         ctx->err = "device allocation failed for the FP64 workspace";
         return CG_ERR_ALLOC;
-    };
-    const size_t elems = ext_elems(ctx, grad), dig = digit_bytes(ctx->nt, ext_blocks(ctx, grad));
-    if (w.cap < B || w.ext_elems < elems || w.dig_bytes < dig) {
-        const int cap = std::max(B, w.cap);
-        const size_t ee = std::max(elems, w.ext_elems), de = std::max(dig, w.dig_bytes);
-        fp64_free(ctx);
-        if (!(alloc((void**)&w.A, sizeof(double) * tiled_elems(ctx->nt) * cap) &&
-              alloc((void**)&w.E, sizeof(double) * ee * cap) && alloc((void**)&w.dig, de * cap) &&
-              alloc((void**)&w.diag, sizeof(double) * (size_t)cap * ctx->N) &&
-              alloc((void**)&w.dvec, sizeof(double) * (size_t)cap * ctx->N) &&
-              alloc((void**)&w.alpha, sizeof(double) * (size_t)cap * ctx->N) &&
-              alloc((void**)&w.gpart, sizeof(double) * (size_t)cap * gpart_elems(ctx)) &&
-              alloc((void**)&w.st, sizeof(int) * (size_t)cap) && alloc((void**)&w.ld, sizeof(double) * (size_t)cap) &&
-              alloc((void**)&w.wfix, sizeof(long long) * (size_t)cap * (ctx->lmax + 1)) &&
-              alloc((void**)&w.wexp, sizeof(int) * (size_t)cap) && alloc((void**)&w.err, sizeof(int))))
-            return fail();
-        w.cap = cap;
-        w.ext_elems = ee;
-        w.dig_bytes = de;
     }
-    if (grad && ctx->harm && !w.Yt) {  // once per workspace: the pixels do not change
-        const int ne = ext_blocks(ctx, true);
-        double* Y = nullptr;
-        if (!alloc((void**)&w.Yt, sizeof(double) * ext_elems(ctx, true)) ||
-            !alloc((void**)&Y, sizeof(double) * ylm_rows(ctx->lmax) * ctx->N)) {
-            cudaFree(Y);
-            return fail();
-        }
-        int rc = ylm_fill(ctx, Y, s);
-        if (!rc) harmonic_tiles<<<dim3(ctx->nt, ne), kThreads, 0, s>>>(ctx->N, ctx->nt, nharm_of(ctx->lmax), Y, w.Yt);
-        const cudaError_t e = cudaStreamSynchronize(s);
-        cudaFree(Y);
-        if (!rc && e != cudaSuccess) { ctx->err = cudaGetErrorString(e); rc = CG_ERR_CUDA; }
-        if (rc) { cudaFree(w.Yt); w.Yt = nullptr; return rc; }
-    }
+    digit_streams(ctx);
+    w.cap = B;
+    return CG_OK;
+}
+
+// The harmonics of the pixels in Yt, by the first gradient call on a workspace (in its stream, by way of E, which the
+// call fills afterwards; a captured call carries them along, and they count as made only when they were run)
+static int fp64_harmonics(cg_ctx* ctx, cudaStream_t s)
+{
+    Fp64Work& w = ctx->w64;
+    if (w.have_yt) return CG_OK;
+    if (int rc = ylm_fill(ctx, w.E, s)) return rc;
+    harmonic_tiles<<<dim3(ctx->nt, ext_blocks(ctx, true)), kThreads, 0, s>>>(ctx->N, ctx->nt, nharm_of(ctx->lmax), w.E, w.Yt);
+    CG_CUDA_TRY(ctx, cudaGetLastError());
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    w.have_yt = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+    cudaGetLastError();
     return CG_OK;
 }
 
@@ -1222,7 +1217,8 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
                  double* d_chi2, double* d_logdet, double* d_grad, int* d_status, cudaStream_t s)
 {
     const bool grad = d_grad != nullptr;
-    int rc = fp64_ensure(ctx, B, grad, s);
+    int rc = fp64_ensure(ctx, B);
+    if (!rc && grad && ctx->harm) rc = fp64_harmonics(ctx, s);
     if (rc) return rc;
     Fp64Work& w = ctx->w64;
     const int nt = ctx->nt, N = ctx->N, n = ctx->n, lmax = ctx->lmax;
