@@ -944,7 +944,8 @@ extern "C" int cg_selftest_wait_timeout(cg_ctx* ctx, int* status)
 {
     if (!ctx || !status) return CG_ERR_BAD_ARG;
     CG_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    return cg::selftest_wait_timeout(ctx, status);
+    const int rc = cg::selftest_wait_timeout(ctx, status);
+    return rc || *status != CG_ERR_TIMEOUT ? rc : cg::digit_selftest_timeout(ctx, status);
 }
 
 extern "C" int cg_probe_fp32_rate(cg_ctx* ctx, int iters, int reps, double* tflops, double* ms)

@@ -165,6 +165,7 @@ struct cg_ctx {
     // the FP64 factorisation's second stream (k_digit.cu) and the events between the two
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_chain[2] = {nullptr, nullptr};
+    bool no_waits = false;       // self-test: the diagonal blocks' and panels' waits (k_digit.cu) give up at once
     std::vector<double> xyz;     // [n][3]
     std::vector<double> noise;   // [n]
     cg::LegConsts leg;
@@ -266,10 +267,12 @@ int fp64_loglike(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int 
 // work: digit_bytes(nt, ne) per matrix, 16-byte aligned; *err is set if a bounded wait gives up.
 enum DigitExt { DIGIT_EXT_ROWS = 0, DIGIT_EXT_IDENTITY = 1, DIGIT_EXT_PRODUCT = 2 };
 size_t digit_bytes(int nt, int ne);
-bool digit_streams(cg_ctx* ctx);  // the context's second stream and its events, where they are not there yet
-void digit_free(cg_ctx* ctx);
+void digit_free(cg_ctx* ctx);  // the context's second stream and its events
 int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t strideA, double* E,
                  size_t strideE, double* diag, int* status, unsigned char* work, int* err, cudaStream_t s);
+// a small factorisation whose diagonal blocks' and panels' waits give up at once, which its updates see: *host_status =
+// CG_ERR_TIMEOUT where that is reported
+int digit_selftest_timeout(cg_ctx* ctx, int* host_status);
 // out += A B for dense square matrices of nt (even) 64-blocks, the same digit products: A and B row-major, B in
 // out's layout with tilesB; out in tiles, (I, J) at I nt + J, element (r, c) at
 // r + 64 c.  A's columns are taken times 2^(-sign scale), B's rows times 2^(sign scale) (digit_scales), so that neither

@@ -31,6 +31,10 @@
 // 32 rows at a time, taken out by a tensor copy as [8][7][4][8][16 bytes], the B operand (the 7 digits of 32
 // rows as N = 224, groups 128 bytes apart).
 //
+// Every wait on a barrier is bounded.  One that gives up sets *err, which all waits watch; its thread and those that see
+// the flag skip their later waits and take no more work (the update after the job in hand), and the copies and products in flight are waited for, bounded
+// too, before their shared and tensor memory is given up.
+//
 // A row with an infinity or a NaN gets the exponent kNonFinite, which makes everything it enters NaN.
 #include <cuda.h>
 
@@ -60,7 +64,7 @@ constexpr int kPiece = 8 * kPieceCore;      // 28672 bytes
 constexpr int kDPlane = 8 * kGroupBytes;    // the same for the 64 rows of an inverted diagonal block
 constexpr int kDCore = kDig * kDPlane;
 constexpr int kDImg = 8 * kDCore;           // 57344 bytes
-constexpr uint32_t kWaits = 1u << 24;
+constexpr uint32_t kWaits = 1u << 22;       // attempts before a wait gives up
 
 // M64 N: bf16 x bf16 -> fp32, both operands K-major
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N)
@@ -147,7 +151,16 @@ struct Dig {
     unsigned char* dimg;      // [B][kDImg]
     int* dex;                 // [B][64]
     int* err;
+    uint32_t waits;           // the diagonal block's and the panel's limit: kWaits, or 0 in the self-test
 };
+
+// a wait that gives up, or finds that another has, sets the flag and clears ok; later ones are skipped
+__device__ __forceinline__ void bounded_wait(bool& ok, uint64_t* bar, uint32_t parity, int* err, uint32_t waits)
+{
+    if (!ok) return;
+    ok = mbar_wait(bar, parity, waits, err);
+    if (!ok) *(volatile int*)err = 1;
+}
 
 __device__ __forceinline__ int dig_pairs(const Dig& g) { return (g.nt + g.ne) / 2; }
 
@@ -251,10 +264,12 @@ __device__ __forceinline__ void arrive_cluster(uint64_t* bar, int rank)
                      mapa(bar, rank))
                  : "memory");
 }
-__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity)
+__device__ __forceinline__ void wait_cluster(bool& ok, uint64_t* bar, uint32_t parity, const Dig& g)
 {
+    if (!ok) return;
     const uint32_t a = smem_u32(bar);
-    for (uint32_t it = 0; it < kWaits; ++it) {
+    const volatile int* err = g.err;
+    for (uint32_t it = 0; it < g.waits; ++it) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
@@ -262,9 +277,11 @@ __device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity)
             : "=r"(done)
             : "r"(a), "r"(parity)
             : "memory");
-        if (done) return true;
+        if (done) return;
+        if ((it & 255) == 255 && *err) break;
     }
-    return false;
+    ok = false;
+    *(volatile int*)g.err = 1;
 }
 
 // v 2^(kFrac - e) rounded to the nearest; false where |v| >= 2^e or v is not finite
@@ -599,7 +616,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
     double w[3] = {0.0, 0.0, 0.0};  // row r's sums, columns 8 block(j) + qi
     bool ok = true;
     for (int grp = 0; grp < 8; ++grp) {
-        ok = wait_cluster(&sh.full[grp], 0) && ok;
+        wait_cluster(ok, &sh.full[grp], 0, g);
         if (rank == 1 && t < 8) {  // L's diagonal
             const int c = 8 * grp + t;
             diag[(size_t)b * g.nt * TS + k * TS + c] = scaled(v.lq[grp][t][c], sh.e[c] - kFrac);
@@ -646,7 +663,6 @@ __global__ void __launch_bounds__(kDiagThreads, 1)
                 }
         }
     }
-    if (!ok) atomicExch(g.err, 1);
     named_sync(1, kDiagOwners);
     // The rows of the scaled factor's inverse in digits, one exponent per row over all these CTAs: thread (row, 8
     // columns).  The panel's rows carry the scales.
@@ -799,17 +815,21 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
     const uint32_t tmem = tptr;
     bool ok = true;
     if (t == 0) {
-        ok = mbar_wait(&full, 0, kWaits, g.err);
+        bounded_wait(ok, &full, 0, g.err, g.waits);
         const uint64_t ad = smem_desc(smem_u32(sm + kPanelA), kCore, kGroupBytes);
         const uint64_t bd = smem_desc(smem_u32(sm + kPanelB), kDCore, kGroupBytes);
-        for (int kc = 0; kc < 4; ++kc)
-            issue_products<TS>(tmem, ad + (uint64_t)kc * (2 * kCore >> 4), bd + (uint64_t)kc * (2 * kDCore >> 4),
-                               kPlane, kDPlane, kc == 0);
+        if (ok)
+            for (int kc = 0; kc < 4; ++kc)
+                issue_products<TS>(tmem, ad + (uint64_t)kc * (2 * kCore >> 4), bd + (uint64_t)kc * (2 * kDCore >> 4),
+                                   kPlane, kDPlane, kc == 0);
         mma_commit(&done);
     }
     __syncwarp();
-    ok = mbar_wait(&done, 0, kWaits, g.err) && ok;
-    if (!ok) atomicExch(g.err, 1);
+    bounded_wait(ok, &done, 0, g.err, g.waits);
+    if (!ok && t == 0) {  // the copy and the products, if they are under way
+        mbar_wait(&full, 0, kWaits);
+        mbar_wait(&done, 0, kWaits);
+    }
     fence_after();
     __syncwarp();
     // this thread's entries in units of 2^(ea + deb[c] - 55), into the place of the rows' digits, and the row's largest
@@ -1025,7 +1045,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
     digit_update(int k, int njobs, int per, UpRange u, Dig g, const __grid_constant__ CUtensorMap map)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    __shared__ uint64_t afull[4], aempty[4], bfull[4], bempty[4], tfull[2], tempty[2], dfull[kUpDescs], dempty[kUpDescs];
+    __shared__ uint64_t afull[4], aempty[4], bfull[4], bempty[4], tfull[2], tempty[2], dfull[kUpDescs], dempty[kUpDescs], fin;
     __shared__ UpDesc desc[kUpDescs];
     __shared__ uint32_t tptr;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -1047,6 +1067,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
             mbar_init(&dfull[i], 1);
             mbar_init(&dempty[i], kUpWarps + 1);
         }
+        mbar_init(&fin, 1);
         fence_mbar_init();
     }
     fence_before();
@@ -1054,14 +1075,17 @@ __global__ void __launch_bounds__(kUpThreads, 1)
     fence_after();
     const uint32_t tmem = tptr;
     bool ok = true;
+    // (a constant: as a parameter the limit took 3 % of the update)
+    auto wait = [&](uint64_t* bar, uint32_t parity) { bounded_wait(ok, bar, parity, g.err, kWaits); };
     // (the jobs are worked out before the wait for the kernel before this one, which precedes every access to memory)
     if (warp == kUpWarps + 1) {
         if (lane == 0) {
-            uint32_t aphase = 0, bphase = 0;  // uses so far, mod 2: of A, of piece i in bit i
+            uint32_t aphase = 0, bphase = 0;  // uses so far, mod 2: of A's and B's piece i in bit i
             // job s into its slot (i1 = 0 past the last)
             auto put = [&](int s, int job, const UpJob& j, bool fresh) {
                 UpDesc& d = desc[s % kUpDescs];
-                ok = mbar_wait(&dempty[s % kUpDescs], ((s / kUpDescs) & 1) ^ 1, kWaits, g.err) && ok;
+                wait(&dempty[s % kUpDescs], ((s / kUpDescs) & 1) ^ 1);
+                if (!ok) return;
                 if (job >= 0) up_desc(g, u, j, k, fresh, d);
                 else d.i0 = d.i1 = 0;
                 mbar_arrive(&dfull[s % kUpDescs]);
@@ -1079,7 +1103,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
             };
             if (job >= 0) ahead(1);
             wait_prior();
-            for (int s = 0; job >= 0; ++s) {
+            for (int s = 0; ok && job >= 0; ++s) {
                 if (g.prefetch && next >= 0) {  // the next job's tiles on their way from DRAM
                     const UpDesc& d = desc[(s + 1) % kUpDescs];
 #pragma unroll 1
@@ -1094,7 +1118,8 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                 for (int ks = 0; ks < nk; ++ks) {
                     const int ia = ks * g.kim + j.b * pairs + j.pa, ib = g.im0 + ks * g.kim + j.b * pairs + j.pb;
                     auto piece = [&](int i) {
-                        ok = mbar_wait(&bempty[i], ((bphase >> i) & 1) ^ 1, kWaits, g.err) && ok;
+                        wait(&bempty[i], ((bphase >> i) & 1) ^ 1);
+                        if (!ok) return;
                         bphase ^= 1u << i;
                         mbar_arrive_expect_tx(&bfull[i], kPiece);
                         tensor_g2s(smem_u32(sm + kUpB + i * kPiece), &map, i, ib, &bfull[i]);
@@ -1102,11 +1127,12 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                     auto rows = [&]() {
                         const unsigned char* a = g.img + (size_t)ia * kImg;
                         for (int kc = 0; kc < 4; ++kc) {
-                            ok = mbar_wait(&aempty[kc], aphase ^ 1, kWaits, g.err) && ok;
+                            wait(&aempty[kc], ((aphase >> kc) & 1) ^ 1);
+                            if (!ok) return;
+                            aphase ^= 1u << kc;
                             mbar_arrive_expect_tx(&afull[kc], 2 * kCore);
                             bulk_g2s(smem_u32(sm + 2 * kc * kCore), a + 2 * kc * kCore, 2 * kCore, &afull[kc]);
                         }
-                        aphase ^= 1;
                     };
                     // in the order in which the places become free
                     const bool first = s == 0 && ks == 0;
@@ -1121,6 +1147,11 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                 fresh = !same;
                 if (job >= 0) ahead(s + 2);
             }
+            if (!ok)  // the copies under way
+                for (int i = 0; i < 4; ++i) {
+                    mbar_wait(&afull[i], ((aphase >> i) & 1) ^ 1, kWaits);
+                    mbar_wait(&bfull[i], ((bphase >> i) & 1) ^ 1, kWaits);
+                }
         }
         __syncwarp();
     } else if (warp == kUpWarps) {
@@ -1128,24 +1159,24 @@ __global__ void __launch_bounds__(kUpThreads, 1)
             uint32_t aphase = 0, bphase = 0, pass = 0;
             for (int s = 0;; ++s) {
                 const UpDesc& d = desc[s % kUpDescs];
-                ok = mbar_wait(&dfull[s % kUpDescs], (s / kUpDescs) & 1, kWaits, g.err) && ok;
+                wait(&dfull[s % kUpDescs], (s / kUpDescs) & 1);
                 const int i0 = d.i0, i1 = ok ? d.i1 : 0;
                 if (i1 == 0) break;
                 const bool fresh = d.fresh;
                 const UpDesc& n = desc[(s + 1) % kUpDescs];  // put there before this job's images were fetched
-                ok = mbar_wait(&dfull[(s + 1) % kUpDescs], ((s + 1) / kUpDescs) & 1, kWaits, g.err) && ok;
+                wait(&dfull[(s + 1) % kUpDescs], ((s + 1) / kUpDescs) & 1);
                 const bool last = n.i1 == 0 || n.fresh;
                 for (int ks = 0; ks < nk; ++ks) {
                     for (int i = i0; i < i1; ++i, ++pass) {
                         const uint32_t buf = pass & 1;
-                        ok = mbar_wait(&tempty[buf], ((pass >> 1) & 1) ^ 1, kWaits, g.err) && ok;
-                        ok = mbar_wait(&bfull[i], (bphase >> i) & 1, kWaits, g.err) && ok;
+                        wait(&tempty[buf], ((pass >> 1) & 1) ^ 1);
+                        wait(&bfull[i], (bphase >> i) & 1);
                         bphase ^= 1u << i;
                         fence_after();
                         const uint64_t ad = smem_desc(smem_u32(sm), kCore, kGroupBytes);
                         const uint64_t bd = smem_desc(smem_u32(sm + kUpB + i * kPiece), kPieceCore, kGroupBytes);
                         for (int kc = 0; kc < 4; ++kc) {
-                            if (fresh && i == i0) ok = mbar_wait(&afull[kc], aphase, kWaits, g.err) && ok;
+                            if (fresh && i == i0) wait(&afull[kc], aphase);
                             issue_products<kPassCols>(tmem + 256 * buf, ad + (uint64_t)kc * (2 * kCore >> 4),
                                                       bd + (uint64_t)kc * (2 * kPieceCore >> 4), kPlane, kPieceRow,
                                                       kc == 0);
@@ -1157,6 +1188,10 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                     if (fresh) aphase ^= 1;
                 }
                 mbar_arrive(&dempty[s % kUpDescs]);
+            }
+            if (!ok) {  // the products under way
+                mma_commit(&fin);
+                mbar_wait(&fin, 0, kWaits);
             }
         }
         __syncwarp();
@@ -1171,7 +1206,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
         double* dst = nullptr;
         double old[8];
         auto open_job = [&]() {  // false: no more jobs
-            ok = mbar_wait(&dfull[s % kUpDescs], (s / kUpDescs) & 1, kWaits, g.err) && ok;
+            wait(&dfull[s % kUpDescs], (s / kUpDescs) & 1);
             const UpDesc& d = desc[s % kUpDescs];
             i0 = d.i0;
             i1 = ok ? d.i1 : 0;
@@ -1185,7 +1220,7 @@ __global__ void __launch_bounds__(kUpThreads, 1)
             dst = desc[s % kUpDescs].tile[half][i >> 1];
             if (dst != nullptr) dst += r + TS * (32 * (i & 1) + 8 * c4);
         };
-        bool more = open_job();
+        bool more = __all_sync(0xffffffffu, open_job());  // a warp leaves as a whole
         if (more) {
             open_pass();
             const bool read = dst != nullptr && !desc[s % kUpDescs].start[half];
@@ -1216,9 +1251,9 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                 open_pass();
                 read = dst != nullptr && !desc[s % kUpDescs].start[half];
             }
-            ok = mbar_wait(&tfull[buf], (pass >> 1) & 1, kWaits, g.err) && ok;
+            wait(&tfull[buf], (pass >> 1) & 1);
             fence_after();
-            __syncwarp();
+            more = __all_sync(0xffffffffu, more);
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 uint32_t acc[8][4];
@@ -1247,7 +1282,6 @@ __global__ void __launch_bounds__(kUpThreads, 1)
             }
         }
     }
-    if (!ok) atomicExch(g.err, 1);
     fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);
@@ -1397,7 +1431,7 @@ static int chain_reserve(const cg_ctx* ctx, int B, int nq, int npe, int v)
     return reserve;
 }
 
-bool digit_streams(cg_ctx* ctx)
+static bool chain_streams(cg_ctx* ctx)
 {
     if (!ctx->aux && cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking) != cudaSuccess) ctx->aux = nullptr;
     bool ok = ctx->aux != nullptr;
@@ -1450,6 +1484,7 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
                         reinterpret_cast<int*>(g.dimg + (size_t)B * kDImg) + (size_t)B * pairs * 128};
     g.dex = ex[1] + (size_t)B * pairs * 128;
     g.err = err;
+    g.waits = ctx->no_waits ? 0 : kWaits;
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DiagShared)));
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem));
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_update<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem));
@@ -1463,7 +1498,7 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
             return rc;
         if (m + npe == 0) continue;
         const int reserve = m > 1 ? chain_reserve(ctx, B, m, npe, v) : 0;
-        const bool beside = reserve > 0 && digit_streams(ctx);
+        const bool beside = reserve > 0 && chain_streams(ctx);
         if (rest && !beside) {
             CG_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_chain[1], 0));
             rest = false;
@@ -1496,6 +1531,42 @@ int digit_factor(cg_ctx* ctx, int B, int nt, int ne, int ext, double* A, size_t 
     return CG_OK;
 }
 
+int digit_selftest_timeout(cg_ctx* ctx, int* host_status)
+{
+    const int nt = 4;
+    const size_t tiled = tiled_elems(nt);
+    double *A = nullptr, *diag = nullptr;
+    unsigned char* work = nullptr;
+    int* st = nullptr;
+    cudaStream_t s = ctx->stream;
+    int rc = CG_OK, h[2] = {0, 0};
+    if (cudaMalloc((void**)&A, 2 * tiled * sizeof(double)) != cudaSuccess ||
+        cudaMalloc((void**)&diag, nt * TS * sizeof(double)) != cudaSuccess ||
+        cudaMalloc((void**)&work, digit_bytes(nt, nt)) != cudaSuccess || cudaMalloc((void**)&st, sizeof h) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->err = "device allocation failed";
+        rc = CG_ERR_ALLOC;
+    }
+    if (!rc && cudaMemsetAsync(st, 0, sizeof h, s) != cudaSuccess) rc = CG_ERR_CUDA;
+    if (!rc) rc = fp64_identity_rows(ctx, 2, nt, A, tiled, s);  // the matrix and E's rows
+    if (!rc) {
+        ctx->no_waits = true;
+        rc = digit_factor(ctx, 1, nt, nt, DIGIT_EXT_IDENTITY, A, tiled, A + tiled, tiled, diag, st, work, st + 1, s);
+        ctx->no_waits = false;
+    }
+    if (!rc) {
+        cudaError_t e = cudaMemcpyAsync(h, st, sizeof h, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) { ctx->err = cudaGetErrorString(e); rc = CG_ERR_CUDA; }
+    }
+    cudaFree(A);
+    cudaFree(diag);
+    cudaFree(work);
+    cudaFree(st);
+    *host_status = h[1] ? CG_ERR_TIMEOUT : CG_OK;
+    return rc;
+}
+
 // K blocks whose images are held at once
 static int gemm_chunk(int nt) { return std::min(nt, 16); }
 
@@ -1524,6 +1595,7 @@ int digit_gemm(cg_ctx* ctx, int nt, const double* A, const double* Bm, bool tile
     g.img = work;
     g.ex = reinterpret_cast<int*>(work + chunk * g.kimg);
     g.err = err;
+    g.waits = ctx->no_waits ? 0 : kWaits;
     CG_CUDA_TRY(ctx, cudaFuncSetAttribute(digit_update<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpSmem));
     CUtensorMap map;
     if (int rc = image_map(ctx, &map, work, (size_t)chunk * nt)) return rc;

@@ -1089,7 +1089,6 @@ static int fp64_ensure(cg_ctx* ctx, int B)
         ctx->err = "device allocation failed for the FP64 workspace";
         return CG_ERR_ALLOC;
     }
-    digit_streams(ctx);
     w.cap = B;
     return CG_OK;
 }

@@ -223,8 +223,9 @@ int cg_mh_run(cg_ctx* ctx, const double* map, int nchains, const double* x0, con
 
 /* ---- instrumentation ------------------------------------------------------ */
 /* self-test of the failure path of the device's bounded waits: one thread waits, with a short
-   limit, on a barrier that nothing completes; *status receives CG_ERR_TIMEOUT when the wait
-   gave up and reported as it should.  Nothing faults or hangs; the context stays usable. */
+   limit, on a barrier that nothing completes, and a small FP64 factorisation runs with
+   waits that give up at once; *status receives CG_ERR_TIMEOUT when both gave up and reported as
+   they should.  Nothing faults or hangs; the context stays usable. */
 int cg_selftest_wait_timeout(cg_ctx* ctx, int* status);
 /* Tensor-core rate probe: one CTA per SM issues iters x 4 tcgen05.mma kind::tf32 M128 N128 K8
    (A in tensor memory, B in shared memory: the form the factorisation kernels issue), reps
