@@ -1047,15 +1047,18 @@ static size_t gpart_elems(const cg_ctx* ctx)
 
 // The harmonics' route takes nh / 128 block-row pairs through every column of the factorisation, the
 // route through C^-1 about 2/3 of the matrix's own pairs and then (lmax - 1) FP64 recurrence steps per
-// pixel pair, 0.8 lmax pairs' worth of time.  The addition theorem needs unit directions (cg_pix2vec's
-// are; a caller's are taken as unit below 1e-14).
+// pixel pair, 0.8 lmax pairs' worth of time.  The addition theorem needs unit directions: what |v|^2
+// lacks to 1 puts the gradient off by l (l + 1) / 2 times that.  cg_pix2vec's are unit vectors; a caller's are taken as
+// such below 1e-15, which leaves what rounding does to a normalised vector (6.7e-16 at most in 3 million of five
+// kinds) and stays within the rounding of the dot products (with the line at 1e-14 the gradient's error at l = 60 was
+// 8e-13 of its terms, 5e-15 through C^-1).
 bool fp64_harmonics_ok(int n, int nt, int lmax, const double* xyz)
 {
     if ((double)nharm_of(lmax) / 128.0 > nt / 3.0 + 0.8 * lmax) return false;
     if (xyz)
         for (int i = 0; i < n; ++i) {
             const double x = xyz[3 * (size_t)i], y = xyz[3 * (size_t)i + 1], z = xyz[3 * (size_t)i + 2];
-            if (!(fabs(x * x + y * y + z * z - 1.0) <= 1e-14)) return false;
+            if (!(fabs(x * x + y * y + z * z - 1.0) <= 1e-15)) return false;
         }
     return true;
 }
