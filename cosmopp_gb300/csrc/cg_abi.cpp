@@ -121,7 +121,7 @@ size_t staging_bytes(int N, int lmax, int max_batch)
 
 void fill_plan(cg_ctx* shape, size_t budget, cg_memory_plan* p)
 {
-    size_t fixed = staging_bytes(shape->N, shape->lmax, shape->max_batch), per = 0;
+    size_t fixed = staging_bytes(shape->N, shape->lmax, shape->max_batch), per = 0, most = (size_t)-1;
     if (shape->precision == CG_PREC_MIXED) {
         size_t f = 0;
         cg::mixed_bytes(shape, &f, &per);
@@ -134,6 +134,17 @@ void fill_plan(cg_ctx* shape, size_t budget, cg_memory_plan* p)
             shape->harm = false;
             cg::fp64_bytes(shape, &f, &per);
         }
+        // The harmonics' rows are 1.3 (nside 32) to 60 times (few pixels, many l) the bytes of the route through C^-1.
+        // From 24 GB on, where a batch has long filled the device, a piece takes no more than that route would for all
+        // of max_batch (with the line at 8 GB 32 elements of 6131 pixels ran as 15, 15 and 2: values 148 -> 168 ms).
+        if (shape->harm) {
+            size_t f1 = 0, per1 = 0;
+            shape->harm = false;
+            cg::fp64_bytes(shape, &f1, &per1);
+            shape->harm = true;
+            const size_t bytes = std::max((size_t)24 << 30, per1 * (size_t)shape->max_batch);
+            most = bytes > f + per ? (bytes - f) / per : 1;
+        }
         fixed += f;
     }
     p->bytes_fixed = fixed;
@@ -143,7 +154,7 @@ void fill_plan(cg_ctx* shape, size_t budget, cg_memory_plan* p)
     const size_t avail = budget > p->bytes_reserve + fixed ? budget - p->bytes_reserve - fixed : 0;
     const size_t fit = per ? avail / per : 0;
     p->max_batch_fit = (int)std::min<size_t>(fit, (size_t)1 << 30);
-    p->chunk = std::min(shape->max_batch, p->max_batch_fit);
+    p->chunk = (int)std::min<size_t>(most, std::min(shape->max_batch, p->max_batch_fit));
 }
 
 // pixel count, padded size and l range of a configuration (the checks cg_create repeats)
@@ -575,7 +586,9 @@ extern "C" int cg_loglike_device(cg_ctx* ctx, int B, const double* d_cl, const d
 static int loglike_chunks(cg_ctx* ctx, int B, const double* d_cl, const double* d_d, int d_stride, double* d_m2lnl,
                           double* d_chi2, double* d_logdet, double* d_grad, int* d_status, cudaStream_t s)
 {
-    const int chunk = ctx->chunk > 0 ? ctx->chunk : B;
+    int chunk = ctx->chunk > 0 ? ctx->chunk : B;
+    // FP64 pieces of one size; the mixed path's stay as they are, which may be re-centred on each
+    if (ctx->precision == CG_PREC_FP64) chunk = (B + (B + chunk - 1) / chunk - 1) / ((B + chunk - 1) / chunk);
     const size_t L1 = (size_t)ctx->lmax + 1;
     for (int b0 = 0; b0 < B; b0 += chunk) {
         const int nb = std::min(chunk, B - b0);

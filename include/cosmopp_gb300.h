@@ -74,9 +74,11 @@ typedef struct cg_config {
    max_batch elements and, for the mixed path, the FP64 reference factor and the whitened
    Legendre table) plus bytes_per_element for every batch element in flight.  Planned against
    bytes_budget less a reserve of 256 MB + 1% (the CUDA context, allocator rounding):
-   max_batch_fit elements fit; chunk = min(max_batch, max_batch_fit) is the piece a call's batch
-   is evaluated in (one piece after another, each its own batch; with CG_RECENTER_BATCH each
-   piece is re-centred on its own mean).  max_batch_fit = 0: nothing fits. */
+   max_batch_fit elements fit; chunk = min(max_batch, max_batch_fit) is the largest piece a call's
+   batch is evaluated in, on the FP64 path less where a piece's workspace would exceed both 24 GB
+   and what max_batch elements take by the gradient's route through C^-1 (one piece after another,
+   each its own batch, FP64 pieces of one size; with CG_RECENTER_BATCH each piece is re-centred on
+   its own mean).  max_batch_fit = 0: nothing fits. */
 typedef struct cg_memory_plan {
     size_t bytes_fixed;
     size_t bytes_per_element;
