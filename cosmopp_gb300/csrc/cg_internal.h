@@ -54,7 +54,7 @@ struct Fp64Work {
     double* E = nullptr;         // [cap][ext_elems] the factorisation's extra rows (k_digit.cu)
     size_t ext_elems = 0;        // doubles of E per element
     unsigned char* dig = nullptr;  // digit images, digit_bytes per element
-    double* Yt = nullptr;        // [ext tiles] harmonics x B_l of the pixels, shared by every element
+    double* Yt = nullptr;        // [ext_elems] behind E: harmonics x B_l of the pixels, shared by every element
     bool have_yt = false;        // Yt is filled
     double* diag = nullptr;      // [cap][N] diagonal of L
     double* dvec = nullptr;      // [cap][N] data maps (padded)

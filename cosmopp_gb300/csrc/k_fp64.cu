@@ -1014,7 +1014,7 @@ void fp64_dot(int n, const double* a, const double* b, double* out, cudaStream_t
 void fp64_free(cg_ctx* ctx)
 {
     Fp64Work& w = ctx->w64;
-    cudaFree(w.A); cudaFree(w.E); cudaFree(w.dig); cudaFree(w.Yt); cudaFree(w.diag); cudaFree(w.dvec);
+    cudaFree(w.A); cudaFree(w.E); cudaFree(w.dig); cudaFree(w.diag); cudaFree(w.dvec);
     cudaFree(w.alpha); cudaFree(w.gpart); cudaFree(w.st); cudaFree(w.ld); cudaFree(w.err);
     cudaFree(w.wfix); cudaFree(w.wexp);
     w = Fp64Work();
@@ -1082,16 +1082,17 @@ static int fp64_ensure(cg_ctx* ctx, int B)
     fp64_free(ctx);
     auto alloc = [](auto** p, size_t count) { return cudaMalloc((void**)p, sizeof(**p) * count) == cudaSuccess; };
     w.ext_elems = ext_elems(ctx);
-    if (!(alloc(&w.A, tiled_elems(ctx->nt) * n) && alloc(&w.E, w.ext_elems * n) &&
+    if (!(alloc(&w.A, tiled_elems(ctx->nt) * n) && alloc(&w.E, w.ext_elems * (n + (ctx->harm ? 1 : 0))) &&
           alloc(&w.dig, digit_bytes(ctx->nt, ext_blocks(ctx, true)) * n) && alloc(&w.diag, ctx->N * n) &&
           alloc(&w.dvec, ctx->N * n) && alloc(&w.alpha, ctx->N * n) && alloc(&w.gpart, gpart_elems(ctx) * n) &&
           alloc(&w.st, n) && alloc(&w.ld, n) && alloc(&w.wfix, (ctx->lmax + 1) * n) && alloc(&w.wexp, n) &&
-          alloc(&w.err, 1) && (!ctx->harm || alloc(&w.Yt, w.ext_elems)))) {
+          alloc(&w.err, 1))) {
         fp64_free(ctx);
         cudaGetLastError();
         ctx->err = "device allocation failed for the FP64 workspace";
         return CG_ERR_ALLOC;
     }
+    w.Yt = ctx->harm ? w.E + w.ext_elems * n : nullptr;
     w.cap = B;
     return CG_OK;
 }
