@@ -134,7 +134,7 @@ void fill_plan(cg_ctx* shape, size_t budget, cg_memory_plan* p)
             shape->harm = false;
             cg::fp64_bytes(shape, &f, &per);
         }
-        // The harmonics' rows are 1.3 (nside 32) to 60 times (few pixels, many l) the bytes of the route through C^-1.
+        // The harmonics' rows take 1.3 (nside 32) to 25 times (190 pixels, lmax 100) the bytes of the route through C^-1.
         // From 24 GB on, where a batch has long filled the device, a piece takes no more than that route would for all
         // of max_batch (with the line at 8 GB 32 elements of 6131 pixels ran as 15, 15 and 2: values 148 -> 168 ms).
         if (shape->harm) {

@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) digit_panel(int k, Dig g)
 // ahead of the next (both images again for every job, and every warp working out the job: 11.1 us a job in a
 // batch of 16 at nside 16, this 9.9).  Per job and SM the tensor cores need 8.7 k cycles, the FP64 pipe (one
 // addition per output, 64 cycles per warp and partition) 8.2 k, the issue slots (about 80 instructions per
-// output and thread, 20 to join, 25 to convert) 10 k; the matrix takes 256 KB of DRAM traffic, 5.4 of the 6.8 TB/s.
+// output and thread, 20 to join, 25 to convert) 10 k; the matrix takes 256 KB of DRAM traffic, 5.0 of the 6.8 TB/s.
 constexpr int kUpB = kImg, kUpSmem = 2 * kImg, kRun = 8;
 constexpr int kUpWarps = 16, kUpThreads = (kUpWarps + 2) * 32, kPassCols = 32;
 
